@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -45,6 +46,30 @@ std::vector<double> k2_axis(int n, double L) {
   for (int i = n / 2; i < n; ++i) k[i] = 2 * kPiRef * (i - n) * 1.0 / d / n;
   for (int i = 0; i < n; ++i) k[i] *= k[i];
   return k;
+}
+
+// Digits per line value of the tensor-core filter.
+int tc_digits(const scft_ctx *ctx) { return ctx->rkind == kRealF32 ? 4 : 7; }
+
+// The tensor-core tables of one pass, rewritten in place when the box changes.
+// A gain that the table cannot hold exactly (tc_build_table) sends the pass
+// back to its FFT kernel; captured graphs are then stale.
+int upload_tc(scft_ctx *ctx, int pi, const std::vector<double> &g, const std::vector<double> &dg) {
+  AxisPlan &ap = ctx->passes[pi];
+  const int nd = tc_digits(ctx);
+  std::vector<unsigned char> t[2];
+  const bool ok = scft::tc_build_table(g.data(), ap.n, nd, t[0], &ctx->row_sum[pi]) &&
+                  scft::tc_build_table(dg.data(), ap.n, nd, t[1], nullptr);
+  unsigned char *mem = static_cast<unsigned char *>(ctx->tc_mem);
+  for (int k = 0; ok && k < 2; ++k)
+    CK(cudaMemcpy(mem + ctx->tc_off[2 * pi + k], t[k].data(), t[k].size(), cudaMemcpyHostToDevice));
+  const void *tc = ok ? mem + ctx->tc_off[2 * pi] : nullptr;
+  if (tc != ap.tc) {
+    ap.tc = tc;
+    ctx->dtc_pass[pi] = ok ? mem + ctx->tc_off[2 * pi + 1] : nullptr;
+    ++ctx->plan_epoch;
+  }
+  return SCFT_OK;
 }
 
 // Gains of the passes (kxyzdz, init_cuda.cu:394-428, split per axis:
@@ -95,6 +120,15 @@ int upload_gains(scft_ctx *ctx) {
       CK(cudaMemcpy(const_cast<void *>(ap.gain), g.data(), 8 * ap.n, cudaMemcpyHostToDevice));
       CK(cudaMemcpy(dptr, dg.data(), 8 * ap.n, cudaMemcpyHostToDevice));
     }
+    if (ctx->tc_want[pi]) {
+      const int rc = upload_tc(ctx, (int)pi, g, dg);
+      if (rc) return rc;
+    }
+  }
+  if (ctx->kbits) {
+    const double growth = ctx->row_sum[0] * ctx->row_sum[1] * ctx->row_sum[2];
+    const int kb = growth > 1.0 ? (int)ceil(log2(growth)) : 0;
+    CK(cudaMemcpy(ctx->kbits, &kb, sizeof kb, cudaMemcpyHostToDevice));
   }
   return SCFT_OK;
 }
@@ -126,6 +160,14 @@ bool axis_ok(int n, bool allow_one) {
 // kernel, or one generic launch per set member.
 template <typename R>
 int launch_set(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R> &ps, cudaStream_t st) {
+  if constexpr (!std::is_same<R, scft::dfloat>::value) {
+    if (ap.tc) {
+      scft::PassSet<R> p = ps;
+      p.err = ctx->dev_err;
+      CKL(scft::launch_tc(ap, p, false, st));
+      return SCFT_OK;
+    }
+  }
   if (ap.use_fast) {
     CKL(scft::launch_fast_line(ap, ps, st));
     return SCFT_OK;
@@ -139,6 +181,23 @@ int launch_set(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R> &ps, cu
                                     ps.pre[k], ps.post[k], ps.w_bs, ps.batch, st));
   return SCFT_OK;
   }
+}
+
+// A fused step pair on one axis's lines: finishes a step (qout) and starts the
+// next one (out).
+template <typename R>
+int launch_pair(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R> &ps, cudaStream_t st) {
+  if constexpr (std::is_same<R, float>::value) {
+    if (ap.tc) {
+      scft::PassSet<R> p = ps;
+      p.err = ctx->dev_err;
+      CKL(scft::launch_tc(ap, p, true, st));
+      return SCFT_OK;
+    }
+  }
+  if (ap.n_fast) CKL(scft::launch_xx(ap, ps, st));
+  else CKL(scft::launch_zz(ap, ps, st));
+  return SCFT_OK;
 }
 
 // A march segment: propagator qi over ns steps in field wf, direction sign,
@@ -250,21 +309,31 @@ int run_chains(scft_ctx *ctx, const Seg *const *chains, const int *nseg, int nch
 // odd and (z, x+y) when k is even, which the commuting axis filters allow.
 // The end of step k and the start of step k+1 are then one kernel
 // (k_zz / k_xyxy): one launch per contour step instead of two.
-// Without the x+y plane (three passes, all register-resident) the same idea
-// gives (x, y, z) for odd and (z, y, x) for even steps: k_zz / k_xx fuse the
-// end of one step with the start of the next, two launches per step instead
-// of three.
+// Without the x+y plane (two or three passes, each with a pair kernel) the same
+// idea gives (x, y, z) for odd and (z, y, x) for even steps: a pair on z or x
+// fuses the end of one step with the start of the next, so three passes take
+// two launches per step instead of three and two passes take one.
 bool fused_possible(const scft_ctx *ctx) {
-  if (!ctx->fuse_steps || ctx->passes.size() != 3) return false;
-  if (ctx->fuse_xy) return ctx->rbytes == 4 && ctx->passes[2].use_fast != 0;
-  return ctx->passes[0].use_fast && ctx->passes[1].use_fast && ctx->passes[2].use_fast;
+  const size_t np = ctx->passes.size();
+  if (!ctx->fuse_steps) return false;
+  if (ctx->fuse_xy && np == 3)
+    return ctx->rbytes == 4 && (ctx->passes[2].use_fast != 0 || ctx->passes[2].tc);
+  if (ctx->fuse_xy || np < 2) return false;
+  // tensor-core passes pair with each other (64-bit contexts: only all of
+  // them), register-resident passes when there are three
+  int tc = 0, fast = 0;
+  for (const AxisPlan &ap : ctx->passes) {
+    if (ap.tc) ++tc;
+    else if (ap.use_fast && np == 3) ++fast;
+  }
+  return tc + fast == (int)np && (ctx->rkind == kRealF32 || tc == 0 || fast == 0);
 }
 
 template <typename R>
 int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, int cidx) {
   const long long M = ctx->M;
   R *tmp[2] = {static_cast<R *>(ctx->tmp[2 * cidx]), static_cast<R *>(ctx->tmp[2 * cidx + 1])};
-  const AxisPlan &apx = ctx->passes[0], &apy = ctx->passes[1], &apz = ctx->passes[2];
+  const int np = (int)ctx->passes.size();
   for (int k = 0; k < nseg; ++k) {
     const Seg &sg = segs[k];
     int rc = seg_boundary<R>(ctx, sg, st);
@@ -285,31 +354,110 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
       ps.out[0] = out;
       ps.out_bs[0] = out_bs;
     };
-    // step 1: x with the pre factor, then y; tmp[0] holds the state between steps
-    reset(slice(0), qbs, tmp[1], M);
+    int cur = 0;   // tmp[cur] holds the state between launches
+    // the passes strictly between a step's first and last (y of x, y, z)
+    auto middle = [&]() {
+      if (np < 3) return (int)SCFT_OK;
+      reset(tmp[cur], M, tmp[cur ^ 1], M);
+      cur ^= 1;
+      return launch_set<R>(ctx, ctx->passes[1], ps, st);
+    };
+    // step 1: x with the pre factor
+    reset(slice(0), qbs, tmp[cur], M);
     ps.pre[0] = W;
-    if ((rc = launch_set<R>(ctx, apx, ps, st))) return rc;
-    reset(tmp[1], M, tmp[0], M);
-    if ((rc = launch_set<R>(ctx, apy, ps, st))) return rc;
+    if ((rc = launch_set<R>(ctx, ctx->passes[0], ps, st))) return rc;
+    if ((rc = middle())) return rc;
     for (int it = 2; it <= sg.ns; ++it) {
-      // finish step it-1 (z when it was odd, x when even) and start step it
-      reset(tmp[0], M, tmp[1], M);
+      // finish step it-1 (last pass when it was odd, x when even), start step it
+      reset(tmp[cur], M, tmp[cur ^ 1], M);
+      cur ^= 1;
       ps.qout[0] = slice(it - 1);
       ps.qout_bs[0] = qbs;
       ps.post[0] = W;
-      if ((it - 1) & 1) CKL(scft::launch_zz(apz, ps, st));
-      else CKL(scft::launch_xx(apx, ps, st));
-      reset(tmp[1], M, tmp[0], M);
-      if ((rc = launch_set<R>(ctx, apy, ps, st))) return rc;
+      if ((rc = launch_pair<R>(ctx, ctx->passes[(it - 1) & 1 ? np - 1 : 0], ps, st))) return rc;
+      if ((rc = middle())) return rc;
     }
-    reset(tmp[0], M, slice(sg.ns), qbs);
+    reset(tmp[cur], M, slice(sg.ns), qbs);
     ps.post[0] = W;
-    if ((rc = launch_set<R>(ctx, (sg.ns & 1) ? apz : apx, ps, st))) return rc;
+    if ((rc = launch_set<R>(ctx, ctx->passes[(sg.ns & 1) ? np - 1 : 0], ps, st))) return rc;
   }
   return SCFT_OK;
 }
 
+// The same schedule with integer intermediates (FP64 contexts whose passes all
+// run on the tensor cores).  v_j = W q_j starts step j+1; its unit follows from
+// the exponent bound of v_{j-1} (two factors on), of q_0 for j = 0.
+int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, int cidx) {
+  const long long M = ctx->M;
+  const int B = ctx->batch, np = (int)ctx->passes.size();
+  int64_t *tmp[2] = {static_cast<int64_t *>(ctx->tmp[2 * cidx]),
+                     static_cast<int64_t *>(ctx->tmp[2 * cidx + 1])};
+  for (int k = 0; k < nseg; ++k) {
+    const Seg &sg = segs[k];
+    int rc = seg_boundary<double>(ctx, sg, st);
+    if (rc) return rc;
+    if (sg.ns == 0) continue;
+    double *q = static_cast<double *>(ctx->q[sg.qi]);
+    const long long qbs = (long long)(ctx->q_ns[sg.qi] + 1) * M;
+    auto slice = [&](int it) { return q + (long long)(sg.sign > 0 ? it : sg.ns - it) * M; };
+    int *exq = ctx->ex[cidx], *ex = exq + B;   // |q_0| and |v_j| bounds, [..][B]
+    CK(cudaMemsetAsync(exq, 0x80, sizeof(int) * (size_t)(sg.ns + 1) * B, st));
+    CKL(scft::launch_slice_exp(slice(0), qbs, M, B, exq, st));
+    scft::FixPass fp;
+    int cur = 0, j = 0;   // tmp[cur] holds v_j, or v_j filtered
+    auto pass = [&](int pi, int mode, const void *in, long long in_bs) {
+      memset(&fp, 0, sizeof fp);
+      fp.batch = B;
+      fp.eref = ctx->eref[sg.wf];
+      fp.kbits = ctx->kbits;
+      fp.w = ctx->wfix[sg.wf];
+      fp.w_bs = M;
+      fp.err = ctx->dev_err;
+      fp.in = in;
+      fp.in_bs = in_bs;
+      auto unit = [&](int v, const int *&u, int &w) {
+        u = v == 0 ? exq : ex + (long long)(v - 1) * B;
+        w = v == 0 ? 1 : 2;
+      };
+      if (mode != scft::kFixFirst) unit(j, fp.u_in, fp.w_in);
+      if (mode == scft::kFixPair || mode == scft::kFixLast) {
+        fp.q = slice(j + 1);
+        fp.q_bs = qbs;
+        ++j;
+      }
+      if (mode != scft::kFixLast) {
+        unit(j, fp.u_out, fp.w_out);
+        fp.out = mode == scft::kFixFirst ? tmp[cur] : tmp[cur ^ 1];
+        fp.out_bs = M;
+        if (mode != scft::kFixFirst) cur ^= 1;
+        if (mode != scft::kFixMid) fp.ex = ex + (long long)j * B;
+      }
+      CKL(scft::launch_fix(ctx->passes[pi], mode, fp, st));
+      return (int)SCFT_OK;
+    };
+    auto middle = [&]() { return np < 3 ? (int)SCFT_OK : pass(1, scft::kFixMid, tmp[cur], M); };
+    if ((rc = pass(0, scft::kFixFirst, slice(0), qbs))) return rc;
+    if ((rc = middle())) return rc;
+    for (int it = 2; it <= sg.ns; ++it) {
+      // finish step it-1 (last pass when it was odd, x when even), start step it
+      if ((rc = pass((it - 1) & 1 ? np - 1 : 0, scft::kFixPair, tmp[cur], M))) return rc;
+      if ((rc = middle())) return rc;
+    }
+    if ((rc = pass((sg.ns & 1) ? np - 1 : 0, scft::kFixLast, tmp[cur], M))) return rc;
+  }
+  return SCFT_OK;
+}
+
+// Whether fused chains of this context run with integer intermediates.
+bool fixed_march(const scft_ctx *ctx) {
+  if (!ctx->kbits) return false;
+  for (const AxisPlan &ap : ctx->passes)
+    if (!ap.tc) return false;
+  return true;
+}
+
 int run_chain_fused(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, int cidx) {
+  if (fixed_march(ctx)) return run_chain_fixed(ctx, segs, nseg, st, cidx);
   if (!ctx->fuse_xy)
     return with_real(ctx, [&](auto r) {
       return run_chain_fused_axes<decltype(r)>(ctx, segs, nseg, st, cidx);
@@ -353,8 +501,11 @@ int run_chain_fused(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, i
       ps.qout[0] = slice(it - 1);
       ps.qout_bs[0] = qbs;
       ps.post[0] = W;
-      if ((it - 1) & 1) CKL(scft::launch_zz(apz, ps, st));     // step it-1 was (x+y, z)
-      else CKL(scft::launch_xyxy(apx, apy, ps, st));            // step it-1 was (z, x+y)
+      if ((it - 1) & 1) {                                       // step it-1 was (x+y, z)
+        if ((rc = launch_pair<float>(ctx, apz, ps, st))) return rc;
+      } else {                                                  // step it-1 was (z, x+y)
+        CKL(scft::launch_xyxy(apx, apy, ps, st));
+      }
       cur ^= 1;
     }
     // finish the last step with its remaining pass and the post factor
@@ -390,6 +541,13 @@ int boltzmann(scft_ctx *ctx, int f, cudaStream_t st) {
     using R = decltype(r);
     CKL(scft::launch_boltzmann<R>(w, static_cast<R *>(ctx->W[f]), ctx->M * ctx->batch,
                                   ctx->p.ds0 / 2, st));
+    if constexpr (std::is_same<R, double>::value) {
+      if (ctx->kbits) {
+        CKL(scft::launch_wfix(static_cast<const double *>(ctx->W[f]), ctx->M, ctx->batch,
+                              ctx->eref[f], ctx->wfix[f], st));
+        ++ctx->launches;
+      }
+    }
     return SCFT_OK;
   });
 }
@@ -422,7 +580,12 @@ int march_phase(scft_ctx *ctx, cudaStream_t st) {
 int march_phase_graph(scft_ctx *ctx) {
   NvtxRange range("scft march phase");
   if (!ctx->use_graph || ctx->capturing) return march_phase(ctx, ctx->st);
+  if (ctx->march_exec && ctx->march_epoch != ctx->plan_epoch) {
+    cudaGraphExecDestroy(ctx->march_exec);
+    ctx->march_exec = nullptr;
+  }
   if (!ctx->march_exec) {
+    ctx->march_epoch = ctx->plan_epoch;
     const long long l0 = ctx->launches;
     CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
     int rc = march_phase(ctx, ctx->st);
@@ -671,7 +834,8 @@ void free_all(scft_ctx *ctx) {
   cudaFree(ctx->fe5); cudaFree(ctx->tables); cudaFree(ctx->dev_err);
   cudaFree(ctx->res); cudaFree(ctx->rpartial); cudaFree(ctx->gram); cudaFree(ctx->and_a);
   cudaFree(ctx->and_lam); cudaFree(ctx->target); cudaFree(ctx->dgain);
-  cudaFree(ctx->shift_alpha);
+  cudaFree(ctx->shift_alpha); cudaFree(ctx->tc_mem);
+  cudaFree(ctx->wfix[0]); cudaFree(ctx->wfix[1]); cudaFree(ctx->kbits);
   scft_internal_adjoint_free(ctx);
   for (float *h : ctx->hist_u) cudaFree(h);
   for (float *h : ctx->hist_d) cudaFree(h);
@@ -695,7 +859,7 @@ int autotune(scft_ctx *ctx) {
   for (size_t i = 1; i < ctx->passes.size(); ++i)
     has_fast_col |= ctx->rbytes == 4 && ctx->passes[i].use_fast != 0;
   const bool can_xy = ctx->fuse_xy;
-  const bool can_fs = (ctx->p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0 && ctx->passes.size() == 3;
+  const bool can_fs = (ctx->p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0 && ctx->passes.size() >= 2;
   int rc;
   if ((rc = boltzmann(ctx, SCFT_FIELD_WA, ctx->st))) return rc;
   if ((rc = boltzmann(ctx, SCFT_FIELD_WB, ctx->st))) return rc;
@@ -841,7 +1005,10 @@ int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long o
     p.pre[0] = pi == 0 ? pre : nullptr;
     p.post[0] = pi == np - 1 ? post : nullptr;
     AxisPlan ap = ctx->passes[pi];
-    if (pi == deriv_pass) ap.gain = ctx->dgain_pass[pi];
+    if (pi == deriv_pass) {
+      ap.gain = ctx->dgain_pass[pi];
+      ap.tc = ctx->dtc_pass[pi];
+    }
     int rc = launch_set<R>(ctx, ap, p, st);
     if (rc) return rc;
   }
@@ -1106,6 +1273,41 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
     ctx->pass_axis[ctx->passes.size()] = a;
     ctx->passes.push_back(ap);
   }
+  if (cudaMemcpy(ctx->tables, host.data(), tab_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
+    return fail(SCFT_ERR_CUDA, "table upload failed");
+  // Passes on the tensor cores: every FP64 line they take, and FP32 lines without
+  // a register kernel.  Measured, ms per SCF iteration with 200 contour steps:
+  // FP64 64^3 22 -> 5.5, 128^3 107 -> 22; FP32 100x80x60 24 -> 5.2.  FP32 and
+  // double-float lines with a register kernel keep it (64^3: FP32 1.2; double-float
+  // 4.0 against 5.6).
+  size_t tc_bytes = 0;
+  for (size_t pi = 0; pi < ctx->passes.size(); ++pi) {
+    const AxisPlan &ap = ctx->passes[pi];
+    ctx->tc_want[pi] = scft::tc_line_possible(ap.n, tc_digits(ctx)) &&
+                       (ctx->rkind == kRealF64 || (ctx->rkind == kRealF32 && !ap.use_fast));
+    for (int k = 0; ctx->tc_want[pi] && k < 2; ++k) {
+      ctx->tc_off[2 * pi + k] = tc_bytes;
+      tc_bytes += (scft::tc_table_bytes(ap.n, tc_digits(ctx)) + 255) & ~(size_t)255;
+    }
+  }
+  if (tc_bytes && scft::tc_prepare() != cudaSuccess)
+    return fail(SCFT_ERR_CUDA, "kernel attribute set-up failed");
+  if (tc_bytes && !alloc(&ctx->tc_mem, tc_bytes))
+    return fail(SCFT_ERR_NO_MEMORY, "table allocation failed");
+  if (ctx->rkind == kRealF64 && (p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0 &&
+      ctx->passes.size() >= 2 && ctx->tc_want[0] && ctx->tc_want[1] &&
+      (ctx->passes.size() == 2 || ctx->tc_want[2])) {
+    // kbits, then eref[2][B], then the exponent bounds of the two chains
+    const size_t steps = (size_t)std::max(ctx->NsA, ctx->dNsB) + 2;
+    if (!alloc((void **)&ctx->kbits, sizeof(int) * (1 + 2 * (size_t)B + 2 * steps * B)) ||
+        !alloc((void **)&ctx->wfix[0], 8 * M * B) || !alloc((void **)&ctx->wfix[1], 8 * M * B))
+      return fail(SCFT_ERR_NO_MEMORY, "device allocation failed");
+    ctx->eref[0] = ctx->kbits + 1;
+    ctx->eref[1] = ctx->eref[0] + B;
+    ctx->ex[0] = ctx->eref[1] + B;
+    ctx->ex[1] = ctx->ex[0] + steps * B;
+  }
+  if (upload_gains(ctx)) return fail(SCFT_ERR_CUDA, "gain table upload failed: " + ctx->err);
   // x and y both as their own passes (no length-1 axis among them) and small
   // enough for a shared-memory plane: fuse them
   ctx->fuse_xy = rb == 4 && (p.flags & SCFT_FLAG_NO_XY) == 0 && ctx->passes.size() >= 2 &&
@@ -1119,9 +1321,6 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
   // kernel takes (measured per SCF iteration: 64^3 1.12 ms against 1.27 ms
   // lockstep, 128^3 4.46 ms against 5.79 ms).
   if (ctx->fuse_steps && (p.flags & SCFT_FLAG_LOCKSTEP) == 0) ctx->two_streams = true;
-  if (cudaMemcpy(ctx->tables, host.data(), tab_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
-    return fail(SCFT_ERR_CUDA, "table upload failed");
-  if (upload_gains(ctx)) return fail(SCFT_ERR_CUDA, "gain table upload failed: " + ctx->err);
   if (cudaDeviceSynchronize() != cudaSuccess) return fail(SCFT_ERR_CUDA, "set-up failed");
   ctx->err = "no error";
   if (p.flags & SCFT_FLAG_AUTOTUNE) {

@@ -69,6 +69,20 @@ struct scft_ctx {
   void *dgain = nullptr;
   const void *dgain_pass[3] = {nullptr, nullptr, nullptr};
   double unit_c[3] = {0.0, 0.0, 0.0};
+  // tensor-core tables (k_tc.cu) of the passes that run there, for the gain
+  // and its box derivative; slot 2*pass + derivative, 0 where a pass has none
+  void *tc_mem = nullptr;
+  size_t tc_off[6] = {0, 0, 0, 0, 0, 0};
+  bool tc_want[3] = {false, false, false};
+  const void *dtc_pass[3] = {nullptr, nullptr, nullptr};
+  // the fused 64-bit march (run_chain_fixed): factors as integers and their
+  // largest exponent per instance, exponent bounds per step [2 chains], and
+  // log2 of the filters' growth
+  int64_t *wfix[2] = {nullptr, nullptr};
+  int *eref[2] = {nullptr, nullptr}, *ex[2] = {nullptr, nullptr}, *kbits = nullptr;
+  double row_sum[3] = {1.0, 1.0, 1.0};
+  int march_epoch = 0;          // plan_epoch that march_exec was captured with
+  int plan_epoch = 0;           // bumped when a pass changes kernels (captured graphs are stale)
   struct AdjointState *adj = nullptr;   // adjoint / stress work buffers (lazy)
   bool have_conc = false;       // propagators, W and Q of a getConc at the current box
   // per-march event timing

@@ -64,10 +64,18 @@ struct scft_group {
   cudaGraphExec_t exec = nullptr;
   long long nodes = 0;
   long long launches = 0;
+  long long epoch = 0;               // the members' plan epochs at capture
   std::string err = "no error";
 };
 
 namespace {
+
+long long plan_epochs(const scft_group *g) {
+  long long s = 0;
+  for (const scft_ctx *c : g->members) s += c->plan_epoch;
+  return s;
+}
+
 
 int gfail(scft_group *g, int st, const std::string &m) {
   g->err = m;
@@ -81,14 +89,20 @@ int gfail(scft_group *g, int st, const std::string &m) {
                                                            cudaGetErrorString(e_));  \
   } while (0)
 
-void release(scft_group *g) {
+void release_graph(scft_group *g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
+  g->exec = nullptr;
   for (GroupBucket &b : g->buckets)
     for (BucketChain &c : b.ch) {
       cudaFree(c.desc);
       if (c.ev) cudaEventDestroy(c.ev);
       if (c.st) cudaStreamDestroy(c.st);
     }
+  g->buckets.clear();
+}
+
+void release(scft_group *g) {
+  release_graph(g);
   for (cudaEvent_t e : g->pre) cudaEventDestroy(e);
   for (cudaEvent_t e : g->joined) cudaEventDestroy(e);
   if (g->fork) cudaEventDestroy(g->fork);
@@ -104,12 +118,14 @@ void release(scft_group *g) {
 // 48^3 (142.3 against 169.4) and 64^3 (172.1 against 196.0).
 constexpr long long kBatchFusedBelow = 1LL << 16;
 int make_buckets(scft_group *g) {
-  std::map<std::tuple<int, int, int>, std::vector<int>> by_grid;
+  std::map<std::tuple<int, int, int, int>, std::vector<int>> by_grid;
   for (size_t i = 0; i < g->members.size(); ++i) {
     const scft_ctx *c = g->members[i];
     if (c->rkind != kRealF32 || c->batch != 1 || c->NsA < 1 || c->dNsB < 1) continue;
     if (c->fuse_steps && c->M >= kBatchFusedBelow) continue;
-    by_grid[std::make_tuple(c->p.nx, c->p.ny, c->p.nz)].push_back((int)i);
+    int tc = 0;   // the passes on the tensor cores (a box can send one back, upload_tc)
+    for (size_t pi = 0; pi < c->passes.size(); ++pi) tc |= (c->passes[pi].tc ? 1 : 0) << pi;
+    by_grid[std::make_tuple(c->p.nx, c->p.ny, c->p.nz, tc)].push_back((int)i);
   }
   g->bucket_of.assign(g->members.size(), -1);
   for (auto &kv : by_grid) {
@@ -153,6 +169,7 @@ int make_buckets(scft_group *g) {
             d.post = pi == bb.npass - 1 ? W : nullptr;
             const int ai = bb.xy ? (pi == 0 ? 0 : pi + 1) : pi;   // the member's axis pass
             d.gain = static_cast<const float *>(c->passes[ai].gain);
+            d.tc = c->passes[ai].tc;
             d.gain_y = bb.xy && pi == 0 ? static_cast<const float *>(c->passes[1].gain) : nullptr;
             step[pi].push_back(d);
           }
@@ -207,7 +224,10 @@ int bucket_march(scft_group *g, GroupBucket &b, int ch, long long *launches) {
       const int ai = b.xy ? (pi == 0 ? 0 : pi + 1) : pi;
       const scft::AxisPlan &ap = c0->passes[ai];
       if (b.xy && pi == 0) e = scft::launch_xy(c0->passes[0], c0->passes[1], ps, bc.st);
-      else if (ap.use_fast) e = scft::launch_fast_line(ap, ps, bc.st);
+      else if (ap.tc) {
+        ps.err = c0->dev_err;
+        e = scft::launch_tc(ap, ps, false, bc.st);
+      } else if (ap.use_fast) e = scft::launch_fast_line(ap, ps, bc.st);
       else e = scft::launch_line_filter_desc(ap, d, n, bc.st);
       if (e != cudaSuccess)
         return gfail(g, SCFT_ERR_CUDA, std::string("batched pass: ") + cudaGetErrorString(e));
@@ -283,6 +303,7 @@ int build_graph(scft_group *g) {
     g->exec = nullptr;
     return gfail(g, SCFT_ERR_CUDA, std::string("group instantiate: ") + cudaGetErrorString(e));
   }
+  g->epoch = plan_epochs(g);
   long long l1 = 0;
   for (scft_ctx *c : g->members) l1 += c->launches;
   g->bucket_launches = bl;
@@ -291,6 +312,13 @@ int build_graph(scft_group *g) {
 }
 
 int iterate_once(scft_group *g) {
+  if (g->epoch != plan_epochs(g)) {   // a member's box sent a pass to another kernel
+    GCK(cudaStreamSynchronize(g->st));
+    release_graph(g);
+    int rc = make_buckets(g);
+    if (rc == SCFT_OK) rc = build_graph(g);
+    if (rc) return rc;
+  }
   GCK(cudaGraphLaunch(g->exec, g->st));
   g->launches += g->nodes;
   GCK(cudaEventRecord(g->done, g->st));

@@ -1,0 +1,1002 @@
+// Tensor-core passes of the propagator march (core and arithmetic: tc_core.cuh).
+//
+// k_real: one axis pass on working reals, out = post * K (pre * in), and for
+// FP32 the fused step pair.  k_fix: the fused march of FP64 and double-float
+// contexts, whose intermediates between passes stay 64-bit integers of one unit
+// per instance and step, so that a pass costs no conversion to or from the
+// working real (those were about half of a pass's 142 instructions per point):
+//   first  v0 = W q0 and the first filter        real in, fixed out
+//   mid    one filter                            fixed in, fixed out
+//   pair   filter, q = W y (stored), v = W q, filter
+//   last   filter, q = W y (stored)              fixed in, real out
+// The unit must be known before the values are: every kernel that forms v
+// reports the largest exponent (ex), and the next one scales by that times the
+// growth one step can bring (W^2 and the kernels' row sums, kbits).  Integers
+// stay below 2^59 (2^61 in registers); each line is rescaled to the digits' 2^54
+// by its own largest value, so a line keeps the accuracy of its own scale.
+#include "tc_core.cuh"
+
+#include <limits.h>
+#include <math.h>
+#include <string.h>
+
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <vector>
+
+namespace scft {
+
+namespace {
+
+using namespace tc;
+
+template <typename T> constexpr int kNd = 7;
+template <> constexpr int kNd<float> = 4;
+
+__device__ __forceinline__ double bad_value(double) { return __longlong_as_double(0x7ff8000000000000LL); }
+__device__ __forceinline__ float bad_value(float) { return __int_as_float(0x7fc00000); }
+
+// filter result -> working real (float: y * 2^ue)
+template <typename T, typename A> __device__ __forceinline__ T finish_real(A y, int ue) {
+  if constexpr (std::is_same<T, float>::value) return scale2(y, ue);
+  else return from_fixed(y, ue, T());
+}
+
+// Geometry of a pass's lines.
+struct Lines {
+  int n, half, kg;
+  long long lines;       // per instance
+  long long row_len;     // column passes: consecutive lines of one row
+  long long s_outer, s_n;
+};
+
+// f(row, column, offset in the tile) over the tile's contiguous rows by the nt
+// computing threads, coalesced
+template <typename F> __device__ __forceinline__ void over_rows(int nt, int n, int nl, F &&f) {
+  int r = (int)threadIdx.x / n, col = (int)threadIdx.x % n;
+  const int dr = nt / n, dc = nt % n;
+  for (int i = threadIdx.x; i < nl * n; i += nt) {
+    f(r, col, i);
+    r += dr;
+    col += dc;
+    if (col >= n) {
+      col -= n;
+      ++r;
+    }
+  }
+}
+
+// f(row, column, offset, src[offset]), four loads in flight per thread
+template <typename F>
+__device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *src, F &&f) {
+  const int total = nl * n;
+  int r = (int)threadIdx.x / n, col = (int)threadIdx.x % n;
+  const int dr = nt / n, dc = nt % n;
+#pragma unroll 1
+  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * nt) {
+    int64_t x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      x[j] = i0 + j * nt < total ? __ldg(reinterpret_cast<const long long *>(src) + (i0 + j * nt)) : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (i0 + j * nt < total) f(r, col, i0 + j * nt, x[j]);
+      r += dr;
+      col += dc;
+      if (col >= n) {
+        col -= n;
+        ++r;
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ k_real
+template <typename T, int MAXT, int PP, bool XP, bool PAIR>
+__global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, PassSet<T> ps) {
+  typedef Tile<kNd<T>, PP> E;
+  typedef typename E::I I;
+  typedef typename E::Acc Acc;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  E e;
+  const void *table = table_;
+  if constexpr (std::is_same<T, float>::value) {
+    if (ps.desc) table = ps.desc[blockIdx.z].tc;
+  }
+  e.setup(smem_raw, ln.n, ln.kg, XP ? (int)sizeof(T) : 0, table);
+  const TcHead head = *static_cast<const TcHead *>(table);
+  const int set = (int)blockIdx.z >= ps.batch ? 1 : 0;
+  const long long b = (long long)blockIdx.z - (long long)set * ps.batch;
+  const long long line0 = (long long)blockIdx.x * kLines;
+  const int nl = (int)min((long long)kLines, ln.lines - line0);
+  const T *in = ps.in[set] + b * ps.in_bs[set];
+  T *out = ps.out[set] + b * ps.out_bs[set];
+  const T *pre = ps.pre[set] ? ps.pre[set] + b * ps.w_bs : nullptr;
+  const T *post = ps.post[set] ? ps.post[set] + b * ps.w_bs : nullptr;
+  T *qo = PAIR ? ps.qout[set] + b * ps.qout_bs[set] : nullptr;
+  if constexpr (std::is_same<T, float>::value && !PAIR) {
+    if (ps.desc) {   // a batched pass: this line set's own buffers
+      const PassDesc d = ps.desc[blockIdx.z];
+      in = d.in;
+      out = d.out;
+      pre = d.pre;
+      post = d.post;
+    }
+  }
+  const int H = ln.half;
+  pdl_wait();      // the input is the previous pass's output
+  pdl_release();
+  if (e.issuer) {
+    e.run_issuer(PAIR ? 2 : 1);
+    e.finish(ps.err);
+    return;
+  }
+  e.run_compute();
+  const bool mine = e.line < nl;
+  const long long c = line0 + e.line;
+  const long long base = XP ? 0 : (mine ? (c / ln.row_len) * ln.s_outer + c % ln.row_len : 0);
+  const long long tile = XP ? line0 * ln.n : 0;   // x pass: contiguous rows
+  const int P = ln.n + 1;                         // staging pitch
+  T *stg = reinterpret_cast<T *>(smem_raw);
+
+  T a[PP], bb[PP];
+  if constexpr (XP) {
+    const T *src = in + tile, *wsrc = pre ? pre + tile : nullptr;
+    over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
+      T x = ldg(src + i);
+      if (wsrc) x = x * ldg(wsrc + i);
+      stg[r * P + col] = x;
+    });
+    e.sync();
+  }
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    const int k = PP * e.u + i;
+    a[i] = bb[i] = T(0.0f);
+    if (mine && k < H) {
+      if constexpr (XP) {
+        a[i] = stg[e.line * P + k];
+        bb[i] = stg[e.line * P + k + H];
+      } else {
+        a[i] = ldg(in + base + (long long)k * ln.s_n);
+        bb[i] = ldg(in + base + (long long)(k + H) * ln.s_n);
+      }
+    }
+  }
+  if constexpr (!XP) {
+    if (pre) {
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int k = PP * e.u + i;
+        if (mine && k < H) {
+          a[i] = a[i] * ldg(pre + base + (long long)k * ln.s_n);
+          bb[i] = bb[i] * ldg(pre + base + (long long)(k + H) * ln.s_n);
+        }
+      }
+    }
+  }
+  int key = 0;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) key = max(key, max(mag_key(a[i]), mag_key(bb[i])));
+  e.start();   // TMEM address, cleared keys; the staging tile is read
+  key = e.line_key(0, key);
+  bool bad = key >= bad_key<T>();
+  int Eb = line_exp(T(0.0f), key);
+  I xa[PP], xb[PP];
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    xa[i] = to_fixed(a[i], Eb);
+    xb[i] = to_fixed(bb[i], Eb);
+  }
+  // results come in units of 2^(unit + shift)
+  const int shift = (kNd<T> == 7 ? 55 : 23) - head.kshift;
+  int ue = unit_exp(T(0.0f), Eb) + shift;
+
+  if constexpr (PAIR) {
+    T ya[PP], yb[PP];
+    e.filter(xa, xb, []() {}, [&](int i, Acc p, Acc q) {
+      ya[i] = bad ? bad_value(T(0.0f)) : finish_real<T>(p, ue);
+      yb[i] = bad ? bad_value(T(0.0f)) : finish_real<T>(q, ue);
+    });
+    if constexpr (XP) {
+      e.sync();
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int k = PP * e.u + i;
+        if (mine && k < H) {
+          stg[e.line * P + k] = ya[i];
+          stg[e.line * P + k + H] = yb[i];
+        }
+      }
+      e.sync();
+      over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
+        const T w = ldg(post + tile + i);
+        const T q = stg[r * P + col] * w;
+        qo[tile + i] = q;
+        stg[r * P + col] = q * w;
+      });
+      e.sync();
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int k = PP * e.u + i;
+        const bool on = mine && k < H;
+        ya[i] = on ? stg[e.line * P + k] : T(0.0f);
+        yb[i] = on ? stg[e.line * P + k + H] : T(0.0f);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int k = PP * e.u + i;
+        if (mine && k < H) {
+          const long long o0 = base + (long long)k * ln.s_n, o1 = o0 + (long long)H * ln.s_n;
+          const T w0 = ldg(post + o0), w1 = ldg(post + o1);
+          const T q0 = ya[i] * w0, q1 = yb[i] * w1;
+          qo[o0] = q0;
+          qo[o1] = q1;
+          ya[i] = q0 * w0;
+          yb[i] = q1 * w1;
+        } else {
+          ya[i] = yb[i] = T(0.0f);
+        }
+      }
+    }
+    int key2 = 0;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) key2 = max(key2, max(mag_key(ya[i]), mag_key(yb[i])));
+    key2 = e.line_key(1, key2);   // (its barrier: the staging tile is read)
+    bad = key2 >= bad_key<T>();
+    Eb = line_exp(T(0.0f), key2);
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      xa[i] = to_fixed(ya[i], Eb);
+      xb[i] = to_fixed(yb[i], Eb);
+    }
+    ue = unit_exp(T(0.0f), Eb) + shift;
+  }
+
+  if constexpr (XP) {
+    // row by row through the staging tile (A is free once the products are done)
+    T ya[PP], yb[PP];
+    e.filter(xa, xb, []() {}, [&](int i, Acc p, Acc q) {
+      ya[i] = bad ? bad_value(T(0.0f)) : finish_real<T>(p, ue);
+      yb[i] = bad ? bad_value(T(0.0f)) : finish_real<T>(q, ue);
+    });
+    e.sync();
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      const int k = PP * e.u + i;
+      if (mine && k < H) {
+        stg[e.line * P + k] = ya[i];
+        stg[e.line * P + k + H] = yb[i];
+      }
+    }
+    e.sync();
+    const T *wd = !PAIR && post ? post + tile : nullptr;
+    over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
+      T x = stg[r * P + col];
+      if (wd) x = x * ldg(wd + i);
+      out[tile + i] = x;
+    });
+  } else {
+    e.filter(xa, xb, []() {}, [&](int i, Acc p, Acc q) {
+      const int k = PP * e.u + i;
+      if (mine && k < H) {
+        const long long o0 = base + (long long)k * ln.s_n, o1 = o0 + (long long)H * ln.s_n;
+        T r0 = bad ? bad_value(T(0.0f)) : finish_real<T>(p, ue);
+        T r1 = bad ? bad_value(T(0.0f)) : finish_real<T>(q, ue);
+        if (!PAIR && post) {
+          r0 = r0 * ldg(post + o0);
+          r1 = r1 * ldg(post + o1);
+        }
+        out[o0] = r0;
+        out[o1] = r1;
+      }
+    });
+  }
+  e.finish(ps.err);
+}
+
+// ------------------------------------------------------------------ k_fix
+enum { FIRST = 0, MID = 1, PAIR = 2, LAST = 3 };
+
+constexpr int kBadExp = 0x7fffffff;         // ex: the values are not finite
+
+// Points per line of the staging memory: x passes stage rows, column passes
+// with 16 points per thread the factor step (32 per thread).
+__host__ __device__ inline int stage_points(const Lines &ln, bool xp, int mode) {
+  if (xp) return ln.n;
+  return ln.kg > 2 && (mode == PAIR || mode == LAST) ? 32 * ln.kg - 1 : 0;
+}
+__device__ __forceinline__ bool unit_bad(int s) { return s >= 0x40000000; }
+
+__device__ __forceinline__ int64_t ld64(const int64_t *p) {
+  return __ldg(reinterpret_cast<const long long *>(p));
+}
+// r = W y as the stored slice's value
+__device__ __forceinline__ double slice_value(int64_t r, int ur) {
+  const int h = (int)(r >> 32);
+  if (h != (h >> 31) && fast_units(ur)) return from_fixed_fast(r, ur);
+  return from_fixed(r, ur, 0.0);
+}
+
+template <int PP, bool XP, int MODE>
+__global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const void *table, FixPass fp) {
+  typedef Tile<7, PP> E;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  E e;
+  e.setup(smem_raw, stage_points(ln, XP, MODE), ln.kg, 8, table);
+  const TcHead head = *static_cast<const TcHead *>(table);
+  const long long b = blockIdx.z;
+  const unsigned line0 = blockIdx.x * kLines;
+  const int nl = (int)min((long long)kLines, ln.lines - line0);
+  const unsigned H = ln.half;
+  const int kbits = *fp.kbits;
+  pdl_wait();      // the input is the previous pass's output
+  pdl_release();
+  if (e.issuer) {
+    e.run_issuer(MODE == PAIR ? 2 : 1);
+    e.finish(fp.err);
+    return;
+  }
+  e.run_compute();
+  const int eref = fp.eref[b];
+  // element offsets within an instance fit 32 bits (at most 128^3 points)
+  const unsigned c = line0 + e.line, rl = (unsigned)ln.row_len;
+  const unsigned base = XP ? c * ln.n : (c / rl) * (unsigned)ln.s_outer + c % rl;
+  const unsigned sn = XP ? 1 : (unsigned)ln.s_n;
+  const unsigned k0 = PP * e.u, tile = line0 * ln.n;
+  const unsigned off = base + k0 * sn, hs = H * sn;
+  const int lim = e.line < nl ? (int)H - (int)k0 : 0;   // this thread's points: i < lim
+  const int P = ln.n + 1;
+  int64_t *stg = reinterpret_cast<int64_t *>(smem_raw);
+  int64_t *row = stg + e.line * P + k0;                 // its points in the staging tile
+  int *ur_row = reinterpret_cast<int *>(smem_raw + e.lay.ur_off);
+  const int64_t *wf = fp.w + b * fp.w_bs;
+  // units: 2^u_in of the input, 2^u_out of the output
+  const int s_in = MODE == FIRST ? 0 : fp.u_in[b], s_out = MODE == LAST ? 0 : fp.u_out[b];
+  bool bad = unit_bad(s_in) || unit_bad(s_out);   // (FIRST: u_out is the input's own)
+  const int u_in = s_in + fp.w_in * (eref - 1022) + kbits - 59;
+  const int u_out = s_out + fp.w_out * (eref - 1022) + kbits - 59;
+  const int shift = 55 - head.kshift;
+
+  int64_t xa[PP], xb[PP];
+  int ue;                       // xa, xb in units of 2^ue
+  if constexpr (MODE == FIRST) {
+    // real slice times the factor; a handful of launches per iteration, so the
+    // x pass reads its rows without staging
+    const double *in = static_cast<const double *>(fp.in) + b * fp.in_bs;
+    double a[PP], bb[PP];
+    int key = 0;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      a[i] = i < lim ? ldg(in + (off + i * sn)) : 0.0;
+      bb[i] = i < lim ? ldg(in + (off + i * sn + hs)) : 0.0;
+      key = max(key, max(mag_key(a[i]), mag_key(bb[i])));
+    }
+    e.start();   // TMEM address, cleared keys
+    key = e.line_key(0, key);
+    const int Eb = line_exp(0.0, key);
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      const int64_t w0 = i < lim ? wf[off + i * sn] : 0, w1 = i < lim ? wf[off + i * sn + hs] : 0;
+      bad |= w0 < 0 || w1 < 0;
+      xa[i] = mul_w62(to_fixed(a[i], Eb) << 6, w0);
+      xb[i] = mul_w62(to_fixed(bb[i], Eb) << 6, w1);
+    }
+    bad = e.any(bad);
+    ue = unit_exp(0.0, Eb) - 6 + eref - 1022;
+  } else {
+    const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs;
+    if constexpr (XP) {
+      over_rows(e.ncomp, ln.n, nl, in + tile,
+                [&](int r, int col, int, int64_t x) { stg[r * P + col] = x; });
+      e.sync();
+    }
+    int key = 0;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      xa[i] = xb[i] = 0;
+      if (i < lim) {
+        xa[i] = XP ? row[i] : ld64(in + (off + i * sn));
+        xb[i] = XP ? row[i + H] : ld64(in + (off + i * sn + hs));
+      }
+      key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
+    }
+    e.start();   // TMEM address, cleared keys; the staging tile is read
+    key = e.line_key(0, key);
+    const int lz = clz32((uint32_t)key | 1u) - 2;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      xa[i] = to_digits54(xa[i], lz);
+      xb[i] = to_digits54(xb[i], lz);
+    }
+    ue = u_in + 8 - lz;
+  }
+
+  // The filters and what follows each.  One copy of the code serves both
+  // filters of a pair: with two a pair was 7450 instructions long (119 KB at
+  // N = 128) and waited for them.
+  int64_t *out = static_cast<int64_t *>(fp.out) + b * fp.out_bs;
+#pragma unroll 1
+  for (int f = 0; f < (MODE == PAIR ? 2 : 1); ++f) {
+    if (MODE == FIRST || (MODE == PAIR && f == 1)) {
+      // the formed v: report its exponent, rescale the lines
+      int key = 0;
+#pragma unroll
+      for (int i = 0; i < PP; ++i) key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
+      key = e.line_key(1, key);   // (its barrier: the staging tile is read)
+      const int clz = clz32((uint32_t)key | 1u);
+      if (e.u == 0) {
+        int x = bad ? kBadExp : (e.line < nl ? ue + 64 - clz : INT_MIN);
+        x = __reduce_max_sync(0xffffffffu, x);
+        if ((threadIdx.x & 31) == 0 && x != INT_MIN) atomicMax(fp.ex + b, x);
+      }
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        xa[i] = to_digits54(xa[i], clz - 2);
+        xb[i] = to_digits54(xb[i], clz - 2);
+      }
+      ue += 10 - clz;
+    }
+    e.filter(xa, xb, []() {});
+    if (MODE == LAST || (MODE == PAIR && f == 0)) {
+      // q = W y to the finished slice, v = W q onwards
+      const int ur = ue + shift + eref - 1022;            // unit of r = W y
+      double *qo = static_cast<double *>(fp.q) + b * fp.q_bs;
+      int wneg = 0;   // the factors' signs: a negative one is not finite
+      if constexpr (XP) {
+        e.sync();   // A is free
+        if (e.u == 0) ur_row[e.line] = ur;
+#pragma unroll
+        for (int i = 0; i < PP; ++i) {
+          if (i < lim) {
+            row[i] = xa[i];
+            row[i + H] = xb[i];
+          }
+        }
+        e.sync();
+        auto factor = [&](int r, int col, int i, int64_t w) {
+          wneg |= (int)(w >> 32);
+          const int64_t v = mul_w62(stg[r * P + col], w);
+          qo[tile + i] = slice_value(v, ur_row[r]);
+          if (MODE == PAIR) stg[r * P + col] = mul_w62(v, w);
+        };
+        over_rows(e.ncomp, ln.n, nl, wf + tile, factor);
+        if (bad || wneg < 0)
+          over_rows(e.ncomp, ln.n, nl, wf + tile, [&](int, int, int i, int64_t w) {
+            if (bad || w < 0) qo[tile + i] = bad_value(0.0);
+          });
+        if constexpr (MODE == PAIR) {
+          if (e.any(wneg < 0)) bad = true;
+#pragma unroll
+          for (int i = 0; i < PP; ++i) {
+            xa[i] = i < lim ? row[i] : 0;
+            xb[i] = i < lim ? row[i + H] : 0;
+          }
+        }
+      } else {
+        auto factor = [&](unsigned o, int64_t &x, int64_t w, bool on) {
+          wneg |= (int)(w >> 32);
+          const int64_t r = mul_w62(x, w);
+          const double q = slice_value(r, ur);
+          if (on) qo[o] = q;
+          x = mul_w62(r, w);
+        };
+        if constexpr (PP == 8) {
+#pragma unroll
+          for (int g = 0; g < PP; g += 4) {
+            int64_t w[8];   // (predicated loads: a branch around a point would
+                            // serialise them)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const unsigned o = off + (g + i) * sn;
+              w[2 * i] = g + i < lim ? ld64(wf + o) : 0;
+              w[2 * i + 1] = g + i < lim ? ld64(wf + (o + hs)) : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const unsigned o = off + (g + i) * sn;
+              factor(o, xa[g + i], w[2 * i], g + i < lim);
+              factor(o + hs, xb[g + i], w[2 * i + 1], g + i < lim);
+            }
+          }
+        } else {
+          // through the thread's own part of the (free) operand memory: as an
+          // unrolled loop over registers this spilled 800 bytes a thread
+          int64_t *own = stg + threadIdx.x;
+#pragma unroll
+          for (int i = 0; i < PP; ++i) {
+            own[2 * i * e.ncomp] = xa[i];
+            own[(2 * i + 1) * e.ncomp] = xb[i];
+          }
+          // (predicated loads, two points ahead)
+          int64_t w[4];
+          auto load_w = [&](int i) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const unsigned o = off + (i + j) * sn;
+              w[2 * j] = i + j < lim ? ld64(wf + o) : 0;
+              w[2 * j + 1] = i + j < lim ? ld64(wf + (o + hs)) : 0;
+            }
+          };
+          load_w(0);
+#pragma unroll 1
+          for (int i = 0; i < PP; i += 2) {
+            const int64_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
+            int64_t y0 = own[2 * i * e.ncomp], y1 = own[(2 * i + 1) * e.ncomp], y2 = own[(2 * i + 2) * e.ncomp], y3 = own[(2 * i + 3) * e.ncomp];
+            if (i + 2 < PP) load_w(i + 2);
+            const unsigned o = off + i * sn;
+            factor(o, y0, w0, i < lim);
+            factor(o + hs, y1, w1, i < lim);
+            factor(o + sn, y2, w2, i + 1 < lim);
+            factor(o + sn + hs, y3, w3, i + 1 < lim);
+            own[2 * i * e.ncomp] = y0;
+            own[(2 * i + 1) * e.ncomp] = y1;
+            own[(2 * i + 2) * e.ncomp] = y2;
+            own[(2 * i + 3) * e.ncomp] = y3;
+          }
+          if (MODE == PAIR) {
+#pragma unroll
+            for (int i = 0; i < PP; ++i) {
+              xa[i] = own[2 * i * e.ncomp];
+              xb[i] = own[(2 * i + 1) * e.ncomp];
+            }
+          }
+        }
+        if (bad || wneg < 0)
+          for (int i = 0; i < lim && i < PP; ++i) {
+            const unsigned o = off + i * sn;
+            if (bad || wf[o] < 0) qo[o] = bad_value(0.0);
+            if (bad || wf[o + hs] < 0) qo[o + hs] = bad_value(0.0);
+          }
+        if constexpr (MODE == PAIR) {
+          if (e.any(wneg < 0)) bad = true;
+        }
+      }
+      ue = ur + eref - 1022;   // v = W r (PAIR)
+    }
+  }
+
+  if constexpr (MODE != LAST) {
+    const Rescale rs(u_out - (ue + shift));   // to the output's unit
+    if constexpr (XP) {
+      e.sync();   // A is free
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        if (i < lim) {
+          row[i] = rs(xa[i]);
+          row[i + H] = rs(xb[i]);
+        }
+      }
+      e.sync();
+      over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) { out[tile + i] = stg[r * P + col]; });
+    } else {
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        if (i < lim) {
+          out[off + i * sn] = rs(xa[i]);
+          out[off + i * sn + hs] = rs(xb[i]);
+        }
+      }
+    }
+  }
+  e.finish(fp.err);
+}
+
+// ------------------------------------------------- factors and slice exponents
+// The largest biased FP64 exponent of each instance's finite factors.
+__global__ void k_wexp(const double *__restrict__ W, long long M, int *__restrict__ eref) {
+  const double *w = W + (long long)blockIdx.y * M;
+  int e = 0;
+  stream_loop<4>(M, [&](long long i) { return w[i]; }, [&](long long, double x) {
+    if (mag_key(x) < bad_key<double>()) e = max(e, line_exp(x, mag_key(x)));
+  });
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0) atomicMax(eref + blockIdx.y, e);
+}
+// W as packed integers: W = wf * 2^(eref - 1084), wf < 2^62; negative where not
+// finite.
+__global__ void k_wfix(const double *__restrict__ W, long long M, const int *__restrict__ eref_,
+                       int64_t *__restrict__ wf) {
+  const long long o = (long long)blockIdx.y * M;
+  const int eref = eref_[blockIdx.y];
+  stream_loop<4>(M, [&](long long i) { return W[o + i]; }, [&](long long i, double x) {
+    // from units of 2^(eref - 1076)
+    wf[o + i] = mag_key(x) >= bad_key<double>() ? -1 : pack_w62(to_fixed(x, eref) << 8);
+  });
+}
+// Exponent bound of a slice: every |q| < 2^ex[b]; kBadExp when not finite.
+__global__ void k_slice_exp(const double *__restrict__ q, long long bs, long long M,
+                            int *__restrict__ ex) {
+  const double *x = q + (long long)blockIdx.y * bs;
+  int key = 0;
+  stream_loop<4>(M, [&](long long i) { return x[i]; },
+                 [&](long long, double v) { key = max(key, mag_key(v)); });
+  key = __reduce_max_sync(0xffffffffu, key);
+  if ((threadIdx.x & 31) == 0 && key != 0) {
+    int e = kBadExp;
+    if (key < bad_key<double>()) e = unit_exp(0.0, line_exp(0.0, key)) + 55;
+    atomicMax(ex + blockIdx.y, e);
+  }
+}
+
+// Geometry of a pass, or false when the kernels do not take it.
+bool lines_of(const AxisPlan &ap, int nd, Lines &ln) {
+  if (!ap.tc || !tc_line_possible(ap.n, nd) || ap.n_real < 1 || ap.n_outer < 1) return false;
+  ln.n = ap.n;
+  ln.half = ap.n / 2;
+  ln.kg = (ln.half + 15) / 16;
+  ln.s_n = ap.s_n;
+  ln.lines = (long long)ap.n_real * ap.n_outer;
+  if (ap.n_fast) {                 // rows
+    ln.row_len = 1;
+    ln.s_outer = ap.n;
+  } else if (ap.flat_nx) {         // columns over (row, outer)
+    ln.row_len = ap.flat_nx;
+    ln.s_outer = ap.s_outer;
+  } else {
+    ln.row_len = ap.n_real;
+    ln.s_outer = ap.s_outer;
+  }
+  return (ln.lines + kLines - 1) / kLines <= 0x7fffffffLL;
+}
+inline int threads_of(const Lines &ln) {
+  const int pp = pairs_per_thread(ln.kg);
+  return kLines * 16 * ln.kg / pp + issuer_threads(pp);
+}
+
+template <typename T, int MAXT, int PP, bool XP, bool PR>
+cudaError_t launch_real_t(const Lines &ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+  dim3 grid((unsigned)((ln.lines + kLines - 1) / kLines), 1, ps.nset * ps.batch);
+  return launch_pdl(k_real<T, MAXT, PP, XP, PR>, grid, dim3(threads_of(ln)),
+                    (size_t)smem_layout(kNd<T>, ln.n, ln.kg, XP ? (int)sizeof(T) : 0).total, st,
+                    ln, tc, ps);
+}
+template <typename T, bool XP, bool PR>
+cudaError_t launch_real_kg(const Lines &ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+  if (ln.kg <= 2) return launch_real_t<T, 544, 8, XP, PR>(ln, tc, ps, st);
+  if constexpr (std::is_same<T, float>::value) {
+    if (ln.kg > 4) return launch_real_t<T, 1024, 16, XP, PR>(ln, tc, ps, st);
+  }
+  return launch_real_t<T, 640, 16, XP, PR>(ln, tc, ps, st);
+}
+template <typename T>
+cudaError_t launch_real(const AxisPlan &ap, const PassSet<T> &ps, bool pair, cudaStream_t st) {
+  Lines ln;
+  const long long sets = (long long)ps.nset * ps.batch;
+  if (!lines_of(ap, kNd<T>, ln) || ps.nset < 1 || ps.nset > kMaxSet || sets < 1 || sets > 65535 ||
+      (ps.desc && (pair || kNd<T> != 4)))
+    return cudaErrorInvalidValue;
+  for (int k = 0; k < ps.nset && !ps.desc; ++k) {
+    if (!ps.in[k] || !ps.out[k] || (pair && (!ps.post[k] || !ps.qout[k])))
+      return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(ps.in[k]) | reinterpret_cast<uintptr_t>(ps.out[k]) |
+         reinterpret_cast<uintptr_t>(ps.pre[k]) | reinterpret_cast<uintptr_t>(ps.post[k]) |
+         reinterpret_cast<uintptr_t>(ps.qout[k])) & (sizeof(T) - 1))
+      return cudaErrorMisalignedAddress;
+  }
+  if constexpr (std::is_same<T, float>::value) {
+    if (pair)
+      return ap.n_fast ? launch_real_kg<T, true, true>(ln, ap.tc, ps, st)
+                       : launch_real_kg<T, false, true>(ln, ap.tc, ps, st);
+  } else {
+    if (pair) return cudaErrorInvalidValue;   // 64-bit pairs run in k_fix
+  }
+  return ap.n_fast ? launch_real_kg<T, true, false>(ln, ap.tc, ps, st)
+                   : launch_real_kg<T, false, false>(ln, ap.tc, ps, st);
+}
+
+template <bool XP, int MODE>
+cudaError_t launch_fix_t(const Lines &ln, const void *tc, const FixPass &fp, cudaStream_t st) {
+  dim3 grid((unsigned)((ln.lines + kLines - 1) / kLines), 1, fp.batch);
+  const size_t smem = smem_layout(7, stage_points(ln, XP, MODE), ln.kg, 8).total;
+  if (ln.kg <= 2)
+    return launch_pdl(k_fix<8, XP, MODE>, grid, dim3(threads_of(ln)), smem, st, ln, tc, fp);
+  return launch_pdl(k_fix<16, XP, MODE>, grid, dim3(threads_of(ln)), smem, st, ln, tc, fp);
+}
+
+// Shared-memory opt-in; a kernel that splits its registers must have been given
+// at least the launch count that the split was added up for.
+template <typename K> cudaError_t opt_in(K *k, bool splits = false) {
+  if (splits) {
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, k);
+    if (e != cudaSuccess) return e;
+    if (at.numRegs != kRegsLaunch) return cudaErrorInvalidConfiguration;
+  }
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+template <typename T, int MAXT, int PP> cudaError_t prep_real() {
+  constexpr bool kSplit = kNd<T> == 7 && PP == 16;
+  cudaError_t e;
+  if ((e = opt_in(k_real<T, MAXT, PP, true, false>, kSplit)) != cudaSuccess) return e;
+  if ((e = opt_in(k_real<T, MAXT, PP, false, false>, kSplit)) != cudaSuccess) return e;
+  if constexpr (std::is_same<T, float>::value) {
+    if ((e = opt_in(k_real<T, MAXT, PP, true, true>, kSplit)) != cudaSuccess) return e;
+    if ((e = opt_in(k_real<T, MAXT, PP, false, true>, kSplit)) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+template <int PP> cudaError_t prep_fix() {
+  cudaError_t e;
+  if ((e = opt_in(k_fix<PP, true, FIRST>, PP == 16)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, FIRST>, PP == 16)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, MID>, PP == 16)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, true, PAIR>, PP == 16)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, PAIR>, PP == 16)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, true, LAST>, PP == 16)) != cudaSuccess) return e;
+  return opt_in(k_fix<PP, false, LAST>, PP == 16);
+}
+
+// ---- host: the convolution kernel in double-double arithmetic
+struct dd {
+  double h, l;
+};
+dd dd_norm(double a, double b) {
+  const double s = a + b, bb = s - a;
+  return {s, (a - (s - bb)) + (b - bb)};
+}
+dd dd_add(dd a, dd b) {
+  dd s = dd_norm(a.h, b.h);
+  return dd_norm(s.h, s.l + (a.l + b.l));
+}
+dd dd_mul(dd a, dd b) {
+  const double p = a.h * b.h, e = fma(a.h, b.h, -p);
+  return dd_norm(p, e + (a.h * b.l + a.l * b.h));
+}
+dd dd_div_small(dd a, double n) {   // a / n, n a small integer
+  const double q = a.h / n, r = fma(-q, n, a.h);
+  return dd_norm(q, (r + a.l) / n);
+}
+// cos(2 pi m / n): Taylor series on [0, pi/4], the symmetries outside
+dd dd_cos2pi(long m, long n) {
+  m %= n;
+  if (2 * m > n) m = n - m;                 // cos is even: m/n in [0, 1/2]
+  bool neg = false;
+  if (4 * m > n) {                          // cos(pi - t) = -cos t
+    m = n - 2 * m;
+    n *= 2;
+    neg = true;
+  }
+  const bool sine = 8 * m > n;              // above 1/8: cos(pi/2 - t) = sin t
+  if (sine) {
+    m = n - 4 * m;
+    n *= 4;
+  }
+  const dd two_pi = {6.283185307179586, 2.4492935982947064e-16};
+  dd x = dd_mul(two_pi, dd_div_small({(double)m, 0.0}, (double)n));
+  dd x2 = dd_mul(x, x), term = sine ? x : dd{1.0, 0.0}, sum = term;
+  for (int i = 1; i < 20; ++i) {
+    const double d = sine ? (2.0 * i) * (2.0 * i + 1.0) : (2.0 * i - 1.0) * (2.0 * i);
+    term = dd_div_small(dd_mul(term, x2), -d);
+    sum = dd_add(sum, term);
+  }
+  return neg ? dd{-sum.h, -sum.l} : sum;
+}
+// a * 2^s as an integer, rounded to nearest (|a 2^s| < 2^62)
+int64_t dd_to_int(dd a, int s) {
+  const double h = ldexp(a.h, s), l = ldexp(a.l, s);
+  const double hi = rint(h);
+  const double r = rint((h - hi) + l);
+  return (int64_t)hi + (int64_t)r;
+}
+// a small integer as f16 bits
+uint16_t f16_of_int(int v) {
+  if (v == 0) return 0;
+  const uint16_t s = v < 0 ? 0x8000 : 0;
+  int a = v < 0 ? -v : v, e = 0;
+  while ((a >> (e + 1)) != 0) ++e;
+  return (uint16_t)(s | ((15 + e) << 10) | (((a << (10 - e)) & 0x3ff)));
+}
+// digit j (0 the top one) of v
+int digit_of(int64_t v, int nd, int j) {
+  const uint64_t z = (uint64_t)v + (nd == 7 ? 0x0080808080808080ULL : 0x80808080ULL);
+  return (int)((z >> (8 * (nd - 1 - j))) & 0xff) - 128;
+}
+
+// The table with K scaled `less` bits below the digits' full range.
+bool build_scaled(const std::vector<dd> &K, int nd, int less, std::vector<unsigned char> &table) {
+  const int n = (int)K.size(), H = n / 2, kg = (H + 15) / 16, kp = 16 * kg;
+  const int bits = 8 * nd;
+  double mx = 0.0;
+  for (int d = 0; d < H; ++d)
+    for (int s = -1; s <= 1; s += 2) mx = fmax(mx, fabs(K[d].h + s * K[d + H].h));
+  TcHead head;
+  memset(&head, 0, sizeof head);
+  int shift = 0;
+  if (mx > 0.0) {
+    int ex;
+    frexp(mx, &ex);                               // mx < 2^ex
+    shift = bits - 1 - ex;
+    // a top digit of at most 127 with any others behind it
+    if (ldexp(mx, shift) > ldexp(126.9, bits - 8)) --shift;
+  }
+  shift -= less;
+  if (shift > 900 || shift < -900) return false;
+  head.kshift = shift;
+  // integers of K, with the zero-frequency sum kept exact: its rounding would
+  // act on every line's mean in every step
+  std::vector<int64_t> Ki(n);
+  dd sum = {0.0, 0.0};
+  int64_t isum = 0;
+  for (int d = 0; d < n; ++d) {
+    Ki[d] = dd_to_int(K[d], shift);
+    isum += Ki[d];
+    sum = dd_add(sum, K[d]);
+  }
+  int64_t miss = dd_to_int(sum, shift) - isum;
+  for (int d = 1; (miss > 1 || miss < -1) && 2 * d < n; ++d) {   // in +-d pairs near the peak
+    const int s = miss > 0 ? 1 : -1;
+    Ki[d] += s;
+    Ki[n - d] += s;
+    miss -= 2 * s;
+  }
+  Ki[0] += miss;
+  table.assign(tc_table_bytes(n, nd), 0);
+  uint16_t *out = reinterpret_cast<uint16_t *>(table.data() + sizeof(TcHead));
+  for (int par = 0; par < 2; ++par) {
+    // t[d], d = n - k in (-H, H): cyclic (c) or negacyclic (d)
+    auto tv = [&](int d) -> int64_t {
+      if (d <= -H || d >= H) return 0;
+      const int m = d < 0 ? d + H : d;
+      const int64_t v = par == 0 ? Ki[m] + Ki[m + H] : Ki[m] - Ki[m + H];
+      return par == 1 && d < 0 ? -v : v;
+    };
+    double worst = 0.0;
+    for (int d = 0; d < H; ++d) {
+      const int64_t v = tv(d);
+      // for d also -v can stand in a row: the larger digit bounds the sums
+      for (int j = 0; j < nd; ++j) {
+        const int a = abs(digit_of(v, nd, j)), c = par == 1 ? abs(digit_of(-v, nd, j)) : 0;
+        worst += 128.0 * std::max(a, c);
+      }
+    }
+    if (!(worst < (nd == 7 ? 4194304.0 : 16777216.0))) return false;
+    uint16_t *half = out + (size_t)par * b_half_bytes(nd, kg) / 2;
+    if (dense_b(kg)) {       // [k block][row block of (round, digit, output)][8 rows][8 k]
+      const int rounds = split_rows(nd, kg) ? 2 : 1, gc = group_cols(nd, kg);
+      for (int rd = 0; rd < rounds; ++rd)
+        for (int j = 0; j < nd; ++j)
+          for (int col = 0; col < gc; ++col) {
+            const int r = rounds == 2 ? col / 8 * 16 + 8 * rd + col % 8 : col;   // the output
+            const int row = (rd * nd + j) * gc + col;
+            for (int k = 0; k < kp; ++k) {
+              const int dj = r < H && k < H ? digit_of(tv(r - k), nd, j) : 0;
+              half[((size_t)(k / 8) * (rounds * nd * gc / 8) + row / 8) * 64 + (row % 8) * 8 +
+                   k % 8] = f16_of_int(dj);
+            }
+          }
+    } else {                 // [digit][n block - k block][8][8]
+      const int NB = 4 * kg - 1;
+      for (int j = 0; j < nd; ++j)
+        for (int blk = 0; blk < NB; ++blk)
+          for (int r = 0; r < 8; ++r)
+            for (int c = 0; c < 8; ++c)
+              half[((size_t)j * NB + blk) * 64 + r * 8 + c] =
+                  f16_of_int(digit_of(tv(8 * (blk - (2 * kg - 1)) + r - c), nd, j));
+    }
+  }
+  memcpy(table.data(), &head, sizeof head);
+  return true;
+}
+
+}  // namespace
+
+bool tc_line_possible(int n, int nd) {
+  return n >= 2 && n % 2 == 0 && (n / 2 + 15) / 16 <= (nd == 4 ? 7 : 4);
+}
+
+size_t tc_table_bytes(int n, int nd) {
+  return sizeof(TcHead) + 2 * (size_t)b_half_bytes(nd, (n / 2 + 15) / 16);
+}
+
+// Digits of the two half-length kernels of gain table g (natural order, real
+// and even, the 1/n of the transform included).  The digits' sizes depend on
+// the scale; the first of a few scales whose accumulators stay in the exact
+// range is taken.  False when none does or the gains are not finite: the
+// caller keeps the FFT pass.  row_sum: sum |K|, the filter's largest growth.
+bool tc_build_table(const double *g, int n, int nd, std::vector<unsigned char> &table,
+                    double *row_sum) {
+  for (int k = 0; k < n; ++k)
+    if (!std::isfinite(g[k])) return false;
+  std::vector<dd> ct(n), K(n);
+  for (int m = 0; m < n; ++m) ct[m] = dd_cos2pi(m, n);
+  double l1 = 0.0;
+  // g and K are even: bins and offsets up to n/2 stand for their mirrors
+  const int h = n / 2;
+  for (int d = 0; d <= h; ++d) {
+    dd s = {0.0, 0.0};
+    for (int k = 1; k < h; ++k) s = dd_add(s, dd_mul({g[k], 0.0}, ct[k * d % n]));
+    s = dd_add({2.0 * s.h, 2.0 * s.l}, {g[0], 0.0});
+    K[d] = dd_add(s, {d & 1 ? -g[h] : g[h], 0.0});
+    if (d > 0 && d < h) K[n - d] = K[d];
+    l1 += fabs(K[d].h) * (d > 0 && d < h ? 2.0 : 1.0);
+  }
+  if (row_sum) *row_sum = l1;
+  for (int less = 0; less < 4; ++less)
+    if (build_scaled(K, nd, less, table)) return true;
+  return false;
+}
+
+namespace {
+cudaError_t prepare_all() {
+  cudaError_t e;
+  if ((e = prep_real<float, 544, 8>()) != cudaSuccess) return e;
+  if ((e = prep_real<float, 640, 16>()) != cudaSuccess) return e;
+  if ((e = prep_real<float, 1024, 16>()) != cudaSuccess) return e;
+  if ((e = prep_real<double, 544, 8>()) != cudaSuccess) return e;
+  if ((e = prep_real<double, 640, 16>()) != cudaSuccess) return e;
+  if ((e = prep_fix<8>()) != cudaSuccess) return e;
+  return prep_fix<16>();
+}
+}  // namespace
+
+// Kernel attributes, set once per device (host threads may race to it).
+cudaError_t tc_prepare() {
+  static std::mutex mu;
+  static bool done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!done[dev]) {
+    if ((e = prepare_all()) != cudaSuccess) return e;
+    done[dev] = true;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float> &ps, bool pair, cudaStream_t st) {
+  return launch_real(ap, ps, pair, st);
+}
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double> &ps, bool pair, cudaStream_t st) {
+  return launch_real(ap, ps, pair, st);
+}
+
+cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStream_t st) {
+  Lines ln;
+  if (!lines_of(ap, 7, ln) || fp.batch < 1 || fp.batch > 65535 || !fp.in || !fp.eref || !fp.kbits ||
+      (mode != LAST && (!fp.out || !fp.u_out)) || (mode != FIRST && !fp.u_in) ||
+      (mode != MID && !fp.w) || ((mode == PAIR || mode == LAST) && !fp.q) ||
+      ((mode == FIRST || mode == PAIR) && !fp.ex))
+    return cudaErrorInvalidValue;
+  const bool x = ap.n_fast != 0;
+  switch (mode) {
+    case FIRST:
+      return x ? launch_fix_t<true, FIRST>(ln, ap.tc, fp, st)
+               : launch_fix_t<false, FIRST>(ln, ap.tc, fp, st);
+    case MID:
+      return x ? cudaErrorInvalidValue : launch_fix_t<false, MID>(ln, ap.tc, fp, st);
+    case PAIR:
+      return x ? launch_fix_t<true, PAIR>(ln, ap.tc, fp, st)
+               : launch_fix_t<false, PAIR>(ln, ap.tc, fp, st);
+    case LAST:
+      return x ? launch_fix_t<true, LAST>(ln, ap.tc, fp, st)
+               : launch_fix_t<false, LAST>(ln, ap.tc, fp, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+// Factors in integers: eref[b] and wf from W (two launches).
+cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
+                        cudaStream_t st) {
+  if (batch > 65535) return cudaErrorInvalidValue;
+  cudaError_t e = cudaMemsetAsync(eref, 0, sizeof(int) * batch, st);
+  if (e != cudaSuccess) return e;
+  const unsigned g = (unsigned)std::min<long long>((M + 1023) / 1024, 608);
+  k_wexp<<<dim3(g, batch), 256, 0, st>>>(W, M, eref);
+  k_wfix<<<dim3(g, batch), 256, 0, st>>>(W, M, eref, wf);
+  return cudaGetLastError();
+}
+// ex[b] (cleared by the caller) from a slice.
+cudaError_t launch_slice_exp(const double *q, long long bs, long long M, int batch, int *ex,
+                             cudaStream_t st) {
+  if (batch > 65535) return cudaErrorInvalidValue;
+  const unsigned g = (unsigned)std::min<long long>((M + 1023) / 1024, 608);
+  k_slice_exp<<<dim3(g, batch), 256, 0, st>>>(q, bs, M, ex);
+  return cudaGetLastError();
+}
+
+}  // namespace scft

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "dfloat.cuh"
 
 namespace scft {
@@ -30,6 +32,7 @@ struct AxisPlan {
   int use_fast;          // FP32 register-resident kernel (k_fast.cu) handles this pass
   const void *twiddle;   // device: n complex, exp(-2*pi*i*m/n), working precision
   const void *gain;      // device: n reals, working precision
+  const void *tc;        // device: the gain's tensor-core table (k_tc.cu), or null
 };
 
 // One pass over up to kMaxSet independent propagators at once (the lockstep
@@ -44,6 +47,7 @@ struct PassDesc {
   const float *pre, *post;   // Boltzmann factor on load / on store, or null
   const float *gain;         // the set's gain table of this pass's axis (x for a plane pass)
   const float *gain_y;       // x+y plane passes: the y axis's gain table
+  const void *tc;            // the set's tensor-core table (passes through launch_tc)
 };
 template <typename R> struct PassSet {
   const R *in[kMaxSet];
@@ -100,6 +104,41 @@ cudaError_t launch_xx(const AxisPlan &ap, const PassSet<double> &ps, cudaStream_
 cudaError_t launch_xx(const AxisPlan &ap, const PassSet<dfloat> &ps, cudaStream_t st);
 cudaError_t launch_xyxy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
                         cudaStream_t st);
+
+// Tensor-core line filter (k_tc.cu): exact integer convolution of lines of any
+// even length, up to 128 points (FP64: 7 digits) or 224 (FP32: 4 digits).  pair (FP32): a fused step pair (qout = post * K(in),
+// out = K(post * qout)).
+bool tc_line_possible(int n, int nd);
+size_t tc_table_bytes(int n, int nd);
+bool tc_build_table(const double *gain, int n, int nd, std::vector<unsigned char> &table,
+                    double *row_sum);
+cudaError_t tc_prepare();
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float> &ps, bool pair, cudaStream_t st);
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double> &ps, bool pair, cudaStream_t st);
+// One pass of the fused FP64 march, whose intermediates are
+// 64-bit integers (batch instances; strides in elements).  The unit of an
+// intermediate is 2^(u[b] + w * (eref[b] - 1022) + kbits - 59): u the exponent
+// bound of the values it was formed from, w the factors applied since.
+struct FixPass {
+  const void *in;            // FIRST: FP64, else integers
+  void *out;                 // integers (not LAST)
+  void *q;                   // PAIR, LAST: the finished slice
+  const int64_t *w;          // the factors as integers (launch_wfix)
+  const int *eref;           // their largest exponent per instance
+  const int *kbits;          // log2 bound of one step's filters' growth
+  const int *u_in, *u_out;   // exponent bounds, [batch]
+  int w_in, w_out;
+  int *ex;                   // FIRST, PAIR: exponent bound of the formed W q (atomic max)
+  long long in_bs, out_bs, q_bs, w_bs;
+  int batch;
+  unsigned *err;             // device error word (bounded-wait timeouts)
+};
+constexpr int kFixFirst = 0, kFixMid = 1, kFixPair = 2, kFixLast = 3;
+cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStream_t st);
+cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
+                        cudaStream_t st);
+cudaError_t launch_slice_exp(const double *q, long long bs, long long M, int batch, int *ex,
+                             cudaStream_t st);
 
 // Generic mixed-radix Stockham line filter (any n whose prime factors are
 // <= 61).  in/out may not alias.  pre multiplies the input, post the output

@@ -1,0 +1,153 @@
+// Fixed-point slices for the tensor-core line filter (k_tc.cu): conversions
+// between the working reals and line-scaled integers, and the integers' signed
+// base-256 digits.  Host and device, integer and FP32 arithmetic only: an FP64
+// instruction on GB300 takes 16 cycles of an SM per warp, the sequences here
+// 3 to 6.
+//
+// A line x is held as integers X with x = X * 2^ue, ue chosen from the line's
+// largest exponent so that |X| <= 2^54 (FP64; 7 digits) or 2^29
+// (FP32; 4 digits).  All roundings are to nearest: a truncation's bias would
+// add up over the contour steps.
+#pragma once
+
+#include <stdint.h>
+#include <string.h>
+
+#include "common.cuh"
+
+namespace scft {
+namespace slices {
+
+#define SL_HD __host__ __device__ __forceinline__
+
+SL_HD uint32_t f2u(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t u; memcpy(&u, &f, 4); return u;
+#endif
+}
+SL_HD float u2f(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f; memcpy(&f, &u, 4); return f;
+#endif
+}
+SL_HD uint64_t d2u(double d) {
+#ifdef __CUDA_ARCH__
+  return (uint64_t)__double_as_longlong(d);
+#else
+  uint64_t u; memcpy(&u, &d, 8); return u;
+#endif
+}
+SL_HD double u2d(uint64_t u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)u);
+#else
+  double d; memcpy(&d, &u, 8); return d;
+#endif
+}
+SL_HD int clz64(uint64_t u) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)u);
+#else
+  return u ? __builtin_clzll(u) : 64;
+#endif
+}
+SL_HD int clz32(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __clz((int)u);
+#else
+  return u ? __builtin_clz(u) : 32;
+#endif
+}
+// y * w / 2^62 rounded to nearest (within 2^-29 of a unit), |y| < 2^61, with the
+// factor 0 <= w < 2^62 packed as two 31-bit halves (high word, low word):
+// three 32-bit products.
+SL_HD int64_t mul_w62(int64_t y, int64_t wp) {
+  const int wh = (int)(wp >> 32), wl = (int)wp;
+  const int yh = (int)(y >> 31), yl = (int)((uint32_t)y & 0x7fffffffu);
+  const int64_t t = (int64_t)yh * wl + ((int64_t)yl * wh + (1 << 30));
+  return (int64_t)yh * wh + (t >> 31);
+}
+SL_HD int64_t pack_w62(int64_t w) {
+  return (int64_t)((uint64_t)(w >> 31) << 32 | (uint64_t)(w & 0x7fffffff));
+}
+
+// 2^e as a float, e clamped to the normal range.
+SL_HD float exp2i(int e) {
+  e = e < -126 ? -126 : (e > 127 ? 127 : e);
+  return u2f((uint32_t)(e + 127) << 23);
+}
+// x * 2^e for any e (two steps keep the factors normal).
+SL_HD float scale2(float x, int e) {
+  const int h = e / 2;
+  return x * exp2i(h) * exp2i(e - h);
+}
+
+// Magnitude keys: ordered like |x|; a key of kBadKey<T> or more marks a NaN or
+// an infinity.
+SL_HD int mag_key(double x) { return (int)((uint32_t)(d2u(x) >> 32) & 0x7fffffffu); }
+SL_HD int mag_key(float x) { return (int)(f2u(x) & 0x7fffffffu); }
+template <typename T> SL_HD constexpr int bad_key() { return sizeof(T) == 8 ? 0x7ff00000 : 0x7f800000; }
+
+// Biased exponent of a line's largest magnitude, and the unit exponent ue.
+SL_HD int line_exp(double, int key) { return key >> 20; }
+SL_HD int line_exp(float, int key) { return key >> 23; }
+SL_HD int unit_exp(double, int E) { return E - 1076; }   // |X| < 2^54
+SL_HD int unit_exp(float, int E) { return (E < 29 ? 29 : E) - 155; }   // |X| <= 2^29
+
+// x / 2^unit_exp(E), rounded to nearest; E is at least x's own exponent.
+SL_HD int64_t to_fixed(double x, int E) {
+  const uint64_t b = d2u(x);
+  const int e = (int)(b >> 52) & 0x7ff;
+  const uint64_t m = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 8;   // 61 bits
+  int sh = E - e;
+  if (e == 0 || sh > 63) sh = 63;                  // zero, or far below the line's unit
+  const int64_t t = (int64_t)(((m >> sh) + 64) >> 7);
+  const int64_t s = (int64_t)b >> 63;
+  return (t ^ s) - s;
+}
+SL_HD int to_fixed(float x, int E) {
+  const float s = x * exp2i(155 - (E < 29 ? 29 : E));
+#ifdef __CUDA_ARCH__
+  return __float2int_rn(s);
+#else
+  return (int)lrintf(s);
+#endif
+}
+
+// y * 2^ue as an FP64 number, |y| < 2^63, rounded to nearest (halves up);
+// results below the normal range become 0.
+SL_HD double from_fixed(int64_t y, int ue, double) {
+  const int64_t sg = y >> 63;
+  const uint64_t u = (uint64_t)((y ^ sg) - sg);
+  const int lz = clz64(u);                         // >= 1
+  const uint64_t m = ((u << ((lz - 1) & 63)) + 0x200) >> 10;   // leading bit 52 (53 after a carry)
+  const int be = 1086 + ue - lz;                   // biased exponent of the leading bit
+  uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(be - 1) << 20);
+  if (u == 0 || be <= 0) hi = 0;
+  if (be >= 2047) hi = 0x7ff00000u;
+  const uint32_t lo = u == 0 || be <= 0 || be >= 2047 ? 0u : (uint32_t)m;
+  return u2d(((uint64_t)(hi | ((uint32_t)(sg >> 32) & 0x80000000u)) << 32) | lo);
+}
+// The same for |y| in [2^32, 2^62) and results in the normal range (fast path;
+// a negative y is taken as ~y, one unit off).
+SL_HD double from_fixed_fast(int64_t y, int ue) {
+  const uint32_t sg = (uint32_t)(y >> 63);
+  const uint32_t h = (uint32_t)(y >> 32) ^ sg, l = (uint32_t)y ^ sg;
+  const int lz = clz32(h);                         // 2 .. 31
+  const uint64_t m = ((((uint64_t)h << 32 | l) << (lz - 1)) + 0x200) >> 10;
+  const uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(1085 + ue - lz) << 20);
+  return u2d((uint64_t)(hi | (sg & 0x80000000u)) << 32 | (uint32_t)m);
+}
+SL_HD bool fast_units(int ue) { return ue > -1000 && ue < 900; }
+// The signed base-256 digits of X (digit i weighs 256^(ND-1-i)) as bytes plus
+// 128: all but the top one are in [0, 255]; the top one, in the high half word,
+// is in [0, 256] (7 digits) or [64, 192] (4 digits).
+SL_HD uint64_t biased_digits(int64_t X) { return (uint64_t)X + 0x0080808080808080ULL; }
+SL_HD uint32_t biased_digits(int X) { return (uint32_t)X + 0x80808080u; }
+
+}  // namespace slices
+}  // namespace scft

@@ -1,0 +1,567 @@
+// Core of the tensor-core line filters (k_tc.cu): one axis of the separable
+// split-step operator as an exact integer convolution.
+//
+// The pass IFFT . diag(g) . FFT along an axis of N points is the circulant
+// convolution y[n] = sum_k K[(n-k) mod N] x[k] with K = IDFT(g).  Splitting it
+// by z^N - 1 = (z^H - 1)(z^H + 1), H = N/2, leaves two H x H Toeplitz products
+//   c = Kc (x[k] + x[k+H]),  d = Kd (x[k] - x[k+H]),   Kc/Kd = K[d] +- K[d+H]
+//   y[n] = (c[n] + d[n])/2,  y[n+H] = (c[n] - d[n])/2 .
+// Each is computed without rounding (the slicing scheme of Ozaki, Ogita, Oishi
+// and Rump, Numer. Algorithms 59, 2012): the line and the kernel are integers
+// of ND base-256 digits (slices.cuh; FP64 7, FP32 4), a digit
+// is an exact f16 number, and the products of digits i and j with i + j = g
+// accumulate in FP32 in one TMEM accumulator per g.  The host checks for each
+// table that no accumulator can reach 2^22 (2^24 for FP32), so every partial
+// sum is an integer that FP32 holds exactly and the order of the sums does not
+// matter.  What is left out (i + j >= ND) is below the last digit's unit.
+//
+// Tile: 128 lines (the M of one tcgen05.mma) x N points per CTA.  Thread t owns
+// line t % 128 (its TMEM lane) and the PP points k = PP*u + i, u = t / 128, with
+// their partners k + H: it writes their digits as A operands (K-major core
+// matrices of 8 lines x 16 bytes, unswizzled) and reads the same outputs back.
+// B holds the digits of Kc or Kd stacked along its rows (digit j, output n), so
+// one instruction multiplies x's digit i with all of K's digits 0 .. ND-1-i and
+// adds into the accumulators i .. ND-1 side by side: up to 256 columns per
+// instruction.  (One instruction per digit pair, 32 or 64 columns wide, took
+// about 76 cycles each whatever its width.)  Lines above 128 points (FP32) have
+// no room for that B; there its 8x8 core matrix (bn, bk), which depends only on
+// bn - bk, is shared by descriptor: with A's k blocks in reverse order both
+// strides are one core matrix.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "slices.cuh"
+
+namespace scft {
+namespace tc {
+
+using namespace slices;
+
+constexpr int kLines = 128;
+
+// Scales of a table, in front of its digits (device memory: a box change
+// rewrites tables in place under captured graphs).
+struct TcHead {
+  int kshift;    // K' = K * 2^kshift
+  int pad[3];
+};
+
+// Accumulators come in two TMEM buffers, so that one is read while the tensor
+// core fills the other.  Where A, B and TMEM have the room (both_halves) a
+// buffer holds all outputs of c or d; else half of the outputs (8 of each
+// thread's 16), and a half takes two rounds.
+__host__ __device__ constexpr bool both_halves(int nd, int kg) { return nd == 7 ? kg <= 2 : kg <= 4; }
+__host__ __device__ constexpr bool split_rows(int nd, int kg) { return nd == 7 && kg > 2; }
+// Accumulator columns of one digit group in one buffer (a multiple of 16), and
+// the outputs they stand for.
+__host__ __device__ constexpr int group_cols(int nd, int kg) { return split_rows(nd, kg) ? 32 : 16 * kg; }
+__host__ __device__ constexpr bool dense_b(int kg) { return kg <= 4; }
+// B of both halves resident (else the half in use is copied in).
+__host__ __device__ constexpr bool b_resident(int nd, int kg) { return nd != 7 || kg <= 3; }
+// Points per thread: 8 where that keeps the CTA at 512 threads.
+__host__ __device__ constexpr int pairs_per_thread(int kg) { return kg <= 2 ? 8 : 16; }
+// The issuing warp; with 16 points per thread a warpgroup of its own, so that
+// the computing ones can take its registers (setmaxnreg: 96 at launch for 640
+// threads, then 112 x 512 + 24 x 128 = 60416 <= 96 x 640 = 61440; with 384 + 128
+// threads 46080 <= 49152).
+__host__ __device__ constexpr int issuer_threads(int pp) { return pp == 16 ? 128 : 32; }
+constexpr int kRegsLaunch = 96, kRegsCompute = 112, kRegsIssue = 24;
+__host__ __device__ constexpr int b_half_bytes(int nd, int kg) {
+  return dense_b(kg) ? nd * group_cols(nd, kg) * (split_rows(nd, kg) ? 2 : 1) * (16 * kg) * 2
+                     : nd * (4 * kg - 1) * 128;
+}
+
+// ---- shared-memory layout (bytes)
+struct Smem {
+  int a_digit, a_half;   // one digit's A operand; one half's
+  int b_off, b_half, key_off, ur_off, bar_off, total;
+};
+__host__ __device__ inline Smem smem_layout(int nd, int n, int kg, int stage_elem) {
+  Smem s;
+  s.a_digit = kLines * kg * 16 * 2;
+  s.a_half = nd * s.a_digit;
+  int big = s.a_half * (both_halves(nd, kg) ? 2 : 1);
+  const int stage = stage_elem ? kLines * (n + 1) * stage_elem : 0;   // row staging, aliases A
+  if (stage > big) big = stage;
+  s.b_off = (big + 127) / 128 * 128;
+  s.b_half = b_half_bytes(nd, kg);
+  s.key_off = s.b_off + (b_resident(nd, kg) ? 2 : 1) * s.b_half;
+  s.ur_off = s.key_off + 2 * kLines * 4;    // keys of the two filters
+  s.bar_off = s.ur_off + kLines * 4;        // per-line units
+  s.total = s.bar_off + 64;                 // six mbarriers, TMEM address
+  return s;
+}
+__host__ __device__ constexpr int tmem_cols(int nd, int kg) {
+  int c = nd * group_cols(nd, kg) * (dense_b(kg) ? 2 : 1), p = 32;
+  while (p < c) p *= 2;
+  return p;
+}
+
+#ifdef __CUDACC__
+// ---- tcgen05 / mbarrier wrappers
+__device__ __forceinline__ uint32_t sm32(const void *p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void tm_alloc(uint32_t slot, int cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot),
+               "r"(cols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tm_free(uint32_t base, int cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols));
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                        int accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.s32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void fence_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// Waits for phase `parity`, at most ~1 s of SM clocks; false on timeout.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity) {
+  const long long t0 = clock64();
+  while (true) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (clock64() - t0 > 2000000000LL) return false;
+  }
+}
+// 1-D bulk copy global -> shared, completing on `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, unsigned bytes,
+                                          uint32_t bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+          dst),
+      "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+// Eight or four consecutive accumulator columns of this thread's lane.
+__device__ __forceinline__ void tm_ld(uint32_t addr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "r"(addr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tm_ld(uint32_t addr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tm_wait_ld() {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// Unswizzled K-major operand: 8-row x 16-byte core matrices, `lbo` bytes
+// between neighbours along K and `sbo` along M/N.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)(lbo >> 4) << 16) |
+         ((uint64_t)(sbo >> 4) << 32) | (1ULL << 46);
+}
+
+// ---- digits -> A operand.  Bytes of two neighbouring k become a half2 of
+// 1024 + byte (exponent byte 0x64), minus 1152.
+__device__ __forceinline__ uint32_t sub1152(uint32_t h2) {
+  const __half2 v = *reinterpret_cast<const __half2 *>(&h2);
+  const __half2 r = __hsub2(v, __half2half2(__ushort_as_half(0x6480)));
+  return *reinterpret_cast<const uint32_t *>(&r);
+}
+__device__ __forceinline__ void bytes_to_f16(uint32_t wa, uint32_t wb, uint32_t (&d)[4]) {
+  const uint32_t p = __byte_perm(wa, wb, 0x5140), q = __byte_perm(wa, wb, 0x7362);
+  d[0] = sub1152(__byte_perm(p, 0x64646464u, 0x4140));   // byte 0 of a, b
+  d[1] = sub1152(__byte_perm(p, 0x64646464u, 0x4342));
+  d[2] = sub1152(__byte_perm(q, 0x64646464u, 0x4140));
+  d[3] = sub1152(__byte_perm(q, 0x64646464u, 0x4342));
+}
+// digit pair words of two neighbouring k: out[digit], digit 0 the top one
+__device__ __forceinline__ void digit_words(int64_t a, int64_t b, uint32_t (&o)[7]) {
+  const uint64_t za = biased_digits(a), zb = biased_digits(b);
+  uint32_t lo[4];
+  bytes_to_f16((uint32_t)za, (uint32_t)zb, lo);
+  const uint32_t ha = (uint32_t)(za >> 32), hb = (uint32_t)(zb >> 32);
+  const uint32_t p = __byte_perm(ha, hb, 0x5140);
+  o[0] = sub1152(__byte_perm(ha, hb, 0x7632) | 0x64006400u);
+  o[1] = sub1152(__byte_perm(p, 0x64646464u, 0x4342));
+  o[2] = sub1152(__byte_perm(p, 0x64646464u, 0x4140));
+  o[3] = lo[3];
+  o[4] = lo[2];
+  o[5] = lo[1];
+  o[6] = lo[0];
+}
+__device__ __forceinline__ void digit_words(int a, int b, uint32_t (&o)[4]) {
+  uint32_t d[4];
+  bytes_to_f16(biased_digits(a), biased_digits(b), d);
+  o[0] = d[3];
+  o[1] = d[2];
+  o[2] = d[1];
+  o[3] = d[0];
+}
+
+// ---- accumulators -> result
+// 7 digits: sum_g D_g 256^(6-g) / 256, rounded.  D_g + 1.5*2^23 has the integer
+// D_g in its low bits (|D_g| < 2^22).
+__device__ __forceinline__ int64_t combine(const float (&D)[7]) {
+  constexpr uint32_t C = 0x4B400000u;
+  uint32_t I[7];
+#pragma unroll
+  for (int g = 0; g < 7; ++g) I[g] = __float_as_uint(D[g] + 12582912.f);
+  const uint32_t p01 = I[0] * 256u + I[1] - C * 257u;
+  const int p23 = (int)(I[2] * 256u + I[3] - C * 257u);
+  const int p45 = (int)(I[4] * 256u + I[5] - C * 257u);
+  const int l6 = ((int)(I[6] - C) + 128) >> 8;
+  return (int64_t)((uint64_t)p01 << 32) + (int64_t)p23 * 65536 + (int64_t)(p45 + l6);
+}
+__device__ __forceinline__ float combine(const float (&D)[4]) {
+  return fmaf(fmaf(fmaf(D[0], 256.f, D[1]), 256.f, D[2]), 256.f, D[3]);
+}
+
+// x << lz, then / 256 rounded to nearest: a line's values from below 2^(62-lz)
+// to the digits' 2^54.
+__device__ __forceinline__ int64_t to_digits54(int64_t x, int lz) {
+  return (int64_t)(((uint64_t)x << lz) + 128) >> 8;
+}
+// A filter result to another unit: p * 2^-s, rounded to nearest.
+struct Rescale {
+  int l, r;
+  int64_t half;
+  __device__ __forceinline__ explicit Rescale(int s) {
+    l = s < 0 ? -s & 63 : 0;
+    r = s < 0 ? 0 : (s > 62 ? 62 : s);
+    half = r ? 1LL << (r - 1) : 0;
+  }
+  __device__ __forceinline__ int64_t operator()(int64_t p) const {
+    return (int64_t)(((uint64_t)p << l) + half) >> r;
+  }
+};
+// high word of |x|, as a magnitude key
+__device__ __forceinline__ int hi_key(int64_t x) { return (int)((uint64_t)(x ^ (x >> 63)) >> 32); }
+
+// mbarriers of a CTA
+enum { kFull0 = 0, kFull1 = 1, kEmpty = 2, kDone0 = 3, kDone1 = 4, kTable = 5 };
+
+// One CTA's filter engine.  ND digits, PP points per thread and half.  The
+// last warp only issues the products: with one of the computing threads issuing
+// them, its warp fell behind the others by the issue time of every round (36 %
+// of all stalls at barriers at N = 128).  Computing warps signal digits written
+// (full) and accumulators read (empty) once per warp and wait for products
+// (done); none of it is a CTA-wide barrier.
+template <int ND, int PP> struct Tile {
+  typedef typename std::conditional<ND == 7, int64_t, int>::type I;
+  typedef typename std::conditional<ND == 7, int64_t, float>::type Acc;
+
+  unsigned char *smem;
+  Smem lay;
+  const unsigned char *table;   // global: the digits of Kc, then of Kd
+  int kg, line, u, warp, ncomp;
+  uint32_t tmem;
+  unsigned phases;              // parities of the products' barriers
+  bool ok, both, issuer;
+
+  __device__ __forceinline__ uint32_t bar(int i) const { return sm32(smem + lay.bar_off) + 8 * i; }
+
+  // Before the dependency wait: barriers, keys and the (constant) tables.
+  __device__ __forceinline__ void setup(unsigned char *sm, int n, int kgs, int stage_elem,
+                                        const void *tab) {
+    smem = sm;
+    kg = kgs;
+    lay = smem_layout(ND, n, kgs, stage_elem);
+    table = static_cast<const unsigned char *>(tab) + sizeof(TcHead);
+    ncomp = blockDim.x - issuer_threads(PP);
+    line = threadIdx.x & 127;
+    u = threadIdx.x >> 7;
+    warp = threadIdx.x >> 5;
+    issuer = (int)threadIdx.x >= ncomp;
+    phases = 0;
+    ok = true;
+    both = both_halves(ND, kg);
+    int *keys = reinterpret_cast<int *>(smem + lay.key_off);
+    for (int i = threadIdx.x; i < 2 * kLines; i += blockDim.x) keys[i] = 0;
+    if ((int)threadIdx.x == ncomp) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(i)),
+                     "r"(i <= kEmpty ? ncomp / 32 : 1)
+                     : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      bulk_load(sm32(smem + lay.b_off), table, (b_resident(ND, kg) ? 2 : 1) * lay.b_half,
+                bar(kTable));
+    }
+  }
+  // The issuing warp's part: after the dependency wait (a CTA that holds TMEM
+  // must not wait for another one) TMEM, then `filters` filters.
+  __device__ __forceinline__ void run_issuer(int filters) {
+    if (ND == 7 && PP == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == ncomp / 32) tm_alloc(bar(6), tmem_cols(ND, kg));
+    __syncthreads();
+    read_tmem();
+    if ((int)threadIdx.x == ncomp) {
+      const bool res = b_resident(ND, kg);
+      unsigned tphase = 0;
+      for (int f = 0; f < filters; ++f)
+        for (int half = 0; half < 2; ++half) {
+          wait_for(kFull0 + half, f & 1);
+          if (!res || (f | half) == 0) wait_for(kTable, tphase++ & 1);
+          fence_after();
+          if (split_rows(ND, kg)) {
+            issue(half, 0);
+            if (half == 1) {
+              wait_for(kEmpty, f & 1);   // c's second round is read
+              fence_after();
+            }
+            issue(half, 1);
+          } else {
+            issue(half, half);
+          }
+          if (!res && (half == 0 || f + 1 < filters)) {
+            // the other half's table, once this half's products are done
+            wait_for(kDone1, half);
+            if (ok) bulk_load(sm32(smem + lay.b_off), table + (half ^ 1) * lay.b_half, lay.b_half, bar(kTable));
+          }
+        }
+    }
+    __syncwarp();
+  }
+  // The computing threads' other side of it.
+  __device__ __forceinline__ void run_compute() {
+    if (ND == 7 && PP == 16) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
+  }
+  // Every computing thread, once its loads are issued.
+  __device__ __forceinline__ void start() {
+    __syncthreads();
+    read_tmem();
+  }
+  __device__ __forceinline__ void read_tmem() {
+    fence_after();
+    tmem = *reinterpret_cast<volatile uint32_t *>(smem + lay.bar_off + 48);
+  }
+  __device__ __forceinline__ void finish(unsigned *err) {
+    if (!ok && err) atomicOr(err, 2u);
+    __syncthreads();
+    if (warp == ncomp / 32) tm_free(tmem, tmem_cols(ND, kg));
+  }
+  // barrier of the computing warps
+  __device__ __forceinline__ void sync() const {
+    asm volatile("bar.sync 1, %0;" ::"r"(ncomp) : "memory");
+  }
+  __device__ __forceinline__ void wait_for(int b, unsigned parity) {
+    if (ok && !bar_wait(bar(b), parity)) ok = false;
+  }
+  __device__ __forceinline__ void signal(int b) {
+    fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(b)) : "memory");
+  }
+  // Accumulator buffer `buf` holds its products.
+  __device__ __forceinline__ void wait_done(int buf) {
+    wait_for(kDone0 + buf, phases >> buf & 1);
+    phases ^= 1u << buf;
+    fence_after();
+    __syncwarp();
+  }
+
+  // digits of this thread's PP values (k = PP*u + i) into A operand `half`
+  __device__ __forceinline__ void put_digits(const I (&v)[PP], int half) {
+    const int kb = 2 * kg;
+    unsigned char *base = smem + (both ? half * lay.a_half : 0) + line * 16;
+#pragma unroll
+    for (int h = 0; h < PP / 8; ++h) {
+      uint32_t w[4][ND];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) digit_words(v[8 * h + 2 * i], v[8 * h + 2 * i + 1], w[i]);
+      const int bk = PP / 8 * u + h;
+      unsigned char *dst = base + (dense_b(kg) ? bk : kb - 1 - bk) * (kLines * 16);
+#pragma unroll
+      for (int d = 0; d < ND; ++d)
+        *reinterpret_cast<uint4 *>(dst + d * lay.a_digit) =
+            make_uint4(w[0][d], w[1][d], w[2][d], w[3][d]);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    signal(kFull0 + half);
+  }
+
+  // The digit products of half `half` (0: c, 1: d) into accumulator buffer
+  // `buf` (also the round, where rows are split).
+  __device__ __forceinline__ void issue(int half, int buf) {
+    if (!ok) return;
+    const uint32_t kp = 16 * kg, gc = group_cols(ND, kg);
+    const uint32_t d0 = tmem + (dense_b(kg) ? buf * ND * gc : 0);
+    const uint32_t id0 = (1u << 4) | ((kLines >> 4) << 24);
+    const uint64_t a0 = smem_desc(sm32(smem) + (both ? half * lay.a_half : 0), kLines * 16, 128);
+    const uint32_t bh = sm32(smem + lay.b_off) + (b_resident(ND, kg) ? half * lay.b_half : 0);
+    if (dense_b(kg)) {
+      const bool split = split_rows(ND, kg);
+      const uint32_t blbo = ND * gc * 16 * (split ? 2 : 1);
+      const uint64_t b0 = smem_desc(bh + (split ? buf * ND * gc * 16 : 0), blbo, 128);
+#pragma unroll 1
+      for (int s = 0; s < kg; ++s) {
+        const uint64_t as = a0 + s * (2 * kLines * 16 >> 4), bs = b0 + s * (2 * blbo >> 4);
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          const uint32_t rows = (ND - i) * gc, n0 = rows < 256 ? rows : 256;
+          const uint64_t ai = as + (uint32_t)(i * lay.a_digit >> 4);
+          mma_f16(d0 + i * gc, ai, bs, id0 | ((n0 >> 3) << 17), (s | i) != 0);
+          if (rows > 256)
+            mma_f16(d0 + i * gc + 256, ai, bs + 256, id0 | ((rows - 256) >> 3 << 17), (s | i) != 0);
+        }
+      }
+    } else {
+      const int bd = (4 * kg - 1) * 128;
+      const uint64_t b0 = smem_desc(bh, 128, 128);
+#pragma unroll 1
+      for (int s = 0; s < kg; ++s) {
+        const uint64_t as = a0 + s * (2 * kLines * 16 >> 4), bs = b0 + s * (256 >> 4);
+#pragma unroll
+        for (int i = 0; i < ND; ++i)
+#pragma unroll
+          for (int j = 0; j < ND - i; ++j)
+            mma_f16(d0 + (i + j) * kp, as + (uint32_t)(i * lay.a_digit >> 4),
+                    bs + (uint32_t)(j * bd >> 4), id0 | ((kp >> 3) << 17), (s | i) != 0);
+      }
+    }
+    mma_commit(bar(kDone0 + buf));
+  }
+
+  // eight outputs of this thread from accumulator buffer `buf`, starting at
+  // column `col` of each group (with 16 points per thread four at a time: 28
+  // accumulators in registers instead of 56, which spilled)
+  __device__ __forceinline__ void get8(int buf, int col, Acc (&y)[8]) {
+    constexpr int L = PP == 16 && ND == 7 ? 4 : 8;
+    const uint32_t gc = group_cols(ND, kg);
+    const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + (dense_b(kg) ? buf * ND * gc : 0) + col;
+#pragma unroll
+    for (int h = 0; h < 8; h += L) {
+      float D[ND][L];
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < ND; ++g) tm_ld(addr + g * gc + h, D[g]);
+      tm_wait_ld();
+#pragma unroll
+      for (int i = 0; i < L; ++i) {
+        float d[ND];
+#pragma unroll
+        for (int g = 0; g < ND; ++g) d[g] = D[g][i];
+        y[h + i] = combine(d);
+      }
+    }
+  }
+
+  // a = x[k], b = x[k+H] -> a = 2 y[k], b = 2 y[k+H] in the accumulators' units
+  // (7 digits).
+  // waiting() runs while the products do.
+  template <typename G> __device__ __forceinline__ void filter(I (&a)[PP], I (&b)[PP], G &&waiting) {
+    filter(a, b, waiting, [&](int i, I p, I q) {
+      a[i] = p;
+      b[i] = q;
+    });
+  }
+  // ... -> out(i, 2 y[k], 2 y[k+H]).
+  template <typename G, typename F>
+  __device__ __forceinline__ void filter(I (&a)[PP], I (&b)[PP], G &&waiting, F &&out) {
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      const I s = a[i] + b[i];
+      b[i] = a[i] - b[i];
+      a[i] = s;
+    }
+    Acc c[PP], y[8];
+    put_digits(a, 0);
+    if constexpr (ND == 7 && PP == 16) {
+      // rounds c0 c1 d0 d1 (points 0-7, 8-15) in buffers 0 1 0 1: while one
+      // buffer is read the other one's products run
+      wait_done(0);
+      get8(0, 8 * u, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i] = y[i];
+      wait_done(1);          // c's products have read A
+      put_digits(b, 1);
+      get8(1, 8 * u, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[8 + i] = y[i];
+      signal(kEmpty);
+      wait_done(0);
+      get8(0, 8 * u, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out(i, c[i] + y[i], c[i] - y[i]);
+      wait_done(1);
+      get8(1, 8 * u, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out(8 + i, c[8 + i] + y[i], c[8 + i] - y[i]);
+    } else {
+      if (both) put_digits(b, 1);
+      waiting();
+      wait_done(0);
+#pragma unroll
+      for (int h = 0; h < PP / 8; ++h) {
+        get8(0, PP * u + 8 * h, y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c[8 * h + i] = y[i];
+      }
+      if (!both) put_digits(b, 1);
+      wait_done(1);
+#pragma unroll
+      for (int h = 0; h < PP / 8; ++h) {
+        get8(1, PP * u + 8 * h, y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out(8 * h + i, c[8 * h + i] + y[i], c[8 * h + i] - y[i]);
+      }
+    }
+    fence_before();
+    __syncwarp();
+  }
+
+  // The largest of the line's keys over its threads (slot 0 or 1); a barrier of
+  // the computing warps.
+  __device__ __forceinline__ int line_key(int slot, int key) {
+    int *k = reinterpret_cast<int *>(smem + lay.key_off) + slot * kLines + line;
+    atomicMax(k, key);
+    sync();
+    return *k;
+  }
+  // Whether any computing thread says so; a barrier of the computing warps.
+  __device__ __forceinline__ bool any(bool v) {
+    int r;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.s32 p, %2, 0;\n barrier.cta.red.or.pred q, 1, %1, p;\n"
+        " selp.s32 %0, 1, 0, q;\n}\n"
+        : "=r"(r)
+        : "r"(ncomp), "r"(v ? 1 : 0)
+        : "memory");
+    return r != 0;
+  }
+};
+#endif  // __CUDACC__
+
+}  // namespace tc
+}  // namespace scft
