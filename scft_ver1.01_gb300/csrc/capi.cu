@@ -367,16 +367,28 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
     ps.pre[0] = W;
     if ((rc = launch_set<R>(ctx, ctx->passes[0], ps, st))) return rc;
     if ((rc = middle())) return rc;
+    // FP32 planes: an x pair takes the middle passes before and after it along
+    const bool planes = std::is_same<R, float>::value && np == 3 && ctx->tc_planes &&
+                        ctx->passes[0].tc && ctx->passes[1].tc;
     for (int it = 2; it <= sg.ns; ++it) {
       // finish step it-1 (last pass when it was odd, x when even), start step it
+      const bool x = ((it - 1) & 1) == 0;
       reset(tmp[cur], M, tmp[cur ^ 1], M);
       cur ^= 1;
       ps.qout[0] = slice(it - 1);
       ps.qout_bs[0] = qbs;
       ps.post[0] = W;
-      if ((rc = launch_pair<R>(ctx, ctx->passes[(it - 1) & 1 ? np - 1 : 0], ps, st))) return rc;
-      if ((rc = middle())) return rc;
+      if constexpr (std::is_same<R, float>::value) {
+        if (planes && x) {
+          ps.err = ctx->dev_err;
+          CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], ps, st));
+          continue;
+        }
+      }
+      if ((rc = launch_pair<R>(ctx, ctx->passes[x ? 0 : np - 1], ps, st))) return rc;
+      if (!planes && (rc = middle())) return rc;
     }
+    if (planes && !(sg.ns & 1) && (rc = middle())) return rc;
     reset(tmp[cur], M, slice(sg.ns), qbs);
     ps.post[0] = W;
     if ((rc = launch_set<R>(ctx, ctx->passes[(sg.ns & 1) ? np - 1 : 0], ps, st))) return rc;
@@ -390,6 +402,7 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
 int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, int cidx) {
   const long long M = ctx->M;
   const int B = ctx->batch, np = (int)ctx->passes.size();
+  const bool planes = ctx->tc_planes;
   int64_t *tmp[2] = {static_cast<int64_t *>(ctx->tmp[2 * cidx]),
                      static_cast<int64_t *>(ctx->tmp[2 * cidx + 1])};
   for (int k = 0; k < nseg; ++k) {
@@ -401,8 +414,6 @@ int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, i
     const long long qbs = (long long)(ctx->q_ns[sg.qi] + 1) * M;
     auto slice = [&](int it) { return q + (long long)(sg.sign > 0 ? it : sg.ns - it) * M; };
     int *exq = ctx->ex[cidx], *ex = exq + B;   // |q_0| and |v_j| bounds, [..][B]
-    CK(cudaMemsetAsync(exq, 0x80, sizeof(int) * (size_t)(sg.ns + 1) * B, st));
-    CKL(scft::launch_slice_exp(slice(0), qbs, M, B, exq, st));
     scft::FixPass fp;
     int cur = 0, j = 0;   // tmp[cur] holds v_j, or v_j filtered
     auto pass = [&](int pi, int mode, const void *in, long long in_bs) {
@@ -432,17 +443,38 @@ int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, i
         if (mode != scft::kFixFirst) cur ^= 1;
         if (mode != scft::kFixMid) fp.ex = ex + (long long)j * B;
       }
-      CKL(scft::launch_fix(ctx->passes[pi], mode, fp, st));
+      // an x pair on planes takes the middle passes before and after it along
+      if (mode == scft::kFixPair && pi == 0 && planes)
+        CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], fp, 0, 0, st));
+      else
+        CKL(scft::launch_fix(ctx->passes[pi], mode, fp, st));
       return (int)SCFT_OK;
     };
     auto middle = [&]() { return np < 3 ? (int)SCFT_OK : pass(1, scft::kFixMid, tmp[cur], M); };
+    if (planes && np == 2) {   // a film: the segment is one launch
+      memset(&fp, 0, sizeof fp);
+      fp.batch = B;
+      fp.eref = ctx->eref[sg.wf];
+      fp.kbits = ctx->kbits;
+      fp.w = ctx->wfix[sg.wf];
+      fp.w_bs = M;
+      fp.err = ctx->dev_err;
+      fp.in = slice(0);
+      fp.in_bs = fp.q_bs = qbs;
+      fp.q = slice(1);
+      CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], fp, sg.ns, sg.sign * M, st));
+      continue;
+    }
+    CK(cudaMemsetAsync(exq, 0x80, sizeof(int) * (size_t)(sg.ns + 1) * B, st));
+    CKL(scft::launch_slice_exp(slice(0), qbs, M, B, exq, st));
     if ((rc = pass(0, scft::kFixFirst, slice(0), qbs))) return rc;
     if ((rc = middle())) return rc;
     for (int it = 2; it <= sg.ns; ++it) {
       // finish step it-1 (last pass when it was odd, x when even), start step it
       if ((rc = pass((it - 1) & 1 ? np - 1 : 0, scft::kFixPair, tmp[cur], M))) return rc;
-      if ((rc = middle())) return rc;
+      if (!planes && (rc = middle())) return rc;
     }
+    if (planes && !(sg.ns & 1) && (rc = middle())) return rc;
     if ((rc = pass((sg.ns & 1) ? np - 1 : 0, scft::kFixLast, tmp[cur], M))) return rc;
   }
   return SCFT_OK;
@@ -1277,9 +1309,9 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
     return fail(SCFT_ERR_CUDA, "table upload failed");
   // Passes on the tensor cores: every FP64 line they take, and FP32 lines without
   // a register kernel.  Measured, ms per SCF iteration with 200 contour steps:
-  // FP64 64^3 22 -> 5.5, 128^3 107 -> 22; FP32 100x80x60 24 -> 5.2.  FP32 and
+  // FP64 64^3 22 -> 3.5, 128^3 107 -> 21; FP32 100x80x60 24 -> 4.8.  FP32 and
   // double-float lines with a register kernel keep it (64^3: FP32 1.2; double-float
-  // 4.0 against 5.6).
+  // 4.0 against 5.5 on passes of the first form).
   size_t tc_bytes = 0;
   for (size_t pi = 0; pi < ctx->passes.size(); ++pi) {
     const AxisPlan &ap = ctx->passes[pi];
@@ -1289,6 +1321,12 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
       ctx->tc_off[2 * pi + k] = tc_bytes;
       tc_bytes += (scft::tc_table_bytes(ap.n, tc_digits(ctx)) + 255) & ~(size_t)255;
     }
+  }
+  if (ctx->passes.size() >= 2 && ctx->tc_want[0] && ctx->tc_want[1] && ctx->pass_axis[0] == 0 &&
+      (p.flags & (SCFT_FLAG_NO_XY | SCFT_FLAG_NO_FUSED_STEPS)) == 0) {
+    const AxisPlan &ay = ctx->passes[1];
+    ctx->tc_planes = ay.s_n == p.nx && (ctx->passes.size() == 3 || rb == 8) &&
+                     scft::tc_planes_wanted(p.nx, ay.n, p.ny * p.nz / ay.n, tc_digits(ctx), p.batch);
   }
   if (tc_bytes && scft::tc_prepare() != cudaSuccess)
     return fail(SCFT_ERR_CUDA, "kernel attribute set-up failed");

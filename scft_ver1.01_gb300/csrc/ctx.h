@@ -74,6 +74,7 @@ struct scft_ctx {
   void *tc_mem = nullptr;
   size_t tc_off[6] = {0, 0, 0, 0, 0, 0};
   bool tc_want[3] = {false, false, false};
+  bool tc_planes = false;       // fused steps run the x and y passes on whole planes
   const void *dtc_pass[3] = {nullptr, nullptr, nullptr};
   // the fused 64-bit march (run_chain_fixed): factors as integers and their
   // largest exponent per instance, exponent bounds per step [2 chains], and

@@ -20,6 +20,7 @@
 // differ in chiN, f, box and Ns, so their step counts differ and the sets
 // drop out as their chains end.  A bucket of n members makes ~2-3 launches
 // per step instead of n x ~2.
+#include <algorithm>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -46,7 +47,7 @@ struct BucketChain {
 };
 struct GroupBucket {
   std::vector<int> mem;             // member indices (same grid)
-  bool xy = false;                  // first pass: the x+y plane kernel
+  bool xy = false;                  // first pass: x and y of whole planes
   int npass = 0;                    // launches per step
   int T = 0;                        // steps of the longest chain
   BucketChain ch[2];
@@ -116,7 +117,13 @@ void release(scft_group *g) {
 // march from 2^16 points up: measured with 21 members per grid, the batched
 // (unfused) march wins at 32^3 (81.6 against 64.5 Gpt*step/s) and loses at
 // 48^3 (142.3 against 169.4) and 64^3 (172.1 against 196.0).
+// Members on the tensor cores keep theirs while the CTAs of all of them, both
+// chains, come to two waves at most: their launches then run side by side, two
+// a step fewer each (ms per iteration, own against batched march: two of 40^3
+// 2.35 / 2.91, three 3.04 / 3.13, five 4.75 / 3.96, 21 of them 20.0 / 13.8; eight of 20^3
+// 1.68 / 2.19, 21 3.38 / 3.38; three of 80 x 10 x 20 3.87 / 4.13, five 4.90 / 4.27).
 constexpr long long kBatchFusedBelow = 1LL << 16;
+constexpr long long kOwnCtas = 2 * 152;
 int make_buckets(scft_group *g) {
   std::map<std::tuple<int, int, int, int>, std::vector<int>> by_grid;
   for (size_t i = 0; i < g->members.size(); ++i) {
@@ -133,8 +140,15 @@ int make_buckets(scft_group *g) {
     GroupBucket b;
     b.mem = kv.second;
     const scft_ctx *c0 = g->members[b.mem[0]];
-    b.xy = c0->passes.size() >= 2 && c0->pass_axis[0] == 0 && c0->pass_axis[1] == 1 &&
-           scft::xy_fusable(c0->passes[0], c0->passes[1]);
+    long long ctas = 0;
+    for (const scft::AxisPlan &ap : c0->passes) ctas = std::max(ctas, scft::tc_pass_ctas(ap, 4));
+    bool fused = true;
+    for (int m : b.mem) fused = fused && g->members[m]->fuse_steps;
+    if (fused && ctas > 0 && 2 * ctas * (long long)b.mem.size() <= kOwnCtas) continue;
+    if (c0->passes.size() >= 2 && c0->pass_axis[0] == 0 && c0->pass_axis[1] == 1)
+      b.xy = c0->passes[0].tc && c0->passes[1].tc
+                 ? scft::tc_planes_wanted(c0->p.nx, c0->p.ny, c0->p.nz, 4, (int)b.mem.size())
+                 : scft::xy_fusable(c0->passes[0], c0->passes[1]);
     b.npass = (int)c0->passes.size() - (b.xy ? 1 : 0);
     for (int m : b.mem) {
       const scft_ctx *c = g->members[m];
@@ -170,6 +184,7 @@ int make_buckets(scft_group *g) {
             const int ai = bb.xy ? (pi == 0 ? 0 : pi + 1) : pi;   // the member's axis pass
             d.gain = static_cast<const float *>(c->passes[ai].gain);
             d.tc = c->passes[ai].tc;
+            d.tc_y = bb.xy && pi == 0 ? c->passes[1].tc : nullptr;
             d.gain_y = bb.xy && pi == 0 ? static_cast<const float *>(c->passes[1].gain) : nullptr;
             step[pi].push_back(d);
           }
@@ -223,11 +238,12 @@ int bucket_march(scft_group *g, GroupBucket &b, int ch, long long *launches) {
       cudaError_t e;
       const int ai = b.xy ? (pi == 0 ? 0 : pi + 1) : pi;
       const scft::AxisPlan &ap = c0->passes[ai];
-      if (b.xy && pi == 0) e = scft::launch_xy(c0->passes[0], c0->passes[1], ps, bc.st);
-      else if (ap.tc) {
-        ps.err = c0->dev_err;
-        e = scft::launch_tc(ap, ps, false, bc.st);
-      } else if (ap.use_fast) e = scft::launch_fast_line(ap, ps, bc.st);
+      if (ap.tc) ps.err = c0->dev_err;
+      if (b.xy && pi == 0)
+        e = ap.tc ? scft::launch_planes(ap, c0->passes[1], ps, bc.st)
+                  : scft::launch_xy(ap, c0->passes[1], ps, bc.st);
+      else if (ap.tc) e = scft::launch_tc(ap, ps, false, bc.st);
+      else if (ap.use_fast) e = scft::launch_fast_line(ap, ps, bc.st);
       else e = scft::launch_line_filter_desc(ap, d, n, bc.st);
       if (e != cudaSuccess)
         return gfail(g, SCFT_ERR_CUDA, std::string("batched pass: ") + cudaGetErrorString(e));
@@ -238,8 +254,8 @@ int bucket_march(scft_group *g, GroupBucket &b, int ch, long long *launches) {
 }
 
 int build_graph(scft_group *g) {
-  long long l0 = 0;
-  for (scft_ctx *c : g->members) l0 += c->launches;
+  std::vector<long long> before;   // the members' counters: captured launches did not run
+  for (scft_ctx *c : g->members) before.push_back(c->launches);
   GCK(cudaStreamBeginCapture(g->st, cudaStreamCaptureModeThreadLocal));
   int rc = SCFT_OK;
   long long bl = 0;
@@ -304,10 +320,12 @@ int build_graph(scft_group *g) {
     return gfail(g, SCFT_ERR_CUDA, std::string("group instantiate: ") + cudaGetErrorString(e));
   }
   g->epoch = plan_epochs(g);
-  long long l1 = 0;
-  for (scft_ctx *c : g->members) l1 += c->launches;
   g->bucket_launches = bl;
-  g->nodes = l1 - l0 + bl;   // kernel nodes per replay (counted while capturing)
+  g->nodes = bl;   // kernel nodes per replay
+  for (size_t i = 0; i < g->members.size(); ++i) {
+    g->nodes += g->members[i]->launches - before[i];
+    g->members[i]->launches = before[i];
+  }
   return SCFT_OK;
 }
 

@@ -1,8 +1,8 @@
 // Tensor-core passes of the propagator march (core and arithmetic: tc_core.cuh).
 //
 // k_real: one axis pass on working reals, out = post * K (pre * in), and for
-// FP32 the fused step pair.  k_fix: the fused march of FP64 and double-float
-// contexts, whose intermediates between passes stay 64-bit integers of one unit
+// FP32 the fused step pair.  k_fix: the fused march of FP64 contexts,
+// whose intermediates between passes stay 64-bit integers of one unit
 // per instance and step, so that a pass costs no conversion to or from the
 // working real (those were about half of a pass's 142 instructions per point):
 //   first  v0 = W q0 and the first filter        real in, fixed out
@@ -45,7 +45,8 @@ template <typename T, typename A> __device__ __forceinline__ T finish_real(A y, 
 
 // Geometry of a pass's lines.
 struct Lines {
-  int n, half, kg;
+  Shape sh;
+  int n;
   long long lines;       // per instance
   long long row_len;     // column passes: consecutive lines of one row
   long long s_outer, s_n;
@@ -104,12 +105,12 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
   if constexpr (std::is_same<T, float>::value) {
     if (ps.desc) table = ps.desc[blockIdx.z].tc;
   }
-  e.setup(smem_raw, ln.n, ln.kg, XP ? (int)sizeof(T) : 0, table);
+  e.setup(smem_raw, ln.sh, table, table);
   const TcHead head = *static_cast<const TcHead *>(table);
   const int set = (int)blockIdx.z >= ps.batch ? 1 : 0;
   const long long b = (long long)blockIdx.z - (long long)set * ps.batch;
-  const long long line0 = (long long)blockIdx.x * kLines;
-  const int nl = (int)min((long long)kLines, ln.lines - line0);
+  const long long line0 = (long long)blockIdx.x * e.ln;
+  const int nl = (int)min((long long)e.ln, ln.lines - line0);
   const T *in = ps.in[set] + b * ps.in_bs[set];
   T *out = ps.out[set] + b * ps.out_bs[set];
   const T *pre = ps.pre[set] ? ps.pre[set] + b * ps.w_bs : nullptr;
@@ -124,11 +125,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
       post = d.post;
     }
   }
-  const int H = ln.half;
+  const int H = ln.sh.half[0];
   pdl_wait();      // the input is the previous pass's output
   pdl_release();
   if (e.issuer) {
-    e.run_issuer(PAIR ? 2 : 1);
+    e.run_issuer(PAIR ? 2 : 1, [](int) { return 0; });
     e.finish(ps.err);
     return;
   }
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
   }
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
-    const int k = PP * e.u + i;
+    const int k = PP * e.blk + i;
     a[i] = bb[i] = T(0.0f);
     if (mine && k < H) {
       if constexpr (XP) {
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     if (pre) {
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
-        const int k = PP * e.u + i;
+        const int k = PP * e.blk + i;
         if (mine && k < H) {
           a[i] = a[i] * ldg(pre + base + (long long)k * ln.s_n);
           bb[i] = bb[i] * ldg(pre + base + (long long)(k + H) * ln.s_n);
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
       e.sync();
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
-        const int k = PP * e.u + i;
+        const int k = PP * e.blk + i;
         if (mine && k < H) {
           stg[e.line * P + k] = ya[i];
           stg[e.line * P + k + H] = yb[i];
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
       e.sync();
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
-        const int k = PP * e.u + i;
+        const int k = PP * e.blk + i;
         const bool on = mine && k < H;
         ya[i] = on ? stg[e.line * P + k] : T(0.0f);
         yb[i] = on ? stg[e.line * P + k + H] : T(0.0f);
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     } else {
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
-        const int k = PP * e.u + i;
+        const int k = PP * e.blk + i;
         if (mine && k < H) {
           const long long o0 = base + (long long)k * ln.s_n, o1 = o0 + (long long)H * ln.s_n;
           const T w0 = ldg(post + o0), w1 = ldg(post + o1);
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     e.sync();
 #pragma unroll
     for (int i = 0; i < PP; ++i) {
-      const int k = PP * e.u + i;
+      const int k = PP * e.blk + i;
       if (mine && k < H) {
         stg[e.line * P + k] = ya[i];
         stg[e.line * P + k + H] = yb[i];
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     });
   } else {
     e.filter(xa, xb, []() {}, [&](int i, Acc p, Acc q) {
-      const int k = PP * e.u + i;
+      const int k = PP * e.blk + i;
       if (mine && k < H) {
         const long long o0 = base + (long long)k * ln.s_n, o1 = o0 + (long long)H * ln.s_n;
         T r0 = bad ? bad_value(T(0.0f)) : finish_real<T>(p, ue);
@@ -302,22 +303,144 @@ enum { FIRST = 0, MID = 1, PAIR = 2, LAST = 3 };
 
 constexpr int kBadExp = 0x7fffffff;         // ex: the values are not finite
 
-// Points per line of the staging memory: x passes stage rows, column passes
-// with 16 points per thread the factor step (32 per thread).
-__host__ __device__ inline int stage_points(const Lines &ln, bool xp, int mode) {
-  if (xp) return ln.n;
-  return ln.kg > 2 && (mode == PAIR || mode == LAST) ? 32 * ln.kg - 1 : 0;
-}
 __device__ __forceinline__ bool unit_bad(int s) { return s >= 0x40000000; }
-
 __device__ __forceinline__ int64_t ld64(const int64_t *p) {
   return __ldg(reinterpret_cast<const long long *>(p));
 }
-// r = W y as the stored slice's value
+// r = W y as the stored slice's value, |r| in the range of from_fixed_fast or not
 __device__ __forceinline__ double slice_value(int64_t r, int ur) {
   const int h = (int)(r >> 32);
   if (h != (h >> 31) && fast_units(ur)) return from_fixed_fast(r, ur);
   return from_fixed(r, ur, 0.0);
+}
+// A thread's points of a column line: PP at off, off + sn, ..., and as many
+// another hs on; the first `lim` exist.
+struct Column {
+  unsigned off, sn, hs;
+  int lim;
+};
+// q = W y to the finished slice and x = W q for N/2 points (x[2j]: y of point
+// g + j of the column, x[2j + 1]: of its partner).  Without a branch in it, so
+// that the N chains (about 190 cycles each) run side by side; a value too small
+// for the fast conversion is stored again afterwards.  Returns the factors'
+// signs: a negative one is not finite.
+template <int N>
+__device__ __forceinline__ int factor_group(int64_t (&x)[N], const int64_t *wf, double *qo,
+                                            const Column &c, int g, int ur) {
+  auto at = [&](int i) { return c.off + (g + i / 2) * c.sn + (i & 1) * c.hs; };
+  int wneg = 0;
+  int64_t r[N], w[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) w[i] = g + i / 2 < c.lim ? ld64(wf + at(i)) : 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    wneg |= (int)(w[i] >> 32);
+    r[i] = mul_w62(x[i], w[i]);
+  }
+  bool slow = !fast_units(ur);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int h = (int)(r[i] >> 32);
+    const bool on = g + i / 2 < c.lim;
+    slow |= on && h == (h >> 31);
+    const double q = from_fixed_fast(r[i], ur);
+    if (on) qo[at(i)] = q;
+    x[i] = mul_w62(r[i], w[i]);
+  }
+  if (slow) {
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) {
+      int64_t ri = r[0];
+#pragma unroll
+      for (int j = 1; j < N; ++j) ri = i == j ? r[j] : ri;
+      if (g + i / 2 < c.lim) qo[at(i)] = slice_value(ri, ur);
+    }
+  }
+  return wneg;
+}
+// The same for all of a thread's points.
+template <int PP>
+__device__ __forceinline__ int factor_points(int64_t (&xa)[PP], int64_t (&xb)[PP],
+                                             const int64_t *wf, double *qo, const Column &c,
+                                             int ur) {
+  int wneg = 0;
+#pragma unroll
+  for (int g = 0; g < PP; g += 4) {
+    int64_t x[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[2 * i] = xa[g + i];
+      x[2 * i + 1] = xb[g + i];
+    }
+    wneg |= factor_group(x, wf, qo, c, g, ur);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      xa[g + i] = x[2 * i];
+      xb[g + i] = x[2 * i + 1];
+    }
+  }
+  return wneg;
+}
+// A thread's points (16 and their partners) in the staging memory, where they
+// cost no registers: as unrolled code over registers the factor step of 16
+// points spilled 560-800 bytes a thread.
+struct Staged {
+  int64_t *own;
+  int stride;
+  __device__ __forceinline__ int64_t &a(int i) const { return own[2 * i * stride]; }
+  __device__ __forceinline__ int64_t &b(int i) const { return own[(2 * i + 1) * stride]; }
+  __device__ __forceinline__ int factor(const int64_t *wf, double *qo, const Column &c,
+                                        int ur) const {
+    int wneg = 0;
+#pragma unroll 1
+    for (int g = 0; g < 16; g += 4) {
+      int64_t x[8];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[2 * i] = a(g + i);
+        x[2 * i + 1] = b(g + i);
+      }
+      wneg |= factor_group(x, wf, qo, c, g, ur);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a(g + i) = x[2 * i];
+        b(g + i) = x[2 * i + 1];
+      }
+    }
+    return wneg;
+  }
+};
+// NaN where the input or the factor is not finite (rare)
+__device__ __forceinline__ void spoil_points(bool bad, const int64_t *wf, double *qo,
+                                             const Column &c, int pp) {
+  for (int i = 0; i < c.lim && i < pp; ++i) {
+    const unsigned o = c.off + i * c.sn;
+    if (bad || wf[o] < 0) qo[o] = bad_value(0.0);
+    if (bad || wf[o + c.hs] < 0) qo[o + c.hs] = bad_value(0.0);
+  }
+}
+// the largest magnitude key of a thread's points
+template <int PP>
+__device__ __forceinline__ int points_key(const int64_t (&xa)[PP], const int64_t (&xb)[PP]) {
+  int key = 0;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
+  return key;
+}
+// a line's values, largest key `clz`, to the digits' 2^54; the unit's change
+template <int PP> __device__ __forceinline__ int to_line_scale(int64_t (&xa)[PP], int64_t (&xb)[PP],
+                                             int clz) {
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    xa[i] = to_digits54(xa[i], clz - 2);
+    xb[i] = to_digits54(xb[i], clz - 2);
+  }
+  return 10 - clz;
+}
+// reports the exponent bound of the CTA's lines (x per line, INT_MIN: none)
+__device__ __forceinline__ void report_exp(int *ex, int x) {
+  x = __reduce_max_sync(0xffffffffu, x);
+  if ((threadIdx.x & 31) == 0 && x != INT_MIN) atomicMax(ex, x);
 }
 
 template <int PP, bool XP, int MODE>
@@ -325,17 +448,17 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
   typedef Tile<7, PP> E;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   E e;
-  e.setup(smem_raw, stage_points(ln, XP, MODE), ln.kg, 8, table);
+  e.setup(smem_raw, ln.sh, table, table);
   const TcHead head = *static_cast<const TcHead *>(table);
   const long long b = blockIdx.z;
-  const unsigned line0 = blockIdx.x * kLines;
-  const int nl = (int)min((long long)kLines, ln.lines - line0);
-  const unsigned H = ln.half;
+  const unsigned line0 = blockIdx.x * e.ln;
+  const int nl = (int)min((long long)e.ln, ln.lines - line0);
+  const unsigned H = ln.sh.half[0];
   const int kbits = *fp.kbits;
   pdl_wait();      // the input is the previous pass's output
   pdl_release();
   if (e.issuer) {
-    e.run_issuer(MODE == PAIR ? 2 : 1);
+    e.run_issuer(MODE == PAIR ? 2 : 1, [](int) { return 0; });
     e.finish(fp.err);
     return;
   }
@@ -345,9 +468,10 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
   const unsigned c = line0 + e.line, rl = (unsigned)ln.row_len;
   const unsigned base = XP ? c * ln.n : (c / rl) * (unsigned)ln.s_outer + c % rl;
   const unsigned sn = XP ? 1 : (unsigned)ln.s_n;
-  const unsigned k0 = PP * e.u, tile = line0 * ln.n;
+  const unsigned k0 = PP * e.blk, tile = line0 * ln.n;
   const unsigned off = base + k0 * sn, hs = H * sn;
   const int lim = e.line < nl ? (int)H - (int)k0 : 0;   // this thread's points: i < lim
+  const Column col{off, sn, hs, lim};
   const int P = ln.n + 1;
   int64_t *stg = reinterpret_cast<int64_t *>(smem_raw);
   int64_t *row = stg + e.line * P + k0;                 // its points in the staging tile
@@ -390,10 +514,9 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
     const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs;
     if constexpr (XP) {
       over_rows(e.ncomp, ln.n, nl, in + tile,
-                [&](int r, int col, int, int64_t x) { stg[r * P + col] = x; });
+                [&](int r, int cc, int, int64_t x) { stg[r * P + cc] = x; });
       e.sync();
     }
-    int key = 0;
 #pragma unroll
     for (int i = 0; i < PP; ++i) {
       xa[i] = xb[i] = 0;
@@ -401,53 +524,53 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
         xa[i] = XP ? row[i] : ld64(in + (off + i * sn));
         xb[i] = XP ? row[i + H] : ld64(in + (off + i * sn + hs));
       }
-      key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
     }
+    int key = points_key(xa, xb);
     e.start();   // TMEM address, cleared keys; the staging tile is read
     key = e.line_key(0, key);
-    const int lz = clz32((uint32_t)key | 1u) - 2;
-#pragma unroll
-    for (int i = 0; i < PP; ++i) {
-      xa[i] = to_digits54(xa[i], lz);
-      xb[i] = to_digits54(xb[i], lz);
-    }
-    ue = u_in + 8 - lz;
+    ue = u_in + to_line_scale(xa, xb, clz32((uint32_t)key | 1u));
   }
 
   // The filters and what follows each.  One copy of the code serves both
   // filters of a pair: with two a pair was 7450 instructions long (119 KB at
   // N = 128) and waited for them.
   int64_t *out = static_cast<int64_t *>(fp.out) + b * fp.out_bs;
+  constexpr bool kStaged = PP == 16 && !XP && (MODE == PAIR || MODE == LAST);
+  const Staged sp{stg + threadIdx.x, e.ncomp};
 #pragma unroll 1
   for (int f = 0; f < (MODE == PAIR ? 2 : 1); ++f) {
     if (MODE == FIRST || (MODE == PAIR && f == 1)) {
       // the formed v: report its exponent, rescale the lines
-      int key = 0;
-#pragma unroll
-      for (int i = 0; i < PP; ++i) key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
-      key = e.line_key(1, key);   // (its barrier: the staging tile is read)
+      const int key = e.line_key(1, points_key(xa, xb));   // (its barrier: the staging tile is read)
       const int clz = clz32((uint32_t)key | 1u);
-      if (e.u == 0) {
-        int x = bad ? kBadExp : (e.line < nl ? ue + 64 - clz : INT_MIN);
-        x = __reduce_max_sync(0xffffffffu, x);
-        if ((threadIdx.x & 31) == 0 && x != INT_MIN) atomicMax(fp.ex + b, x);
-      }
-#pragma unroll
-      for (int i = 0; i < PP; ++i) {
-        xa[i] = to_digits54(xa[i], clz - 2);
-        xb[i] = to_digits54(xb[i], clz - 2);
-      }
-      ue += 10 - clz;
+      if (e.blk == 0) report_exp(fp.ex + b, bad ? kBadExp : (e.line < nl ? ue + 64 - clz : INT_MIN));
+      ue += to_line_scale(xa, xb, clz);
     }
-    e.filter(xa, xb, []() {});
+    if constexpr (kStaged) {
+      e.filter(xa, xb, []() {}, [&](int i, int64_t p, int64_t q) {
+        if (i < 8) {
+          xa[i] = p;
+          xb[i] = q;
+        } else {   // the last products are done: A is free
+          sp.a(i) = p;
+          sp.b(i) = q;
+        }
+      });
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        sp.a(i) = xa[i];
+        sp.b(i) = xb[i];
+      }
+    } else {
+      e.filter(xa, xb, []() {});
+    }
     if (MODE == LAST || (MODE == PAIR && f == 0)) {
-      // q = W y to the finished slice, v = W q onwards
       const int ur = ue + shift + eref - 1022;            // unit of r = W y
       double *qo = static_cast<double *>(fp.q) + b * fp.q_bs;
-      int wneg = 0;   // the factors' signs: a negative one is not finite
+      int wneg = 0;
       if constexpr (XP) {
         e.sync();   // A is free
-        if (e.u == 0) ur_row[e.line] = ur;
+        if (e.blk == 0) ur_row[e.line] = ur;
 #pragma unroll
         for (int i = 0; i < PP; ++i) {
           if (i < lim) {
@@ -456,13 +579,12 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
           }
         }
         e.sync();
-        auto factor = [&](int r, int col, int i, int64_t w) {
+        over_rows(e.ncomp, ln.n, nl, wf + tile, [&](int r, int cc, int i, int64_t w) {
           wneg |= (int)(w >> 32);
-          const int64_t v = mul_w62(stg[r * P + col], w);
+          const int64_t v = mul_w62(stg[r * P + cc], w);
           qo[tile + i] = slice_value(v, ur_row[r]);
-          if (MODE == PAIR) stg[r * P + col] = mul_w62(v, w);
-        };
-        over_rows(e.ncomp, ln.n, nl, wf + tile, factor);
+          if (MODE == PAIR) stg[r * P + cc] = mul_w62(v, w);
+        });
         if (bad || wneg < 0)
           over_rows(e.ncomp, ln.n, nl, wf + tile, [&](int, int, int i, int64_t w) {
             if (bad || w < 0) qo[tile + i] = bad_value(0.0);
@@ -476,80 +598,17 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
           }
         }
       } else {
-        auto factor = [&](unsigned o, int64_t &x, int64_t w, bool on) {
-          wneg |= (int)(w >> 32);
-          const int64_t r = mul_w62(x, w);
-          const double q = slice_value(r, ur);
-          if (on) qo[o] = q;
-          x = mul_w62(r, w);
-        };
-        if constexpr (PP == 8) {
+        if constexpr (kStaged) {
+          wneg = sp.factor(wf, qo, col, ur);
 #pragma unroll
-          for (int g = 0; g < PP; g += 4) {
-            int64_t w[8];   // (predicated loads: a branch around a point would
-                            // serialise them)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const unsigned o = off + (g + i) * sn;
-              w[2 * i] = g + i < lim ? ld64(wf + o) : 0;
-              w[2 * i + 1] = g + i < lim ? ld64(wf + (o + hs)) : 0;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const unsigned o = off + (g + i) * sn;
-              factor(o, xa[g + i], w[2 * i], g + i < lim);
-              factor(o + hs, xb[g + i], w[2 * i + 1], g + i < lim);
-            }
+          for (int i = 0; i < PP && MODE == PAIR; ++i) {
+            xa[i] = sp.a(i);
+            xb[i] = sp.b(i);
           }
         } else {
-          // through the thread's own part of the (free) operand memory: as an
-          // unrolled loop over registers this spilled 800 bytes a thread
-          int64_t *own = stg + threadIdx.x;
-#pragma unroll
-          for (int i = 0; i < PP; ++i) {
-            own[2 * i * e.ncomp] = xa[i];
-            own[(2 * i + 1) * e.ncomp] = xb[i];
-          }
-          // (predicated loads, two points ahead)
-          int64_t w[4];
-          auto load_w = [&](int i) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const unsigned o = off + (i + j) * sn;
-              w[2 * j] = i + j < lim ? ld64(wf + o) : 0;
-              w[2 * j + 1] = i + j < lim ? ld64(wf + (o + hs)) : 0;
-            }
-          };
-          load_w(0);
-#pragma unroll 1
-          for (int i = 0; i < PP; i += 2) {
-            const int64_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-            int64_t y0 = own[2 * i * e.ncomp], y1 = own[(2 * i + 1) * e.ncomp], y2 = own[(2 * i + 2) * e.ncomp], y3 = own[(2 * i + 3) * e.ncomp];
-            if (i + 2 < PP) load_w(i + 2);
-            const unsigned o = off + i * sn;
-            factor(o, y0, w0, i < lim);
-            factor(o + hs, y1, w1, i < lim);
-            factor(o + sn, y2, w2, i + 1 < lim);
-            factor(o + sn + hs, y3, w3, i + 1 < lim);
-            own[2 * i * e.ncomp] = y0;
-            own[(2 * i + 1) * e.ncomp] = y1;
-            own[(2 * i + 2) * e.ncomp] = y2;
-            own[(2 * i + 3) * e.ncomp] = y3;
-          }
-          if (MODE == PAIR) {
-#pragma unroll
-            for (int i = 0; i < PP; ++i) {
-              xa[i] = own[2 * i * e.ncomp];
-              xb[i] = own[(2 * i + 1) * e.ncomp];
-            }
-          }
+          wneg = factor_points(xa, xb, wf, qo, col, ur);
         }
-        if (bad || wneg < 0)
-          for (int i = 0; i < lim && i < PP; ++i) {
-            const unsigned o = off + i * sn;
-            if (bad || wf[o] < 0) qo[o] = bad_value(0.0);
-            if (bad || wf[o + hs] < 0) qo[o + hs] = bad_value(0.0);
-          }
+        if (bad || wneg < 0) spoil_points(bad, wf, qo, col, PP);
         if constexpr (MODE == PAIR) {
           if (e.any(wneg < 0)) bad = true;
         }
@@ -570,7 +629,15 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
         }
       }
       e.sync();
-      over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) { out[tile + i] = stg[r * P + col]; });
+      over_rows(e.ncomp, ln.n, nl, [&](int r, int cc, int i) { out[tile + i] = stg[r * P + cc]; });
+    } else if constexpr (kStaged) {
+#pragma unroll 4
+      for (int i = 0; i < PP; ++i) {
+        if (i < lim) {
+          out[off + i * sn] = rs(sp.a(i));
+          out[off + i * sn + hs] = rs(sp.b(i));
+        }
+      }
     } else {
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
@@ -582,6 +649,274 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
     }
   }
   e.finish(fp.err);
+}
+
+// ---------------------------------------------------------------- k_planes
+// Whole planes per CTA (up to 64 points a line): both axes of a step in one
+// launch.  What a launch costs beside its filters (2.7 us until the next one may
+// read, 1.5 us to load and store a tile) was about half of a 64^3 step.  ms per
+// SCF iteration with 200 steps, one launch per pass against planes: FP64 32^3 2.5 /
+// 2.1, 64^3 3.86 / 3.48.  Above 64 points the planes' one CTA each takes as long as the
+// passes' more evenly filled ones (128^3 22.5 / 22.4, 96^3 10.1 / 12.3; FP32 80^3 5.4 /
+// 6.2): those keep their passes.
+//
+// FILM false: x filter, y filter, q = W y (stored), v = W q, y filter, x filter
+// (the middle pass, the pair and the next middle pass of k_fix's schedule).
+// FILM true (nz = 1): a whole march segment, step after step, in one launch of
+// one CTA per instance: nothing of a film leaves the CTA but its slices.
+//
+// Between its filters the planes lie in shared memory as integers of one unit
+// (rows of nx + 1: conflict-free along both axes).  q and W are read and written
+// from the y lines, where consecutive lines are consecutive in memory.
+struct PlaneArgs {
+  Shape sh;
+  int nx, ny, nz, per;   // per: planes per CTA
+  int steps;             // FILM: contour steps of the segment
+  long long q_step;      // FILM: from one slice to the next
+};
+
+template <int PP, bool FILM>
+__global__ void __launch_bounds__(544, 1)
+    k_planes(PlaneArgs pa, const void *tx, const void *ty, FixPass fp) {
+  typedef Tile<7, PP> E;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  E e;
+  e.setup(smem_raw, pa.sh, tx, ty);
+  const int shift_x = 55 - static_cast<const TcHead *>(tx)->kshift;
+  const int shift_y = 55 - static_cast<const TcHead *>(ty)->kshift;
+  const long long b = blockIdx.z;
+  const int kbits = *fp.kbits;
+  const int filters = FILM ? 2 * pa.steps : 4;
+  auto axis_of = [](int f) { return FILM ? f & 1 : (f == 1 || f == 2 ? 1 : 0); };
+  pdl_wait();
+  pdl_release();
+  if (e.issuer) {
+    e.run_issuer(filters, axis_of);
+    e.finish(fp.err);
+    return;
+  }
+  e.run_compute();
+  const int eref = fp.eref[b];
+  const int nx = pa.nx, ny = pa.ny, P = nx + 1;
+  const int z0 = blockIdx.x * pa.per, np = min(pa.per, pa.nz - z0);
+  const unsigned tile = (unsigned)z0 * ny * nx;
+  const int k0 = PP * e.blk, pl = e.line / nx, xx = e.line - pl * nx;
+  int64_t *S = reinterpret_cast<int64_t *>(smem_raw);
+  const int64_t *wf = fp.w + b * fp.w_bs;
+  // this thread's points as x line (row `line`) and as y line (plane pl, x)
+  const int lim_x = e.line < np * ny ? pa.sh.half[0] - k0 : 0;
+  const int lim_y = e.line < np * nx ? pa.sh.half[1] - k0 : 0;
+  const int at_x = e.line * P + k0, at_y = (pl * ny + k0) * P + xx;
+  const Column col{tile + (unsigned)(pl * ny + k0) * nx + xx, (unsigned)nx,
+                   (unsigned)(pa.sh.half[1] * nx), lim_y};
+
+  int us, u_out = 0;            // the unit of what lies in S
+  bool bad;
+  if constexpr (FILM) {
+    // v0 = W q0, scaled by the slice's largest magnitude
+    const double *in = static_cast<const double *>(fp.in) + b * fp.in_bs + tile;
+    int *top = reinterpret_cast<int *>(smem_raw + e.lay.ur_off);
+    if (threadIdx.x == 0) top[0] = top[1] = 0;
+    e.start();
+    int key = 0;
+    for (int i = threadIdx.x; i < ny * nx; i += e.ncomp) key = max(key, mag_key(ldg(in + i)));
+    key = __reduce_max_sync(0xffffffffu, key);
+    if ((threadIdx.x & 31) == 0) atomicMax(top, key);
+    e.sync();
+    key = top[0];
+    bad = key >= bad_key<double>();
+    const int Eb = line_exp(0.0, key);
+    bool wbad = false;
+    over_rows(e.ncomp, nx, ny, wf + tile, [&](int r, int cc, int i, int64_t w) {
+      wbad |= w < 0;
+      S[r * P + cc] = mul_w62(to_fixed(ldg(in + i), Eb) << 5, w);
+    });
+    if (e.any(wbad)) bad = true;
+    us = unit_exp(0.0, Eb) - 5 + eref - 1022;
+  } else {
+    const int s_in = fp.u_in[b], s_out = fp.u_out[b];
+    bad = unit_bad(s_in) || unit_bad(s_out);
+    us = s_in + fp.w_in * (eref - 1022) + kbits - 59;
+    u_out = s_out + fp.w_out * (eref - 1022) + kbits - 59;
+    const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs;
+    over_rows(e.ncomp, nx, np * ny, in + tile,
+              [&](int r, int cc, int, int64_t x) { S[r * P + cc] = x; });
+    e.start();
+  }
+
+  double *qo = static_cast<double *>(fp.q) + b * fp.q_bs;
+  int64_t xa[PP], xb[PP];
+  int ue = us;
+#pragma unroll 1
+  for (int f = 0; f < filters; ++f) {
+    const int ax = axis_of(f);
+    e.set_axis(ax);
+    const int lim = ax ? lim_y : lim_x, at = ax ? at_y : at_x, st = ax ? P : 1, hs = e.H * st;
+    if (FILM || f != 2) {
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        xa[i] = i < lim ? S[at + i * st] : 0;
+        xb[i] = i < lim ? S[at + i * st + hs] : 0;
+      }
+      ue = us;
+    }
+    const int key = e.line_key(f & 3, points_key(xa, xb));   // (its barrier: S is read)
+    if (e.blk == 0) e.clear_key((f + 2) & 3);
+    const int clz = clz32((uint32_t)key | 1u);
+    if (!FILM && f == 2 && e.blk == 0)
+      report_exp(fp.ex + b, bad ? kBadExp : (lim_y > 0 ? ue + 64 - clz : INT_MIN));
+    ue += to_line_scale(xa, xb, clz);
+    e.filter(xa, xb, []() {});
+    ue += ax ? shift_y : shift_x;
+    int target = us;
+    if (FILM ? ax == 1 : f == 1) {
+      const int ur = ue + eref - 1022;
+      const int wneg = factor_points(xa, xb, wf, qo, col, ur);
+      if (bad || wneg < 0) spoil_points(bad, wf, qo, col, PP);
+      if (e.any(wneg < 0)) bad = true;
+      ue = ur + eref - 1022;
+      if (!FILM) continue;     // v goes on along y
+      if (f + 1 == filters) break;
+      qo += pa.q_step;
+      // the next unit from the largest v (two slots in turn)
+      int *top = reinterpret_cast<int *>(smem_raw + e.lay.ur_off) + 2;
+      const int slot = f >> 1 & 1;
+      int x = ue + 64 - clz32((uint32_t)points_key(xa, xb) | 1u);
+      x = __reduce_max_sync(0xffffffffu, lim > 0 ? x : INT_MIN);
+      if (threadIdx.x == 0) top[slot ^ 1] = INT_MIN;
+      if (f == 1 && threadIdx.x == 0) top[slot] = INT_MIN;
+      e.sync();
+      if ((threadIdx.x & 31) == 0) atomicMax(top + slot, x);
+      e.sync();
+      target = us = top[slot] + kbits - 59;
+    } else if (!FILM && f >= 2) {
+      target = us = u_out;
+    }
+    const Rescale rs(target - ue);
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      if (i < lim) {
+        S[at + i * st] = rs(xa[i]);
+        S[at + i * st + hs] = rs(xb[i]);
+      }
+    }
+    e.sync();
+  }
+  if constexpr (!FILM) {
+    int64_t *out = static_cast<int64_t *>(fp.out) + b * fp.out_bs;
+    over_rows(e.ncomp, nx, np * ny, [&](int r, int cc, int i) { out[tile + i] = S[r * P + cc]; });
+  }
+  e.finish(fp.err);
+}
+
+// The same on FP32 planes (working reals between the filters).  A batched pass
+// (ps.desc) is the first half only: pre, x filter, y filter.
+template <int PP>
+__global__ void __launch_bounds__(544, 1)
+    k_planes_f32(PlaneArgs pa, const void *tx, const void *ty, PassSet<float> ps) {
+  typedef Tile<4, PP> E;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  E e;
+  const bool half = ps.desc != nullptr;
+  if (half) {
+    tx = ps.desc[blockIdx.z].tc;
+    ty = ps.desc[blockIdx.z].tc_y;
+  }
+  e.setup(smem_raw, pa.sh, tx, ty);
+  const int shift_x = 23 - static_cast<const TcHead *>(tx)->kshift;
+  const int shift_y = 23 - static_cast<const TcHead *>(ty)->kshift;
+  const long long b = blockIdx.z;
+  const int filters = half ? 2 : 4;
+  auto axis_of = [](int f) { return f == 1 || f == 2 ? 1 : 0; };
+  pdl_wait();
+  pdl_release();
+  if (e.issuer) {
+    e.run_issuer(filters, axis_of);
+    e.finish(ps.err);
+    return;
+  }
+  e.run_compute();
+  const int nx = pa.nx, ny = pa.ny, P = nx + 1;
+  const int z0 = blockIdx.x * pa.per, np = min(pa.per, pa.nz - z0);
+  const unsigned tile = (unsigned)z0 * ny * nx;
+  const int k0 = PP * e.blk, pl = e.line / nx, xx = e.line - pl * nx;
+  float *S = reinterpret_cast<float *>(smem_raw);
+  const float *in = ps.in[0] + b * ps.in_bs[0], *w = ps.post[0] + b * ps.w_bs, *pre = nullptr;
+  float *out = ps.out[0] + b * ps.out_bs[0], *qo = ps.qout[0] + b * ps.qout_bs[0];
+  if (half) {
+    const PassDesc d = ps.desc[b];
+    in = d.in;
+    out = d.out;
+    pre = d.pre;
+  }
+  const int lim_x = e.line < np * ny ? pa.sh.half[0] - k0 : 0;
+  const int lim_y = e.line < np * nx ? pa.sh.half[1] - k0 : 0;
+  const int at_x = e.line * P + k0, at_y = (pl * ny + k0) * P + xx;
+  const unsigned off = tile + (unsigned)(pl * ny + k0) * nx + xx, ghs = pa.sh.half[1] * nx;
+  over_rows(e.ncomp, nx, np * ny, [&](int r, int cc, int i) {
+    const float x = __ldg(in + tile + i);
+    S[r * P + cc] = pre ? x * __ldg(pre + tile + i) : x;
+  });
+  e.start();
+#pragma unroll 1
+  for (int f = 0; f < filters; ++f) {
+    const int ax = axis_of(f);
+    e.set_axis(ax);
+    const int lim = ax ? lim_y : lim_x, at = ax ? at_y : at_x, st = ax ? P : 1, hs = e.H * st;
+    float ya[PP], yb[PP];
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      ya[i] = i < lim ? S[at + i * st] : 0.f;
+      yb[i] = i < lim ? S[at + i * st + hs] : 0.f;
+    }
+    int key = 0;
+#pragma unroll
+    for (int i = 0; i < PP; ++i) key = max(key, max(mag_key(ya[i]), mag_key(yb[i])));
+    key = e.line_key(f, key);   // (its barrier: S is read)
+    const bool bad = key >= bad_key<float>();
+    const int Eb = line_exp(0.f, key), ue = unit_exp(0.f, Eb) + (ax ? shift_y : shift_x);
+    int xa[PP], xb[PP];
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      xa[i] = to_fixed(ya[i], Eb);
+      xb[i] = to_fixed(yb[i], Eb);
+    }
+    e.filter(xa, xb, []() {}, [&](int i, float p, float q) {
+      ya[i] = bad ? bad_value(0.f) : scale2(p, ue);
+      yb[i] = bad ? bad_value(0.f) : scale2(q, ue);
+    });
+    if (f == 1 && !half) {
+#pragma unroll
+      for (int g = 0; g < PP; g += 4) {
+        float w0[4], w1[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          w0[i] = g + i < lim ? __ldg(w + (off + (g + i) * nx)) : 0.f;
+          w1[i] = g + i < lim ? __ldg(w + (off + (g + i) * nx + ghs)) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float q0 = ya[g + i] * w0[i], q1 = yb[g + i] * w1[i];
+          if (g + i < lim) {
+            qo[off + (g + i) * nx] = q0;
+            qo[off + (g + i) * nx + ghs] = q1;
+          }
+          ya[g + i] = q0 * w0[i];
+          yb[g + i] = q1 * w1[i];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < PP; ++i) {
+      if (i < lim) {
+        S[at + i * st] = ya[i];
+        S[at + i * st + hs] = yb[i];
+      }
+    }
+    e.sync();
+  }
+  over_rows(e.ncomp, nx, np * ny, [&](int r, int cc, int i) { out[tile + i] = S[r * P + cc]; });
+  e.finish(ps.err);
 }
 
 // ------------------------------------------------- factors and slice exponents
@@ -624,9 +959,15 @@ __global__ void k_slice_exp(const double *__restrict__ q, long long bs, long lon
 // Geometry of a pass, or false when the kernels do not take it.
 bool lines_of(const AxisPlan &ap, int nd, Lines &ln) {
   if (!ap.tc || !tc_line_possible(ap.n, nd) || ap.n_real < 1 || ap.n_outer < 1) return false;
+  const int kg = line_blocks(ap.n);
+  memset(&ln.sh, 0, sizeof ln.sh);
+  ln.sh.nd = nd;
+  ln.sh.pp = pairs_per_thread(kg);
+  ln.sh.rep = 1;
+  ln.sh.axes = 1;
+  ln.sh.half[0] = ln.sh.half[1] = ap.n / 2;
+  ln.sh.kg[0] = ln.sh.kg[1] = kg;
   ln.n = ap.n;
-  ln.half = ap.n / 2;
-  ln.kg = (ln.half + 15) / 16;
   ln.s_n = ap.s_n;
   ln.lines = (long long)ap.n_real * ap.n_outer;
   if (ap.n_fast) {                 // rows
@@ -641,23 +982,38 @@ bool lines_of(const AxisPlan &ap, int nd, Lines &ln) {
   }
   return (ln.lines + kLines - 1) / kLines <= 0x7fffffffLL;
 }
-inline int threads_of(const Lines &ln) {
-  const int pp = pairs_per_thread(ln.kg);
-  return kLines * 16 * ln.kg / pp + issuer_threads(pp);
+
+// Copies of each line per CTA, and with them 4 points per thread, so that small
+// launches of lines of up to 64 points spread over the SMs: doubled while both
+// chains' CTAs still fit there side by side (ms per SCF iteration, one copy
+// against this: FP64 16^3 3.3 / 2.4, 32^3 3.6 / 2.6, 64^3 5.1 / 4.1).  With 16 points per
+// thread two copies were slower (FP32 100 x 80 x 60 5.7 against 5.2).
+void spread(Shape &sh, long long lines) {
+  if (sh.pp == 16) return;
+  const int kg = sh.axes == 2 ? std::max(sh.kg[0], sh.kg[1]) : sh.kg[0];
+  while (sh.rep < 4 && 2 * ((lines + kLines / (2 * sh.rep) - 1) / (kLines / (2 * sh.rep))) <= 152 &&
+         16 * kg >= 8 * sh.rep)
+    sh.rep *= 2;
+  if (sh.rep > 1 && sh.pp == 8) sh.pp = 4;
 }
+inline int lines_per_cta(const Shape &sh) { return kLines / sh.rep; }
 
 template <typename T, int MAXT, int PP, bool XP, bool PR>
-cudaError_t launch_real_t(const Lines &ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
-  dim3 grid((unsigned)((ln.lines + kLines - 1) / kLines), 1, ps.nset * ps.batch);
-  return launch_pdl(k_real<T, MAXT, PP, XP, PR>, grid, dim3(threads_of(ln)),
-                    (size_t)smem_layout(kNd<T>, ln.n, ln.kg, XP ? (int)sizeof(T) : 0).total, st,
-                    ln, tc, ps);
+cudaError_t launch_real_t(Lines ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+  const int lc = lines_per_cta(ln.sh);
+  dim3 grid((unsigned)((ln.lines + lc - 1) / lc), 1, ps.nset * ps.batch);
+  ln.sh.stage = XP ? lc * (ln.n + 1) * (int)sizeof(T) : 0;
+  ln.sh.finish();
+  return launch_pdl(k_real<T, MAXT, PP, XP, PR>, grid, dim3(ln.sh.threads),
+                    (size_t)ln.sh.lay.total, st, ln, tc, ps);
 }
 template <typename T, bool XP, bool PR>
-cudaError_t launch_real_kg(const Lines &ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
-  if (ln.kg <= 2) return launch_real_t<T, 544, 8, XP, PR>(ln, tc, ps, st);
+cudaError_t launch_real_kg(Lines ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+  spread(ln.sh, ln.lines * ps.nset * ps.batch);
+  if (ln.sh.pp == 4) return launch_real_t<T, 544, 4, XP, PR>(ln, tc, ps, st);
+  if (ln.sh.pp == 8) return launch_real_t<T, 544, 8, XP, PR>(ln, tc, ps, st);
   if constexpr (std::is_same<T, float>::value) {
-    if (ln.kg > 4) return launch_real_t<T, 1024, 16, XP, PR>(ln, tc, ps, st);
+    if (ln.sh.kg[0] > 4) return launch_real_t<T, 1024, 16, XP, PR>(ln, tc, ps, st);
   }
   return launch_real_t<T, 640, 16, XP, PR>(ln, tc, ps, st);
 }
@@ -688,12 +1044,57 @@ cudaError_t launch_real(const AxisPlan &ap, const PassSet<T> &ps, bool pair, cud
 }
 
 template <bool XP, int MODE>
-cudaError_t launch_fix_t(const Lines &ln, const void *tc, const FixPass &fp, cudaStream_t st) {
-  dim3 grid((unsigned)((ln.lines + kLines - 1) / kLines), 1, fp.batch);
-  const size_t smem = smem_layout(7, stage_points(ln, XP, MODE), ln.kg, 8).total;
-  if (ln.kg <= 2)
-    return launch_pdl(k_fix<8, XP, MODE>, grid, dim3(threads_of(ln)), smem, st, ln, tc, fp);
-  return launch_pdl(k_fix<16, XP, MODE>, grid, dim3(threads_of(ln)), smem, st, ln, tc, fp);
+cudaError_t launch_fix_t(Lines ln, const void *tc, const FixPass &fp, cudaStream_t st) {
+  spread(ln.sh, ln.lines * fp.batch);
+  const int lc = lines_per_cta(ln.sh);
+  dim3 grid((unsigned)((ln.lines + lc - 1) / lc), 1, fp.batch);
+  // x passes stage rows; column passes with 16 points per thread the factor step
+  if (XP) ln.sh.stage = lc * (ln.n + 1) * 8;
+  else if (ln.sh.pp == 16 && (MODE == PAIR || MODE == LAST))
+    ln.sh.stage = kLines * ln.sh.kg[0] * 256;
+  ln.sh.finish();
+  const size_t smem = ln.sh.lay.total;
+  if (ln.sh.pp == 4)
+    return launch_pdl(k_fix<4, XP, MODE>, grid, dim3(ln.sh.threads), smem, st, ln, tc, fp);
+  if (ln.sh.pp == 8)
+    return launch_pdl(k_fix<8, XP, MODE>, grid, dim3(ln.sh.threads), smem, st, ln, tc, fp);
+  return launch_pdl(k_fix<16, XP, MODE>, grid, dim3(ln.sh.threads), smem, st, ln, tc, fp);
+}
+
+// Planes of nx x ny points, nz of them per instance (film: a march segment).
+void plane_shape(int nx, int ny, int nz, int nd, int batch, bool film, PlaneArgs &pa) {
+  memset(&pa, 0, sizeof pa);
+  pa.nx = nx;
+  pa.ny = ny;
+  pa.nz = nz;
+  pa.sh.nd = nd;
+  pa.sh.pp = 8;
+  pa.sh.rep = 1;
+  pa.sh.axes = 2;
+  pa.sh.half[0] = nx / 2;
+  pa.sh.half[1] = ny / 2;
+  pa.sh.kg[0] = line_blocks(nx);
+  pa.sh.kg[1] = line_blocks(ny);
+  const int m = std::max(nx, ny), per = kLines / m;
+  // a film's one plane: as many copies of its lines as fit; else by the lines
+  // that the planes fill if a CTA takes 128 of them
+  spread(pa.sh, film ? 1 : (long long)((nz + per - 1) / per) * kLines * batch);
+  while (lines_per_cta(pa.sh) < m) pa.sh.rep /= 2;
+  pa.sh.pp = pa.sh.rep > 1 ? 4 : 8;
+  const int lc = lines_per_cta(pa.sh);
+  pa.per = lc / m;
+  pa.sh.stage = lc * (nx + 1) * (nd == 7 ? 8 : 4);
+  pa.sh.finish();
+}
+// ... of passes apx (x) and apy (lines nx apart), or false.
+bool planes_of(const AxisPlan &apx, const AxisPlan &apy, int nd, int batch, bool film,
+               PlaneArgs &pa) {
+  Lines lx, ly;
+  if (!lines_of(apx, nd, lx) || !lines_of(apy, nd, ly) || !apx.n_fast || apy.n_fast ||
+      apy.s_n != apx.n || lx.sh.pp > 8 || ly.sh.pp > 8)
+    return false;
+  plane_shape(apx.n, apy.n, (int)(lx.lines / apy.n), nd, batch, film, pa);
+  return true;
 }
 
 // Shared-memory opt-in; a kernel that splits its registers must have been given
@@ -720,6 +1121,11 @@ template <typename T, int MAXT, int PP> cudaError_t prep_real() {
 }
 template <int PP> cudaError_t prep_fix() {
   cudaError_t e;
+  if constexpr (PP <= 8) {
+    if ((e = opt_in(k_planes<PP, false>)) != cudaSuccess) return e;
+    if ((e = opt_in(k_planes<PP, true>)) != cudaSuccess) return e;
+    if ((e = opt_in(k_planes_f32<PP>)) != cudaSuccess) return e;
+  }
   if ((e = opt_in(k_fix<PP, true, FIRST>, PP == 16)) != cudaSuccess) return e;
   if ((e = opt_in(k_fix<PP, false, FIRST>, PP == 16)) != cudaSuccess) return e;
   if ((e = opt_in(k_fix<PP, false, MID>, PP == 16)) != cudaSuccess) return e;
@@ -796,8 +1202,9 @@ int digit_of(int64_t v, int nd, int j) {
 }
 
 // The table with K scaled `less` bits below the digits' full range.
-bool build_scaled(const std::vector<dd> &K, int nd, int less, std::vector<unsigned char> &table) {
-  const int n = (int)K.size(), H = n / 2, kg = (H + 15) / 16, kp = 16 * kg;
+bool build_scaled(const std::vector<dd> &K, int nd, int kg, int less,
+                  std::vector<unsigned char> &table) {
+  const int n = (int)K.size(), H = n / 2, kp = 16 * kg;
   const int bits = 8 * nd;
   double mx = 0.0;
   for (int d = 0; d < H; ++d)
@@ -884,11 +1291,55 @@ bool build_scaled(const std::vector<dd> &K, int nd, int less, std::vector<unsign
 }  // namespace
 
 bool tc_line_possible(int n, int nd) {
-  return n >= 2 && n % 2 == 0 && (n / 2 + 15) / 16 <= (nd == 4 ? 7 : 4);
+  return n >= 2 && n % 2 == 0 && line_blocks(n) <= (nd == 4 ? 7 : 4);
 }
 
 size_t tc_table_bytes(int n, int nd) {
-  return sizeof(TcHead) + 2 * (size_t)b_half_bytes(nd, (n / 2 + 15) / 16);
+  const int kg = line_blocks(n);
+  return sizeof(TcHead) + 2 * (size_t)b_half_bytes(nd, kg);
+}
+
+// CTAs of a pass of one instance.
+long long tc_pass_ctas(const AxisPlan &ap, int nd) {
+  Lines ln;
+  if (!lines_of(ap, nd, ln)) return 0;
+  spread(ln.sh, ln.lines);
+  const int lc = lines_per_cta(ln.sh);
+  return (ln.lines + lc - 1) / lc;
+}
+
+// Whether a step's x and y passes run on whole planes.  A film's do when a
+// segment can stay in one CTA's 128 threads' reach, that is at up to 32 x 32
+// (ms per SCF iteration with 200 steps, planes against passes: 32 x 32 1.17 / 1.53,
+// 500 of them 4.6 / 8.1; 40 x 36 1.95 / 1.84, 64 x 64 2.01 / 1.94).  Otherwise
+// planes save two launches in two steps, but a plane does not split over CTAs,
+// its lines leave part of the 128 rows idle, and its CTAs may need one wave
+// more.  The filters' time on both sides is taken as the waves of both chains'
+// CTAs times 2 + 4/rep; in that unit (0.6 us for 7 digits, 0.35 us for 4) a launch
+// saved is worth 2 and 4.  Measured: 64^3 FP64 3.48 / 3.86 and 60^3 FP32 2.31 / 2.82,
+// 48^3 FP64 3.20 / 3.43, 36^3 FP32 1.84 / 2.17; against planes (12, 20, 28) x 8 FP64
+// 2.63 / 2.31, (64, 40, 30) x 4 FP64 4.55 / 4.23, (36, 36, 38) x 20 FP64 14.2 / 12.9
+// and FP32 8.8 / 8.6.
+bool tc_planes_wanted(int nx, int ny, int nz, int nd, int batch) {
+  if (nx > kLines / 2 || ny > kLines / 2 || nx < 2 || ny < 2) return false;
+  if (nz == 1) return nx <= 32 && ny <= 32;
+  auto cost = [&](long long ctas, int rep) {
+    return (double)((2 * ctas + 151) / 152) * (2.0 + 4.0 / rep);
+  };
+  auto pass = [&](int n, long long lines) {
+    Shape sh = {};
+    sh.nd = nd;
+    sh.pp = 8;
+    sh.rep = sh.axes = 1;
+    sh.kg[0] = line_blocks(n);
+    spread(sh, lines * batch);
+    const int lc = lines_per_cta(sh);
+    return cost((lines + lc - 1) / lc * batch, sh.rep);
+  };
+  PlaneArgs pa;
+  plane_shape(nx, ny, nz, nd, batch, false, pa);
+  const double planes = 2.0 * cost((long long)((nz + pa.per - 1) / pa.per) * batch, pa.sh.rep);
+  return planes < pass(nx, (long long)ny * nz) + pass(ny, (long long)nx * nz) + (nd == 7 ? 2.0 : 4.0);
 }
 
 // Digits of the two half-length kernels of gain table g (natural order, real
@@ -915,13 +1366,16 @@ bool tc_build_table(const double *g, int n, int nd, std::vector<unsigned char> &
   }
   if (row_sum) *row_sum = l1;
   for (int less = 0; less < 4; ++less)
-    if (build_scaled(K, nd, less, table)) return true;
+    if (build_scaled(K, nd, line_blocks(n), less, table)) return true;
   return false;
 }
 
 namespace {
 cudaError_t prepare_all() {
   cudaError_t e;
+  if ((e = prep_real<float, 544, 4>()) != cudaSuccess) return e;
+  if ((e = prep_real<double, 544, 4>()) != cudaSuccess) return e;
+  if ((e = prep_fix<4>()) != cudaSuccess) return e;
   if ((e = prep_real<float, 544, 8>()) != cudaSuccess) return e;
   if ((e = prep_real<float, 640, 16>()) != cudaSuccess) return e;
   if ((e = prep_real<float, 1024, 16>()) != cudaSuccess) return e;
@@ -977,6 +1431,34 @@ cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStre
                : launch_fix_t<false, LAST>(ln, ap.tc, fp, st);
     default: return cudaErrorInvalidValue;
   }
+}
+
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+                          cudaStream_t st) {
+  PlaneArgs pa;
+  if (!planes_of(apx, apy, 4, ps.batch, false, pa) || ps.nset != 1 || ps.batch < 1 || ps.batch > 65535 ||
+      (!ps.desc && (!ps.in[0] || !ps.out[0] || !ps.post[0] || !ps.qout[0])))
+    return cudaErrorInvalidValue;
+  dim3 grid((pa.nz + pa.per - 1) / pa.per, 1, ps.batch);
+  const size_t smem = pa.sh.lay.total;
+  return launch_pdl(pa.sh.pp == 4 ? k_planes_f32<4> : k_planes_f32<8>, grid, dim3(pa.sh.threads), smem, st, pa, apx.tc, apy.tc, ps);
+}
+// steps 0: the fused step on planes; else a film's segment of that many steps
+// (fp.q: the first finished slice, q_step to the next one).
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPass &fp, int steps,
+                          long long q_step, cudaStream_t st) {
+  PlaneArgs pa;
+  if (!planes_of(apx, apy, 7, fp.batch, steps > 0, pa) || fp.batch < 1 || fp.batch > 65535 || !fp.in || !fp.eref ||
+      !fp.kbits || !fp.w || !fp.q || (steps == 0 && (!fp.u_in || !fp.u_out || !fp.ex || !fp.out)) ||
+      steps < 0 || (steps > 0 && pa.nz != 1))
+    return cudaErrorInvalidValue;
+  pa.steps = steps;
+  pa.q_step = q_step;
+  dim3 grid((pa.nz + pa.per - 1) / pa.per, 1, fp.batch);
+  const size_t smem = pa.sh.lay.total;
+  auto k = steps ? (pa.sh.pp == 4 ? k_planes<4, true> : k_planes<8, true>)
+                 : (pa.sh.pp == 4 ? k_planes<4, false> : k_planes<8, false>);
+  return launch_pdl(k, grid, dim3(pa.sh.threads), smem, st, pa, apx.tc, apy.tc, fp);
 }
 
 // Factors in integers: eref[b] and wf from W (two launches).

@@ -47,7 +47,7 @@ struct PassDesc {
   const float *pre, *post;   // Boltzmann factor on load / on store, or null
   const float *gain;         // the set's gain table of this pass's axis (x for a plane pass)
   const float *gain_y;       // x+y plane passes: the y axis's gain table
-  const void *tc;            // the set's tensor-core table (passes through launch_tc)
+  const void *tc, *tc_y;     // the set's tensor-core tables (tc_y: plane passes)
 };
 template <typename R> struct PassSet {
   const R *in[kMaxSet];
@@ -109,6 +109,8 @@ cudaError_t launch_xyxy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<
 // even length, up to 128 points (FP64: 7 digits) or 224 (FP32: 4 digits).  pair (FP32): a fused step pair (qout = post * K(in),
 // out = K(post * qout)).
 bool tc_line_possible(int n, int nd);
+long long tc_pass_ctas(const AxisPlan &ap, int nd);
+bool tc_planes_wanted(int nx, int ny, int nz, int nd, int batch);
 size_t tc_table_bytes(int n, int nd);
 bool tc_build_table(const double *gain, int n, int nd, std::vector<unsigned char> &table,
                     double *row_sum);
@@ -135,6 +137,13 @@ struct FixPass {
 };
 constexpr int kFixFirst = 0, kFixMid = 1, kFixPair = 2, kFixLast = 3;
 cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStream_t st);
+// Both axes of whole planes in one launch: x, y, the factor (q stored), the
+// factor, y, x (ps.desc: x, y of a batched pass); FP64 also a film's whole march
+// segment.
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+                          cudaStream_t st);
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPass &fp, int steps,
+                          long long q_step, cudaStream_t st);
 cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
                         cudaStream_t st);
 cudaError_t launch_slice_exp(const double *q, long long bs, long long M, int batch, int *ex,

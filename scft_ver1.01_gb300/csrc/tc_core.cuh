@@ -15,10 +15,13 @@
 // sum is an integer that FP32 holds exactly and the order of the sums does not
 // matter.  What is left out (i + j >= ND) is below the last digit's unit.
 //
-// Tile: 128 lines (the M of one tcgen05.mma) x N points per CTA.  Thread t owns
-// line t % 128 (its TMEM lane) and the PP points k = PP*u + i, u = t / 128, with
-// their partners k + H: it writes their digits as A operands (K-major core
-// matrices of 8 lines x 16 bytes, unswizzled) and reads the same outputs back.
+// Tile: the 128 rows (M) of one tcgen05.mma x N points per CTA.  A row holds one
+// of LN = 128/rep lines; with rep > 1 every line stands in rep rows, because a
+// thread reaches only its own TMEM lane: the threads of a line's copies share
+// its points out, so that a small grid spreads over rep times as many CTAs.
+// Thread t owns row t % 128 and the PP points k = PP*blk + i with their partners
+// k + H: it writes their digits as A operands, once per copy (K-major core
+// matrices of 8 rows x 16 bytes, unswizzled), and reads the same outputs back.
 // B holds the digits of Kc or Kd stacked along its rows (digit j, output n), so
 // one instruction multiplies x's digit i with all of K's digits 0 .. ND-1-i and
 // adds into the accumulators i .. ND-1 side by side: up to 256 columns per
@@ -51,56 +54,80 @@ struct TcHead {
   int pad[3];
 };
 
-// Accumulators come in two TMEM buffers, so that one is read while the tensor
-// core fills the other.  Where A, B and TMEM have the room (both_halves) a
-// buffer holds all outputs of c or d; else half of the outputs (8 of each
-// thread's 16), and a half takes two rounds.
-__host__ __device__ constexpr bool both_halves(int nd, int kg) { return nd == 7 ? kg <= 2 : kg <= 4; }
-__host__ __device__ constexpr bool split_rows(int nd, int kg) { return nd == 7 && kg > 2; }
-// Accumulator columns of one digit group in one buffer (a multiple of 16), and
-// the outputs they stand for.
-__host__ __device__ constexpr int group_cols(int nd, int kg) { return split_rows(nd, kg) ? 32 : 16 * kg; }
-__host__ __device__ constexpr bool dense_b(int kg) { return kg <= 4; }
-// B of both halves resident (else the half in use is copied in).
-__host__ __device__ constexpr bool b_resident(int nd, int kg) { return nd != 7 || kg <= 3; }
-// Points per thread: 8 where that keeps the CTA at 512 threads.
+// 16-point blocks of a half line
+__host__ __device__ constexpr int line_blocks(int n) { return (n / 2 + 15) / 16; }
+// Points per thread: 16 on lines above 64 points (512 computing threads at 128),
+// else 8, or 4 in CTAs of fewer lines.
 __host__ __device__ constexpr int pairs_per_thread(int kg) { return kg <= 2 ? 8 : 16; }
-// The issuing warp; with 16 points per thread a warpgroup of its own, so that
-// the computing ones can take its registers (setmaxnreg: 96 at launch for 640
-// threads, then 112 x 512 + 24 x 128 = 60416 <= 96 x 640 = 61440; with 384 + 128
-// threads 46080 <= 49152).
-__host__ __device__ constexpr int issuer_threads(int pp) { return pp == 16 ? 128 : 32; }
-constexpr int kRegsLaunch = 96, kRegsCompute = 112, kRegsIssue = 24;
+__host__ __device__ constexpr bool dense_b(int kg) { return kg <= 4; }
+// Accumulators come in two TMEM buffers, so that one is read while the tensor
+// core fills the other.  A buffer holds all outputs of c or d (whose A operands
+// then lie side by side); for 7 digits and 16 points per thread TMEM and shared
+// memory have no room for that: a buffer holds half of the outputs (8 of each
+// thread's 16), a half takes two rounds, and c's operand memory serves d.
+__host__ __device__ constexpr bool split_rows(int nd, int kg) { return nd == 7 && kg > 2; }
+__host__ __device__ constexpr bool both_halves(int nd, int kg) {
+  return !split_rows(nd, kg) && dense_b(kg);
+}
+// Accumulator columns of one digit group in one buffer (a multiple of 16).
+__host__ __device__ constexpr int group_cols(int nd, int kg) {
+  return split_rows(nd, kg) ? 32 : 16 * kg;
+}
 __host__ __device__ constexpr int b_half_bytes(int nd, int kg) {
   return dense_b(kg) ? nd * group_cols(nd, kg) * (split_rows(nd, kg) ? 2 : 1) * (16 * kg) * 2
                      : nd * (4 * kg - 1) * 128;
 }
+// The issuing warp; with 16 points per thread and 7 digits a warpgroup of its
+// own, so that the computing ones can take its registers (setmaxnreg: 96 at
+// launch for 640 threads, then 104 x 512 + 56 x 128 = 60416 <= 96 x 640 = 61440;
+// with 384 + 128 threads 47104 <= 49152, with 256 + 128 33792 <= 36864).  112 + 24
+// left the issuing warp too few: it kept its loop in local memory.
+__host__ __device__ constexpr int issuer_threads(int pp) { return pp == 16 ? 128 : 32; }
+constexpr int kRegsLaunch = 96, kRegsCompute = 104, kRegsIssue = 56;
 
 // ---- shared-memory layout (bytes)
+constexpr int kKeySlots = 4;
 struct Smem {
-  int a_digit, a_half;   // one digit's A operand; one half's
-  int b_off, b_half, key_off, ur_off, bar_off, total;
+  int b_off, key_off, ur_off, bar_off, total;
 };
-__host__ __device__ inline Smem smem_layout(int nd, int n, int kg, int stage_elem) {
-  Smem s;
-  s.a_digit = kLines * kg * 16 * 2;
-  s.a_half = nd * s.a_digit;
-  int big = s.a_half * (both_halves(nd, kg) ? 2 : 1);
-  const int stage = stage_elem ? kLines * (n + 1) * stage_elem : 0;   // row staging, aliases A
-  if (stage > big) big = stage;
-  s.b_off = (big + 127) / 128 * 128;
-  s.b_half = b_half_bytes(nd, kg);
-  s.key_off = s.b_off + (b_resident(nd, kg) ? 2 : 1) * s.b_half;
-  s.ur_off = s.key_off + 2 * kLines * 4;    // keys of the two filters
-  s.bar_off = s.ur_off + kLines * 4;        // per-line units
-  s.total = s.bar_off + 64;                 // six mbarriers, TMEM address
-  return s;
-}
-__host__ __device__ constexpr int tmem_cols(int nd, int kg) {
-  int c = nd * group_cols(nd, kg) * (dense_b(kg) ? 2 : 1), p = 32;
-  while (p < c) p *= 2;
-  return p;
-}
+// What a CTA filters: lines of one axis, or of the two axes of its planes.
+// finish() lays it out on the host: computed by each CTA it cost the launch
+// about 0.1 us, which nothing hides (a CTA starts when the one before it has
+// left the SM's shared memory).
+struct Shape {
+  int nd, pp, rep, axes;
+  int half[2], kg[2];    // H, and 16-point blocks of it
+  int stage;             // staging memory, bytes (aliases the A operands)
+  Smem lay;
+  int cols, threads;     // TMEM columns
+  int a_digit[2], b_half[2];   // bytes of a digit's A operand, of a half's table
+
+  __host__ void finish() {
+    int big = stage, bsum = 0, need = 0, blocks = 0;
+    const bool res = nd == 4 || pp <= 8;   // tables of both halves resident, or one
+    for (int i = 0; i < axes; ++i) {
+      a_digit[i] = kLines * kg[i] * 32;
+      b_half[i] = b_half_bytes(nd, kg[i]);
+      const int a = nd * a_digit[i] * (both_halves(nd, kg[i]) ? 2 : 1);
+      const int c = nd * group_cols(nd, kg[i]) * (dense_b(kg[i]) ? 2 : 1);
+      big = a > big ? a : big;
+      bsum += (res ? 2 : 1) * b_half[i];
+      need = c > need ? c : need;
+      blocks = kg[i] > blocks ? kg[i] : blocks;
+    }
+    for (int i = axes; i < 2; ++i) {
+      a_digit[i] = a_digit[0];
+      b_half[i] = b_half[0];
+    }
+    lay.b_off = (big + 127) / 128 * 128;
+    lay.key_off = lay.b_off + bsum;
+    lay.ur_off = lay.key_off + kKeySlots * kLines * 4;   // line keys
+    lay.bar_off = lay.ur_off + kLines * 4;               // per-line units, or CTA scratch
+    lay.total = lay.bar_off + 64;                        // six mbarriers, TMEM address
+    for (cols = 32; cols < need;) cols *= 2;
+    threads = kLines * ((16 * blocks + pp * rep - 1) / (pp * rep)) + issuer_threads(pp);
+  }
+};
 
 #ifdef __CUDACC__
 // ---- tcgen05 / mbarrier wrappers
@@ -149,11 +176,13 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, unsigned parity) {
     if (clock64() - t0 > 2000000000LL) return false;
   }
 }
-// 1-D bulk copy global -> shared, completing on `bar`.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, unsigned bytes,
-                                          uint32_t bar) {
+__device__ __forceinline__ void expect_bytes(uint32_t bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
+}
+// 1-D bulk copy global -> shared, counted on `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, unsigned bytes,
+                                          uint32_t bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
           dst),
@@ -282,31 +311,57 @@ template <int ND, int PP> struct Tile {
 
   unsigned char *smem;
   Smem lay;
-  const unsigned char *table;   // global: the digits of Kc, then of Kd
-  int kg, line, u, warp, ncomp;
+  // per axis: blocks, H, bytes of a digit's A operand and of a half's table (no
+  // arrays: an index at run time is a memory access)
+  int kg0, kg1, half0, half1, ad0, ad1, bh0, bh1;
+  const unsigned char *table;      // global (one axis): the digits of Kc, then of Kd
+  int kg, H, a_digit, a_half, b_half, b_at;   // of the axis in hand
+  int line, blk, rep, ln, warp, ncomp, cols;
   uint32_t tmem;
-  unsigned phases;              // parities of the products' barriers
+  unsigned phases;                 // parities of the products' barriers
   bool ok, both, issuer;
+  static constexpr bool kSplit = ND == 7 && PP == 16;   // split_rows
+  static constexpr bool kRes = ND == 4 || PP <= 8;   // both halves' tables resident
 
   __device__ __forceinline__ uint32_t bar(int i) const { return sm32(smem + lay.bar_off) + 8 * i; }
 
+  __device__ __forceinline__ void set_axis(int ax) {
+    kg = ax ? kg1 : kg0;
+    H = ax ? half1 : half0;
+    both = both_halves(ND, kg);
+    a_digit = ax ? ad1 : ad0;
+    a_half = ND * a_digit;
+    b_half = ax ? bh1 : bh0;
+    b_at = ax ? 2 * bh0 : 0;
+  }
+
   // Before the dependency wait: barriers, keys and the (constant) tables.
-  __device__ __forceinline__ void setup(unsigned char *sm, int n, int kgs, int stage_elem,
-                                        const void *tab) {
+  __device__ __forceinline__ void setup(unsigned char *sm, const Shape &sh, const void *tab0,
+                                        const void *tab1) {
     smem = sm;
-    kg = kgs;
-    lay = smem_layout(ND, n, kgs, stage_elem);
-    table = static_cast<const unsigned char *>(tab) + sizeof(TcHead);
+    lay = sh.lay;
+    cols = sh.cols;
+    table = static_cast<const unsigned char *>(tab0) + sizeof(TcHead);
+    kg0 = sh.kg[0];
+    kg1 = sh.kg[1];
+    half0 = sh.half[0];
+    half1 = sh.half[1];
+    ad0 = sh.a_digit[0];
+    ad1 = sh.a_digit[1];
+    bh0 = sh.b_half[0];
+    bh1 = sh.b_half[1];
+    set_axis(0);
     ncomp = blockDim.x - issuer_threads(PP);
-    line = threadIdx.x & 127;
-    u = threadIdx.x >> 7;
+    rep = PP == 4 ? sh.rep : 1;
+    ln = kLines / rep;
+    line = (threadIdx.x & 127) % ln;
+    blk = (threadIdx.x & 127) / ln + rep * (threadIdx.x >> 7);
     warp = threadIdx.x >> 5;
     issuer = (int)threadIdx.x >= ncomp;
     phases = 0;
     ok = true;
-    both = both_halves(ND, kg);
     int *keys = reinterpret_cast<int *>(smem + lay.key_off);
-    for (int i = threadIdx.x; i < 2 * kLines; i += blockDim.x) keys[i] = 0;
+    for (int i = threadIdx.x; i < kKeySlots * kLines; i += blockDim.x) keys[i] = 0;
     if ((int)threadIdx.x == ncomp) {
 #pragma unroll
       for (int i = 0; i < 6; ++i)
@@ -314,26 +369,40 @@ template <int ND, int PP> struct Tile {
                      "r"(i <= kEmpty ? ncomp / 32 : 1)
                      : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      bulk_load(sm32(smem + lay.b_off), table, (b_resident(ND, kg) ? 2 : 1) * lay.b_half,
-                bar(kTable));
+      if (kRes) {
+        const unsigned b0 = 2 * bh0, b1 = sh.axes == 2 ? 2 * bh1 : 0;
+        expect_bytes(bar(kTable), b0 + b1);
+        bulk_load(sm32(smem + lay.b_off), table, b0, bar(kTable));
+        if (b1)
+          bulk_load(sm32(smem + lay.b_off) + b0,
+                    static_cast<const unsigned char *>(tab1) + sizeof(TcHead), b1, bar(kTable));
+      } else {
+        load_half(0);
+      }
     }
   }
+  // The table of one half into the (free) B memory.
+  __device__ __forceinline__ void load_half(int half) {
+    expect_bytes(bar(kTable), bh0);
+    bulk_load(sm32(smem + lay.b_off), table + half * bh0, bh0, bar(kTable));
+  }
   // The issuing warp's part: after the dependency wait (a CTA that holds TMEM
-  // must not wait for another one) TMEM, then `filters` filters.
-  __device__ __forceinline__ void run_issuer(int filters) {
-    if (ND == 7 && PP == 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
-    if (warp == ncomp / 32) tm_alloc(bar(6), tmem_cols(ND, kg));
+  // must not wait for another one) TMEM, then `filters` filters, the f-th along
+  // axis_of(f).
+  template <typename F> __device__ __forceinline__ void run_issuer(int filters, F &&axis_of) {
+    if (kSplit) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+    if (warp == ncomp / 32) tm_alloc(bar(6), cols);
     __syncthreads();
     read_tmem();
     if ((int)threadIdx.x == ncomp) {
-      const bool res = b_resident(ND, kg);
       unsigned tphase = 0;
-      for (int f = 0; f < filters; ++f)
+      for (int f = 0; f < filters; ++f) {
+        set_axis(axis_of(f));
         for (int half = 0; half < 2; ++half) {
           wait_for(kFull0 + half, f & 1);
-          if (!res || (f | half) == 0) wait_for(kTable, tphase++ & 1);
+          if (!kRes || (f | half) == 0) wait_for(kTable, tphase++ & 1);
           fence_after();
-          if (split_rows(ND, kg)) {
+          if (kSplit) {
             issue(half, 0);
             if (half == 1) {
               wait_for(kEmpty, f & 1);   // c's second round is read
@@ -343,18 +412,20 @@ template <int ND, int PP> struct Tile {
           } else {
             issue(half, half);
           }
-          if (!res && (half == 0 || f + 1 < filters)) {
-            // the other half's table, once this half's products are done
-            wait_for(kDone1, half);
-            if (ok) bulk_load(sm32(smem + lay.b_off), table + (half ^ 1) * lay.b_half, lay.b_half, bar(kTable));
+          if (!kRes && (half == 0 || f + 1 < filters)) {
+            // the next half's table, once this half's products are done
+            wait_for(kSplit ? kDone1 : kDone0 + half,
+                     kSplit ? half : f & 1);
+            if (ok) load_half(half ^ 1);
           }
         }
+      }
     }
     __syncwarp();
   }
   // The computing threads' other side of it.
   __device__ __forceinline__ void run_compute() {
-    if (ND == 7 && PP == 16) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
+    if (kSplit) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsCompute));
   }
   // Every computing thread, once its loads are issued.
   __device__ __forceinline__ void start() {
@@ -368,7 +439,7 @@ template <int ND, int PP> struct Tile {
   __device__ __forceinline__ void finish(unsigned *err) {
     if (!ok && err) atomicOr(err, 2u);
     __syncthreads();
-    if (warp == ncomp / 32) tm_free(tmem, tmem_cols(ND, kg));
+    if (warp == ncomp / 32) tm_free(tmem, cols);
   }
   // barrier of the computing warps
   __device__ __forceinline__ void sync() const {
@@ -391,77 +462,102 @@ template <int ND, int PP> struct Tile {
     __syncwarp();
   }
 
-  // digits of this thread's PP values (k = PP*u + i) into A operand `half`
+  // digits of this thread's PP values (k = PP*blk + i) into A operand `half`
   __device__ __forceinline__ void put_digits(const I (&v)[PP], int half) {
-    const int kb = 2 * kg;
-    unsigned char *base = smem + (both ? half * lay.a_half : 0) + line * 16;
+    unsigned char *base = smem + (both ? half * a_half : 0) + line * 16;
+    if (PP * blk < 16 * kg) {   // (planes: this axis may be shorter than the other one)
+      constexpr int G = PP < 8 ? PP : 8;
 #pragma unroll
-    for (int h = 0; h < PP / 8; ++h) {
-      uint32_t w[4][ND];
+      for (int h = 0; h < PP / G; ++h) {
+        uint32_t w[G / 2][ND];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) digit_words(v[8 * h + 2 * i], v[8 * h + 2 * i + 1], w[i]);
-      const int bk = PP / 8 * u + h;
-      unsigned char *dst = base + (dense_b(kg) ? bk : kb - 1 - bk) * (kLines * 16);
+        for (int i = 0; i < G / 2; ++i) digit_words(v[G * h + 2 * i], v[G * h + 2 * i + 1], w[i]);
+        const int k = PP * blk + G * h, bk = k / 8;
+        unsigned char *dst =
+            base + (dense_b(kg) ? bk : 2 * kg - 1 - bk) * (kLines * 16) + k % 8 * 2;
+        for (int c = 0; c < (PP == 4 ? rep : 1); ++c) {
 #pragma unroll
-      for (int d = 0; d < ND; ++d)
-        *reinterpret_cast<uint4 *>(dst + d * lay.a_digit) =
-            make_uint4(w[0][d], w[1][d], w[2][d], w[3][d]);
+          for (int d = 0; d < ND; ++d) {
+            if constexpr (G == 8)
+              *reinterpret_cast<uint4 *>(dst + d * a_digit) =
+                  make_uint4(w[0][d], w[1][d], w[2][d], w[3][d]);
+            else
+              *reinterpret_cast<uint2 *>(dst + d * a_digit) = make_uint2(w[0][d], w[1][d]);
+          }
+          dst += ln * 16;
+        }
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     signal(kFull0 + half);
   }
 
   // The digit products of half `half` (0: c, 1: d) into accumulator buffer
-  // `buf` (also the round, where rows are split).
+  // `buf` (also the round, where rows are split).  The block count is a constant
+  // in each copy: with it read at run time an instruction took about 170 cycles
+  // to issue among the computing warps, and 116 to run.
   __device__ __forceinline__ void issue(int half, int buf) {
     if (!ok) return;
-    const uint32_t kp = 16 * kg, gc = group_cols(ND, kg);
-    const uint32_t d0 = tmem + (dense_b(kg) ? buf * ND * gc : 0);
-    const uint32_t id0 = (1u << 4) | ((kLines >> 4) << 24);
-    const uint64_t a0 = smem_desc(sm32(smem) + (both ? half * lay.a_half : 0), kLines * 16, 128);
-    const uint32_t bh = sm32(smem + lay.b_off) + (b_resident(ND, kg) ? half * lay.b_half : 0);
-    if (dense_b(kg)) {
-      const bool split = split_rows(ND, kg);
-      const uint32_t blbo = ND * gc * 16 * (split ? 2 : 1);
-      const uint64_t b0 = smem_desc(bh + (split ? buf * ND * gc * 16 : 0), blbo, 128);
-#pragma unroll 1
-      for (int s = 0; s < kg; ++s) {
-        const uint64_t as = a0 + s * (2 * kLines * 16 >> 4), bs = b0 + s * (2 * blbo >> 4);
-#pragma unroll
-        for (int i = 0; i < ND; ++i) {
-          const uint32_t rows = (ND - i) * gc, n0 = rows < 256 ? rows : 256;
-          const uint64_t ai = as + (uint32_t)(i * lay.a_digit >> 4);
-          mma_f16(d0 + i * gc, ai, bs, id0 | ((n0 >> 3) << 17), (s | i) != 0);
-          if (rows > 256)
-            mma_f16(d0 + i * gc + 256, ai, bs + 256, id0 | ((rows - 256) >> 3 << 17), (s | i) != 0);
-        }
-      }
-    } else {
-      const int bd = (4 * kg - 1) * 128;
-      const uint64_t b0 = smem_desc(bh, 128, 128);
-#pragma unroll 1
-      for (int s = 0; s < kg; ++s) {
-        const uint64_t as = a0 + s * (2 * kLines * 16 >> 4), bs = b0 + s * (256 >> 4);
-#pragma unroll
-        for (int i = 0; i < ND; ++i)
-#pragma unroll
-          for (int j = 0; j < ND - i; ++j)
-            mma_f16(d0 + (i + j) * kp, as + (uint32_t)(i * lay.a_digit >> 4),
-                    bs + (uint32_t)(j * bd >> 4), id0 | ((kp >> 3) << 17), (s | i) != 0);
-      }
+    const uint32_t a0 = sm32(smem) + (both ? half * a_half : 0);
+    const uint32_t b0 = sm32(smem + lay.b_off) + b_at + (kRes ? half * b_half : 0);
+    switch (kg) {
+      case 1: issue_kg<1>(a0, b0, buf); break;
+      case 2: issue_kg<2>(a0, b0, buf); break;
+      case 3: issue_kg<3>(a0, b0, buf); break;
+      case 4: issue_kg<4>(a0, b0, buf); break;
+      default: issue_shared(a0, b0); break;
     }
     mma_commit(bar(kDone0 + buf));
   }
-
-  // eight outputs of this thread from accumulator buffer `buf`, starting at
-  // column `col` of each group (with 16 points per thread four at a time: 28
-  // accumulators in registers instead of 56, which spilled)
-  __device__ __forceinline__ void get8(int buf, int col, Acc (&y)[8]) {
-    constexpr int L = PP == 16 && ND == 7 ? 4 : 8;
-    const uint32_t gc = group_cols(ND, kg);
-    const uint32_t addr = tmem + ((uint32_t)(warp & 3) << 21) + (dense_b(kg) ? buf * ND * gc : 0) + col;
+  template <int KG> __device__ __forceinline__ void issue_kg(uint32_t a, uint32_t b, int buf) {
+    if constexpr ((KG <= 2) == (PP <= 8)) {
+      constexpr uint32_t gc = group_cols(ND, KG), id0 = (1u << 4) | ((kLines >> 4) << 24);
+      constexpr uint32_t blbo = ND * gc * 16 * (kSplit ? 2 : 1), adig = kLines * KG * 32;
+      const uint64_t ad = smem_desc(a, kLines * 16, 128);
+      const uint64_t bd = smem_desc(b + (kSplit ? buf * ND * gc * 16 : 0), blbo, 128);
+      const uint32_t d = tmem + buf * ND * gc;
 #pragma unroll
-    for (int h = 0; h < 8; h += L) {
+      for (int s = 0; s < KG; ++s)
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+          constexpr uint32_t kstep = 2 * kLines * 16 >> 4, bstep = 2 * blbo >> 4;
+          const uint32_t rows = (ND - i) * gc, n0 = rows < 256 ? rows : 256;
+          const uint64_t ai = ad + (s * kstep + (i * adig >> 4)), bs = bd + s * bstep;
+          mma_f16(d + i * gc, ai, bs, id0 | ((n0 >> 3) << 17), s + i != 0);
+          if (rows > 256)
+            mma_f16(d + i * gc + 256, ai, bs + 256, id0 | ((rows - 256) >> 3 << 17), s + i != 0);
+        }
+    }
+  }
+  // lines above 128 points: one instruction per digit pair (see the top)
+  __device__ __forceinline__ void issue_shared(uint32_t a, uint32_t b) {
+    const uint32_t kp = 16 * kg, bdig = (4 * kg - 1) * 128;
+    const uint32_t id = (1u << 4) | ((kLines >> 4) << 24) | ((kp >> 3) << 17);
+    const uint64_t a0 = smem_desc(a, kLines * 16, 128), b0 = smem_desc(b, 128, 128);
+#pragma unroll 1
+    for (int s = 0; s < kg; ++s) {
+      const uint64_t as = a0 + s * (2 * kLines * 16 >> 4), bs = b0 + s * (256 >> 4);
+#pragma unroll
+      for (int i = 0; i < ND; ++i)
+#pragma unroll
+        for (int j = 0; j < ND - i; ++j)
+          mma_f16(tmem + (i + j) * kp, as + (uint32_t)(i * a_digit >> 4),
+                  bs + (uint32_t)(j * bdig >> 4), id, (s | i) != 0);
+    }
+  }
+
+  // GO outputs of this thread from accumulator buffer `buf`, starting at column
+  // `col` of each group (with 16 points per thread four at a time: 28
+  // accumulators in registers instead of 56, which spilled)
+  static constexpr int GO = PP < 8 ? PP : 8;
+  __device__ __forceinline__ void get(int buf, int col, Acc (&y)[GO]) {
+    constexpr int L = PP == 16 ? 4 : GO;
+    const uint32_t gc = group_cols(ND, kg);
+    const uint32_t lane0 = tmem + ((uint32_t)(warp & 3) << 21);
+    uint32_t addr = lane0 + (dense_b(kg) ? buf * ND * gc : 0) + col;
+    if (col >= (int)gc) addr = lane0;   // (no such outputs: not used)
+#pragma unroll
+    for (int h = 0; h < GO; h += L) {
       float D[ND][L];
       __syncwarp();
 #pragma unroll
@@ -495,27 +591,27 @@ template <int ND, int PP> struct Tile {
       b[i] = a[i] - b[i];
       a[i] = s;
     }
-    Acc c[PP], y[8];
+    Acc c[PP], y[GO];
     put_digits(a, 0);
     if constexpr (ND == 7 && PP == 16) {
       // rounds c0 c1 d0 d1 (points 0-7, 8-15) in buffers 0 1 0 1: while one
       // buffer is read the other one's products run
       wait_done(0);
-      get8(0, 8 * u, y);
+      get(0, 8 * blk, y);
 #pragma unroll
       for (int i = 0; i < 8; ++i) c[i] = y[i];
       wait_done(1);          // c's products have read A
       put_digits(b, 1);
-      get8(1, 8 * u, y);
+      get(1, 8 * blk, y);
 #pragma unroll
       for (int i = 0; i < 8; ++i) c[8 + i] = y[i];
       signal(kEmpty);
       wait_done(0);
-      get8(0, 8 * u, y);
+      get(0, 8 * blk, y);
 #pragma unroll
       for (int i = 0; i < 8; ++i) out(i, c[i] + y[i], c[i] - y[i]);
       wait_done(1);
-      get8(1, 8 * u, y);
+      get(1, 8 * blk, y);
 #pragma unroll
       for (int i = 0; i < 8; ++i) out(8 + i, c[8 + i] + y[i], c[8 + i] - y[i]);
     } else {
@@ -523,31 +619,35 @@ template <int ND, int PP> struct Tile {
       waiting();
       wait_done(0);
 #pragma unroll
-      for (int h = 0; h < PP / 8; ++h) {
-        get8(0, PP * u + 8 * h, y);
+      for (int h = 0; h < PP / GO; ++h) {
+        get(0, PP * blk + GO * h, y);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) c[8 * h + i] = y[i];
+        for (int i = 0; i < GO; ++i) c[GO * h + i] = y[i];
       }
       if (!both) put_digits(b, 1);
       wait_done(1);
 #pragma unroll
-      for (int h = 0; h < PP / 8; ++h) {
-        get8(1, PP * u + 8 * h, y);
+      for (int h = 0; h < PP / GO; ++h) {
+        get(1, PP * blk + GO * h, y);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) out(8 * h + i, c[8 * h + i] + y[i], c[8 * h + i] - y[i]);
+        for (int i = 0; i < GO; ++i) out(GO * h + i, c[GO * h + i] + y[i], c[GO * h + i] - y[i]);
       }
     }
     fence_before();
     __syncwarp();
   }
 
-  // The largest of the line's keys over its threads (slot 0 or 1); a barrier of
-  // the computing warps.
+  // The largest of the line's keys over its threads; a barrier of the computing
+  // warps.
   __device__ __forceinline__ int line_key(int slot, int key) {
     int *k = reinterpret_cast<int *>(smem + lay.key_off) + slot * kLines + line;
     atomicMax(k, key);
     sync();
     return *k;
+  }
+  // A slot for reuse two filters on (every thread has read it; by blk == 0).
+  __device__ __forceinline__ void clear_key(int slot) {
+    reinterpret_cast<int *>(smem + lay.key_off)[slot * kLines + line] = 0;
   }
   // Whether any computing thread says so; a barrier of the computing warps.
   __device__ __forceinline__ bool any(bool v) {
