@@ -109,85 +109,192 @@ __global__ void k_sum_slots(const double *__restrict__ partial, int nblk, double
   if (threadIdx.x == 0) out[b] = v;
 }
 
-// adjoint seed at one contour point: out = ffl (cA phibarA + cB phibarB) * v
-// (v == null: 1), and the point's contour-weight terms of phi: S += c q q+
-template <typename R>
-__global__ void k_seed(R *__restrict__ out, const R *__restrict__ v, long long v_bs,
-                       const double *__restrict__ pbA, const double *__restrict__ pbB, double cA,
-                       double cB, const double *__restrict__ ffl, const R *__restrict__ q,
-                       long long q_bs, const R *__restrict__ qc, long long qc_bs,
-                       double *__restrict__ SA, double *__restrict__ SB, long long M) {
+// x in FP64.  A conversion costs the FP64 pipe as much as an FMA (16 cycles a
+// warp and SM), rebuilding the exponent in integers about a tenth of it.
+// (Denormal, infinite and NaN values go out of line: predicated in place the
+// conversion would take the pipe for every value.)
+__device__ __noinline__ double widen_rare(float x) { return (double)x; }
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(scft::dfloat x) { return (double)x; }
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return widen_rare(x);
+  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+// x rounded to the working precision, to nearest even (float: in integers, again)
+__device__ __noinline__ float narrow_rare(double x) { return (float)x; }
+__device__ __forceinline__ void narrow(double x, double &r) { r = x; }
+__device__ __forceinline__ void narrow(double x, scft::dfloat &r) { r = scft::dfloat(x); }
+__device__ __forceinline__ void narrow(double x, float &r) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t m = hi & 0x7fffffffu;
+  if (m - 0x38100000u >= 0x0fd00000u && (m | lo) != 0u) {   // below 2^-126, near the top, inf, nan
+    r = narrow_rare(x);
+    return;
+  }
+  // 23 bits and the rest below them; a carry moves into the exponent as it should
+  const uint32_t f = m ? ((m - 0x38000000u) << 3) | (lo >> 29) : 0u, rest = lo & 0x1fffffffu;
+  const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
+  r = __uint_as_float((hi & 0x80000000u) | (f + up));
+}
+// Two neighbouring points (grids have an even first axis).
+template <typename R> struct alignas(2 * sizeof(R)) Two {
+  R v[2];
+};
+template <typename R> __device__ __forceinline__ Two<R> two(const R *p) {
+  return *reinterpret_cast<const Two<R> *>(p);
+}
+template <typename R> __device__ __forceinline__ void put(R *p, const Two<R> &x) {
+  *reinterpret_cast<Two<R> *>(p) = x;
+}
+// One contour point's weights in the accumulators of sums of q q+ (S: the density
+// sums; G: the sums of the Q part, Simpson only) and in the adjoint seed.  How they
+// are used is decided on the host: comparisons of doubles take the FP64 pipe too.
+enum { kNone = 0, kOne = 1, kSome = 2 };   // weight 0 (arrays not touched), 1, other
+struct Point {
+  double c[2], g[2];          // blocks A, B
+  int cm[2], gm[2], in;       // in: the block that the point lies inside of, or -1
+  double *S[2], *G[2];
+  const double *pb[2];        // ffl * phibar
+};
+// the point's seed, (cA phibarA + cB phibarB) ffl
+__device__ __forceinline__ void seed_at(const Point &pt, long long o, double (&s)[2]) {
+  s[0] = s[1] = 0.0;
+#pragma unroll
+  for (int f = 0; f < 2; ++f)
+    if (pt.cm[f]) {
+      const Two<double> b = two(pt.pb[f] + o);
+      if (pt.cm[f] == kOne) {   // (within a block, where the other one's weight is 0)
+        s[0] = b.v[0];
+        s[1] = b.v[1];
+      } else {
+        s[0] += pt.c[f] * b.v[0];
+        s[1] += pt.c[f] * b.v[1];
+      }
+    }
+}
+// the accumulators of a point, read before anything is written; then with q q+ added
+struct Sums {
+  Two<double> s[2], g[2];
+};
+__device__ __forceinline__ void load_sums(const Point &pt, long long o, Sums &u) {
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    if (pt.cm[f]) u.s[f] = two(pt.S[f] + o);
+    if (pt.gm[f]) u.g[f] = two(pt.G[f] + o);
+  }
+}
+__device__ __forceinline__ void add_sum(double *acc, Two<double> &a, int mode, double c,
+                                        const double (&x)[2], const double (&y)[2]) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (mode == kOne) a.v[k] = fma(x[k], y[k], a.v[k]);
+    else a.v[k] += c * (x[k] * y[k]);
+  }
+  put(acc, a);
+}
+__device__ __forceinline__ void store_sums(const Point &pt, long long o, Sums &u,
+                                           const double (&x)[2], const double (&y)[2]) {
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    if (pt.cm[f]) add_sum(pt.S[f] + o, u.s[f], pt.cm[f], pt.c[f], x, y);
+    if (pt.gm[f]) add_sum(pt.G[f] + o, u.g[f], pt.gm[f], pt.g[f], x, y);
+  }
+}
+
+// out = c[b] * in
+__global__ void k_scale(double *__restrict__ out, const double *__restrict__ in,
+                        const double *__restrict__ c, long long M) {
   const long long b = blockIdx.y;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M;
-       i += (long long)gridDim.x * blockDim.x) {
+       i += (long long)gridDim.x * blockDim.x)
+    out[b * M + i] = c[b] * in[b * M + i];
+}
+
+// The end point of a chain: the adjoint seed there; with q also its sums (q+ = 1).
+template <typename R>
+__global__ void k_seed(Point pt, R *__restrict__ out, const R *__restrict__ q, long long q_bs,
+                       long long M) {
+  const long long b = blockIdx.y;
+  for (long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < M;
+       i += 2 * (long long)gridDim.x * blockDim.x) {
     const long long o = b * M + i;
-    const double vv = v ? (double)v[b * v_bs + i] : 1.0;
-    out[o] = (R)(ffl[b] * (cA * pbA[o] + cB * pbB[o]) * vv);
-    if (SA) {
-      const double qq = (double)q[b * q_bs + i] * (qc ? (double)qc[b * qc_bs + i] : 1.0);
-      SA[o] += cA * qq;
-      SB[o] += cB * qq;
+    double s[2];
+    seed_at(pt, o, s);
+    Two<R> r;
+    r.v[0] = (R)s[0];
+    r.v[1] = (R)s[1];
+    put(out + o, r);
+    if (q) {
+      Sums u;
+      load_sums(pt, o, u);
+      const Two<R> x = two(q + b * q_bs + i);
+      const double xx[2] = {widen(x.v[0]), widen(x.v[1])}, one[2] = {1.0, 1.0};
+      store_sums(pt, o, u, xx, one);
     }
   }
 }
 
-// One step of the reverse sweep over the q chain, s -> s-1:
-//   wbar += -ds/2 (lam(s) q(s) + (A lam(s)) q(s-1))     (field of step s)
-//   G    += q+(s) q(s) + q+(s-1) q(s-1)                (Q part, scaled later)
-//   S    += c(s-1) q(s-1) q+(s-1)                        (phi)
-//   lam(s-1) = A lam(s) + ffl (cA phibarA + cB phibarB)(s-1) q+(s-1)
-template <typename R>
-__global__ void k_adj_q(const R *__restrict__ p, const R *__restrict__ lam,
-                        const R *__restrict__ qs, const R *__restrict__ qsm1, long long seg_bs,
-                        const R *__restrict__ qcs, const R *__restrict__ qcsm1,
-                        const double *__restrict__ pbA, const double *__restrict__ pbB,
-                        double cA, double cB, const double *__restrict__ ffl, double hds,
-                        double *__restrict__ wbar, double *__restrict__ G,
-                        double *__restrict__ SA, double *__restrict__ SB, R *__restrict__ lam_out,
-                        long long M) {
+// One step of a reverse sweep.  Over the q chain, s -> s-1 (SUMS; a = lam, x1 = q(s),
+// x0 = q(s-1), y = q+(s-1)), with the sums at s-1; over the q+ chain, s-1 -> s
+// (a = mu, x1 = q+(s-1), x0 = q+(s), y = q(s)):
+//   wbar += a x1 + (A a) x0                        (field of step s; the caller's -ds/2)
+//   a_out = A a + ffl (cA phibarA + cB phibarB) y    at the point reached
+// FP64 pipe and memory latency bound it: with the sums of the Q part taken from the
+// density sums (trapezoid: one is twice the other), only the block's own arrays
+// touched, the constant factors outside and conversions in integers it has 4 FP64
+// operations a point instead of 19 and moves 64 bytes instead of 108, all loads first
+// (64^3: 8.4 us with 8 operations, 12.6 with 16).
+// INNER: the point lies inside block pt.in, with weight 1 (trapezoid).
+template <typename R, bool SUMS, bool INNER>
+__global__ void __launch_bounds__(kT)
+    k_sweep(Point pt, const R *__restrict__ p, const R *__restrict__ a, const R *__restrict__ x1_,
+            long long x1_bs, const R *__restrict__ x0_, long long x0_bs, const R *__restrict__ y_,
+            double *__restrict__ wbar, R *__restrict__ a_out, long long M) {
+  scft::pdl_wait();
+  scft::pdl_release();
   const long long b = blockIdx.y;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long o = b * M + i, so = b * seg_bs + i;
-    const double l = (double)lam[o], pp = (double)p[o], q1 = (double)qs[so],
-                 q0 = (double)qsm1[so];
-    const double c1 = (double)qcs[o], c0 = (double)qcsm1[o];
-    wbar[o] -= hds * (l * q1 + pp * q0);
-    G[o] += c1 * q1 + c0 * q0;
-    const double qq = q0 * c0;
-    SA[o] += cA * qq;
-    SB[o] += cB * qq;
-    lam_out[o] = (R)(pp + ffl[b] * (cA * pbA[o] + cB * pbB[o]) * c0);
+  for (long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < M;
+       i += 2 * (long long)gridDim.x * blockDim.x) {
+    const long long o = b * M + i;
+    const Two<R> tp = two(p + o), ta = two(a + o), t1 = two(x1_ + b * x1_bs + i),
+                 t0 = two(x0_ + b * x0_bs + i), ty = two(y_ + o);
+    Two<double> w = two(wbar + o);
+    Sums u;
+    double s[2], x0[2], y[2];
+    if constexpr (INNER) {
+      if (SUMS) u.s[0] = two(pt.S[pt.in] + o);
+      const Two<double> sd = two(pt.pb[pt.in] + o);
+      s[0] = sd.v[0];
+      s[1] = sd.v[1];
+    } else {
+      if (SUMS) load_sums(pt, o, u);
+      seed_at(pt, o, s);
+    }
+    Two<R> out;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double pp = widen(tp.v[k]);
+      x0[k] = widen(t0.v[k]);
+      y[k] = widen(ty.v[k]);
+      w.v[k] = fma(pp, x0[k], fma(widen(ta.v[k]), widen(t1.v[k]), w.v[k]));
+      narrow(fma(s[k], y[k], pp), out.v[k]);
+    }
+    put(wbar + o, w);
+    put(a_out + o, out);
+    if constexpr (SUMS && INNER) add_sum(pt.S[pt.in] + o, u.s[0], kOne, 1.0, x0, y);
+    else if constexpr (SUMS) store_sums(pt, o, u, x0, y);
   }
 }
 
-// One step of the forward sweep over the q+ chain, s-1 -> s:
-//   wbar += -ds/2 (mu(s-1) q+(s-1) + (A mu(s-1)) q+(s))
-//   mu(s) = A mu(s-1) + ffl (cA phibarA + cB phibarB)(s) q(s)
-template <typename R>
-__global__ void k_adj_qc(const R *__restrict__ p, const R *__restrict__ mu,
-                         const R *__restrict__ qcsm1, const R *__restrict__ qcs, long long seg_bs,
-                         const R *__restrict__ qs, const double *__restrict__ pbA,
-                         const double *__restrict__ pbB, double cA, double cB,
-                         const double *__restrict__ ffl, double hds, double *__restrict__ wbar,
-                         R *__restrict__ mu_out, long long M) {
-  const long long b = blockIdx.y;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long o = b * M + i, so = b * seg_bs + i;
-    const double m = (double)mu[o], pp = (double)p[o];
-    wbar[o] -= hds * (m * (double)qcsm1[so] + pp * (double)qcs[so]);
-    mu_out[o] = (R)(pp + ffl[b] * (cA * pbA[o] + cB * pbB[o]) * (double)qs[o]);
-  }
-}
-
-// wbar += coef[b] * G
-__global__ void k_axpy_inst(double *__restrict__ wbar, const double *__restrict__ G,
-                            const double *__restrict__ coef, long long M) {
+// wbar = -hds wbar + coef[b] * G
+__global__ void k_finish(double *__restrict__ wbar, const double *__restrict__ G, double hds,
+                         const double *__restrict__ coef, long long M) {
   const long long b = blockIdx.y;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < M;
        i += (long long)gridDim.x * blockDim.x)
-    wbar[b * M + i] += coef[b] * G[b * M + i];
+    wbar[b * M + i] = coef[b] * G[b * M + i] - hds * wbar[b * M + i];
 }
 
 
@@ -287,13 +394,14 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   R *ck1 = static_cast<R *>(A.ck1), *ck2 = static_cast<R *>(A.ck2);
   R *seg = static_cast<R *>(A.seg);
   R *W[2] = {static_cast<R *>(A.v[0]), static_cast<R *>(A.v[1])};
-  R *va = static_cast<R *>(A.v[2]), *vb = static_cast<R *>(A.v[3]);    // marching pair
-  R *x = static_cast<R *>(A.v[4]), *y = static_cast<R *>(A.v[5]);      // on-the-fly chain
+  R *va = static_cast<R *>(A.v[2]), *vb = static_cast<R *>(A.v[3]);    // marching pairs
+  R *x = static_cast<R *>(A.v[4]), *y = static_cast<R *>(A.v[5]);
   R *l0 = static_cast<R *>(A.v[6]), *l1 = static_cast<R *>(A.v[7]);    // adjoint pair
   R *p = static_cast<R *>(A.v[8]), *t = static_cast<R *>(A.v[9]);
   R *s0 = static_cast<R *>(A.v[10]), *s1 = static_cast<R *>(A.v[11]);
+  void *scratch[scft::kStepSet] = {s0, s1, t};
   double *wa_avg = A.d[0], *wbar[2] = {A.d[1], A.d[2]}, *G[2] = {A.d[3], A.d[4]};
-  double *SA = A.d[5], *SB = A.d[6], *pbA = A.d[7], *pbB = A.d[8];
+  double *S[2] = {A.d[5], A.d[6]}, *pb[2] = {A.d[7], A.d[8]}, *pbs[2] = {A.d[0], A.d[9]};
   double *acc = A.acc;
   double *Q = A.small, *ffl = A.small + B, *sum = A.small + 2 * B, *coef = A.small + 3 * B;
   double *sums = A.small + 8 * B;   // [kinds][B]
@@ -309,43 +417,90 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   CKL(scft::launch_minus_average(wa_avg, sum, M, B, st));
   CKL(scft::launch_boltzmann<R>(wa_avg, W[0], M * B, hds, st));
   CKL(scft::launch_boltzmann<R>(ctx->wb, W[1], M * B, hds, st));
-  if (h_pbA) CK(cudaMemcpyAsync(pbA, h_pbA, dbytes, cudaMemcpyHostToDevice, st));
-  else CK(cudaMemsetAsync(pbA, 0, dbytes, st));
-  if (h_pbB) CK(cudaMemcpyAsync(pbB, h_pbB, dbytes, cudaMemcpyHostToDevice, st));
-  else CK(cudaMemsetAsync(pbB, 0, dbytes, st));
-  for (double *z : {wbar[0], wbar[1], G[0], G[1], SA, SB}) CK(cudaMemsetAsync(z, 0, dbytes, st));
+  const double *h_pb[2] = {h_pbA, h_pbB};
+  for (int f = 0; f < 2; ++f) {
+    if (h_pb[f]) CK(cudaMemcpyAsync(pb[f], h_pb[f], dbytes, cudaMemcpyHostToDevice, st));
+    else CK(cudaMemsetAsync(pb[f], 0, dbytes, st));
+  }
+  for (double *z : {wbar[0], wbar[1], G[0], G[1], S[0], S[1]}) CK(cudaMemsetAsync(z, 0, dbytes, st));
   CK(cudaMemsetAsync(acc, 0, sizeof(double) * kAccKinds * B * nblk, st));
 
-  auto step = [&](const R *in, long long in_bs, R *out, long long out_bs, int f) {
-    return scft_internal_filter(ctx, in, in_bs, out, out_bs, W[f], W[f], M, B, -1, s0, s1, st);
+  // Steps that do not depend on each other run as one set of launches: the two
+  // chains' forward marches, and in a sweep the companion chain, the adjoint and
+  // the next segment's recomputation: 3 N steps in sequence instead of 8 N, with
+  // two launches each where the x and y passes share one.  What bounds it is the
+  // launches in sequence (about 4 us each at 64^3).  N = 200 steps, ms a call:
+  // FP32 32^3 12.0 -> 5.0, 64^3 16.9 -> 7.7, 128 x 128 x 64 41.5 -> 17.8; FP64 64^3
+  // 118 -> 24.
+  StepIO io[scft::kStepSet];
+  int nio = 0;
+  auto add = [&](const R *in, long long in_bs, R *out, long long out_bs, int f) {
+    io[nio++] = StepIO{in, W[f], out, in_bs, out_bs};
   };
-  const dim3 eg(grid_for(M), B);
+  auto run = [&]() {
+    const int n = nio;
+    nio = 0;
+    return scft_internal_steps(ctx, io, n, M, B, scratch, st);
+  };
+  const dim3 eg(grid_for(M), B), eg2(grid_for(M / 2), B);
 
-  // ---- forward: checkpoints of both chains every K steps
+  // ---- segments between checkpoints, in the order the sweeps take them.  Of a
+  // segment's slices 0 .. len the first and the last are checkpoints; the others
+  // lie in seg, upwards from its first slot or downwards from its last one, in
+  // turn: the next segment grows into the slots the present one has left behind.
+  struct Segm { const R *ck; long long ckbs; int chain, j, lo, len; };
+  std::vector<Segm> segs;
+  for (int c = 0; c < 2; ++c) {
+    const std::vector<int> &pos = c == 0 ? A.pos1 : A.pos2;
+    for (int j = (int)pos.size() - 2; j >= 0; --j)
+      segs.push_back(Segm{c == 0 ? ck1 : ck2, c == 0 ? ckbs1 : ckbs2, c, j, pos[j],
+                          pos[j + 1] - pos[j]});
+  }
+  auto slice = [&](size_t i, int k, long long *bs) -> R * {
+    const Segm &g = segs[i];
+    if (k == 0 || k == g.len) {
+      *bs = g.ckbs;
+      return const_cast<R *>(g.ck) + (long long)(g.j + (k ? 1 : 0)) * M;
+    }
+    *bs = segbs;
+    return seg + (long long)(i & 1 ? K + 1 - k : k - 1) * M;
+  };
+  // the step of a chain from its distance u-1 to u: q(u-1) -> q(u), q+(s) -> q+(s-1)
+  auto step_of = [&](int chain, int u) { return chain == 0 ? u : N - u + 1; };
+  auto recompute = [&](size_t i, int k) {   // slice k of segment i
+    long long ibs, obs;
+    const R *in = slice(i, k - 1, &ibs);
+    R *out = slice(i, k, &obs);
+    add(in, ibs, out, obs, field_of_step(ctx, step_of(segs[i].chain, segs[i].lo + k)));
+  };
+
+  // ---- forward: checkpoints of both chains every K steps; the q chain's last
+  // segment straight into its slots
   CKL(scft::launch_fill<R>(ck1, M, R(1), ckbs1, B, st));
   CKL(scft::launch_fill<R>(ck2, M, R(1), ckbs2, B, st));
-  for (int chain = 0; chain < 2; ++chain) {
-    R *ck = chain == 0 ? ck1 : ck2;
-    const long long ckbs = chain == 0 ? ckbs1 : ckbs2;
-    const std::vector<int> &pos = chain == 0 ? A.pos1 : A.pos2;
-    const R *cur = ck;
-    long long cur_bs = ckbs;
+  {
+    const R *cur[2] = {ck1, ck2};
+    long long cur_bs[2] = {ckbs1, ckbs2};
+    R *ck[2] = {ck1, ck2}, *pair[2][2] = {{va, vb}, {x, y}};
+    const long long ckbs[2] = {ckbs1, ckbs2};
     size_t j = 1;
     for (int u = 1; u <= N; ++u) {
-      const int s = chain == 0 ? u : N - u + 1;   // step applied: q(u-1)->q(u) / q+(s)->q+(s-1)
-      R *dst;
-      long long dst_bs;
-      if (j < pos.size() && pos[j] == u) {
-        dst = ck + (long long)j * M;
-        dst_bs = ckbs;
-        ++j;
-      } else {
-        dst = (cur == va) ? vb : va;
-        dst_bs = M;
+      const bool at = j < A.pos1.size() && A.pos1[j] == u;   // (pos1 and pos2 are the same)
+      for (int c = 0; c < 2; ++c) {
+        long long bs = M;
+        R *dst = cur[c] == pair[c][0] ? pair[c][1] : pair[c][0];
+        if (at) {
+          dst = ck[c] + (long long)j * M;
+          bs = ckbs[c];
+        } else if (c == 0 && u > segs[0].lo) {
+          dst = slice(0, u - segs[0].lo, &bs);
+        }
+        add(cur[c], cur_bs[c], dst, bs, field_of_step(ctx, step_of(c, u)));
+        cur[c] = dst;
+        cur_bs[c] = bs;
       }
-      RC(step(cur, cur_bs, dst, dst_bs, field_of_step(ctx, s)));
-      cur = dst;
-      cur_bs = dst_bs;
+      RC(run());
+      if (at) ++j;
     }
   }
   // Q = <q(N)>, ffl = ds/Q (cal_ql and getConc's host lines, cuda_scft.cu:118-125)
@@ -353,6 +508,11 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   CKL(scft::launch_partial_sum<R>(qN, ckbs1, M, B, ctx->partial, nblk, st));
   CKL(scft::launch_finalize_sum(ctx->partial, nblk, B, 1.0, sum, st));
   CKL(scft::launch_q_ffl(sum, M, ds, B, Q, ffl, st));
+  for (int f = 0; f < 2; ++f) {
+    k_scale<<<eg, kT, 0, st>>>(pbs[f], pb[f], ffl, M);
+    ++ctx->launches;
+  }
+  CK(cudaGetLastError());
 
   auto dot = [&](const R *a, long long a_bs, const R *c1, long long c1_bs, const R *c2,
                  long long c2_bs, double *acc1, double *acc2) {
@@ -361,91 +521,78 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
     ++ctx->launches;
     return cudaGetLastError();
   };
-
-  // ---- reverse sweep of the q chain (s = N .. 1), q+ marched alongside
-  {
-    double cA, cB;
-    weights(ctx, N, &cA, &cB);
-    k_seed<R><<<eg, kT, 0, st>>>(l0, nullptr, 0, pbA, pbB, cA, cB, ffl, qN, ckbs1, nullptr, 0,
-                                 SA, SB, M);
-    ++ctx->launches;
-    CK(cudaGetLastError());
-    CKL(scft::launch_fill<R>(x, M * B, R(1), 0, 1, st));
-    R *lam = l0, *lam_n = l1, *qc = x, *qc_n = y;
-    for (int j = A.nck1 - 2; j >= 0; --j) {
-      const int s_lo = A.pos1[j], len = A.pos1[j + 1] - s_lo;
-      CKL(scft::launch_copy_slice<R>(seg, segbs, ck1 + (long long)j * M, ckbs1, M, B, st));
-      for (int k = 1; k <= len; ++k)
-        RC(step(seg + (long long)(k - 1) * M, segbs, seg + (long long)k * M, segbs,
-                field_of_step(ctx, s_lo + k)));
-      for (int k = len; k >= 1; --k) {
-        const int s = s_lo + k, f = field_of_step(ctx, s);
-        const R *q1 = seg + (long long)k * M, *q0 = seg + (long long)(k - 1) * M;
-        RC(step(qc, M, qc_n, M, f));          // q+(s-1)
-        RC(step(lam, M, p, M, f));            // A lam(s)
-        if (want_L) {
-          for (int pi = 0; pi < np; ++pi) {
-            RC(scft_internal_filter(ctx, q0, segbs, t, M, W[f], W[f], M, B, pi, s0, s1, st));
-            CK(dot(t, M, lam, M, qc, M, accp(ACC_L1 + pi), accp(ACC_Q + pi)));
-          }
-          if (has_unit) CK(dot(q1, segbs, lam, M, qc, M, accp(ACC_U1), accp(ACC_UQ)));
-        }
-        double cA, cB;
-        weights(ctx, s - 1, &cA, &cB);
-        k_adj_q<R><<<eg, kT, 0, st>>>(p, lam, q1, q0, segbs, qc, qc_n, pbA, pbB, cA, cB, ffl,
-                                      hds, wbar[f], G[f], SA, SB, lam_n, M);
-        ++ctx->launches;
-        CK(cudaGetLastError());
-        std::swap(lam, lam_n);
-        std::swap(qc, qc_n);
-      }
+  // The sum over a block's steps of q+(s) q(s) + q+(s-1) q(s-1) is twice its
+  // trapezoid sum: S itself, or G beside Simpson's S.
+  const bool simpson = (ctx->p.flags & SCFT_FLAG_SIMPSON) != 0;
+  auto point = [&](int s, bool sums) {
+    Point pt;
+    weights(ctx, s, &pt.c[0], &pt.c[1]);
+    const int n[2] = {ctx->NsA, ctx->dNsB};
+    pt.in = -1;
+    for (int f = 0; f < 2; ++f) {
+      const int at = f == 0 ? s : s - ctx->NsA;
+      pt.g[f] = sums && simpson ? scft::contour_weight(at, n[f], false) : 0.0;
+      auto mode = [](double w) { return w == 0.0 ? kNone : (w == 1.0 ? kOne : kSome); };
+      pt.cm[f] = mode(pt.c[f]);
+      pt.gm[f] = mode(pt.g[f]);
+      pt.S[f] = S[f];
+      pt.G[f] = G[f];
+      pt.pb[f] = pbs[f];
+      if (!simpson && pt.cm[f] == kOne) pt.in = f;   // (the other block's weight is 0)
     }
-  }
-  // ---- forward sweep of the q+ chain (s = 1 .. N), q marched alongside
-  {
-    double cA, cB;
-    weights(ctx, 0, &cA, &cB);
-    k_seed<R><<<eg, kT, 0, st>>>(l0, nullptr, 0, pbA, pbB, cA, cB, ffl, nullptr, 0, nullptr, 0,
-                                 nullptr, nullptr, M);
-    ++ctx->launches;
-    CK(cudaGetLastError());
-    CKL(scft::launch_fill<R>(x, M * B, R(1), 0, 1, st));
-    R *mu = l0, *mu_n = l1, *qv = x, *qv_n = y;
-    for (int j = A.nck2 - 2; j >= 0; --j) {
-      // segment of q+ at distances t in [pos2[j], pos2[j+1]] from the end
-      const int t_lo = A.pos2[j], len = A.pos2[j + 1] - t_lo;
-      CKL(scft::launch_copy_slice<R>(seg, segbs, ck2 + (long long)j * M, ckbs2, M, B, st));
-      for (int k = 1; k <= len; ++k)
-        RC(step(seg + (long long)(k - 1) * M, segbs, seg + (long long)k * M, segbs,
-                field_of_step(ctx, N - (t_lo + k) + 1)));
-      for (int k = len; k >= 1; --k) {
-        const int s = N - (t_lo + k) + 1, f = field_of_step(ctx, s);
-        const R *qc0 = seg + (long long)k * M;         // q+(s-1)
-        const R *qc1 = seg + (long long)(k - 1) * M;   // q+(s)
-        RC(step(qv, M, qv_n, M, f));          // q(s)
-        RC(step(mu, M, p, M, f));             // A mu(s-1)
-        if (want_L) {
-          for (int pi = 0; pi < np; ++pi) {
-            RC(scft_internal_filter(ctx, qc1, segbs, t, M, W[f], W[f], M, B, pi, s0, s1, st));
-            CK(dot(t, M, mu, M, nullptr, 0, accp(ACC_L2 + pi), nullptr));
-          }
-          if (has_unit) CK(dot(qc0, segbs, mu, M, nullptr, 0, accp(ACC_U2), nullptr));
+    return pt;
+  };
+
+  // ---- the sweeps: the q chain's in reverse (s = N .. 1, q+ marched alongside),
+  // then the q+ chain's (s = 1 .. N, q marched alongside)
+  R *a = l0, *a_n = l1, *co = x, *co_n = y;   // adjoint, companion chain
+  for (size_t i = 0; i < segs.size(); ++i) {
+    const Segm &g = segs[i];
+    const bool q_chain = g.chain == 0, more = i + 1 < segs.size();
+    if (i == 0 || segs[i - 1].chain != g.chain) {
+      k_seed<R><<<eg2, kT, 0, st>>>(point(q_chain ? N : 0, q_chain), a, q_chain ? qN : nullptr,
+                                    ckbs1, M);
+      ++ctx->launches;
+      CK(cudaGetLastError());
+      CKL(scft::launch_fill<R>(co, M * B, R(1), 0, 1, st));
+    }
+    for (int k = g.len; k >= 1; --k) {
+      const int s = step_of(g.chain, g.lo + k), f = field_of_step(ctx, s);
+      long long bs1, bs0;
+      const R *x1 = slice(i, k, &bs1), *x0 = slice(i, k - 1, &bs0);
+      add(co, M, co_n, M, f);                  // q+(s-1) / q(s)
+      add(a, M, p, M, f);                      // A a
+      const int rec = g.len - k + 1;
+      if (more && rec < segs[i + 1].len) recompute(i + 1, rec);
+      RC(run());
+      if (want_L) {
+        const int L = q_chain ? ACC_L1 : ACC_L2;
+        for (int pi = 0; pi < np; ++pi) {
+          RC(scft_internal_filter(ctx, x0, bs0, t, M, W[f], W[f], M, B, pi, s0, s1, st));
+          CK(dot(t, M, a, M, q_chain ? co : nullptr, M, accp(L + pi),
+                 q_chain ? accp(ACC_Q + pi) : nullptr));
         }
-        double cA, cB;
-        weights(ctx, s, &cA, &cB);
-        k_adj_qc<R><<<eg, kT, 0, st>>>(p, mu, qc0, qc1, segbs, qv_n, pbA, pbB, cA, cB, ffl, hds,
-                                       wbar[f], mu_n, M);
-        ++ctx->launches;
-        CK(cudaGetLastError());
-        std::swap(mu, mu_n);
-        std::swap(qv, qv_n);
+        if (has_unit)
+          CK(dot(x1, bs1, a, M, q_chain ? co : nullptr, M, accp(q_chain ? ACC_U1 : ACC_U2),
+                 q_chain ? accp(ACC_UQ) : nullptr));
       }
+      const Point pt = point(q_chain ? s - 1 : s, q_chain);
+      auto k_step = pt.in >= 0 ? (q_chain ? k_sweep<R, true, true> : k_sweep<R, false, true>)
+                               : (q_chain ? k_sweep<R, true, false> : k_sweep<R, false, false>);
+      CKL(scft::launch_pdl(k_step, eg2, dim3(kT), 0, st, pt,
+                           p, a, x1, bs1, x0, bs0, co_n, wbar[f], a_n, M));
+      std::swap(a, a_n);
+      std::swap(co, co_n);
+    }
+    for (int rec = g.len + 1; more && rec < segs[i + 1].len; ++rec) {
+      recompute(i + 1, rec);
+      RC(run());
     }
   }
   // ---- the Q part: Qbar_tot = Qbar - fflbar ds / Q^2, fflbar = <phibar, S>
-  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pbA, M, SA, M, nullptr, 0, M, 1,
+  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[0], M, S[0], M, nullptr, 0, M, 1,
                                                           accp(ACC_FFL), nullptr);
-  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pbB, M, SB, M, nullptr, 0, M, 1,
+  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[1], M, S[1], M, nullptr, 0, M, 1,
                                                           accp(ACC_FFL), nullptr);
   ctx->launches += 2;
   CK(cudaGetLastError());
@@ -460,11 +607,12 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   for (int b = 0; b < B; ++b) {
     const double fflbar = sums_h[(size_t)ACC_FFL * B + b];
     qtot[b] = (h_Qbar ? h_Qbar[b] : 0.0) - fflbar * ds / (hQ[b] * hQ[b]);
-    cf[b] = -hds * qtot[b] / (double)M;
+    cf[b] = -ds * qtot[b] / (double)M;   // (2 S: see point)
   }
   CK(cudaMemcpyAsync(coef, cf.data(), 8 * B, cudaMemcpyHostToDevice, st));
   for (int f = 0; f < 2; ++f) {
-    k_axpy_inst<<<eg, kT, 0, st>>>(wbar[f], G[f], coef, M);
+    if ((f == 0 ? ctx->NsA : ctx->dNsB) == 0) continue;
+    k_finish<<<eg, kT, 0, st>>>(wbar[f], simpson ? G[f] : S[f], hds, coef, M);
     ++ctx->launches;
     CK(cudaGetLastError());
   }

@@ -158,11 +158,11 @@ bool axis_ok(int n, bool allow_one) {
 
 // One pass over a set of propagators: a single launch of the register
 // kernel, or one generic launch per set member.
-template <typename R>
-int launch_set(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R> &ps, cudaStream_t st) {
+template <typename R, int NS>
+int launch_set(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R, NS> &ps, cudaStream_t st) {
   if constexpr (!std::is_same<R, scft::dfloat>::value) {
     if (ap.tc) {
-      scft::PassSet<R> p = ps;
+      auto p = scft::with_sets<scft::kStepSet>(ps);
       p.err = ctx->dev_err;
       CKL(scft::launch_tc(ap, p, false, st));
       return SCFT_OK;
@@ -189,7 +189,7 @@ template <typename R>
 int launch_pair(scft_ctx *ctx, const AxisPlan &ap, const scft::PassSet<R> &ps, cudaStream_t st) {
   if constexpr (std::is_same<R, float>::value) {
     if (ap.tc) {
-      scft::PassSet<R> p = ps;
+      auto p = scft::with_sets<scft::kStepSet>(ps);
       p.err = ctx->dev_err;
       CKL(scft::launch_tc(ap, p, true, st));
       return SCFT_OK;
@@ -235,7 +235,7 @@ template <typename R>
 int run_chains(scft_ctx *ctx, const Seg *const *chains, const int *nseg, int nchain,
                cudaStream_t st, int chain_base) {
   const long long M = ctx->M;
-  int total[scft::kMaxSet] = {0, 0};
+  int total[scft::kMaxSet] = {};
   int maxT = 0;
   for (int c = 0; c < nchain; ++c) {
     for (int k = 0; k < nseg[c]; ++k) total[c] += chains[c][k].ns;
@@ -297,7 +297,7 @@ int run_chains(scft_ctx *ctx, const Seg *const *chains, const int *nseg, int nch
           continue;
         }
       }
-      rc = launch_set<R>(ctx, ctx->passes[xy ? pi + 1 : pi], p, st);
+      rc = launch_set(ctx, ctx->passes[xy ? pi + 1 : pi], p, st);
       if (rc) return rc;
     }
   }
@@ -360,12 +360,12 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
       if (np < 3) return (int)SCFT_OK;
       reset(tmp[cur], M, tmp[cur ^ 1], M);
       cur ^= 1;
-      return launch_set<R>(ctx, ctx->passes[1], ps, st);
+      return launch_set(ctx, ctx->passes[1], ps, st);
     };
     // step 1: x with the pre factor
     reset(slice(0), qbs, tmp[cur], M);
     ps.pre[0] = W;
-    if ((rc = launch_set<R>(ctx, ctx->passes[0], ps, st))) return rc;
+    if ((rc = launch_set(ctx, ctx->passes[0], ps, st))) return rc;
     if ((rc = middle())) return rc;
     // FP32 planes: an x pair takes the middle passes before and after it along
     const bool planes = std::is_same<R, float>::value && np == 3 && ctx->tc_planes &&
@@ -381,7 +381,8 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
       if constexpr (std::is_same<R, float>::value) {
         if (planes && x) {
           ps.err = ctx->dev_err;
-          CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], ps, st));
+          CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1],
+                                  scft::with_sets<scft::kStepSet>(ps), st));
           continue;
         }
       }
@@ -391,7 +392,7 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
     if (planes && !(sg.ns & 1) && (rc = middle())) return rc;
     reset(tmp[cur], M, slice(sg.ns), qbs);
     ps.post[0] = W;
-    if ((rc = launch_set<R>(ctx, ctx->passes[(sg.ns & 1) ? np - 1 : 0], ps, st))) return rc;
+    if ((rc = launch_set(ctx, ctx->passes[(sg.ns & 1) ? np - 1 : 0], ps, st))) return rc;
   }
   return SCFT_OK;
 }
@@ -1041,12 +1042,55 @@ int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long o
       ap.gain = ctx->dgain_pass[pi];
       ap.tc = ctx->dtc_pass[pi];
     }
-    int rc = launch_set<R>(ctx, ap, p, st);
+    int rc = launch_set(ctx, ap, p, st);
     if (rc) return rc;
   }
   return SCFT_OK;
 }
 }  // namespace
+
+// One split step of up to kStepSet chains side by side, each with its own factor:
+// the same passes, with the x and y passes on whole planes where the march has
+// them so.  scratch: one [nb][M] buffer per chain (`out` is the other one).
+int scft_internal_steps(scft_ctx *ctx, const StepIO *io, int n, long long w_bs, int nb,
+                        void *const *scratch, cudaStream_t st) {
+  return with_real(ctx, [&](auto r) {
+    using R = decltype(r);
+    const int all = (int)ctx->passes.size();
+    const bool fp32 = std::is_same<R, float>::value;
+    const bool planes = fp32 && all == 3 && ctx->tc_planes && ctx->passes[0].tc && ctx->passes[1].tc;
+    const bool xy = planes || (fp32 && ctx->fuse_xy);
+    const int np = all - (xy ? 1 : 0);
+    for (int pi = 0; pi < np; ++pi) {
+      scft::PassSet<R, scft::kStepSet> p = {};
+      p.nset = n;
+      p.batch = nb;
+      p.w_bs = w_bs;
+      for (int k = 0; k < n; ++k) {
+        auto buf = [&](int i) { return (np - 1 - i) & 1 ? static_cast<R *>(scratch[k])
+                                                         : static_cast<R *>(io[k].out); };
+        auto bs = [&](int i) { return (np - 1 - i) & 1 ? ctx->M : io[k].out_bs; };
+        p.in[k] = pi == 0 ? static_cast<const R *>(io[k].in) : buf(pi - 1);
+        p.in_bs[k] = pi == 0 ? io[k].in_bs : bs(pi - 1);
+        p.out[k] = buf(pi);
+        p.out_bs[k] = bs(pi);
+        p.pre[k] = pi == 0 ? static_cast<const R *>(io[k].w) : nullptr;
+        p.post[k] = pi == np - 1 ? static_cast<const R *>(io[k].w) : nullptr;
+      }
+      if constexpr (std::is_same<R, float>::value) {
+        if (xy && pi == 0) {
+          if (planes) p.err = ctx->dev_err;
+          CKL(planes ? scft::launch_planes(ctx->passes[0], ctx->passes[1], p, st)
+                     : scft::launch_xy(ctx->passes[0], ctx->passes[1], p, st));
+          continue;
+        }
+      }
+      int rc = launch_set(ctx, ctx->passes[xy ? pi + 1 : pi], p, st);
+      if (rc) return rc;
+    }
+    return (int)SCFT_OK;
+  });
+}
 
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,

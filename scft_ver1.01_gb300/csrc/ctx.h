@@ -121,6 +121,15 @@ int scft_fail(scft_ctx *ctx, int status, const std::string &msg);
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,
                          int nb, int deriv_pass, void *s0, void *s1, cudaStream_t st);
+// One split step W K W of up to kStepSet chains side by side (x and y fused where
+// the march has them so).  scratch[k]: [nb][M]; nothing may overlap.
+struct StepIO {
+  const void *in, *w;
+  void *out;
+  long long in_bs, out_bs;
+};
+int scft_internal_steps(scft_ctx *ctx, const StepIO *io, int n, long long w_bs, int nb,
+                        void *const *scratch, cudaStream_t st);
 // getConc (cuda_scft.cu:61-138) on the context's fields.
 int scft_internal_get_conc(scft_ctx *ctx);
 // Releases the adjoint work buffers (adjoint.cu).

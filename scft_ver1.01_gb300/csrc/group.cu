@@ -240,9 +240,9 @@ int bucket_march(scft_group *g, GroupBucket &b, int ch, long long *launches) {
       const scft::AxisPlan &ap = c0->passes[ai];
       if (ap.tc) ps.err = c0->dev_err;
       if (b.xy && pi == 0)
-        e = ap.tc ? scft::launch_planes(ap, c0->passes[1], ps, bc.st)
+        e = ap.tc ? scft::launch_planes(ap, c0->passes[1], scft::with_sets<scft::kStepSet>(ps), bc.st)
                   : scft::launch_xy(ap, c0->passes[1], ps, bc.st);
-      else if (ap.tc) e = scft::launch_tc(ap, ps, false, bc.st);
+      else if (ap.tc) e = scft::launch_tc(ap, scft::with_sets<scft::kStepSet>(ps), false, bc.st);
       else if (ap.use_fast) e = scft::launch_fast_line(ap, ps, bc.st);
       else e = scft::launch_line_filter_desc(ap, d, n, bc.st);
       if (e != cudaSuccess)

@@ -71,8 +71,8 @@ template <typename T, int N, bool XP> __host__ __device__ constexpr size_t fast_
 }
 
 
-template <typename T, int N, int P, bool XP>
-__global__ void __launch_bounds__(P * 32) k_fast_line(AxisPlan ap, PassSet<T> ps) {
+template <typename T, int N, int P, bool XP, int NS>
+__global__ void __launch_bounds__(P * 32) k_fast_line(AxisPlan ap, PassSet<T, NS> ps) {
   using C = typename cplx<T>::type;
   constexpr int R1 = N / P;
   constexpr int NT = P * 32;
@@ -81,14 +81,14 @@ __global__ void __launch_bounds__(P * 32) k_fast_line(AxisPlan ap, PassSet<T> ps
   C *ex = reinterpret_cast<C *>(smem_raw);
   const int lane = threadIdx.x & 31, p = threadIdx.x >> 5;
   // blockIdx.z = set * batch + instance
-  const int set = (int)blockIdx.z >= ps.batch ? 1 : 0;
+  const int set = set_of(ps);
   long long b = (long long)blockIdx.z - (long long)set * ps.batch;
-  const T *in = set ? ps.in[1] : ps.in[0];
-  T *out = set ? ps.out[1] : ps.out[0];
-  const T *pre = set ? ps.pre[1] : ps.pre[0];
-  const T *post = set ? ps.post[1] : ps.post[0];
-  const long long in_bs = set ? ps.in_bs[1] : ps.in_bs[0];
-  const long long out_bs = set ? ps.out_bs[1] : ps.out_bs[0];
+  const T *in = of_set(ps.in, set);
+  T *out = of_set(ps.out, set);
+  const T *pre = of_set(ps.pre, set);
+  const T *post = of_set(ps.post, set);
+  const long long in_bs = of_set(ps.in_bs, set);
+  const long long out_bs = of_set(ps.out_bs, set);
   const long long w_bs = ps.w_bs;
   const T *gain_n = reinterpret_cast<const T *>(ap.gain);
   if constexpr (std::is_same<T, float>::value) {
@@ -409,9 +409,9 @@ template <int NX, int NY, int G> constexpr size_t xy_smem() {
          (size_t)(filter_table_reals<NX>() + filter_table_reals<NY>()) * 4;
 }
 
-template <int NX, int NY, int G>
+template <int NX, int NY, int G, int NS>
 __global__ void __launch_bounds__(256 * G, G == 1 ? 2 : 1)
-    k_xy_plane(AxisPlan apx, AxisPlan apy, PassSet<float> ps) {
+    k_xy_plane(AxisPlan apx, AxisPlan apy, PassSet<float, NS> ps) {
   constexpr int P = 8, NT = 256 * G, PITCH = NX + 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *plane = reinterpret_cast<float *>(smem_raw);
@@ -424,13 +424,13 @@ __global__ void __launch_bounds__(256 * G, G == 1 ? 2 : 1)
   float *gy = gx + NX;
   const int lane = threadIdx.x & 31, p = (threadIdx.x >> 5) & 7;
   const int bar_id = G == 1 ? 0 : 1 + grp;
-  const int set = (int)blockIdx.z >= ps.batch ? 1 : 0;
+  const int set = set_of(ps);
   const long long b = (long long)blockIdx.z - (long long)set * ps.batch;
   const long long base = (long long)blockIdx.x * NX * NY;
-  const float *in = (set ? ps.in[1] : ps.in[0]) + b * (set ? ps.in_bs[1] : ps.in_bs[0]) + base;
-  float *out = (set ? ps.out[1] : ps.out[0]) + b * (set ? ps.out_bs[1] : ps.out_bs[0]) + base;
-  const float *pre = set ? ps.pre[1] : ps.pre[0];
-  const float *post = set ? ps.post[1] : ps.post[0];
+  const float *in = of_set(ps.in, set) + b * of_set(ps.in_bs, set) + base;
+  float *out = of_set(ps.out, set) + b * of_set(ps.out_bs, set) + base;
+  const float *pre = of_set(ps.pre, set);
+  const float *post = of_set(ps.post, set);
   if (pre) pre += b * ps.w_bs + base;
   if (post) post += b * ps.w_bs + base;
   const float *gxn = reinterpret_cast<const float *>(apx.gain);
@@ -835,31 +835,35 @@ template <typename T, int N, int P, bool XP> size_t fast_smem() {
 // the kernel's compile-time line length matches the plan, the 64-line tiles
 // cover the lines exactly, and the grid fits CUDA's limits.  A failed check
 // is an error status, never a launch.
-template <typename T>
-bool tiles_ok(const AxisPlan &ap, int n, bool outer_in_y, const PassSet<T> &ps) {
+template <typename T, int NS>
+bool tiles_ok(const AxisPlan &ap, int n, bool outer_in_y, const PassSet<T, NS> &ps) {
   const long long sets = (long long)ps.nset * ps.batch;
   return ap.n == n && ap.n_real > 0 && ap.n_real % 64 == 0 && sets >= 1 && sets <= 65535 &&
          (!outer_in_y || (ap.n_outer >= 1 && ap.n_outer <= 65535));
 }
-inline bool planes_ok(const AxisPlan &apx, const AxisPlan &apy, int nx, int ny,
-                      const PassSet<float> &ps) {
+template <int NS>
+bool planes_ok(const AxisPlan &apx, const AxisPlan &apy, int nx, int ny,
+               const PassSet<float, NS> &ps) {
   const long long sets = (long long)ps.nset * ps.batch;
   return apx.n == nx && apy.n == ny && apy.s_n == nx && apy.n_outer >= 1 && sets >= 1 &&
          sets <= 65535;
 }
 
-template <typename T, int N, int P, bool XP>
-cudaError_t launch_one(const AxisPlan &ap, const PassSet<T> &ps, cudaStream_t st) {
+template <typename T, int N, int P, bool XP, int NS>
+cudaError_t launch_one(const AxisPlan &ap, const PassSet<T, NS> &ps, cudaStream_t st) {
   if (!tiles_ok(ap, N, !XP, ps)) return cudaErrorInvalidValue;
   dim3 grid(ap.n_real / 64, XP ? 1 : ap.n_outer, ps.nset * ps.batch);
-  return launch_k(kPdl<T>, k_fast_line<T, N, P, XP>, grid, dim3(P * 32), fast_smem<T, N, P, XP>(), st,
+  return launch_k(kPdl<T>, k_fast_line<T, N, P, XP, NS>, grid, dim3(P * 32), fast_smem<T, N, P, XP>(), st,
                     ap, ps);
 }
 
 template <typename T, int N, int P, bool XP> cudaError_t prep_one() {
-  return cudaFuncSetAttribute(k_fast_line<T, N, P, XP>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)fast_smem<T, N, P, XP>());
+  const int smem = (int)fast_smem<T, N, P, XP>();
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_fast_line<T, N, P, XP, kMaxSet>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_fast_line<T, N, P, XP, kStepSet>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
 }  // namespace
@@ -908,16 +912,20 @@ template <int NX, int NY> constexpr int xy_groups() { return (NX >= 128 && NY >=
 
 template <int NX, int NY> cudaError_t prep_xy() {
   constexpr int G = xy_groups<NX, NY>();
-  return cudaFuncSetAttribute(k_xy_plane<NX, NY, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)xy_smem<NX, NY, G>());
+  const int smem = (int)xy_smem<NX, NY, G>();
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_xy_plane<NX, NY, G, kMaxSet>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_xy_plane<NX, NY, G, kStepSet>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
-template <int NX, int NY>
-cudaError_t launch_xy_t(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+template <int NX, int NY, int NS>
+cudaError_t launch_xy_t(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float, NS> &ps,
                         cudaStream_t st) {
   if (!planes_ok(apx, apy, NX, NY, ps)) return cudaErrorInvalidValue;
   constexpr int G = xy_groups<NX, NY>();
   dim3 grid(apy.n_outer, 1, ps.nset * ps.batch);   // one CTA per z-plane
-  return launch_pdl(k_xy_plane<NX, NY, G>, grid, dim3(256 * G), xy_smem<NX, NY, G>(), st, apx,
+  return launch_pdl(k_xy_plane<NX, NY, G, NS>, grid, dim3(256 * G), xy_smem<NX, NY, G>(), st, apx,
                     apy, ps);
 }
 template <int NX, int NY> cudaError_t prep_xyxy() {
@@ -1013,9 +1021,9 @@ cudaError_t launch_zz_wide(const AxisPlan &ap, const PassSet<T> &ps, cudaStream_
   }
   return cudaErrorInvalidValue;
 }
-template <typename T>
-cudaError_t launch_fast_line_wide(const AxisPlan &ap, const PassSet<T> &ps, cudaStream_t st) {
-  if (ps.nset < 1 || ps.nset > kMaxSet) return cudaErrorInvalidValue;
+template <typename T, int NS>
+cudaError_t launch_fast_line_wide(const AxisPlan &ap, const PassSet<T, NS> &ps, cudaStream_t st) {
+  if (ps.nset < 1 || ps.nset > NS) return cudaErrorInvalidValue;
   for (int k = 0; k < ps.nset; ++k)
     if ((reinterpret_cast<uintptr_t>(ps.post[k]) | reinterpret_cast<uintptr_t>(ps.pre[k]) |
          reinterpret_cast<uintptr_t>(ps.in[k]) | reinterpret_cast<uintptr_t>(ps.out[k])) & 15)
@@ -1091,16 +1099,25 @@ bool xy_fusable(const AxisPlan &apx, const AxisPlan &apy) {
          (apy.n == 64 || apy.n == 128) && apy.s_n == apx.n && !apy.flat_nx;
 }
 
-cudaError_t launch_xy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+template <int NS>
+cudaError_t launch_xy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float, NS> &ps,
                       cudaStream_t st) {
-  if (ps.nset < 1 || ps.nset > kMaxSet) return cudaErrorInvalidValue;
+  if (ps.nset < 1 || ps.nset > NS) return cudaErrorInvalidValue;
   if (apx.n == 128 && apy.n == 128) return launch_xy_t<128, 128>(apx, apy, ps, st);
   if (apx.n == 64 && apy.n == 64) return launch_xy_t<64, 64>(apx, apy, ps, st);
   if (apx.n == 128 && apy.n == 64) return launch_xy_t<128, 64>(apx, apy, ps, st);
   if (apx.n == 64 && apy.n == 128) return launch_xy_t<64, 128>(apx, apy, ps, st);
-  if (plane256_fusable(apx, apy)) return launch_xy256(apx, apy, ps, st);
-  return cudaErrorInvalidValue;
+  if (!plane256_fusable(apx, apy)) return cudaErrorInvalidValue;
+  for (int k = 0; k < ps.nset; k += kMaxSet) {
+    const cudaError_t e = launch_xy256(apx, apy, with_sets<kMaxSet>(ps, k), st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
+template cudaError_t launch_xy(const AxisPlan &, const AxisPlan &, const PassSet<float, kMaxSet> &,
+                               cudaStream_t);
+template cudaError_t launch_xy(const AxisPlan &, const AxisPlan &, const PassSet<float, kStepSet> &,
+                               cudaStream_t);
 
 cudaError_t fast_line_prepare() {
   cudaError_t e = cudaSuccess;
@@ -1159,8 +1176,10 @@ cudaError_t fast_line_prepare() {
   return e;
 }
 
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<float> &ps, cudaStream_t st) {
-  if (ps.nset < 1 || ps.nset > kMaxSet) return cudaErrorInvalidValue;
+template <int NS>
+static cudaError_t launch_fast_line_f32(const AxisPlan &ap, const PassSet<float, NS> &ps,
+                                        cudaStream_t st) {
+  if (ps.nset < 1 || ps.nset > NS) return cudaErrorInvalidValue;
   // column passes copy their post-factor tile with 16-byte cp.async and move
   // lines as float2: refuse misaligned buffers instead of faulting
   for (int k = 0; k < ps.nset; ++k)
@@ -1170,13 +1189,15 @@ cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<float> &ps, cudaS
   const bool xp = ap.n_fast != 0;
   // column passes: the persistent pipelined kernel when the caller supplied
   // an error word for its bounded waits
-  if (!xp && ps.err && !ap.flat_nx) {
-    switch (ap.n) {
-      case 32: return launch_pipe<32, 4>(ap, ps, st, 0);
-      case 64: return launch_pipe<64, 8>(ap, ps, st, 1);
-      case 128: return launch_pipe<128, 8>(ap, ps, st, 2);
-      case 256: return launch_pipe<256, 16>(ap, ps, st, 3);
-      default: break;
+  if constexpr (NS == kMaxSet) {
+    if (!xp && ps.err && !ap.flat_nx) {
+      switch (ap.n) {
+        case 32: return launch_pipe<32, 4>(ap, ps, st, 0);
+        case 64: return launch_pipe<64, 8>(ap, ps, st, 1);
+        case 128: return launch_pipe<128, 8>(ap, ps, st, 2);
+        case 256: return launch_pipe<256, 16>(ap, ps, st, 3);
+        default: break;
+      }
     }
   }
   switch (ap.n) {
@@ -1202,11 +1223,19 @@ cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<float> &ps, cudaS
   }
 }
 
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<double> &ps, cudaStream_t st) {
-  return launch_fast_line_wide(ap, ps, st);
+template <typename R, int NS>
+cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<R, NS> &ps, cudaStream_t st) {
+  if constexpr (std::is_same<R, float>::value) return launch_fast_line_f32(ap, ps, st);
+  else return launch_fast_line_wide(ap, ps, st);
 }
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<dfloat> &ps, cudaStream_t st) {
-  return launch_fast_line_wide(ap, ps, st);
-}
+#define LINE(R, NS) \
+  template cudaError_t launch_fast_line(const AxisPlan &, const PassSet<R, NS> &, cudaStream_t);
+LINE(float, kMaxSet)
+LINE(float, kStepSet)
+LINE(double, kMaxSet)
+LINE(double, kStepSet)
+LINE(dfloat, kMaxSet)
+LINE(dfloat, kStepSet)
+#undef LINE
 
 }  // namespace scft

@@ -95,7 +95,7 @@ __device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *
 
 // ------------------------------------------------------------------ k_real
 template <typename T, int MAXT, int PP, bool XP, bool PAIR>
-__global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, PassSet<T> ps) {
+__global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, PassSet<T, kStepSet> ps) {
   typedef Tile<kNd<T>, PP> E;
   typedef typename E::I I;
   typedef typename E::Acc Acc;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
   }
   e.setup(smem_raw, ln.sh, table, table);
   const TcHead head = *static_cast<const TcHead *>(table);
-  const int set = (int)blockIdx.z >= ps.batch ? 1 : 0;
+  const int set = set_of(ps);
   const long long b = (long long)blockIdx.z - (long long)set * ps.batch;
   const long long line0 = (long long)blockIdx.x * e.ln;
   const int nl = (int)min((long long)e.ln, ln.lines - line0);
@@ -809,23 +809,25 @@ __global__ void __launch_bounds__(544, 1)
   e.finish(fp.err);
 }
 
-// The same on FP32 planes (working reals between the filters).  A batched pass
-// (ps.desc) is the first half only: pre, x filter, y filter.
+// The same on FP32 planes (working reals between the filters).  Without a slice
+// to finish (ps.qout, or a batched pass) it is the first half only: pre, x filter,
+// y filter.
 template <int PP>
 __global__ void __launch_bounds__(544, 1)
-    k_planes_f32(PlaneArgs pa, const void *tx, const void *ty, PassSet<float> ps) {
+    k_planes_f32(PlaneArgs pa, const void *tx, const void *ty, PassSet<float, kStepSet> ps) {
   typedef Tile<4, PP> E;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   E e;
-  const bool half = ps.desc != nullptr;
-  if (half) {
+  const bool half = ps.desc || !ps.qout[0];
+  if (ps.desc) {
     tx = ps.desc[blockIdx.z].tc;
     ty = ps.desc[blockIdx.z].tc_y;
   }
   e.setup(smem_raw, pa.sh, tx, ty);
   const int shift_x = 23 - static_cast<const TcHead *>(tx)->kshift;
   const int shift_y = 23 - static_cast<const TcHead *>(ty)->kshift;
-  const long long b = blockIdx.z;
+  const int set = set_of(ps);
+  const long long b = (long long)blockIdx.z - (long long)set * ps.batch;
   const int filters = half ? 2 : 4;
   auto axis_of = [](int f) { return f == 1 || f == 2 ? 1 : 0; };
   pdl_wait();
@@ -841,10 +843,11 @@ __global__ void __launch_bounds__(544, 1)
   const unsigned tile = (unsigned)z0 * ny * nx;
   const int k0 = PP * e.blk, pl = e.line / nx, xx = e.line - pl * nx;
   float *S = reinterpret_cast<float *>(smem_raw);
-  const float *in = ps.in[0] + b * ps.in_bs[0], *w = ps.post[0] + b * ps.w_bs, *pre = nullptr;
-  float *out = ps.out[0] + b * ps.out_bs[0], *qo = ps.qout[0] + b * ps.qout_bs[0];
-  if (half) {
-    const PassDesc d = ps.desc[b];
+  const float *in = ps.in[set] + b * ps.in_bs[set], *w = ps.post[set] + b * ps.w_bs;
+  const float *pre = ps.pre[set] ? ps.pre[set] + b * ps.w_bs : nullptr;
+  float *out = ps.out[set] + b * ps.out_bs[set], *qo = ps.qout[set] + b * ps.qout_bs[set];
+  if (ps.desc) {
+    const PassDesc d = ps.desc[blockIdx.z];
     in = d.in;
     out = d.out;
     pre = d.pre;
@@ -999,7 +1002,7 @@ void spread(Shape &sh, long long lines) {
 inline int lines_per_cta(const Shape &sh) { return kLines / sh.rep; }
 
 template <typename T, int MAXT, int PP, bool XP, bool PR>
-cudaError_t launch_real_t(Lines ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+cudaError_t launch_real_t(Lines ln, const void *tc, const PassSet<T, kStepSet> &ps, cudaStream_t st) {
   const int lc = lines_per_cta(ln.sh);
   dim3 grid((unsigned)((ln.lines + lc - 1) / lc), 1, ps.nset * ps.batch);
   ln.sh.stage = XP ? lc * (ln.n + 1) * (int)sizeof(T) : 0;
@@ -1008,7 +1011,7 @@ cudaError_t launch_real_t(Lines ln, const void *tc, const PassSet<T> &ps, cudaSt
                     (size_t)ln.sh.lay.total, st, ln, tc, ps);
 }
 template <typename T, bool XP, bool PR>
-cudaError_t launch_real_kg(Lines ln, const void *tc, const PassSet<T> &ps, cudaStream_t st) {
+cudaError_t launch_real_kg(Lines ln, const void *tc, const PassSet<T, kStepSet> &ps, cudaStream_t st) {
   spread(ln.sh, ln.lines * ps.nset * ps.batch);
   if (ln.sh.pp == 4) return launch_real_t<T, 544, 4, XP, PR>(ln, tc, ps, st);
   if (ln.sh.pp == 8) return launch_real_t<T, 544, 8, XP, PR>(ln, tc, ps, st);
@@ -1018,10 +1021,10 @@ cudaError_t launch_real_kg(Lines ln, const void *tc, const PassSet<T> &ps, cudaS
   return launch_real_t<T, 640, 16, XP, PR>(ln, tc, ps, st);
 }
 template <typename T>
-cudaError_t launch_real(const AxisPlan &ap, const PassSet<T> &ps, bool pair, cudaStream_t st) {
+cudaError_t launch_real(const AxisPlan &ap, const PassSet<T, kStepSet> &ps, bool pair, cudaStream_t st) {
   Lines ln;
   const long long sets = (long long)ps.nset * ps.batch;
-  if (!lines_of(ap, kNd<T>, ln) || ps.nset < 1 || ps.nset > kMaxSet || sets < 1 || sets > 65535 ||
+  if (!lines_of(ap, kNd<T>, ln) || ps.nset < 1 || ps.nset > kStepSet || sets < 1 || sets > 65535 ||
       (ps.desc && (pair || kNd<T> != 4)))
     return cudaErrorInvalidValue;
   for (int k = 0; k < ps.nset && !ps.desc; ++k) {
@@ -1402,10 +1405,10 @@ cudaError_t tc_prepare() {
   return cudaSuccess;
 }
 
-cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float> &ps, bool pair, cudaStream_t st) {
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float, kStepSet> &ps, bool pair, cudaStream_t st) {
   return launch_real(ap, ps, pair, st);
 }
-cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double> &ps, bool pair, cudaStream_t st) {
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double, kStepSet> &ps, bool pair, cudaStream_t st) {
   return launch_real(ap, ps, pair, st);
 }
 
@@ -1433,13 +1436,18 @@ cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStre
   }
 }
 
-cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float, kStepSet> &ps,
                           cudaStream_t st) {
   PlaneArgs pa;
-  if (!planes_of(apx, apy, 4, ps.batch, false, pa) || ps.nset != 1 || ps.batch < 1 || ps.batch > 65535 ||
-      (!ps.desc && (!ps.in[0] || !ps.out[0] || !ps.post[0] || !ps.qout[0])))
+  const long long sets = (long long)ps.nset * ps.batch;
+  if (ps.nset < 1 || ps.nset > kStepSet || sets < 1 || sets > 65535 ||
+      !planes_of(apx, apy, 4, (int)sets, false, pa))
     return cudaErrorInvalidValue;
-  dim3 grid((pa.nz + pa.per - 1) / pa.per, 1, ps.batch);
+  for (int k = 0; k < ps.nset && !ps.desc; ++k)
+    if (!ps.in[k] || !ps.out[k] || !ps.qout[k] != !ps.qout[0] || (ps.qout[0] && !ps.post[k]) ||
+        (ps.qout[0] && ps.pre[k]) || (!ps.qout[0] && ps.post[k]))
+      return cudaErrorInvalidValue;
+  dim3 grid((pa.nz + pa.per - 1) / pa.per, 1, (unsigned)sets);
   const size_t smem = pa.sh.lay.total;
   return launch_pdl(pa.sh.pp == 4 ? k_planes_f32<4> : k_planes_f32<8>, grid, dim3(pa.sh.threads), smem, st, pa, apx.tc, apy.tc, ps);
 }

@@ -38,7 +38,7 @@ struct AxisPlan {
 // One pass over up to kMaxSet independent propagators at once (the lockstep
 // march chains): set k reads in[k] (+ b*in_bs), multiplies by pre[k], filters,
 // multiplies by post[k] and writes out[k] (+ b*out_bs), for every instance b.
-constexpr int kMaxSet = 2;
+constexpr int kMaxSet = 2, kStepSet = 3;
 // One line set of a batched pass over several contexts (a group's lockstep
 // march, FP32): the set's buffers (one instance each) and gain tables.
 struct PassDesc {
@@ -49,31 +49,71 @@ struct PassDesc {
   const float *gain_y;       // x+y plane passes: the y axis's gain table
   const void *tc, *tc_y;     // the set's tensor-core tables (tc_y: plane passes)
 };
-template <typename R> struct PassSet {
-  const R *in[kMaxSet];
-  R *out[kMaxSet];
-  const R *pre[kMaxSet];
-  const R *post[kMaxSet];
-  long long in_bs[kMaxSet], out_bs[kMaxSet];
+// (NS: sets it has room for; kStepSet only in scft_internal_steps, since the
+// longer arguments cost every launch about 1 % of a small pass)
+template <typename R, int NS = kMaxSet> struct PassSet {
+  const R *in[NS];
+  R *out[NS];
+  const R *pre[NS];
+  const R *post[NS];
+  long long in_bs[NS], out_bs[NS];
   long long w_bs;
   int nset;
   int batch;
   unsigned *err;   // device error word (bounded-wait timeouts), may be null for non-pipelined kernels
   // fused step pairs only (launch_zz / launch_xyxy): where the finished
   // propagator slice goes; `out` then receives the next step's intermediate
-  R *qout[kMaxSet];
-  long long qout_bs[kMaxSet];
+  R *qout[NS];
+  long long qout_bs[NS];
   // FP32 per-axis and x+y plane passes: when set, line set blockIdx.z takes
   // its buffers and gains from desc[blockIdx.z] (nset 1, batch = sets)
   const PassDesc *desc;
 };
+
+#ifdef __CUDACC__
+// The line set of a CTA (blockIdx.z = set * batch + instance), and its entry of
+// one of the set's arrays: selected, not indexed, which is a load behind a load.
+template <typename R, int NS>
+__device__ __forceinline__ int set_of(const PassSet<R, NS> &ps) {
+  const int z = blockIdx.z;
+  if (NS == 2) return z >= ps.batch ? 1 : 0;
+  return z < ps.batch ? 0 : (z < 2 * ps.batch ? 1 : 2);
+}
+template <typename V> __device__ __forceinline__ V of_set(const V (&a)[2], int set) {
+  return set ? a[1] : a[0];
+}
+template <typename V> __device__ __forceinline__ V of_set(const V (&a)[3], int set) {
+  return set == 0 ? a[0] : (set == 1 ? a[1] : a[2]);
+}
+#endif
+// The first sets of a set for more, or the other way round (as many as fit).
+template <int NS, typename R, int MS> PassSet<R, NS> with_sets(const PassSet<R, MS> &a, int first = 0) {
+  PassSet<R, NS> p = {};
+  for (int k = 0; k < NS && first + k < MS; ++k) {
+    p.in[k] = a.in[first + k];
+    p.out[k] = a.out[first + k];
+    p.pre[k] = a.pre[first + k];
+    p.post[k] = a.post[first + k];
+    p.in_bs[k] = a.in_bs[first + k];
+    p.out_bs[k] = a.out_bs[first + k];
+    p.qout[k] = a.qout[first + k];
+    p.qout_bs[k] = a.qout_bs[first + k];
+  }
+  p.nset = a.nset - first < NS ? a.nset - first : NS;
+  p.w_bs = a.w_bs;
+  p.batch = a.batch;
+  p.err = a.err;
+  p.desc = a.desc;
+  return p;
+}
 
 // Register-resident pass (k_fast.cu): n in {32, 64, 128, 256} (FP32) or
 // {32, 64, 128} (FP64), and n_real a multiple of 64.
 bool fast_line_supported(const AxisPlan &ap, size_t real_bytes = 4);
 // Fused x+y pass over whole z-planes (k_fast.cu): Nx, Ny in {64, 128}.
 bool xy_fusable(const AxisPlan &apx, const AxisPlan &apy);
-cudaError_t launch_xy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
+template <int NS>
+cudaError_t launch_xy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float, NS> &ps,
                       cudaStream_t st);
 cudaError_t fast_line_prepare();
 // x+y passes of 256 x 256 planes (k_plane256.cu): a cluster of two CTAs per
@@ -87,9 +127,8 @@ cudaError_t launch_xyxy256(const AxisPlan &apx, const AxisPlan &apy, const PassS
                            cudaStream_t st);
 // bounded-wait self-test: sets bit 4 of *err after `limit` clocks
 cudaError_t launch_wait_selftest(unsigned *err, long long limit, cudaStream_t st);
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<float> &ps, cudaStream_t st);
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<double> &ps, cudaStream_t st);
-cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<dfloat> &ps, cudaStream_t st);
+template <typename R, int NS>
+cudaError_t launch_fast_line(const AxisPlan &ap, const PassSet<R, NS> &ps, cudaStream_t st);
 // Fused step pairs.  The axis filters commute, so consecutive contour steps
 // can run their passes in alternating order (x+y then z, z then x+y); the
 // end of one step and the start of the next are then the same pass type and
@@ -115,8 +154,10 @@ size_t tc_table_bytes(int n, int nd);
 bool tc_build_table(const double *gain, int n, int nd, std::vector<unsigned char> &table,
                     double *row_sum);
 cudaError_t tc_prepare();
-cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float> &ps, bool pair, cudaStream_t st);
-cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double> &ps, bool pair, cudaStream_t st);
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float, kStepSet> &ps, bool pair,
+                      cudaStream_t st);
+cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double, kStepSet> &ps, bool pair,
+                      cudaStream_t st);
 // One pass of the fused FP64 march, whose intermediates are
 // 64-bit integers (batch instances; strides in elements).  The unit of an
 // intermediate is 2^(u[b] + w * (eref[b] - 1022) + kbits - 59): u the exponent
@@ -138,10 +179,10 @@ struct FixPass {
 constexpr int kFixFirst = 0, kFixMid = 1, kFixPair = 2, kFixLast = 3;
 cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStream_t st);
 // Both axes of whole planes in one launch: x, y, the factor (q stored), the
-// factor, y, x (ps.desc: x, y of a batched pass); FP64 also a film's whole march
+// factor, y, x (without qout, or batched: pre, x, y); FP64 also a film's whole march
 // segment.
-cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSet<float> &ps,
-                          cudaStream_t st);
+cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy,
+                          const PassSet<float, kStepSet> &ps, cudaStream_t st);
 cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPass &fp, int steps,
                           long long q_step, cudaStream_t st);
 cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
