@@ -19,6 +19,8 @@
 // The Gram matrix, the solve and the fields stay FP64.
 // An instance whose max|d| is still above `start` (or with no history yet)
 // takes the simple step w_new = w_c + wopt d_c, decided on the device.
+#include <algorithm>
+
 #include "common.cuh"
 #include "dfloat.cuh"
 #include "kernels.h"
@@ -29,18 +31,21 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// Sum over the block (kThreads threads) in thread 0; sh: kHalf doubles.  Halves
+// fold through shared memory: 12 additions of a warp where eight warps' shuffles
+// took 45, and an FP64 addition is 16 cycles of the SM.
+constexpr int kHalf = kThreads / 2;
 __device__ __forceinline__ double blk_sum(double v, double *sh) {
-  v = warp_sum(v);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (wid == 0) {
-    r = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-    r = warp_sum(r);
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int h = kHalf; h >= 32; h /= 2) {
+    __syncthreads();
+    if (t >= h && t < 2 * h) sh[t - h] = v;
+    __syncthreads();
+    if (t < h) v += sh[t];
   }
-  return r;
+  if (t < 32) v = warp_sum(v);
+  return v;
 }
 __device__ __forceinline__ double blk_max(double v, double *sh) {
   v = warp_max(v);
@@ -83,17 +88,32 @@ __device__ __forceinline__ unsigned long long blk_max_key(unsigned long long v,
   return r;
 }
 
-// phi_w's update direction (cuda_aid.cu:398-408).  It is affine in
-// (wA, wB, phiA, phiB), so the instance mean of the direction is the
-// direction of the instance means.
+// phi_w's update direction (cuda_aid.cu:398-408), its terms gathered so that a
+// point takes 7 FP64 operations instead of 13.  It is affine in (wA, wB, phiA,
+// phiB), so the instance mean of the direction is the direction of the means.
 __device__ __forceinline__ void phi_w_dir(double a, double c, double pa, double pb, double hAB,
                                           double wcmp, double &da, double &db) {
-  const double eta = (a + c - hAB) / 2;
-  const double psum = 1.0 - pa - pb;
-  da = hAB * pb + eta - a;
-  db = hAB * pa + eta - c;
-  da -= wcmp * psum;
-  db -= wcmp * psum;
+  const double m = fma(wcmp, pa + pb, -(0.5 * hAB + wcmp)), t = c - a;
+  da = fma(hAB, pb, fma(0.5, t, m));
+  db = fma(hAB, pa, fma(-0.5, t, m));
+}
+
+// dfloat(x) in integers (bit for bit): the four FP64 operations of the
+// conversion took a third of the residual's time.  Zero, values outside 2^-60 ..
+// 2^120, infinities and NaN go out of line.
+__device__ __noinline__ dfloat pair_rare(double x) { return dfloat(x); }
+__device__ __forceinline__ dfloat pair_of(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t m = hi & 0x7fffffffu;
+  if (m - ((1023u - 60u) << 20) >= 180u << 20) return pair_rare(x);
+  const uint32_t f = ((m - 0x38000000u) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
+  const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
+  int r = (int)rest - (int)(up << 29);           // x - hi, in units of 2^(e - 52)
+  r = (int)hi < 0 ? -r : r;
+  dfloat d;
+  d.hi = __uint_as_float((hi & 0x80000000u) | (f + up));
+  d.lo = __int2float_rn(r) * __uint_as_float(((m >> 20) - (1023u - 127u) - 52u) << 23);
+  return d;
 }
 
 // Per-instance sums of wA, wB, phiA, phiB: partial[(b*4 + f)*nblk + blk].
@@ -102,7 +122,7 @@ __device__ __forceinline__ void phi_w_dir(double a, double c, double pa, double 
 __global__ void k_residual_sum(const double *__restrict__ wa, const double *__restrict__ wb,
                                const double *__restrict__ pha, const double *__restrict__ phb,
                                long long M, double *__restrict__ partial) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   const long long b = blockIdx.y, o = b * M;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   auto load = [&](long long i) { return dquad{wa[o + i], wb[o + i], pha[o + i], phb[o + i]}; };
@@ -118,18 +138,24 @@ __global__ void k_residual_sum(const double *__restrict__ wa, const double *__re
 }
 
 // dmean[b*2 + f] = mean of dA / dB = the direction of the field means
+// (two warps a field, so that no chain of additions is longer than nblk / 64)
 __global__ void k_residual_mean(const double *__restrict__ partial, int nblk, long long M,
                                 double hAB, double wcmp, double *__restrict__ dmean) {
-  __shared__ double sh[32];
-  const int b = blockIdx.x;
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x)
-    for (int f = 0; f < 4; ++f) s[f] += partial[(b * 4 + f) * nblk + i];
-  for (int f = 0; f < 4; ++f) s[f] = blk_sum(s[f], sh);
+  __shared__ double part[8];
+  const int b = blockIdx.x, warp = threadIdx.x >> 5;
+  const double *p = partial + (b * 4 + warp / 2) * (long long)nblk;
+  double s0 = 0.0, s1 = 0.0;
+  for (int i = threadIdx.x & 63; i < nblk; i += 128) {
+    s0 += p[i];
+    if (i + 64 < nblk) s1 += p[i + 64];
+  }
+  const double s = warp_sum(s0 + s1);
+  if ((threadIdx.x & 31) == 0) part[warp] = s;
+  __syncthreads();
   if (threadIdx.x == 0) {
     const double m = (double)M;
-    phi_w_dir(s[0] / m, s[1] / m, s[2] / m, s[3] / m, hAB, wcmp, dmean[b * 2 + 0],
-              dmean[b * 2 + 1]);
+    phi_w_dir((part[0] + part[1]) / m, (part[2] + part[3]) / m, (part[4] + part[5]) / m,
+              (part[6] + part[7]) / m, hAB, wcmp, dmean[b * 2 + 0], dmean[b * 2 + 1]);
   }
 }
 
@@ -141,38 +167,51 @@ __global__ void k_residual_mean(const double *__restrict__ partial, int nblk, lo
 // double-float pairs), copies w to wprev ([b][2][M] FP64) and applies the
 // simple step in place (wopt != 0).
 // partial[(b*2 + {0: max|d|, 1: sum d^2})*nblk + blk]
+// FP64 operations bound it (16 cycles of an SM each per warp; 128^3: 33 a point
+// 160 us, 12 a point 65 us): kernels without the parts not asked for (HIST: the
+// history slot; STEP: the simple step), the means in the constants without STEP,
+// conversions in integers.
+template <bool HIST, bool STEP>
 __global__ void k_residual(double *__restrict__ wa, double *__restrict__ wb,
                            const double *__restrict__ pha, const double *__restrict__ phb,
                            double hAB, double wcmp, double wopt, long long M,
                            const double *__restrict__ dmean, dfloat *__restrict__ hu,
                            dfloat *__restrict__ hd, double lam_u, double *__restrict__ wprev,
                            double *__restrict__ partial) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   __shared__ unsigned long long shk[32];
   const long long b = blockIdx.y, o = b * M;
   const double ma = dmean[b * 2 + 0], mb = dmean[b * 2 + 1];
+  const double ka = -(0.5 * hAB + wcmp) - ma, kb = -(0.5 * hAB + wcmp) - mb;
   unsigned long long mx = 0;
   double ss = 0.0;
   auto load = [&](long long i) { return dquad{wa[o + i], wb[o + i], pha[o + i], phb[o + i]}; };
   stream_loop<4>(M, load,
                  [&](long long i, dquad v) {
     const double a = v.x, c = v.y;
-    double da, db;
-    phi_w_dir(a, c, v.z, v.w, hAB, wcmp, da, db);   // cuda_aid.cu:398-408
-    const double ca = da - ma, cb = db - mb;
+    double da, db, ca, cb;
+    if (STEP) {
+      phi_w_dir(a, c, v.z, v.w, hAB, wcmp, da, db);   // cuda_aid.cu:398-408
+      ca = da - ma;
+      cb = db - mb;
+    } else {
+      const double ps = v.z + v.w, t = c - a;
+      ca = fma(hAB, v.w, fma(0.5, t, fma(wcmp, ps, ka)));
+      cb = fma(hAB, v.z, fma(-0.5, t, fma(wcmp, ps, kb)));
+    }
     mx = key_max(mx, key_max(abs_key(ca), abs_key(cb)));
-    ss += ca * ca + cb * cb;
-    if (hu) {
-      hu[(2 * b) * M + i] = dfloat(fma(lam_u, ca, a));
-      hu[(2 * b + 1) * M + i] = dfloat(fma(lam_u, cb, c));
-      hd[(2 * b) * M + i] = dfloat(ca);
-      hd[(2 * b + 1) * M + i] = dfloat(cb);
+    ss = fma(ca, ca, fma(cb, cb, ss));
+    if (HIST) {
+      hu[(2 * b) * M + i] = pair_of(fma(lam_u, ca, a));
+      hu[(2 * b + 1) * M + i] = pair_of(fma(lam_u, cb, c));
+      hd[(2 * b) * M + i] = pair_of(ca);
+      hd[(2 * b + 1) * M + i] = pair_of(cb);
     }
     if (wprev) {
       wprev[(2 * b) * M + i] = a;
       wprev[(2 * b + 1) * M + i] = c;
     }
-    if (wopt != 0.0) {
+    if (STEP) {
       wa[o + i] = a + wopt * da;   // phi_w, cuda_aid.cu:410-412
       wb[o + i] = c + wopt * db;
     }
@@ -188,7 +227,7 @@ __global__ void k_residual(double *__restrict__ wa, double *__restrict__ wb,
 // err[b*2 + 0] = max|d|, err[b*2 + 1] = rms
 __global__ void k_residual_finalize(const double *__restrict__ partial, int nblk, long long M,
                                     double *__restrict__ err) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   __shared__ unsigned long long shk[32];
   const int b = blockIdx.x;
   unsigned long long mx = 0;
@@ -228,40 +267,64 @@ struct SlotList {
   int slot[kMaxSlots];
   int n;
 };
-// Grid row blockIdx.y takes the kChunk list entries from blockIdx.y*kChunk:
-// few accumulators keep the occupancy high and each thread has kChunk + 1
-// loads in flight per element; d_c is read once per chunk (an L2 hit while
-// it fits).
-constexpr int kChunk = 8;
-__global__ void k_gram_row(const dfloat *__restrict__ dc, SlotList sl, long long M,
-                           double *__restrict__ partial) {
-  __shared__ double sh[32];
+// x in FP64, the exponent rebuilt in integers (see pair_of)
+__device__ __noinline__ double wide_rare(float x) { return (double)x; }
+__device__ __forceinline__ double wide(float x) {
+  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return wide_rare(x);   // denormal, inf, nan
+  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+// Two pairs of a slot (grids have an even number of points).
+struct __align__(16) Pair2 {
+  dfloat v[2];
+};
+__device__ __forceinline__ Pair2 ld_pair2(const dfloat *p) {
+  const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+  Pair2 r;
+  r.v[0] = dfloat(v.x, v.y);
+  r.v[1] = dfloat(v.z, v.w);
+  return r;
+}
+// Grid row blockIdx.y takes the kChunk list entries from blockIdx.y*kChunk: few
+// accumulators keep the occupancy high and each thread has kChunk + 1 16-byte
+// loads in flight; d_c is read once per chunk.  HBM bounds it: 21 slots of 128^3
+// points 153 us -> 101 (6.3 TB/s), with one wave of blocks and their last sums
+// cheaper, which had taken 60 us of FP64 additions.  (All slots in one pass read
+// d_c once but ran at 2.2 TB/s: too few threads, each with a long chain.)
+constexpr int kChunk = 5;
+__global__ void __launch_bounds__(kThreads, 4)
+    k_gram_row(const dfloat *__restrict__ dc, SlotList sl, long long M, double *__restrict__ partial) {
+  __shared__ double sh[kHalf];
   const long long b = blockIdx.z;
   const int k0 = blockIdx.y * kChunk;
   const long long n2 = 2 * M;
   const dfloat *dk[kChunk];
-  dfloat acc[kChunk];
+  dfloat acc[kChunk][2];
 #pragma unroll
-  for (int kk = 0; kk < kChunk; ++kk)
-    dk[kk] = k0 + kk < sl.n ? sl.d[k0 + kk] + b * n2 : nullptr;
+  for (int k = 0; k < kChunk; ++k) dk[k] = k0 + k < sl.n ? sl.d[k0 + k] + b * n2 : nullptr;
   const dfloat *x = dc + b * n2;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2;
-       i += (long long)gridDim.x * blockDim.x) {
-    dfloat y[kChunk];
+  const long long S = 2 * (long long)gridDim.x * blockDim.x;
+  for (long long i = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i < n2; i += S) {
+    Pair2 y[kChunk];
 #pragma unroll
-    for (int kk = 0; kk < kChunk; ++kk)
-      if (dk[kk]) y[kk] = ld_pair(dk[kk] + i);
-    const dfloat xi = ld_pair(x + i);
+    for (int k = 0; k < kChunk; ++k)
+      if (dk[k]) y[k] = ld_pair2(dk[k] + i);
+    const Pair2 xi = ld_pair2(x + i);
 #pragma unroll
-    for (int kk = 0; kk < kChunk; ++kk)
-      if (dk[kk]) df_fma_acc(acc[kk], xi, y[kk]);
+    for (int k = 0; k < kChunk; ++k)
+      if (dk[k]) {
+        df_fma_acc(acc[k][0], xi.v[0], y[k].v[0]);
+        df_fma_acc(acc[k][1], xi.v[1], y[k].v[1]);
+      }
   }
 #pragma unroll
-  for (int kk = 0; kk < kChunk; ++kk) {
-    if (dk[kk]) {
-      const double r = blk_sum((double)acc[kk], sh);
-      if (threadIdx.x == 0)
-        partial[(b * kMaxSlots + k0 + kk) * gridDim.x + blockIdx.x] = r;
+  for (int k = 0; k < kChunk; ++k) {
+    if (dk[k]) {
+      const double r = blk_sum((wide(acc[k][0].hi) + wide(acc[k][1].hi)) +
+                                   (wide(acc[k][0].lo) + wide(acc[k][1].lo)),
+                               sh);
+      if (threadIdx.x == 0) partial[(b * kMaxSlots + k0 + k) * gridDim.x + blockIdx.x] = r;
     }
   }
 }
@@ -269,7 +332,7 @@ __global__ void k_gram_row(const dfloat *__restrict__ dc, SlotList sl, long long
 // Finalise the Gram row into the ring matrix G[b][(m+1)x(m+1)] (symmetric).
 __global__ void k_gram_finalize(const double *__restrict__ partial, int nblk, SlotList sl, int c,
                                 int m1, double *__restrict__ G) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   const int b = blockIdx.y, k = blockIdx.x;
   if (k >= sl.n) return;
   double s = 0.0;
@@ -291,7 +354,6 @@ __global__ void k_anderson_solve(const double *__restrict__ G, const double *__r
                                  double wopt, double *__restrict__ a, double *__restrict__ lam,
                                  double *__restrict__ mode) {
   __shared__ double U[32][33];
-  __shared__ double V[32];
   const int b = blockIdx.x, lane = threadIdx.x;
   const double *Gb = G + (long long)b * m1 * m1;
   double *ab = a + (long long)b * m1;
@@ -307,60 +369,80 @@ __global__ void k_anderson_solve(const double *__restrict__ G, const double *__r
     return;
   }
   const int n = hist;
-  auto slot = [&](int i) { return ((c - i) % m1 + m1) % m1; };   // i = 1..n
-  const double gcc = Gb[c * m1 + c];
+  // lane i: the slot of entry i (slot c - i - 1 of the ring)
+  const int mine = ((c - lane - 1) % m1 + m1) % m1;
+  const double gcc = Gb[c * m1 + c], gcj = lane < n ? Gb[c * m1 + mine] : 0.0;
+  double diag = 0.0;
+#pragma unroll 4
   for (int i = 0; i < n; ++i) {
+    const int si = __shfl_sync(0xffffffffu, mine, i);
+    const double gci = __shfl_sync(0xffffffffu, gcj, i);
     if (lane < n) {
-      const int si = slot(i + 1), sj = slot(lane + 1);
-      U[i][lane] = gcc - Gb[c * m1 + si] - Gb[c * m1 + sj] + Gb[si * m1 + sj];
+      const double u = gcc - gci - gcj + Gb[si * m1 + mine];
+      U[i][lane] = u;
+      if (i == lane) diag = u;
     }
   }
-  if (lane < n) V[lane] = gcc - Gb[c * m1 + slot(lane + 1)];
-  __syncwarp();
+  double vl = lane < n ? gcc - gcj : 0.0;         // lane r: row r's right-hand side
   // Tikhonov shift relative to the largest diagonal entry keeps U invertible
-  // when two histories are nearly parallel.
-  double dmax = 0.0;
-  for (int i = 0; i < n; ++i) dmax = fmax(dmax, fabs(U[i][i]));
-  if (lane < n) U[lane][lane] += 1e-12 * dmax + 1e-300;
+  // when two histories are nearly parallel (a NaN counts as none).
+  unsigned long long dkey = abs_key(diag);
+  if (dkey > 0x7ff0000000000000ULL) dkey = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dkey = key_max(dkey, __shfl_xor_sync(0xffffffffu, dkey, o));
+  if (lane < n) U[lane][lane] = diag + (1e-12 * __longlong_as_double((long long)dkey) + 1e-300);
   __syncwarp();
-  // Gaussian elimination with partial pivoting; lane r owns row r.
+  // Gaussian elimination with partial pivoting.  Lane r finds row r's factor (one
+  // division a step for all rows), then lane j updates column j of every row; the
+  // back substitution goes by columns, with the divisions done beforehand.  (With
+  // a row per lane and a serial pivot search and substitution the solve took
+  // 68 us of an update at 20 histories.)
   for (int k = 0; k < n; ++k) {
-    int piv = k;
-    if (lane == 0) {
-      double best = fabs(U[k][k]);
-      for (int r = k + 1; r < n; ++r)
-        if (fabs(U[r][k]) > best) { best = fabs(U[r][k]); piv = r; }
-    }
-    piv = __shfl_sync(0xffffffffu, piv, 0);
+    // the first largest |U[r][k]|, r >= k; a NaN is never larger than U[k][k]
+    unsigned long long key = 0;
+    if (lane >= k && lane < n) key = abs_key(U[lane][k]);
+    if (key > 0x7ff0000000000000ULL) key = lane == k ? ~0ULL : 0ULL;
+    const unsigned kh = (unsigned)(key >> 32), top = __reduce_max_sync(0xffffffffu, kh);
+    const unsigned kl = kh == top ? (unsigned)key : 0u, low = __reduce_max_sync(0xffffffffu, kl);
+    const unsigned at = __ballot_sync(0xffffffffu, kh == top && (unsigned)key == low && lane >= k);
+    const int piv = __ffs(at) - 1;
     if (piv != k) {
-      if (lane <= n) {
-        if (lane < n) {
-          const double t = U[k][lane]; U[k][lane] = U[piv][lane]; U[piv][lane] = t;
-        }
+      if (lane < n) {
+        const double t = U[k][lane];
+        U[k][lane] = U[piv][lane];
+        U[piv][lane] = t;
       }
-      if (lane == 0) { const double t = V[k]; V[k] = V[piv]; V[piv] = t; }
+      const double vk = __shfl_sync(0xffffffffu, vl, k), vp = __shfl_sync(0xffffffffu, vl, piv);
+      if (lane == k) vl = vp;
+      if (lane == piv) vl = vk;
     }
     __syncwarp();
-    const double pk = U[k][k];
+    const double vk = __shfl_sync(0xffffffffu, vl, k);
+    double f = 0.0;
     if (lane > k && lane < n) {
-      const double f = U[lane][k] / pk;
-      for (int j = k; j < n; ++j) U[lane][j] -= f * U[k][j];
-      V[lane] -= f * V[k];
+      f = U[lane][k] / U[k][k];
+      vl -= f * vk;
+    }
+    const double uk = U[k][lane];                // (lanes from n on: unused columns)
+    __syncwarp();
+#pragma unroll 4
+    for (int r = k + 1; r < n; ++r) {
+      const double fr = __shfl_sync(0xffffffffu, f, r);
+      if (lane >= k && lane < n) U[r][lane] -= fr * uk;
     }
     __syncwarp();
   }
+  const double inv = lane < n ? 1.0 / U[lane][lane] : 0.0;
+  double x = 0.0;                                // lane i: x[i]
+  for (int j = n - 1; j >= 0; --j) {
+    if (lane == j) x = vl * inv;
+    const double xj = __shfl_sync(0xffffffffu, x, j);
+    if (lane < j) vl -= U[lane][j] * xj;
+  }
+  if (lane < n) ab[mine] = x;
+  double sx = 0.0;
+  for (int i = 0; i < n; ++i) sx += __shfl_sync(0xffffffffu, x, i);
   if (lane == 0) {
-    double x[32];
-    double sx = 0.0;
-    for (int i = n - 1; i >= 0; --i) {
-      double s = V[i];
-      for (int j = i + 1; j < n; ++j) s -= U[i][j] * x[j];
-      x[i] = s / U[i][i];
-    }
-    for (int i = 0; i < n; ++i) {
-      ab[slot(i + 1)] = x[i];
-      sx += x[i];
-    }
     ab[c] = 1.0 - sx;
     lam[b] = lambda;
     mode[b] = 1.0;
@@ -368,7 +450,7 @@ __global__ void k_anderson_solve(const double *__restrict__ G, const double *__r
 }
 
 // Anderson step: w_new = sum_j a_j u_j over the listed slots, in pair
-// arithmetic; simple step (mode 0): w_new = w + lam d_c in FP64 from the live
+// arithmetic, two points a thread (128^3, 20 slots: 126 us -> 101, 6.6 TB/s); simple step (mode 0): w_new = w + lam d_c in FP64 from the live
 // fields.  kUChunk slots' loads are in flight per element.
 struct SlotRing {
   const dfloat *u[kMaxSlots];
@@ -396,19 +478,23 @@ __global__ void k_anderson_update(double *__restrict__ wa, double *__restrict__ 
   }
   for (int k = threadIdx.x; k < sr.n; k += blockDim.x) s_a[k] = dfloat(a[b * m1 + sr.idx[k]]);
   __syncthreads();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2; i += S) {
-    dfloat s;
+  for (long long i = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); i < n2; i += 2 * S) {
+    dfloat s0, s1;
     for (int k0 = 0; k0 < sr.n; k0 += kUChunk) {
-      dfloat y[kUChunk];
+      Pair2 y[kUChunk];
 #pragma unroll
       for (int kk = 0; kk < kUChunk; ++kk)
-        if (k0 + kk < sr.n) y[kk] = ld_pair(sr.u[k0 + kk] + b * n2 + i);
+        if (k0 + kk < sr.n) y[kk] = ld_pair2(sr.u[k0 + kk] + b * n2 + i);
 #pragma unroll
       for (int kk = 0; kk < kUChunk; ++kk)
-        if (k0 + kk < sr.n) df_fma_acc(s, s_a[k0 + kk], y[kk]);
+        if (k0 + kk < sr.n) {
+          df_fma_acc(s0, s_a[k0 + kk], y[kk].v[0]);
+          df_fma_acc(s1, s_a[k0 + kk], y[kk].v[1]);
+        }
     }
-    if (i < M) wab[i] = (double)s;
-    else wbb[i - M] = (double)s;
+    double *w = i < M ? wab + i : wbb + (i - M);   // (both points in one field: M is even)
+    *reinterpret_cast<double2 *>(w) =
+        make_double2(wide(s0.hi) + wide(s0.lo), wide(s1.hi) + wide(s1.lo));
   }
 }
 
@@ -439,7 +525,7 @@ __device__ __forceinline__ void shift_gen(const double *__restrict__ w0, long lo
 __global__ void k_shift_dots(const double *__restrict__ wa1, const double *__restrict__ wb1,
                              const double *__restrict__ w0, long long M, Grid3 g,
                              double *__restrict__ partial) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   const long long b = blockIdx.y;
   double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
@@ -472,7 +558,7 @@ __global__ void k_shift_dots(const double *__restrict__ wa1, const double *__res
 // one point (the normal equations with a 1e-14 relative diagonal shift).
 __global__ void k_shift_solve(const double *__restrict__ partial, int nblk, Grid3 g,
                               double *__restrict__ alpha) {
-  __shared__ double sh[32];
+  __shared__ double sh[kHalf];
   const int b = blockIdx.x;
   double s[9];
   for (int k = 0; k < 9; ++k) {
@@ -546,7 +632,9 @@ cudaError_t launch_residual(double *wa, double *wb, const double *pha, const dou
   double *dmean = err + 2 * batch;
   k_residual_sum<<<dim3(nblk, batch), kThreads, 0, st>>>(wa, wb, pha, phb, M, partial);
   k_residual_mean<<<batch, kThreads, 0, st>>>(partial, nblk, M, hAB, wcmp, dmean);
-  k_residual<<<dim3(nblk, batch), kThreads, 0, st>>>(
+  auto k = hu ? (wopt != 0.0 ? k_residual<true, true> : k_residual<true, false>)
+              : (wopt != 0.0 ? k_residual<false, true> : k_residual<false, false>);
+  k<<<dim3(nblk, batch), kThreads, 0, st>>>(
       wa, wb, pha, phb, hAB, wcmp, wopt, M, dmean, static_cast<dfloat *>(hu),
       static_cast<dfloat *>(hd), lam_u, wprev, partial);
   k_residual_finalize<<<batch, kThreads, 0, st>>>(partial, nblk, M, err);
@@ -563,9 +651,12 @@ cudaError_t launch_gram_row(const void *dc, const void *const *dj, const int *sl
     sl.d[k] = static_cast<const dfloat *>(dj[k]);
     sl.slot[k] = slots[k];
   }
-  k_gram_row<<<dim3(nblk, (n + kChunk - 1) / kChunk, batch), kThreads, 0, st>>>(
-      static_cast<const dfloat *>(dc), sl, M, partial);
-  k_gram_finalize<<<dim3(n, batch), kThreads, 0, st>>>(partial, nblk, sl, c, m1, G);
+  // one wave of four blocks an SM: a block's end costs 36 FP64 additions a slot
+  const int chunks = (n + kChunk - 1) / kChunk;
+  const int g = std::min(nblk, std::max(1, 4 * 152 / chunks));
+  k_gram_row<<<dim3(g, chunks, batch), kThreads, 0, st>>>(static_cast<const dfloat *>(dc), sl, M,
+                                                          partial);
+  k_gram_finalize<<<dim3(n, batch), kThreads, 0, st>>>(partial, g, sl, c, m1, G);
   return cudaGetLastError();
 }
 
@@ -598,7 +689,7 @@ cudaError_t launch_anderson_update(double *wa, double *wb, const void *const *hu
     sr.u[k] = static_cast<const dfloat *>(hu[k]);
     sr.idx[k] = idx[k];
   }
-  k_anderson_update<<<dim3(grid_for(2 * M), batch), kThreads, 0, st>>>(
+  k_anderson_update<<<dim3(grid_for(M), batch), kThreads, 0, st>>>(
       wa, wb, sr, static_cast<const dfloat *>(dc), a, lam, lam + batch, m1, M);
   return cudaGetLastError();
 }
