@@ -15,6 +15,13 @@
 // with the axis-a gain multiplied by 2 ds k_a^2 / L_a (k_a ~ 1/L_a), or, for
 // a length-1 axis (whose k is the constant 2 pi / L), the whole K times that
 // factor.  Hence dQ/dL_a = (1/M) sum_s <q+(s), W (dK/dL_a) W q(s-1)>.
+//
+// dK/dL_a = K D_a with D_a along axis a alone, and K W q(s-1) = q(s) / W, so that
+//   <q+(s), W (dK/dL_a) W q(s-1)> = <W^-1 D_a W q+(s), q(s)> :
+// one pass an axis and step instead of one an axis for every axis.  The whole
+// operator W K D_a W is applied where W or 1/W leaves 2^-60 .. 2^60, since the
+// quotient could lose what q(s) has left, and on axes that the tensor cores filter,
+// which have the one table of K_a D_a.
 #include <math.h>
 #include <string.h>
 
@@ -54,42 +61,62 @@ int grid_for(long long n) {
   return (int)std::min<long long>(g, 1 << 20);
 }
 
+// Sum over the block (kT threads) in thread 0, halves folding through shared memory
+// (sh: kT / 2 doubles): 12 FP64 additions of a warp where shuffles in every warp
+// take 45.
 __device__ __forceinline__ double block_sum(double v, double *sh) {
-  v = warp_sum(v);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (wid == 0) {
-    r = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-    r = warp_sum(r);
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int h = kT / 2; h >= 32; h /= 2) {
+    __syncthreads();
+    if (t >= h && t < 2 * h) sh[t - h] = v;
+    __syncthreads();
+    if (t < h) v += sh[t];
   }
-  __syncthreads();
-  return r;
+  if (t < 32) v = warp_sum(v);
+  return v;
 }
 
-// acc1[b*nblk + blk] += sum_{j<cnt, r} a[b,j,r] * c1[b,j,r]  (and acc2 with c2)
-// Slices j are M apart; every (b, blk) slot has one writer, so repeated
-// calls accumulate in a fixed order (bit-reproducible).
+// x in FP64.  A conversion costs the FP64 pipe as much as an FMA (16 cycles a
+// warp and SM), rebuilding the exponent in integers about a tenth of it.
+// (Denormal, infinite and NaN values go out of line: predicated in place the
+// conversion would take the pipe for every value.)
+__device__ __noinline__ double widen_rare(float x) { return (double)x; }
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return widen_rare(x);
+  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
+  return __hiloint2double((int)hi, (int)(u << 29));
+}
+__device__ __forceinline__ double widen(scft::dfloat x) { return widen(x.hi) + widen(x.lo); }
+
+// Two neighbouring points (grids have an even first axis).
+template <typename R> struct alignas(2 * sizeof(R)) Two {
+  R v[2];
+};
+template <typename R> __device__ __forceinline__ Two<R> two(const R *p) {
+  return *reinterpret_cast<const Two<R> *>(p);
+}
+template <typename R> __device__ __forceinline__ void put(R *p, const Two<R> &x) {
+  *reinterpret_cast<Two<R> *>(p) = x;
+}
+// acc1[b*nblk + blk] += sum_r a[b,r] * c1[b,r]  (and acc2 with c2).  Every (b, blk)
+// slot has one writer, so repeated calls accumulate in a fixed order
+// (bit-reproducible).
 template <typename R, typename S>
 __global__ void k_dot_acc(const R *__restrict__ a, long long a_bs, const S *__restrict__ c1,
                           long long c1_bs, const S *__restrict__ c2, long long c2_bs,
-                          long long M, int cnt, double *__restrict__ acc1,
-                          double *__restrict__ acc2) {
-  __shared__ double sh[32];
+                          long long M, double *__restrict__ acc1, double *__restrict__ acc2) {
+  __shared__ double sh[kT / 2];
   const long long b = blockIdx.y;
   const int nblk = gridDim.x;
   double v1 = 0.0, v2 = 0.0;
-  for (int j = 0; j < cnt; ++j) {
-    const R *aj = a + b * a_bs + (long long)j * M;
-    const S *c1j = c1 + b * c1_bs + (long long)j * M;
-    const S *c2j = c2 ? c2 + b * c2_bs + (long long)j * M : nullptr;
-    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < M;
-         r += (long long)nblk * blockDim.x) {
-      const double x = (double)aj[r];
-      v1 += x * (double)c1j[r];
-      if (c2j) v2 += x * (double)c2j[r];
-    }
+  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < M;
+       r += (long long)nblk * blockDim.x) {
+    const double x = widen(a[b * a_bs + r]);
+    v1 += x * widen(c1[b * c1_bs + r]);
+    if (c2) v2 += x * widen(c2[b * c2_bs + r]);
   }
   v1 = block_sum(v1, sh);
   if (threadIdx.x == 0) acc1[b * nblk + blockIdx.x] += v1;
@@ -99,9 +126,72 @@ __global__ void k_dot_acc(const R *__restrict__ a, long long a_bs, const S *__re
   }
 }
 
+// acc[k][blk] += sum_{r < n} x[k][r] * y[r] for N arrays x.  The FP64 pipe bounds it
+// (two operations a product of double-float values, y converted once for all), or
+// HBM: two points a load and U loads of each array in flight.  Its blocks do not
+// follow the grid's size: 64 slices of 30 x 16 x 32 on the 15 blocks of a single
+// slice took 52 us.
+constexpr int kDotBlocks = 3 * 152;
+template <typename R> struct DotArgs {
+  const R *x[4];
+  double *acc[4];
+  int n;
+};
+template <typename R, int N, int U>
+__global__ void __launch_bounds__(kT) k_dots(DotArgs<R> d, const R *__restrict__ y, long long n) {
+  __shared__ double sh[kT / 2];
+  double v[N][2] = {};
+  const long long S = 2 * (long long)gridDim.x * blockDim.x;
+  for (long long r0 = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); r0 < n; r0 += U * S) {
+    Two<R> tx[U][N], ty[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r0 + u * S < n) {
+        ty[u] = two(y + (r0 + u * S));
+#pragma unroll
+        for (int k = 0; k < N; ++k) tx[u][k] = two(d.x[k] + (r0 + u * S));
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r0 + u * S < n) {
+        const double y0 = widen(ty[u].v[0]), y1 = widen(ty[u].v[1]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          v[k][0] = fma(widen(tx[u][k].v[0]), y0, v[k][0]);
+          v[k][1] = fma(widen(tx[u][k].v[1]), y1, v[k][1]);
+        }
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double s = block_sum(v[k][0] + v[k][1], sh);
+    if (threadIdx.x == 0) d.acc[k][blockIdx.x] += s;
+  }
+}
+
+// out = 1 / W; *wide is set where W is not within 2^-60 .. 2^60.
+__device__ __forceinline__ float inverse(float w) { return 1.0f / w; }
+__device__ __forceinline__ double inverse(double w) { return 1.0 / w; }
+__device__ __forceinline__ scft::dfloat inverse(scft::dfloat w) {
+  return scft::dfloat(1.0 / (double)w);
+}
+__device__ __forceinline__ double size_of(float w) { return w; }
+__device__ __forceinline__ double size_of(double w) { return w; }
+__device__ __forceinline__ double size_of(scft::dfloat w) { return w.hi; }
+template <typename R>
+__global__ void k_inverse(const R *__restrict__ W, R *__restrict__ out, long long n,
+                          int *__restrict__ wide) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    const R w = W[i];
+    if (!(size_of(w) > 0x1p-60 && size_of(w) < 0x1p60)) *wide = 1;
+    out[i] = inverse(w);
+  }
+}
+
 // out[b] = sum_k partial[b*nblk + k]
 __global__ void k_sum_slots(const double *__restrict__ partial, int nblk, double *__restrict__ out) {
-  __shared__ double sh[32];
+  __shared__ double sh[kT / 2];
   const int b = blockIdx.x;
   double v = 0.0;
   for (int k = threadIdx.x; k < nblk; k += blockDim.x) v += partial[(long long)b * nblk + k];
@@ -109,19 +199,6 @@ __global__ void k_sum_slots(const double *__restrict__ partial, int nblk, double
   if (threadIdx.x == 0) out[b] = v;
 }
 
-// x in FP64.  A conversion costs the FP64 pipe as much as an FMA (16 cycles a
-// warp and SM), rebuilding the exponent in integers about a tenth of it.
-// (Denormal, infinite and NaN values go out of line: predicated in place the
-// conversion would take the pipe for every value.)
-__device__ __noinline__ double widen_rare(float x) { return (double)x; }
-__device__ __forceinline__ double widen(double x) { return x; }
-__device__ __forceinline__ double widen(scft::dfloat x) { return (double)x; }
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return widen_rare(x);
-  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
-  return __hiloint2double((int)hi, (int)(u << 29));
-}
 // x rounded to the working precision, to nearest even (float: in integers, again)
 __device__ __noinline__ float narrow_rare(double x) { return (float)x; }
 __device__ __forceinline__ void narrow(double x, double &r) { r = x; }
@@ -137,16 +214,6 @@ __device__ __forceinline__ void narrow(double x, float &r) {
   const uint32_t f = m ? ((m - 0x38000000u) << 3) | (lo >> 29) : 0u, rest = lo & 0x1fffffffu;
   const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
   r = __uint_as_float((hi & 0x80000000u) | (f + up));
-}
-// Two neighbouring points (grids have an even first axis).
-template <typename R> struct alignas(2 * sizeof(R)) Two {
-  R v[2];
-};
-template <typename R> __device__ __forceinline__ Two<R> two(const R *p) {
-  return *reinterpret_cast<const Two<R> *>(p);
-}
-template <typename R> __device__ __forceinline__ void put(R *p, const Two<R> &x) {
-  *reinterpret_cast<Two<R> *>(p) = x;
 }
 // One contour point's weights in the accumulators of sums of q q+ (S: the density
 // sums; G: the sums of the Q part, Simpson only) and in the adjoint seed.  How they
@@ -314,7 +381,7 @@ struct AdjointState {
   double *small = nullptr;      // [8][B]
   // stress chunk buffers
   size_t sbytes = 0, sacc_off = 0;
-  void *smem = nullptr;          // chunk x 3 slices, then reduction slots
+  void *smem = nullptr;          // chunk x 3 slices, 1/W, then reduction slots
   int chunk = 0;
 };
 
@@ -376,6 +443,23 @@ int ensure_adjoint(scft_ctx *ctx, int K) {
   A.acc = static_cast<double *>(take(8 * (size_t)kAccKinds * B * ctx->nblk));
   A.small = static_cast<double *>(take(8 * (8 + (size_t)kAccKinds) * B));
   return SCFT_OK;
+}
+
+// Whether axis pass pi takes W K D_a W; out = that of `in` (s0, s1: scratch, `out`
+// the result's place among them).
+bool whole_axis(const scft_ctx *ctx, int pi, int wide) { return wide || ctx->passes[pi].tc; }
+template <typename R>
+int whole_term(scft_ctx *ctx, int pi, const R *in, long long in_bs, const R *W, long long w_bs,
+               int nb, R *t, R *s0, R *s1, const R **out, cudaStream_t st) {
+  const long long M = ctx->M;
+  if (ctx->passes[pi].tc) {
+    *out = t;
+    return scft_internal_filter(ctx, in, in_bs, t, M, W, W, w_bs, nb, pi, s0, s1, st);
+  }
+  RC(scft_internal_deriv(ctx, pi, in, in_bs, t, M, W, nullptr, w_bs, nb, st));
+  R *o = ctx->passes.size() == 1 ? s0 : t;
+  *out = o;
+  return scft_internal_filter(ctx, t, M, o, M, nullptr, W, w_bs, nb, -1, o == s0 ? s1 : s0, s1, st);
 }
 
 template <typename R>
@@ -516,8 +600,7 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
 
   auto dot = [&](const R *a, long long a_bs, const R *c1, long long c1_bs, const R *c2,
                  long long c2_bs, double *acc1, double *acc2) {
-    k_dot_acc<R, R><<<dim3(nblk, B), kT, 0, st>>>(a, a_bs, c1, c1_bs, c2, c2_bs, M, 1, acc1,
-                                                   acc2);
+    k_dot_acc<R, R><<<dim3(nblk, B), kT, 0, st>>>(a, a_bs, c1, c1_bs, c2, c2_bs, M, acc1, acc2);
     ++ctx->launches;
     return cudaGetLastError();
   };
@@ -542,6 +625,21 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
     }
     return pt;
   };
+
+  // the box derivatives' 1/W (the marching pair is free), and whether it will do
+  R *Winv[2] = {va, vb};
+  int wide = 0;
+  if (want_L) {
+    int *flag = reinterpret_cast<int *>(A.small + 4 * B);
+    CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    for (int f = 0; f < 2; ++f) {
+      k_inverse<R><<<grid_for(M * B), kT, 0, st>>>(W[f], Winv[f], M * B, flag);
+      ++ctx->launches;
+    }
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
 
   // ---- the sweeps: the q chain's in reverse (s = N .. 1, q+ marched alongside),
   // then the q+ chain's (s = 1 .. N, q marched alongside)
@@ -568,8 +666,13 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
       if (want_L) {
         const int L = q_chain ? ACC_L1 : ACC_L2;
         for (int pi = 0; pi < np; ++pi) {
-          RC(scft_internal_filter(ctx, x0, bs0, t, M, W[f], W[f], M, B, pi, s0, s1, st));
-          CK(dot(t, M, a, M, q_chain ? co : nullptr, M, accp(L + pi),
+          const R *d = t;
+          const bool whole = whole_axis(ctx, pi, wide);
+          if (whole)   // <a, W K D W x0>
+            RC(whole_term<R>(ctx, pi, x0, bs0, W[f], M, B, t, s0, s1, &d, st));
+          else         // = <A a, W^-1 D W x0>
+            RC(scft_internal_deriv(ctx, pi, x0, bs0, t, M, W[f], Winv[f], M, B, st));
+          CK(dot(d, M, whole ? a : p, M, q_chain ? (whole ? co : co_n) : nullptr, M, accp(L + pi),
                  q_chain ? accp(ACC_Q + pi) : nullptr));
         }
         if (has_unit)
@@ -590,9 +693,9 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
     }
   }
   // ---- the Q part: Qbar_tot = Qbar - fflbar ds / Q^2, fflbar = <phibar, S>
-  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[0], M, S[0], M, nullptr, 0, M, 1,
+  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[0], M, S[0], M, nullptr, 0, M,
                                                           accp(ACC_FFL), nullptr);
-  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[1], M, S[1], M, nullptr, 0, M, 1,
+  k_dot_acc<double, double><<<dim3(nblk, B), kT, 0, st>>>(pb[1], M, S[1], M, nullptr, 0, M,
                                                           accp(ACC_FFL), nullptr);
   ctx->launches += 2;
   CK(cudaGetLastError());
@@ -639,61 +742,106 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   return SCFT_OK;
 }
 
-// Box stress from the propagators stored by the last getConc: for every
-// contour step s (all independent, so batched `chunk` steps per launch),
-// t = W (dK/dL_a) W q(s-1), contracted with q+(s) in FP64.
+// Box stress from the propagators stored by the last getConc (200 steps, ms: 128 x
+// 128 x 64 pairs 22.2 -> 10.2, FP64 24 x 32 x 32 0.81 -> 0.50): for every contour step s (all independent, so batched `chunk` steps per launch) and axis a,
+// W^-1 D_a W q+(s) contracted with q(s) in FP64, or (whole_axis) W K D_a W q(s-1)
+// with q+(s).
 template <typename R>
-int stress_impl(scft_ctx *ctx, double *h_out) {
+int stress_sums(scft_ctx *ctx, bool wide, double *acc, int *flag) {
   AdjointState &A = *ctx->adj;
   const long long M = ctx->M;
-  const int B = ctx->batch, nblk = ctx->nblk, np = (int)ctx->passes.size();
+  const int B = ctx->batch, nblk = kDotBlocks, np = (int)ctx->passes.size();
   cudaStream_t st = ctx->st;
   const int chunk = A.chunk;
-  R *tb = static_cast<R *>(A.smem);
-  R *s0 = tb + (long long)chunk * M, *s1 = s0 + (long long)chunk * M;
-  // [4 kinds][B][nblk]: passes 0..2 and the unit term, then [4][B] sums
-  double *acc = reinterpret_cast<double *>(static_cast<unsigned char *>(A.smem) + A.sacc_off);
-  double *sums = acc + (size_t)4 * B * nblk;
+  R *t[3];
+  for (int k = 0; k < 3; ++k) t[k] = static_cast<R *>(A.smem) + (long long)k * chunk * M;
+  R *winv = t[2] + (long long)chunk * M;
   CK(cudaMemsetAsync(acc, 0, sizeof(double) * 4 * B * nblk, st));
   struct Block { int q, qc, f, ns; };
   const Block blocks[2] = {{SCFT_Q_A, SCFT_Q_CA, 0, ctx->NsA}, {SCFT_Q_B, SCFT_Q_CB, 1, ctx->dNsB}};
   bool has_unit = false;
   for (int a = 0; a < 3; ++a) has_unit |= ctx->unit_c[a] != 0.0;
+  bool quotient = false;
+  for (int pi = 0; pi < np; ++pi) quotient |= !whole_axis(ctx, pi, wide);
+  auto dots = [&](const DotArgs<R> &d, const R *y, int cnt) {
+    const long long n = cnt * M;
+    switch (d.n) {
+      case 1: k_dots<R, 1, 4><<<nblk, kT, 0, st>>>(d, y, n); break;
+      case 2: k_dots<R, 2, 2><<<nblk, kT, 0, st>>>(d, y, n); break;
+      case 3: k_dots<R, 3, 2><<<nblk, kT, 0, st>>>(d, y, n); break;
+      default: k_dots<R, 4, 1><<<nblk, kT, 0, st>>>(d, y, n); break;
+    }
+    ++ctx->launches;
+    return cudaGetLastError();
+  };
   for (const Block &bl : blocks) {
     const R *q = static_cast<const R *>(ctx->q[bl.q]);
     const R *qc = static_cast<const R *>(ctx->q[bl.qc]);
     const long long qbs = (long long)(bl.ns + 1) * M;
-    const R *Wf = static_cast<const R *>(ctx->W[bl.f]);
-    for (int b = 0; b < B; ++b)
+    for (int b = 0; b < B && bl.ns > 0; ++b) {
+      const R *W = static_cast<const R *>(ctx->W[bl.f]) + b * M;
+      if (quotient) {
+        k_inverse<R><<<grid_for(M), kT, 0, st>>>(W, winv, M, flag);
+        ++ctx->launches;
+        CK(cudaGetLastError());
+      }
+      auto slots = [&](int kind) { return acc + ((size_t)kind * B + b) * nblk; };
       for (int s1st = 1; s1st <= bl.ns; s1st += chunk) {
         const int cnt = std::min(chunk, bl.ns - s1st + 1);
         const R *qin = q + b * qbs + (long long)(s1st - 1) * M;    // q(s-1)
         const R *qcs = qc + b * qbs + (long long)s1st * M;         // q+(s)
+        // the whole operators one after the other, then the quotient forms, which
+        // keep a buffer each, with one reading of q(s)
         for (int pi = 0; pi < np; ++pi) {
-          RC(scft_internal_filter(ctx, qin, M, tb, M, Wf + b * M, Wf + b * M, 0, cnt, pi, s0, s1,
-                                  st));
-          k_dot_acc<R, R><<<dim3(nblk, 1), kT, 0, st>>>(tb, 0, qcs, 0, nullptr, 0, M, cnt,
-                                                        acc + ((size_t)pi * B + b) * nblk,
-                                                        nullptr);
-          ++ctx->launches;
-          CK(cudaGetLastError());
+          if (!whole_axis(ctx, pi, wide)) continue;
+          DotArgs<R> one = {};
+          RC(whole_term<R>(ctx, pi, qin, M, W, 0, cnt, t[0], t[1], t[2], &one.x[0], st));
+          one.acc[0] = slots(pi);
+          one.n = 1;
+          CK(dots(one, qcs, cnt));
         }
-        if (has_unit) {   // W K W q(s-1) = q(s)
-          k_dot_acc<R, R><<<dim3(nblk, 1), kT, 0, st>>>(qin + M, 0, qcs, 0, nullptr, 0, M, cnt,
-                                                        acc + ((size_t)3 * B + b) * nblk,
-                                                        nullptr);
-          ++ctx->launches;
-          CK(cudaGetLastError());
+        DotArgs<R> d = {};
+        for (int pi = 0; pi < np; ++pi) {
+          if (whole_axis(ctx, pi, wide)) continue;
+          RC(scft_internal_deriv(ctx, pi, qcs, M, t[pi], M, W, winv, 0, cnt, st));
+          d.x[d.n] = t[pi];
+          d.acc[d.n++] = slots(pi);
         }
+        if (has_unit) {   // <q+(s), W K W q(s-1)>
+          d.x[d.n] = qcs;
+          d.acc[d.n++] = slots(3);
+        }
+        if (d.n) CK(dots(d, qin + M, cnt));
       }
+    }
   }
+  return SCFT_OK;
+}
+
+template <typename R>
+int stress_impl(scft_ctx *ctx, double *h_out) {
+  AdjointState &A = *ctx->adj;
+  const long long M = ctx->M;
+  const int B = ctx->batch, nblk = kDotBlocks, np = (int)ctx->passes.size();
+  cudaStream_t st = ctx->st;
+  // [4 kinds][B][nblk]: passes 0..2 and the unit term, then [4][B] sums, a flag
+  double *acc = reinterpret_cast<double *>(static_cast<unsigned char *>(A.smem) + A.sacc_off);
+  double *sums = acc + (size_t)4 * B * nblk;
+  int *flag = reinterpret_cast<int *>(sums + 4 * B);
+  CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
   std::vector<double> s_h(4 * (size_t)B), hQ(B);
-  k_sum_slots<<<4 * B, kT, 0, st>>>(acc, nblk, sums);
-  ++ctx->launches;
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(s_h.data(), sums, 8 * 4 * B, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(hQ.data(), ctx->Q, 8 * B, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  int wide = 0;
+  for (int again = 0; again < 2; ++again) {
+    RC(stress_sums<R>(ctx, again != 0, acc, flag));
+    k_sum_slots<<<4 * B, kT, 0, st>>>(acc, nblk, sums);
+    ++ctx->launches;
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(s_h.data(), sums, 8 * 4 * B, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hQ.data(), ctx->Q, 8 * B, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (!wide) break;
+  }
   for (int b = 0; b < B; ++b) {
     const double scale = -1.0 / ((double)M * hQ[b]);   // -d ln Q / dL
     for (int a = 0; a < 3; ++a) h_out[3 * b + a] = 0.0;
@@ -748,14 +896,19 @@ int scft_stress(scft_ctx *ctx, double *dF_dL) {
   if (!ctx->adj) ctx->adj = new AdjointState();
   AdjointState &A = *ctx->adj;
   if (!A.smem) {
-    // up to 64 contour steps per launch, the three chunk buffers <= 768 MB
+    // up to 64 contour steps per launch.  FFT passes: the three chunk buffers <= 96
+    // MB, with the slices that they are made from and contracted with in the L2.
+    // Tensor-core passes, one CTA an SM, want long launches (128 x 128 x 64 FP64: 32
+    // steps a launch 24 ms, 4 steps 32 ms): <= 768 MB.
     const long long per = ctx->M * ctx->rbytes;
-    int chunk = (int)std::min<long long>(64, std::max<long long>(1, (256LL << 20) / per));
+    bool tc = false;
+    for (const scft::AxisPlan &ap : ctx->passes) tc |= ap.tc != nullptr;
+    int chunk = (int)std::min<long long>(64, std::max<long long>(1, ((tc ? 256LL : 32LL) << 20) / per));
     chunk = std::min(chunk, std::max(ctx->NsA, ctx->dNsB));
     chunk = std::max(chunk, 1);
     A.chunk = chunk;
-    A.sacc_off = ((size_t)3 * chunk * per + 255) & ~(size_t)255;
-    A.sbytes = A.sacc_off + 8 * ((size_t)4 * ctx->batch * ctx->nblk + 4 * ctx->batch);
+    A.sacc_off = ((size_t)(3 * chunk + 1) * per + 255) & ~(size_t)255;
+    A.sbytes = A.sacc_off + 8 * ((size_t)4 * ctx->batch * kDotBlocks + 4 * ctx->batch + 1);
     CK(cudaMalloc(&A.smem, A.sbytes));
   }
   return with_real(ctx, [&](auto r) { return stress_impl<decltype(r)>(ctx, dF_dL); });

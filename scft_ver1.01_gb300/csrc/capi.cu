@@ -74,8 +74,11 @@ int upload_tc(scft_ctx *ctx, int pi, const std::vector<double> &g, const std::ve
 
 // Gains of the passes (kxyzdz, init_cuda.cu:394-428, split per axis:
 // exp(-ds0 k^2)/n, with the constant factors of length-1 axes folded into the
-// first pass) and their box derivatives: d/dL_a of exp(-ds0 k_a^2) is
-// exp(-ds0 k_a^2) * 2 ds0 k_a^2 / L_a because k_a is proportional to 1/L_a.
+// first pass) and their logarithmic box derivatives: d/dL_a of exp(-ds0 k_a^2) is
+// exp(-ds0 k_a^2) * 2 ds0 k_a^2 / L_a because k_a is proportional to 1/L_a; dgain
+// holds (2 ds0 k_a^2 / L_a) / n, the operator D_a with dK/dL_a = K D_a, and the
+// tensor-core table of an axis K_a D_a (D_a's own range of sizes would leave its
+// low wave numbers few bits: stresses 1e-13 off instead of 1e-15).
 // Rewritten in place when the box changes.
 int upload_gains(scft_ctx *ctx) {
   const scft_params &p = ctx->p;
@@ -99,11 +102,12 @@ int upload_gains(scft_ctx *ctx) {
     const AxisPlan &ap = ctx->passes[pi];
     const int a = ctx->pass_axis[pi];
     const std::vector<double> k2 = k2_axis(ap.n, lens[a]);
-    std::vector<double> g(ap.n), dg(ap.n);
+    std::vector<double> g(ap.n), dg(ap.n), kdg(ap.n);
     for (int m = 0; m < ap.n; ++m) {
       g[m] = exp(-p.ds0 * k2[m]) / ap.n;
       if (pi == 0) g[m] *= scalar;
-      dg[m] = g[m] * 2.0 * p.ds0 * k2[m] / lens[a];
+      dg[m] = 2.0 * p.ds0 * k2[m] / lens[a] / ap.n;
+      kdg[m] = g[m] * 2.0 * p.ds0 * k2[m] / lens[a];
     }
     void *dptr = static_cast<unsigned char *>(ctx->dgain) + doff;
     ctx->dgain_pass[pi] = dptr;
@@ -121,7 +125,7 @@ int upload_gains(scft_ctx *ctx) {
       CK(cudaMemcpy(dptr, dg.data(), 8 * ap.n, cudaMemcpyHostToDevice));
     }
     if (ctx->tc_want[pi]) {
-      const int rc = upload_tc(ctx, (int)pi, g, dg);
+      const int rc = upload_tc(ctx, (int)pi, g, kdg);
       if (rc) return rc;
     }
   }
@@ -1021,8 +1025,8 @@ int scft_internal_get_conc(scft_ctx *ctx) { return get_conc(ctx); }
 namespace {
 template <typename R>
 int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long out_bs,
-                const R *pre, const R *post, long long w_bs, int nb, int deriv_pass, R *s0,
-                R *s1, cudaStream_t st) {
+                const R *pre, const R *post, long long w_bs, int nb, int tc_deriv, R *s0, R *s1,
+                cudaStream_t st) {
   const long long M = ctx->M;
   const int np = (int)ctx->passes.size();
   for (int pi = 0; pi < np; ++pi) {
@@ -1038,10 +1042,7 @@ int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long o
     p.pre[0] = pi == 0 ? pre : nullptr;
     p.post[0] = pi == np - 1 ? post : nullptr;
     AxisPlan ap = ctx->passes[pi];
-    if (pi == deriv_pass) {
-      ap.gain = ctx->dgain_pass[pi];
-      ap.tc = ctx->dtc_pass[pi];
-    }
+    if (pi == tc_deriv) ap.tc = ctx->dtc_pass[pi];
     int rc = launch_set(ctx, ap, p, st);
     if (rc) return rc;
   }
@@ -1094,11 +1095,34 @@ int scft_internal_steps(scft_ctx *ctx, const StepIO *io, int n, long long w_bs, 
 
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,
-                         int nb, int deriv_pass, void *s0, void *s1, cudaStream_t st) {
+                         int nb, int tc_deriv, void *s0, void *s1, cudaStream_t st) {
   return with_real(ctx, [&](auto r) {
     using R = decltype(r);
     return filter_impl<R>(ctx, (const R *)in, in_bs, (R *)out, out_bs, (const R *)pre,
-                          (const R *)post, w_bs, nb, deriv_pass, (R *)s0, (R *)s1, st);
+                          (const R *)post, w_bs, nb, tc_deriv, (R *)s0, (R *)s1, st);
+  });
+}
+
+int scft_internal_deriv(scft_ctx *ctx, int pi, const void *in, long long in_bs, void *out,
+                        long long out_bs, const void *pre, const void *post, long long w_bs, int nb,
+                        cudaStream_t st) {
+  return with_real(ctx, [&](auto r) {
+    using R = decltype(r);
+    scft::PassSet<R> p;
+    memset(&p, 0, sizeof(p));
+    p.nset = 1;
+    p.batch = nb;
+    p.w_bs = w_bs;
+    p.in[0] = (const R *)in;
+    p.in_bs[0] = in_bs;
+    p.out[0] = (R *)out;
+    p.out_bs[0] = out_bs;
+    p.pre[0] = (const R *)pre;
+    p.post[0] = (const R *)post;
+    AxisPlan ap = ctx->passes[pi];
+    ap.gain = ctx->dgain_pass[pi];
+    ap.tc = nullptr;
+    return launch_set(ctx, ap, p, st);
   });
 }
 

@@ -115,12 +115,17 @@ int scft_fail(scft_ctx *ctx, int status, const std::string &msg);
 
 // One application of the step operator's diffusion part to nb slices:
 // out = post * K (pre * in), K = the per-axis line filters of the context
-// (x, y, z passes, no plane fusion).  deriv_pass >= 0 swaps that pass's gain
-// for its box-derivative gain.  s0 and s1 hold the intermediates (nb slices
-// of M each); in, out, s0 and s1 must not overlap.  Working precision.
+// (x, y, z passes, no plane fusion).  tc_deriv >= 0: pass tc_deriv (on the tensor
+// cores) with its table of K_a D_a, D_a = d ln K / dL_a.  s0 and s1 hold the
+// intermediates (nb slices of M each); in, out, s0 and s1 must not overlap (with
+// one or two passes s1 is not used).  Working precision.
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,
-                         int nb, int deriv_pass, void *s0, void *s1, cudaStream_t st);
+                         int nb, int tc_deriv, void *s0, void *s1, cudaStream_t st);
+// out = post * D_a (pre * in): one FFT pass along pass pi's axis.
+int scft_internal_deriv(scft_ctx *ctx, int pi, const void *in, long long in_bs, void *out,
+                        long long out_bs, const void *pre, const void *post, long long w_bs, int nb,
+                        cudaStream_t st);
 // One split step W K W of up to kStepSet chains side by side (x and y fused where
 // the march has them so).  scratch[k]: [nb][M]; nothing may overlap.
 struct StepIO {
