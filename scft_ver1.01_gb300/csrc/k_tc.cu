@@ -68,20 +68,23 @@ template <typename F> __device__ __forceinline__ void over_rows(int nt, int n, i
   }
 }
 
-// f(row, column, offset, src[offset]), four loads in flight per thread
-template <typename F>
-__device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *src, F &&f) {
+// f(row, column, offset, load(offset)) with U loads in flight per thread.  One at a
+// time the FP32 x passes waited for them (100 x 80 x 60: 26 us where a column pass
+// takes 10; 4.8 ms per SCF iteration, with 8 in flight 4.3).  64-bit values take 4:
+// 8 were no faster (96^3 9.7 against 9.4 ms) and spilled.
+template <int U, typename L, typename F>
+__device__ __forceinline__ void over_rows(int nt, int n, int nl, L &&load, F &&f) {
+  typedef decltype(load(0)) V;
   const int total = nl * n;
   int r = (int)threadIdx.x / n, col = (int)threadIdx.x % n;
   const int dr = nt / n, dc = nt % n;
 #pragma unroll 1
-  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * nt) {
-    int64_t x[4];
+  for (int i0 = threadIdx.x; i0 < total; i0 += U * nt) {
+    V x[U];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      x[j] = i0 + j * nt < total ? __ldg(reinterpret_cast<const long long *>(src) + (i0 + j * nt)) : 0;
+    for (int j = 0; j < U; ++j) x[j] = i0 + j * nt < total ? load(i0 + j * nt) : V();
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < U; ++j) {
       if (i0 + j * nt < total) f(r, col, i0 + j * nt, x[j]);
       r += dr;
       col += dc;
@@ -92,6 +95,14 @@ __device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *
     }
   }
 }
+template <typename F>
+__device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *src, F &&f) {
+  over_rows<4>(nt, n, nl,
+               [&](int i) { return (int64_t)__ldg(reinterpret_cast<const long long *>(src) + i); }, f);
+}
+template <typename T> struct WithFactor {
+  T x, w;
+};
 
 // ------------------------------------------------------------------ k_real
 template <typename T, int MAXT, int PP, bool XP, bool PAIR>
@@ -144,11 +155,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
   T a[PP], bb[PP];
   if constexpr (XP) {
     const T *src = in + tile, *wsrc = pre ? pre + tile : nullptr;
-    over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
-      T x = ldg(src + i);
-      if (wsrc) x = x * ldg(wsrc + i);
-      stg[r * P + col] = x;
-    });
+    constexpr int U = sizeof(T) == 4 ? 8 : 4;
+    if (wsrc)
+      over_rows<U>(e.ncomp, ln.n, nl, [&](int i) { return WithFactor<T>{ldg(src + i), ldg(wsrc + i)}; },
+                   [&](int r, int col, int, WithFactor<T> v) { stg[r * P + col] = v.x * v.w; });
+    else
+      over_rows<U>(e.ncomp, ln.n, nl, [&](int i) { return ldg(src + i); },
+                   [&](int r, int col, int, T x) { stg[r * P + col] = x; });
     e.sync();
   }
 #pragma unroll
@@ -211,8 +224,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
         }
       }
       e.sync();
-      over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
-        const T w = ldg(post + tile + i);
+      over_rows<8>(e.ncomp, ln.n, nl, [&](int i) { return ldg(post + tile + i); },
+                   [&](int r, int col, int i, T w) {
         const T q = stg[r * P + col] * w;
         qo[tile + i] = q;
         stg[r * P + col] = q * w;
@@ -274,11 +287,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     }
     e.sync();
     const T *wd = !PAIR && post ? post + tile : nullptr;
-    over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) {
-      T x = stg[r * P + col];
-      if (wd) x = x * ldg(wd + i);
-      out[tile + i] = x;
-    });
+    if (wd)
+      over_rows<4>(e.ncomp, ln.n, nl, [&](int i) { return ldg(wd + i); },
+                   [&](int r, int col, int i, T w) { out[tile + i] = stg[r * P + col] * w; });
+    else
+      over_rows(e.ncomp, ln.n, nl, [&](int r, int col, int i) { out[tile + i] = stg[r * P + col]; });
   } else {
     e.filter(xa, xb, []() {}, [&](int i, Acc p, Acc q) {
       const int k = PP * e.blk + i;
@@ -856,10 +869,13 @@ __global__ void __launch_bounds__(544, 1)
   const int lim_y = e.line < np * nx ? pa.sh.half[1] - k0 : 0;
   const int at_x = e.line * P + k0, at_y = (pl * ny + k0) * P + xx;
   const unsigned off = tile + (unsigned)(pl * ny + k0) * nx + xx, ghs = pa.sh.half[1] * nx;
-  over_rows(e.ncomp, nx, np * ny, [&](int r, int cc, int i) {
-    const float x = __ldg(in + tile + i);
-    S[r * P + cc] = pre ? x * __ldg(pre + tile + i) : x;
-  });
+  if (pre)
+    over_rows<8>(e.ncomp, nx, np * ny,
+                 [&](int i) { return WithFactor<float>{__ldg(in + tile + i), __ldg(pre + tile + i)}; },
+                 [&](int r, int cc, int, WithFactor<float> v) { S[r * P + cc] = v.x * v.w; });
+  else
+    over_rows<8>(e.ncomp, nx, np * ny, [&](int i) { return __ldg(in + tile + i); },
+                 [&](int r, int cc, int, float x) { S[r * P + cc] = x; });
   e.start();
 #pragma unroll 1
   for (int f = 0; f < filters; ++f) {
