@@ -1377,7 +1377,7 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
     return fail(SCFT_ERR_CUDA, "table upload failed");
   // Passes on the tensor cores: every FP64 line they take, and FP32 lines without
   // a register kernel.  Measured, ms per SCF iteration with 200 contour steps:
-  // FP64 64^3 22 -> 3.5, 128^3 107 -> 22; FP32 100x80x60 24 -> 4.4.  FP32 and
+  // FP64 64^3 22 -> 3.5, 128^3 107 -> 22; FP32 100x80x60 24 -> 4.2.  FP32 and
   // double-float lines with a register kernel keep it (64^3: FP32 1.2; double-float
   // 4.0 against 5.5 on passes of the first form).
   size_t tc_bytes = 0;
