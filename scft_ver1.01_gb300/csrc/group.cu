@@ -145,9 +145,11 @@ int make_buckets(scft_group *g) {
     bool fused = true;
     for (int m : b.mem) fused = fused && g->members[m]->fuse_steps;
     if (fused && ctas > 0 && 2 * ctas * (long long)b.mem.size() <= kOwnCtas) continue;
+    // (the tensor cores' batched planes are pre, x, y: a later pass closes the step)
     if (c0->passes.size() >= 2 && c0->pass_axis[0] == 0 && c0->pass_axis[1] == 1)
       b.xy = c0->passes[0].tc && c0->passes[1].tc
-                 ? scft::tc_planes_wanted(c0->p.nx, c0->p.ny, c0->p.nz, 4, (int)b.mem.size())
+                 ? c0->passes.size() == 3 &&
+                       scft::tc_planes_wanted(c0->p.nx, c0->p.ny, c0->p.nz, 4, (int)b.mem.size())
                  : scft::xy_fusable(c0->passes[0], c0->passes[1]);
     b.npass = (int)c0->passes.size() - (b.xy ? 1 : 0);
     for (int m : b.mem) {
