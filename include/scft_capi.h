@@ -146,6 +146,10 @@ int scft_get_field(scft_ctx *ctx, int field, double *dst);
  * wait gave up and reported through the device error word (the kernel returns;
  * nothing traps or hangs).  Returns SCFT_OK while the device stays usable. */
 int scft_selftest_bounded_wait(int device, double seconds, int *timed_out);
+/* Sets the context's device error word, as a kernel does that gives up a bounded
+ * wait (word 1 or 2): the next call that waits for results, of the context or of
+ * a group that it is in, must return SCFT_ERR_CUDA. */
+int scft_selftest_set_error(scft_ctx *ctx, unsigned word);
 
 /* Zero-copy access (no reference counterpart; the reference hands out its
  * per-GPU device pointers through CUFFT_INFO, struct.h:94-121): the device

@@ -43,7 +43,8 @@ EXPORTS = [
     "scft_save_checkpoint", "scft_load_checkpoint", "scft_set_metrics_file",
     "scft_phi_w_constrained", "scft_set_box", "scft_stress", "scft_adjoint",
     "scft_adjoint_checkpoints", "scft_relax_cell", "scft_get_box", "scft_field_device_ptr",
-    "scft_get_stream", "scft_copy_q_reference_layout", "scft_selftest_bounded_wait", "scft_spline", "scft_spline_eval",
+    "scft_get_stream", "scft_copy_q_reference_layout", "scft_selftest_bounded_wait",
+    "scft_selftest_set_error", "scft_spline", "scft_spline_eval",
     "scft_spline_deriv", "scft_spline_integral", "scft_spline_eval_device",
     "scft_shard_plan", "scft_free_shards",
 ]
@@ -142,6 +143,7 @@ def load_library(path: str | None = None):
         "scft_get_stream": (C.c_int, [vp, C.POINTER(vp)]),
         "scft_copy_q_reference_layout": (C.c_int, [vp, C.c_int, vp]),
         "scft_selftest_bounded_wait": (C.c_int, [C.c_int, C.c_double, C.POINTER(C.c_int)]),
+        "scft_selftest_set_error": (C.c_int, [vp, C.c_uint]),
         "scft_spline": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_double, C.c_double, dp, dp, dp,
                                   dp, dp, C.POINTER(C.c_int)]),
         "scft_spline_eval": (C.c_double, [C.c_int, C.c_double, dp, dp, dp, dp, dp,

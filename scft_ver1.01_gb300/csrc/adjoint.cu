@@ -725,7 +725,7 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
   CKL(scft::launch_minus_average(wbar[0], sum, M, B, st));
   if (h_wabar) CK(cudaMemcpyAsync(h_wabar, wbar[0], dbytes, cudaMemcpyDeviceToHost, st));
   if (h_wbbar) CK(cudaMemcpyAsync(h_wbbar, wbar[1], dbytes, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  RC(scft_internal_sync_check(ctx));
   if (want_L) {
     for (int b = 0; b < B; ++b) {
       for (int a = 0; a < 3; ++a) h_Lbar[3 * b + a] = 0.0;
@@ -839,7 +839,7 @@ int stress_impl(scft_ctx *ctx, double *h_out) {
     CK(cudaMemcpyAsync(s_h.data(), sums, 8 * 4 * B, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hQ.data(), ctx->Q, 8 * B, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    RC(scft_internal_sync_check(ctx));
     if (!wide) break;
   }
   for (int b = 0; b < B; ++b) {

@@ -819,20 +819,7 @@ int free_energy_dev(scft_ctx *ctx) {
   return SCFT_OK;
 }
 
-// Synchronise the stream and check the device error word that the pipelined
-// kernels set when a bounded wait gives up.
-int sync_check(scft_ctx *ctx) {
-  CK(cudaStreamSynchronize(ctx->st));
-  unsigned w = 0;
-  CK(cudaMemcpy(&w, ctx->dev_err, sizeof(w), cudaMemcpyDeviceToHost));
-  if (w) {
-    cudaMemset(ctx->dev_err, 0, sizeof(unsigned));
-    return scft_fail(ctx, SCFT_ERR_CUDA,
-                     "a pipelined kernel timed out waiting for its bulk copies (error word " +
-                         std::to_string(w) + "); results of that launch are invalid");
-  }
-  return SCFT_OK;
-}
+int sync_check(scft_ctx *ctx) { return scft_internal_sync_check(ctx); }
 
 int read_fe(scft_ctx *ctx, double *out5) {
   CK(cudaMemcpyAsync(out5, ctx->fe5, sizeof(double) * 5 * ctx->batch, cudaMemcpyDeviceToHost,
@@ -885,6 +872,26 @@ void free_all(scft_ctx *ctx) {
 }
 
 }  // namespace
+
+int scft_internal_sync_check(scft_ctx *ctx) {
+  CK(cudaStreamSynchronize(ctx->st));
+  unsigned w = 0;
+  CK(cudaMemcpy(&w, ctx->dev_err, sizeof(w), cudaMemcpyDeviceToHost));
+  if (w) {
+    CK(cudaMemset(ctx->dev_err, 0, sizeof(unsigned)));
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
+    return scft_internal_wait_failed(ctx, w);
+  }
+  return SCFT_OK;
+}
+int scft_internal_wait_failed(scft_ctx *ctx, unsigned word) {
+  ctx->have_conc = false;   // the propagators may be that launch's
+  return scft_fail(ctx, SCFT_ERR_CUDA, scft_internal_wait_message(word));
+}
+std::string scft_internal_wait_message(unsigned word) {
+  return "a kernel gave up waiting for its copies or products (error word " +
+         std::to_string(word) + "); results of that launch are invalid";
+}
 
 // Schedule autotuner: every legal combination of chain schedule (lockstep /
 // two streams), x+y fusion and column-pass kernel (one tile per CTA /
@@ -1523,8 +1530,7 @@ int scft_get_q(scft_ctx *ctx, int q, int s, double *dst) {
   }
   CK(cudaMemcpyAsync(dst, stage, sizeof(double) * M * ctx->batch, cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaFreeAsync(stage, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
-  return SCFT_OK;
+  return sync_check(ctx);
 }
 
 int scft_get_conc(scft_ctx *ctx) {
@@ -1535,8 +1541,7 @@ int scft_get_conc(scft_ctx *ctx) {
 int scft_get_Q(scft_ctx *ctx, double *dst) {
   if (!ctx || !dst) return SCFT_ERR_INVALID_ARG;
   CK(cudaMemcpyAsync(dst, ctx->Q, sizeof(double) * ctx->batch, cudaMemcpyDeviceToHost, ctx->st));
-  CK(cudaStreamSynchronize(ctx->st));
-  return SCFT_OK;
+  return sync_check(ctx);
 }
 
 int scft_phi_w(scft_ctx *ctx) {
@@ -1730,6 +1735,12 @@ int scft_copy_q_reference_layout(scft_ctx *ctx, int q, double *dst_device) {
     return SCFT_OK;
   });
   if (rc) return rc;
+  return sync_check(ctx);
+}
+
+int scft_selftest_set_error(scft_ctx *ctx, unsigned word) {
+  if (!ctx) return SCFT_ERR_INVALID_ARG;
+  CK(cudaMemcpyAsync(ctx->dev_err, &word, sizeof word, cudaMemcpyHostToDevice, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   return SCFT_OK;
 }
@@ -1837,7 +1848,8 @@ int scft_copy_fields(scft_ctx *dst, const scft_ctx *src) {
   if (dst->M != src->M || dst->batch != src->batch)
     return scft_fail(dst, SCFT_ERR_INVALID_ARG, "contexts differ in grid or batch");
   const size_t bytes = sizeof(double) * dst->M * dst->batch;
-  CK(cudaStreamSynchronize(src->st));
+  scft_ctx *from = const_cast<scft_ctx *>(src);
+  if (int rc = sync_check(from)) return from == dst ? rc : scft_fail(dst, rc, from->err);
   CK(cudaMemcpyAsync(dst->wa, src->wa, bytes, cudaMemcpyDeviceToDevice, dst->st));
   CK(cudaMemcpyAsync(dst->wb, src->wb, bytes, cudaMemcpyDeviceToDevice, dst->st));
   CK(cudaMemcpyAsync(dst->pha, src->pha, bytes, cudaMemcpyDeviceToDevice, dst->st));
@@ -1866,7 +1878,8 @@ int scft_time_iterations(scft_ctx *ctx, int n_iter, double *ms) {
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   *ms = f;
-  return rc;
+  const int rc2 = sync_check(ctx);
+  return rc ? rc : rc2;
 }
 
 int scft_profile_enable(scft_ctx *ctx, int enable) {

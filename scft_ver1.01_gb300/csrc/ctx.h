@@ -113,6 +113,13 @@ struct NvtxRange {
 // Set ctx->err and return status.
 int scft_fail(scft_ctx *ctx, int status, const std::string &msg);
 
+// Synchronises the context's stream and takes the device error word, which a
+// kernel sets when a bounded wait gives up: every call that hands out results ends
+// with it.  wait_failed: the failure of a word that was taken elsewhere.
+int scft_internal_sync_check(scft_ctx *ctx);
+int scft_internal_wait_failed(scft_ctx *ctx, unsigned word);
+std::string scft_internal_wait_message(unsigned word);
+
 // One application of the step operator's diffusion part to nb slices:
 // out = post * K (pre * in), K = the per-axis line filters of the context
 // (x, y, z passes, no plane fusion).  tc_deriv >= 0: pass tc_deriv (on the tensor

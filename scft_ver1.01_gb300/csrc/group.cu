@@ -66,6 +66,7 @@ struct scft_group {
   long long nodes = 0;
   long long launches = 0;
   long long epoch = 0;               // the members' plan epochs at capture
+  unsigned **words = nullptr;        // device: the members' error words, then their union
   std::string err = "no error";
 };
 
@@ -106,6 +107,7 @@ void release(scft_group *g) {
   release_graph(g);
   for (cudaEvent_t e : g->pre) cudaEventDestroy(e);
   for (cudaEvent_t e : g->joined) cudaEventDestroy(e);
+  cudaFree(g->words);
   if (g->fork) cudaEventDestroy(g->fork);
   if (g->done) cudaEventDestroy(g->done);
   if (g->st) cudaStreamDestroy(g->st);
@@ -331,6 +333,27 @@ int build_graph(scft_group *g) {
   return SCFT_OK;
 }
 
+// One warp: the members' error words, taken and put together.
+__global__ void k_take_words(unsigned **words, int n) {
+  unsigned w = 0;
+  for (int i = threadIdx.x; i < n; i += 32) w |= atomicExch(words[i], 0u);
+  w = __reduce_or_sync(0xffffffffu, w);
+  if (threadIdx.x == 0) *reinterpret_cast<unsigned *>(words + n) = w;
+}
+// Waits for the members.  A batched launch reports into its first member's word but
+// spoils all of them, so a word anywhere fails the group's call.
+int sync_check(scft_group *g) {
+  const int n = (int)g->members.size();
+  unsigned w = 0;
+  k_take_words<<<1, 32, 0, g->st>>>(g->words, n);
+  GCK(cudaGetLastError());
+  GCK(cudaMemcpyAsync(&w, g->words + n, sizeof w, cudaMemcpyDeviceToHost, g->st));
+  GCK(cudaStreamSynchronize(g->st));
+  if (!w) return SCFT_OK;
+  for (scft_ctx *c : g->members) scft_internal_wait_failed(c, w);
+  return gfail(g, SCFT_ERR_CUDA, scft_internal_wait_message(w));
+}
+
 int iterate_once(scft_group *g) {
   if (g->epoch != plan_epochs(g)) {   // a member's box sent a pass to another kernel
     GCK(cudaStreamSynchronize(g->st));
@@ -378,6 +401,12 @@ int scft_group_create(scft_ctx *const *ctxs, int n, scft_group **out) {
   for (int i = 0; ok && i < n; ++i)
     ok = cudaEventCreateWithFlags(&g->joined[i], cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&g->pre[i], cudaEventDisableTiming) == cudaSuccess;
+  std::vector<unsigned *> words;
+  for (scft_ctx *c : g->members) words.push_back(c->dev_err);
+  words.push_back(nullptr);
+  ok = ok && cudaMalloc((void **)&g->words, sizeof(unsigned *) * words.size()) == cudaSuccess &&
+       cudaMemcpyAsync(g->words, words.data(), sizeof(unsigned *) * words.size(),
+                       cudaMemcpyHostToDevice, g->st) == cudaSuccess;
   if (!ok) {
     release(g);
     delete g;
@@ -411,8 +440,7 @@ int scft_group_iterate(scft_group *g, int n_iter) {
     int rc = iterate_once(g);
     if (rc) return rc;
   }
-  GCK(cudaStreamSynchronize(g->st));
-  return SCFT_OK;
+  return sync_check(g);
 }
 
 int scft_group_time_iterations(scft_group *g, int n_iter, double *ms) {
@@ -430,7 +458,8 @@ int scft_group_time_iterations(scft_group *g, int n_iter, double *ms) {
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   *ms = f;
-  return rc;
+  const int rc2 = sync_check(g);
+  return rc ? rc : rc2;
 }
 
 // Graph-replayed kernel launches so far (the members' own counters hold

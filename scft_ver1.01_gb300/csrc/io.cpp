@@ -124,10 +124,9 @@ int scft_write_pha_dat(scft_ctx *ctx, const char *path, int inst) {
   const double *src[4] = {ctx->pha, ctx->phb, ctx->wa, ctx->wb};
   std::vector<double> *dst[4] = {&a, &b, &c, &d};
   cudaSetDevice(ctx->p.device);
-  cudaError_t e = cudaStreamSynchronize(ctx->st);
-  if (e != cudaSuccess) return scft_fail(ctx, SCFT_ERR_CUDA, cudaGetErrorString(e));
+  if (int rc = scft_internal_sync_check(ctx)) return rc;
   for (int k = 0; k < 4; ++k) {
-    e = cudaMemcpy(dst[k]->data(), src[k] + (long long)inst * M, sizeof(double) * M,
+    cudaError_t e = cudaMemcpy(dst[k]->data(), src[k] + (long long)inst * M, sizeof(double) * M,
                    cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return scft_fail(ctx, SCFT_ERR_CUDA, cudaGetErrorString(e));
   }
@@ -225,10 +224,9 @@ int scft_write_vtk(scft_ctx *ctx, const char *path, int inst, const char *source
   const long long M = ctx->M;
   std::vector<double> a(M), b(M);
   cudaSetDevice(ctx->p.device);
-  cudaError_t e = cudaStreamSynchronize(ctx->st);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(a.data(), ctx->pha + (long long)inst * M, sizeof(double) * M,
-                   cudaMemcpyDeviceToHost);
+  if (int rc = scft_internal_sync_check(ctx)) return rc;
+  cudaError_t e = cudaMemcpy(a.data(), ctx->pha + (long long)inst * M, sizeof(double) * M,
+                             cudaMemcpyDeviceToHost);
   if (e == cudaSuccess)
     e = cudaMemcpy(b.data(), ctx->phb + (long long)inst * M, sizeof(double) * M,
                    cudaMemcpyDeviceToHost);
@@ -308,8 +306,7 @@ extern "C" {
 int scft_save_checkpoint(scft_ctx *ctx, const char *path, int with_history) {
   if (!ctx || !path) return SCFT_ERR_INVALID_ARG;
   cudaSetDevice(ctx->p.device);
-  cudaError_t e = cudaStreamSynchronize(ctx->st);
-  if (e != cudaSuccess) return scft_fail(ctx, SCFT_ERR_CUDA, cudaGetErrorString(e));
+  if (int rc = scft_internal_sync_check(ctx)) return rc;
   const scft_params &p = ctx->p;
   CkptHeader h;
   memset(&h, 0, sizeof h);
