@@ -1388,10 +1388,12 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
   // double-float lines with a register kernel keep it (64^3: FP32 1.2; double-float
   // 4.0 against 5.5 on passes of the first form).
   size_t tc_bytes = 0;
+  if (ctx->rkind != kRealDF && scft::tc_prepare() != cudaSuccess)
+    return fail(SCFT_ERR_CUDA, "kernel attribute set-up failed");
   for (size_t pi = 0; pi < ctx->passes.size(); ++pi) {
     const AxisPlan &ap = ctx->passes[pi];
-    ctx->tc_want[pi] = scft::tc_line_possible(ap.n, tc_digits(ctx)) &&
-                       (ctx->rkind == kRealF64 || (ctx->rkind == kRealF32 && !ap.use_fast));
+    ctx->tc_want[pi] = (ctx->rkind == kRealF64 || (ctx->rkind == kRealF32 && !ap.use_fast)) &&
+                       scft::tc_line_usable(ap.n, tc_digits(ctx));
     for (int k = 0; ctx->tc_want[pi] && k < 2; ++k) {
       ctx->tc_off[2 * pi + k] = tc_bytes;
       tc_bytes += (scft::tc_table_bytes(ap.n, tc_digits(ctx)) + 255) & ~(size_t)255;
@@ -1403,8 +1405,6 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
     ctx->tc_planes = ay.s_n == p.nx && (ctx->passes.size() == 3 || rb == 8) &&
                      scft::tc_planes_wanted(p.nx, ay.n, p.ny * p.nz / ay.n, tc_digits(ctx), p.batch);
   }
-  if (tc_bytes && scft::tc_prepare() != cudaSuccess)
-    return fail(SCFT_ERR_CUDA, "kernel attribute set-up failed");
   if (tc_bytes && !alloc(&ctx->tc_mem, tc_bytes))
     return fail(SCFT_ERR_NO_MEMORY, "table allocation failed");
   if (ctx->rkind == kRealF64 && (p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0 &&

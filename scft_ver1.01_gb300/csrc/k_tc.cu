@@ -1145,42 +1145,43 @@ bool planes_of(const AxisPlan &apx, const AxisPlan &apy, int nd, int batch, bool
   return true;
 }
 
-// Shared-memory opt-in; a kernel that splits its registers must have been given
-// at least the launch count that the split was added up for.
-template <typename K> cudaError_t opt_in(K *k, bool splits = false) {
-  if (splits) {
+// Shared-memory opt-in; *fits goes false where the compiler's register count of a
+// kernel that splits them does not hold the split.
+template <typename K> cudaError_t opt_in(K *k, bool *fits = nullptr) {
+  if (fits) {
     cudaFuncAttributes at;
     const cudaError_t e = cudaFuncGetAttributes(&at, k);
     if (e != cudaSuccess) return e;
-    if (at.numRegs != kRegsLaunch) return cudaErrorInvalidConfiguration;
+    for (int c = 2; c <= 4; ++c) *fits = *fits && split_fits(at.numRegs, c);
   }
   return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
-template <typename T, int MAXT, int PP> cudaError_t prep_real() {
-  constexpr bool kSplit = kNd<T> == 7 && PP == 16;
+template <typename T, int MAXT, int PP> cudaError_t prep_real(bool *split) {
+  bool *fits = kNd<T> == 7 && PP == 16 ? split : nullptr;
   cudaError_t e;
-  if ((e = opt_in(k_real<T, MAXT, PP, true, false>, kSplit)) != cudaSuccess) return e;
-  if ((e = opt_in(k_real<T, MAXT, PP, false, false>, kSplit)) != cudaSuccess) return e;
+  if ((e = opt_in(k_real<T, MAXT, PP, true, false>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_real<T, MAXT, PP, false, false>, fits)) != cudaSuccess) return e;
   if constexpr (std::is_same<T, float>::value) {
-    if ((e = opt_in(k_real<T, MAXT, PP, true, true>, kSplit)) != cudaSuccess) return e;
-    if ((e = opt_in(k_real<T, MAXT, PP, false, true>, kSplit)) != cudaSuccess) return e;
+    if ((e = opt_in(k_real<T, MAXT, PP, true, true>, fits)) != cudaSuccess) return e;
+    if ((e = opt_in(k_real<T, MAXT, PP, false, true>, fits)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
-template <int PP> cudaError_t prep_fix() {
+template <int PP> cudaError_t prep_fix(bool *split) {
+  bool *fits = PP == 16 ? split : nullptr;
   cudaError_t e;
   if constexpr (PP <= 8) {
     if ((e = opt_in(k_planes<PP, false>)) != cudaSuccess) return e;
     if ((e = opt_in(k_planes<PP, true>)) != cudaSuccess) return e;
     if ((e = opt_in(k_planes_f32<PP>)) != cudaSuccess) return e;
   }
-  if ((e = opt_in(k_fix<PP, true, FIRST>, PP == 16)) != cudaSuccess) return e;
-  if ((e = opt_in(k_fix<PP, false, FIRST>, PP == 16)) != cudaSuccess) return e;
-  if ((e = opt_in(k_fix<PP, false, MID>, PP == 16)) != cudaSuccess) return e;
-  if ((e = opt_in(k_fix<PP, true, PAIR>, PP == 16)) != cudaSuccess) return e;
-  if ((e = opt_in(k_fix<PP, false, PAIR>, PP == 16)) != cudaSuccess) return e;
-  if ((e = opt_in(k_fix<PP, true, LAST>, PP == 16)) != cudaSuccess) return e;
-  return opt_in(k_fix<PP, false, LAST>, PP == 16);
+  if ((e = opt_in(k_fix<PP, true, FIRST>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, FIRST>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, MID>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, true, PAIR>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, false, PAIR>, fits)) != cudaSuccess) return e;
+  if ((e = opt_in(k_fix<PP, true, LAST>, fits)) != cudaSuccess) return e;
+  return opt_in(k_fix<PP, false, LAST>, fits);
 }
 
 // ---- host: the convolution kernel in double-double arithmetic
@@ -1428,35 +1429,53 @@ bool tc_build_table(const double *g, int n, int nd, std::vector<unsigned char> &
 }
 
 namespace {
-cudaError_t prepare_all() {
+cudaError_t prepare_all(bool *split) {
   cudaError_t e;
-  if ((e = prep_real<float, 544, 4>()) != cudaSuccess) return e;
-  if ((e = prep_real<double, 544, 4>()) != cudaSuccess) return e;
-  if ((e = prep_fix<4>()) != cudaSuccess) return e;
-  if ((e = prep_real<float, 544, 8>()) != cudaSuccess) return e;
-  if ((e = prep_real<float, 640, 16>()) != cudaSuccess) return e;
-  if ((e = prep_real<float, 1024, 16>()) != cudaSuccess) return e;
-  if ((e = prep_real<double, 544, 8>()) != cudaSuccess) return e;
-  if ((e = prep_real<double, 640, 16>()) != cudaSuccess) return e;
-  if ((e = prep_fix<8>()) != cudaSuccess) return e;
-  return prep_fix<16>();
+  if ((e = prep_real<float, 544, 4>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<double, 544, 4>(split)) != cudaSuccess) return e;
+  if ((e = prep_fix<4>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<float, 544, 8>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<float, 640, 16>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<float, 1024, 16>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<double, 544, 8>(split)) != cudaSuccess) return e;
+  if ((e = prep_real<double, 640, 16>(split)) != cudaSuccess) return e;
+  if ((e = prep_fix<8>(split)) != cudaSuccess) return e;
+  return prep_fix<16>(split);
+}
+struct Prepared {
+  std::mutex mu;
+  bool done[64] = {}, split[64] = {};
+};
+Prepared &prepared() {
+  static Prepared p;
+  return p;
 }
 }  // namespace
 
 // Kernel attributes, set once per device (host threads may race to it).
 cudaError_t tc_prepare() {
-  static std::mutex mu;
-  static bool done[64];
+  Prepared &p = prepared();
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!done[dev]) {
-    if ((e = prepare_all()) != cudaSuccess) return e;
-    done[dev] = true;
+  std::lock_guard<std::mutex> lock(p.mu);
+  if (!p.done[dev]) {
+    p.split[dev] = true;
+    if ((e = prepare_all(&p.split[dev])) != cudaSuccess) return e;
+    p.done[dev] = true;
   }
   return cudaSuccess;
+}
+// Whether the kernels of such lines can run on the current device (prepared):
+// without the register split 64-bit lines above 64 points keep their FFT passes.
+bool tc_line_usable(int n, int nd) {
+  if (!tc_line_possible(n, nd)) return false;
+  Prepared &p = prepared();
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  std::lock_guard<std::mutex> lock(p.mu);
+  return p.done[dev] && (p.split[dev] || !split_rows(nd, line_blocks(n)));
 }
 
 cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float, kStepSet> &ps, bool pair, cudaStream_t st) {

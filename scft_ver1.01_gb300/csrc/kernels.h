@@ -148,6 +148,7 @@ cudaError_t launch_xyxy(const AxisPlan &apx, const AxisPlan &apy, const PassSet<
 // even length, up to 128 points (FP64: 7 digits) or 224 (FP32: 4 digits).  pair (FP32): a fused step pair (qout = post * K(in),
 // out = K(post * qout)).
 bool tc_line_possible(int n, int nd);
+bool tc_line_usable(int n, int nd);   // on this device, after tc_prepare
 long long tc_pass_ctas(const AxisPlan &ap, int nd);
 bool tc_planes_wanted(int nx, int ny, int nz, int nd, int batch);
 size_t tc_table_bytes(int n, int nd);

@@ -78,12 +78,18 @@ __host__ __device__ constexpr int b_half_bytes(int nd, int kg) {
                      : nd * (4 * kg - 1) * 128;
 }
 // The issuing warp; with 16 points per thread and 7 digits a warpgroup of its
-// own, so that the computing ones can take its registers (setmaxnreg: 96 at
-// launch for 640 threads, then 104 x 512 + 56 x 128 = 60416 <= 96 x 640 = 61440;
-// with 384 + 128 threads 47104 <= 49152, with 256 + 128 33792 <= 36864).  112 + 24
+// own, so that the computing ones can take its registers (setmaxnreg).  112 + 24
 // left the issuing warp too few: it kept its loop in local memory.
 __host__ __device__ constexpr int issuer_threads(int pp) { return pp == 16 ? 128 : 32; }
-constexpr int kRegsLaunch = 96, kRegsCompute = 104, kRegsIssue = 56;
+constexpr int kRegsCompute = 104, kRegsIssue = 56;
+// Whether a block of 128 c computing threads and the issuing 128, launched with
+// `regs` registers a thread, holds what the split asks for (the computing threads
+// would wait for ever otherwise): 96 do for every c (104 x 512 + 56 x 128 = 60416 <= 96 x
+// 640 = 61440; 47104 <= 49152 for 3, 33792 <= 36864 for 2).
+__host__ __device__ constexpr bool split_fits(int regs, int c) {
+  return regs >= kRegsIssue && regs <= kRegsCompute &&
+         128 * c * kRegsCompute + 128 * kRegsIssue <= 128 * (c + 1) * regs;
+}
 
 // ---- shared-memory layout (bytes)
 constexpr int kKeySlots = 4;
