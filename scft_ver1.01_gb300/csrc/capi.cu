@@ -134,6 +134,9 @@ int upload_gains(scft_ctx *ctx) {
     const int kb = growth > 1.0 ? (int)ceil(log2(growth)) : 0;
     CK(cudaMemcpy(ctx->kbits, &kb, sizeof kb, cudaMemcpyHostToDevice));
   }
+  // a copy from pageable memory may return before it has landed, and the streams
+  // that read the tables do not wait for the default one
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
   return SCFT_OK;
 }
 

@@ -202,8 +202,8 @@ int make_buckets(scft_group *g) {
         cudaGetLastError();
         return gfail(g, SCFT_ERR_NO_MEMORY, "batched-march descriptor allocation failed");
       }
-      GCK(cudaMemcpy(bc.desc, host.data(), sizeof(scft::PassDesc) * host.size(),
-                     cudaMemcpyHostToDevice));
+      GCK(cudaMemcpyAsync(bc.desc, host.data(), sizeof(scft::PassDesc) * host.size(),
+                          cudaMemcpyHostToDevice, g->st));   // (in front of the graph)
       GCK(cudaStreamCreateWithFlags(&bc.st, cudaStreamNonBlocking));
       GCK(cudaEventCreateWithFlags(&bc.ev, cudaEventDisableTiming));
     }

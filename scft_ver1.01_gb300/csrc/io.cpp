@@ -12,6 +12,13 @@
 
 #include "ctx.h"
 
+// Copies from pageable memory may return before they have landed, and the
+// context's streams do not wait for the default one.
+static int landed(scft_ctx *ctx) {
+  const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+  return e == cudaSuccess ? SCFT_OK : scft_fail(ctx, SCFT_ERR_CUDA, cudaGetErrorString(e));
+}
+
 extern "C" {
 
 int scft_read_ab_txt(const char *path, scft_params *p, int *intag) {
@@ -113,7 +120,7 @@ int scft_read_phi_dat(scft_ctx *ctx, const char *path, int inst) {
                                cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return scft_fail(ctx, SCFT_ERR_CUDA, cudaGetErrorString(e));
   }
-  return SCFT_OK;
+  return landed(ctx);
 }
 
 int scft_write_pha_dat(scft_ctx *ctx, const char *path, int inst) {
@@ -408,7 +415,7 @@ int scft_load_checkpoint(scft_ctx *ctx, const char *path) {
     }
   }
   fclose(fp);
-  return rc;
+  return rc == SCFT_OK ? landed(ctx) : rc;
 }
 
 }  // extern "C"
