@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "convert.cuh"
 #include "ctx.h"
 
 #define CK(call)                                                                        \
@@ -53,43 +54,14 @@
 
 namespace {
 
-using scft::warp_sum;
+using scft::narrow;
+using scft::widen;
 constexpr int kT = 256;
 
 int grid_for(long long n) {
   long long g = (n + kT - 1) / kT;
   return (int)std::min<long long>(g, 1 << 20);
 }
-
-// Sum over the block (kT threads) in thread 0, halves folding through shared memory
-// (sh: kT / 2 doubles): 12 FP64 additions of a warp where shuffles in every warp
-// take 45.
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int h = kT / 2; h >= 32; h /= 2) {
-    __syncthreads();
-    if (t >= h && t < 2 * h) sh[t - h] = v;
-    __syncthreads();
-    if (t < h) v += sh[t];
-  }
-  if (t < 32) v = warp_sum(v);
-  return v;
-}
-
-// x in FP64.  A conversion costs the FP64 pipe as much as an FMA (16 cycles a
-// warp and SM), rebuilding the exponent in integers about a tenth of it.
-// (Denormal, infinite and NaN values go out of line: predicated in place the
-// conversion would take the pipe for every value.)
-__device__ __noinline__ double widen_rare(float x) { return (double)x; }
-__device__ __forceinline__ double widen(double x) { return x; }
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return widen_rare(x);
-  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
-  return __hiloint2double((int)hi, (int)(u << 29));
-}
-__device__ __forceinline__ double widen(scft::dfloat x) { return widen(x.hi) + widen(x.lo); }
 
 // Two neighbouring points (grids have an even first axis).
 template <typename R> struct alignas(2 * sizeof(R)) Two {
@@ -118,10 +90,10 @@ __global__ void k_dot_acc(const R *__restrict__ a, long long a_bs, const S *__re
     v1 += x * widen(c1[b * c1_bs + r]);
     if (c2) v2 += x * widen(c2[b * c2_bs + r]);
   }
-  v1 = block_sum(v1, sh);
+  v1 = scft::block_sum<kT>(v1, sh);
   if (threadIdx.x == 0) acc1[b * nblk + blockIdx.x] += v1;
   if (c2) {
-    v2 = block_sum(v2, sh);
+    v2 = scft::block_sum<kT>(v2, sh);
     if (threadIdx.x == 0) acc2[b * nblk + blockIdx.x] += v2;
   }
 }
@@ -164,7 +136,7 @@ __global__ void __launch_bounds__(kT) k_dots(DotArgs<R> d, const R *__restrict__
   }
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    const double s = block_sum(v[k][0] + v[k][1], sh);
+    const double s = scft::block_sum<kT>(v[k][0] + v[k][1], sh);
     if (threadIdx.x == 0) d.acc[k][blockIdx.x] += s;
   }
 }
@@ -195,26 +167,10 @@ __global__ void k_sum_slots(const double *__restrict__ partial, int nblk, double
   const int b = blockIdx.x;
   double v = 0.0;
   for (int k = threadIdx.x; k < nblk; k += blockDim.x) v += partial[(long long)b * nblk + k];
-  v = block_sum(v, sh);
+  v = scft::block_sum<kT>(v, sh);
   if (threadIdx.x == 0) out[b] = v;
 }
 
-// x rounded to the working precision, to nearest even (float: in integers, again)
-__device__ __noinline__ float narrow_rare(double x) { return (float)x; }
-__device__ __forceinline__ void narrow(double x, double &r) { r = x; }
-__device__ __forceinline__ void narrow(double x, scft::dfloat &r) { r = scft::dfloat(x); }
-__device__ __forceinline__ void narrow(double x, float &r) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t m = hi & 0x7fffffffu;
-  if (m - 0x38100000u >= 0x0fd00000u && (m | lo) != 0u) {   // below 2^-126, near the top, inf, nan
-    r = narrow_rare(x);
-    return;
-  }
-  // 23 bits and the rest below them; a carry moves into the exponent as it should
-  const uint32_t f = m ? ((m - 0x38000000u) << 3) | (lo >> 29) : 0u, rest = lo & 0x1fffffffu;
-  const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
-  r = __uint_as_float((hi & 0x80000000u) | (f + up));
-}
 // One contour point's weights in the accumulators of sums of q q+ (S: the density
 // sums; G: the sums of the Q part, Simpson only) and in the adjoint seed.  How they
 // are used is decided on the host: comparisons of doubles take the FP64 pipe too.

@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "convert.cuh"
 #include "dfloat.cuh"
 #include "kernels.h"
 
@@ -31,22 +32,8 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Sum over the block (kThreads threads) in thread 0; sh: kHalf doubles.  Halves
-// fold through shared memory: 12 additions of a warp where eight warps' shuffles
-// took 45, and an FP64 addition is 16 cycles of the SM.
 constexpr int kHalf = kThreads / 2;
-__device__ __forceinline__ double blk_sum(double v, double *sh) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int h = kHalf; h >= 32; h /= 2) {
-    __syncthreads();
-    if (t >= h && t < 2 * h) sh[t - h] = v;
-    __syncthreads();
-    if (t < h) v += sh[t];
-  }
-  if (t < 32) v = warp_sum(v);
-  return v;
-}
+__device__ __forceinline__ double blk_sum(double v, double *sh) { return block_sum<kThreads>(v, sh); }
 __device__ __forceinline__ double blk_max(double v, double *sh) {
   v = warp_max(v);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -96,24 +83,6 @@ __device__ __forceinline__ void phi_w_dir(double a, double c, double pa, double 
   const double m = fma(wcmp, pa + pb, -(0.5 * hAB + wcmp)), t = c - a;
   da = fma(hAB, pb, fma(0.5, t, m));
   db = fma(hAB, pa, fma(-0.5, t, m));
-}
-
-// dfloat(x) in integers (bit for bit): the four FP64 operations of the
-// conversion took a third of the residual's time.  Zero, values outside 2^-60 ..
-// 2^120, infinities and NaN go out of line.
-__device__ __noinline__ dfloat pair_rare(double x) { return dfloat(x); }
-__device__ __forceinline__ dfloat pair_of(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t m = hi & 0x7fffffffu;
-  if (m - ((1023u - 60u) << 20) >= 180u << 20) return pair_rare(x);
-  const uint32_t f = ((m - 0x38000000u) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
-  const uint32_t up = rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
-  int r = (int)rest - (int)(up << 29);           // x - hi, in units of 2^(e - 52)
-  r = (int)hi < 0 ? -r : r;
-  dfloat d;
-  d.hi = __uint_as_float((hi & 0x80000000u) | (f + up));
-  d.lo = __int2float_rn(r) * __uint_as_float(((m >> 20) - (1023u - 127u) - 52u) << 23);
-  return d;
 }
 
 // Per-instance sums of wA, wB, phiA, phiB: partial[(b*4 + f)*nblk + blk].
@@ -170,7 +139,8 @@ __global__ void k_residual_mean(const double *__restrict__ partial, int nblk, lo
 // FP64 operations bound it (16 cycles of an SM each per warp; 128^3: 33 a point
 // 160 us, 12 a point 65 us): kernels without the parts not asked for (HIST: the
 // history slot; STEP: the simple step), the means in the constants without STEP,
-// conversions in integers.
+// conversions in integers (the four FP64 operations of the pairs' own took a third
+// of the time).
 template <bool HIST, bool STEP>
 __global__ void k_residual(double *__restrict__ wa, double *__restrict__ wb,
                            const double *__restrict__ pha, const double *__restrict__ phb,
@@ -267,14 +237,6 @@ struct SlotList {
   int slot[kMaxSlots];
   int n;
 };
-// x in FP64, the exponent rebuilt in integers (see pair_of)
-__device__ __noinline__ double wide_rare(float x) { return (double)x; }
-__device__ __forceinline__ double wide(float x) {
-  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u && m != 0u) return wide_rare(x);   // denormal, inf, nan
-  const uint32_t hi = (u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u);
-  return __hiloint2double((int)hi, (int)(u << 29));
-}
 // Two pairs of a slot (grids have an even number of points).
 struct __align__(16) Pair2 {
   dfloat v[2];
@@ -321,8 +283,8 @@ __global__ void __launch_bounds__(kThreads, 4)
 #pragma unroll
   for (int k = 0; k < kChunk; ++k) {
     if (dk[k]) {
-      const double r = blk_sum((wide(acc[k][0].hi) + wide(acc[k][1].hi)) +
-                                   (wide(acc[k][0].lo) + wide(acc[k][1].lo)),
+      const double r = blk_sum((widen(acc[k][0].hi) + widen(acc[k][1].hi)) +
+                                   (widen(acc[k][0].lo) + widen(acc[k][1].lo)),
                                sh);
       if (threadIdx.x == 0) partial[(b * kMaxSlots + k0 + k) * gridDim.x + blockIdx.x] = r;
     }
@@ -494,7 +456,7 @@ __global__ void k_anderson_update(double *__restrict__ wa, double *__restrict__ 
     }
     double *w = i < M ? wab + i : wbb + (i - M);   // (both points in one field: M is even)
     *reinterpret_cast<double2 *>(w) =
-        make_double2(wide(s0.hi) + wide(s0.lo), wide(s1.hi) + wide(s1.lo));
+        make_double2(widen(s0.hi) + widen(s0.lo), widen(s1.hi) + widen(s1.lo));
   }
 }
 
