@@ -7,7 +7,7 @@
 // A line x is held as integers X with x = X * 2^ue, ue chosen from the line's
 // largest exponent so that |X| <= 2^54 (FP64; 7 digits) or 2^29
 // (FP32; 4 digits).  All roundings are to nearest: a truncation's bias would
-// add up over the contour steps.
+// add up over the contour steps.  Denormals are kept.
 #pragma once
 
 #include <stdint.h>
@@ -92,25 +92,27 @@ SL_HD int mag_key(double x) { return (int)((uint32_t)(d2u(x) >> 32) & 0x7fffffff
 SL_HD int mag_key(float x) { return (int)(f2u(x) & 0x7fffffffu); }
 template <typename T> SL_HD constexpr int bad_key() { return sizeof(T) == 8 ? 0x7ff00000 : 0x7f800000; }
 
-// Biased exponent of a line's largest magnitude, and the unit exponent ue.
-SL_HD int line_exp(double, int key) { return key >> 20; }
-SL_HD int line_exp(float, int key) { return key >> 23; }
+// Biased exponent of a line's largest magnitude, and the unit exponent ue
+// (denormals count as exponent 1, which is their unit).
+SL_HD int line_exp(double, int key) { return key < 1 << 21 ? 1 : key >> 20; }
+SL_HD int line_exp(float, int key) { return key < 1 << 24 ? 1 : key >> 23; }
 SL_HD int unit_exp(double, int E) { return E - 1076; }   // |X| < 2^54
-SL_HD int unit_exp(float, int E) { return (E < 29 ? 29 : E) - 155; }   // |X| <= 2^29
+SL_HD int unit_exp(float, int E) { return E - 155; }     // |X| <= 2^29
 
 // x / 2^unit_exp(E), rounded to nearest; E is at least x's own exponent.
 SL_HD int64_t to_fixed(double x, int E) {
   const uint64_t b = d2u(x);
   const int e = (int)(b >> 52) & 0x7ff;
-  const uint64_t m = ((b & 0xfffffffffffffULL) | 0x10000000000000ULL) << 8;   // 61 bits
-  int sh = E - e;
-  if (e == 0 || sh > 63) sh = 63;                  // zero, or far below the line's unit
+  const uint64_t m = ((b & 0xfffffffffffffULL) | (e ? 0x10000000000000ULL : 0)) << 8;   // 61 bits
+  int sh = E - (e ? e : 1);
+  if (sh > 63) sh = 63;                            // far below the line's unit
   const int64_t t = (int64_t)(((m >> sh) + 64) >> 7);
   const int64_t s = (int64_t)b >> 63;
   return (t ^ s) - s;
 }
 SL_HD int to_fixed(float x, int E) {
-  const float s = x * exp2i(155 - (E < 29 ? 29 : E));
+  // (2^154 at most: two factors)
+  const float s = x * exp2i(E < 29 ? 126 : 155 - E) * exp2i(E < 29 ? 29 - E : 0);
 #ifdef __CUDA_ARCH__
   return __float2int_rn(s);
 #else
@@ -118,18 +120,22 @@ SL_HD int to_fixed(float x, int E) {
 #endif
 }
 
-// y * 2^ue as an FP64 number, |y| < 2^63, rounded to nearest (halves up);
-// results below the normal range become 0.
+// y * 2^ue as an FP64 number, |y| < 2^63, rounded to nearest (halves up).
 SL_HD double from_fixed(int64_t y, int ue, double) {
   const int64_t sg = y >> 63;
   const uint64_t u = (uint64_t)((y ^ sg) - sg);
   const int lz = clz64(u);                         // >= 1
   const uint64_t m = ((u << ((lz - 1) & 63)) + 0x200) >> 10;   // leading bit 52 (53 after a carry)
   const int be = 1086 + ue - lz;                   // biased exponent of the leading bit
-  uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(be - 1) << 20);
-  if (u == 0 || be <= 0) hi = 0;
-  if (be >= 2047) hi = 0x7ff00000u;
-  const uint32_t lo = u == 0 || be <= 0 || be >= 2047 ? 0u : (uint32_t)m;
+  uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(be - 1) << 20), lo = (uint32_t)m;
+  if (u == 0) hi = lo = 0;
+  else if (be >= 2047) { hi = 0x7ff00000u; lo = 0; }
+  else if (be <= 0) {                              // in units of 2^-1074
+    const int s = -1074 - ue;                      // (> 0 for |y| >= 2^52)
+    const uint64_t d = s > 63 ? 0 : (s > 0 ? (u + (1ULL << (s - 1))) >> s : u << -s);
+    hi = (uint32_t)(d >> 32);
+    lo = (uint32_t)d;
+  }
   return u2d(((uint64_t)(hi | ((uint32_t)(sg >> 32) & 0x80000000u)) << 32) | lo);
 }
 // The same for |y| in [2^32, 2^62) and results in the normal range (fast path;
