@@ -58,7 +58,7 @@ int upload_tc(scft_ctx *ctx, int pi, const std::vector<double> &g, const std::ve
   AxisPlan &ap = ctx->passes[pi];
   const int nd = tc_digits(ctx);
   std::vector<unsigned char> t[2];
-  const bool ok = scft::tc_build_table(g.data(), ap.n, nd, t[0], &ctx->row_sum[pi]) &&
+  const bool ok = scft::tc_build_table(g.data(), ap.n, nd, t[0], nullptr) &&
                   scft::tc_build_table(dg.data(), ap.n, nd, t[1], nullptr);
   unsigned char *mem = static_cast<unsigned char *>(ctx->tc_mem);
   for (int k = 0; ok && k < 2; ++k)
@@ -128,11 +128,6 @@ int upload_gains(scft_ctx *ctx) {
       const int rc = upload_tc(ctx, (int)pi, g, kdg);
       if (rc) return rc;
     }
-  }
-  if (ctx->kbits) {
-    const double growth = ctx->row_sum[0] * ctx->row_sum[1] * ctx->row_sum[2];
-    const int kb = growth > 1.0 ? (int)ceil(log2(growth)) : 0;
-    CK(cudaMemcpy(ctx->kbits, &kb, sizeof kb, cudaMemcpyHostToDevice));
   }
   // a copy from pageable memory may return before it has landed, and the streams
   // that read the tables do not wait for the default one
@@ -405,14 +400,11 @@ int run_chain_fused_axes(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t 
 }
 
 // The same schedule with integer intermediates (FP64 contexts whose passes all
-// run on the tensor cores).  v_j = W q_j starts step j+1; its unit follows from
-// the exponent bound of v_{j-1} (two factors on), of q_0 for j = 0.
+// run on the tensor cores), each with the units of its lines in ctx->units.
 int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, int cidx) {
   const long long M = ctx->M;
-  const int B = ctx->batch, np = (int)ctx->passes.size();
+  const int B = ctx->batch, np = (int)ctx->passes.size(), nx = ctx->p.nx, ny = ctx->p.ny;
   const bool planes = ctx->tc_planes;
-  int64_t *tmp[2] = {static_cast<int64_t *>(ctx->tmp[2 * cidx]),
-                     static_cast<int64_t *>(ctx->tmp[2 * cidx + 1])};
   for (int k = 0; k < nseg; ++k) {
     const Seg &sg = segs[k];
     int rc = seg_boundary<double>(ctx, sg, st);
@@ -421,36 +413,47 @@ int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, i
     double *q = static_cast<double *>(ctx->q[sg.qi]);
     const long long qbs = (long long)(ctx->q_ns[sg.qi] + 1) * M;
     auto slice = [&](int it) { return q + (long long)(sg.sign > 0 ? it : sg.ns - it) * M; };
-    int *exq = ctx->ex[cidx], *ex = exq + B;   // |q_0| and |v_j| bounds, [..][B]
     scft::FixPass fp;
-    int cur = 0, j = 0;   // tmp[cur] holds v_j, or v_j filtered
-    auto pass = [&](int pi, int mode, const void *in, long long in_bs) {
-      memset(&fp, 0, sizeof fp);
-      fp.batch = B;
-      fp.eref = ctx->eref[sg.wf];
-      fp.kbits = ctx->kbits;
-      fp.w = ctx->wfix[sg.wf];
-      fp.w_bs = M;
-      fp.err = ctx->dev_err;
-      fp.in = in;
-      fp.in_bs = in_bs;
-      auto unit = [&](int v, const int *&u, int &w) {
-        u = v == 0 ? exq : ex + (long long)(v - 1) * B;
-        w = v == 0 ? 1 : 2;
-      };
-      if (mode != scft::kFixFirst) unit(j, fp.u_in, fp.w_in);
-      if (mode == scft::kFixPair || mode == scft::kFixLast) {
-        fp.q = slice(j + 1);
-        fp.q_bs = qbs;
-        ++j;
+    memset(&fp, 0, sizeof fp);
+    fp.batch = B;
+    fp.w = static_cast<const double *>(ctx->W[sg.wf]);
+    fp.w_bs = M;
+    fp.q_bs = qbs;
+    fp.out_bs = M;
+    fp.u_in_bs = fp.u_out_bs = ctx->unit_bs;
+    fp.err = ctx->dev_err;
+    if (planes && np == 2) {   // a film: the segment is one launch
+      fp.in = slice(0);
+      fp.in_bs = qbs;
+      fp.q = slice(1);
+      CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], fp, sg.ns, sg.sign * M, st));
+      continue;
+    }
+    // tmp[cur] holds the state between launches, filtered last along axis `from`
+    int cur = 2 * cidx, from = -1, it = 0;
+    auto pass = [&](int pi, int mode) {
+      const int axis = ctx->pass_axis[pi];
+      fp.in = mode == scft::kFixFirst ? (const void *)slice(0) : ctx->tmp[cur];
+      fp.in_bs = mode == scft::kFixFirst ? qbs : M;
+      fp.u_in = mode == scft::kFixFirst ? nullptr : ctx->units[cur];
+      if (mode != scft::kFixFirst) cur ^= 1;
+      fp.out = mode == scft::kFixLast ? nullptr : ctx->tmp[cur];
+      fp.u_out = mode == scft::kFixLast ? nullptr : ctx->units[cur];
+      fp.q = mode == scft::kFixPair || mode == scft::kFixLast ? slice(++it) : nullptr;
+      // lines are counted x: y + ny z, y: x + nx z, z: x + nx y
+      fp.u_div = axis == 0 ? ny : nx;
+      fp.u_quo = fp.u_rem = 0;
+      if (axis == 0) {
+        (from == 1 ? fp.u_quo : fp.u_rem) = nx;
+        fp.u_step = 1;
+      } else if (from == 0) {
+        fp.u_quo = axis == 1 ? ny : 1;
+        fp.u_step = axis == 1 ? 1 : ny;
+      } else {
+        fp.u_rem = 1;
+        fp.u_step = nx;
       }
-      if (mode != scft::kFixLast) {
-        unit(j, fp.u_out, fp.w_out);
-        fp.out = mode == scft::kFixFirst ? tmp[cur] : tmp[cur ^ 1];
-        fp.out_bs = M;
-        if (mode != scft::kFixFirst) cur ^= 1;
-        if (mode != scft::kFixMid) fp.ex = ex + (long long)j * B;
-      }
+      from = axis;
       // an x pair on planes takes the middle passes before and after it along
       if (mode == scft::kFixPair && pi == 0 && planes)
         CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], fp, 0, 0, st));
@@ -458,39 +461,23 @@ int run_chain_fixed(scft_ctx *ctx, const Seg *segs, int nseg, cudaStream_t st, i
         CKL(scft::launch_fix(ctx->passes[pi], mode, fp, st));
       return (int)SCFT_OK;
     };
-    auto middle = [&]() { return np < 3 ? (int)SCFT_OK : pass(1, scft::kFixMid, tmp[cur], M); };
-    if (planes && np == 2) {   // a film: the segment is one launch
-      memset(&fp, 0, sizeof fp);
-      fp.batch = B;
-      fp.eref = ctx->eref[sg.wf];
-      fp.kbits = ctx->kbits;
-      fp.w = ctx->wfix[sg.wf];
-      fp.w_bs = M;
-      fp.err = ctx->dev_err;
-      fp.in = slice(0);
-      fp.in_bs = fp.q_bs = qbs;
-      fp.q = slice(1);
-      CKL(scft::launch_planes(ctx->passes[0], ctx->passes[1], fp, sg.ns, sg.sign * M, st));
-      continue;
-    }
-    CK(cudaMemsetAsync(exq, 0x80, sizeof(int) * (size_t)(sg.ns + 1) * B, st));
-    CKL(scft::launch_slice_exp(slice(0), qbs, M, B, exq, st));
-    if ((rc = pass(0, scft::kFixFirst, slice(0), qbs))) return rc;
+    auto middle = [&]() { return np < 3 ? (int)SCFT_OK : pass(1, scft::kFixMid); };
+    if ((rc = pass(0, scft::kFixFirst))) return rc;
     if ((rc = middle())) return rc;
-    for (int it = 2; it <= sg.ns; ++it) {
-      // finish step it-1 (last pass when it was odd, x when even), start step it
-      if ((rc = pass((it - 1) & 1 ? np - 1 : 0, scft::kFixPair, tmp[cur], M))) return rc;
+    for (int step = 2; step <= sg.ns; ++step) {
+      // finish step - 1 (last pass when it was odd, x when even), start this one
+      if ((rc = pass((step - 1) & 1 ? np - 1 : 0, scft::kFixPair))) return rc;
       if (!planes && (rc = middle())) return rc;
     }
     if (planes && !(sg.ns & 1) && (rc = middle())) return rc;
-    if ((rc = pass((sg.ns & 1) ? np - 1 : 0, scft::kFixLast, tmp[cur], M))) return rc;
+    if ((rc = pass((sg.ns & 1) ? np - 1 : 0, scft::kFixLast))) return rc;
   }
   return SCFT_OK;
 }
 
 // Whether fused chains of this context run with integer intermediates.
 bool fixed_march(const scft_ctx *ctx) {
-  if (!ctx->kbits) return false;
+  if (!ctx->units[0]) return false;
   for (const AxisPlan &ap : ctx->passes)
     if (!ap.tc) return false;
   return true;
@@ -581,13 +568,6 @@ int boltzmann(scft_ctx *ctx, int f, cudaStream_t st) {
     using R = decltype(r);
     CKL(scft::launch_boltzmann<R>(w, static_cast<R *>(ctx->W[f]), ctx->M * ctx->batch,
                                   ctx->p.ds0 / 2, st));
-    if constexpr (std::is_same<R, double>::value) {
-      if (ctx->kbits) {
-        CKL(scft::launch_wfix(static_cast<const double *>(ctx->W[f]), ctx->M, ctx->batch,
-                              ctx->eref[f], ctx->wfix[f], st));
-        ++ctx->launches;
-      }
-    }
     return SCFT_OK;
   });
 }
@@ -862,7 +842,7 @@ void free_all(scft_ctx *ctx) {
   cudaFree(ctx->res); cudaFree(ctx->rpartial); cudaFree(ctx->gram); cudaFree(ctx->and_a);
   cudaFree(ctx->and_lam); cudaFree(ctx->target); cudaFree(ctx->dgain);
   cudaFree(ctx->shift_alpha); cudaFree(ctx->tc_mem);
-  cudaFree(ctx->wfix[0]); cudaFree(ctx->wfix[1]); cudaFree(ctx->kbits);
+  for (int i = 0; i < 4; ++i) cudaFree(ctx->units[i]);
   scft_internal_adjoint_free(ctx);
   for (float *h : ctx->hist_u) cudaFree(h);
   for (float *h : ctx->hist_d) cudaFree(h);
@@ -1413,15 +1393,12 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
   if (ctx->rkind == kRealF64 && (p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0 &&
       ctx->passes.size() >= 2 && ctx->tc_want[0] && ctx->tc_want[1] &&
       (ctx->passes.size() == 2 || ctx->tc_want[2])) {
-    // kbits, then eref[2][B], then the exponent bounds of the two chains
-    const size_t steps = (size_t)std::max(ctx->NsA, ctx->dNsB) + 2;
-    if (!alloc((void **)&ctx->kbits, sizeof(int) * (1 + 2 * (size_t)B + 2 * steps * B)) ||
-        !alloc((void **)&ctx->wfix[0], 8 * M * B) || !alloc((void **)&ctx->wfix[1], 8 * M * B))
-      return fail(SCFT_ERR_NO_MEMORY, "device allocation failed");
-    ctx->eref[0] = ctx->kbits + 1;
-    ctx->eref[1] = ctx->eref[0] + B;
-    ctx->ex[0] = ctx->eref[1] + B;
-    ctx->ex[1] = ctx->ex[0] + steps * B;
+    int shortest = ctx->passes[0].n;
+    for (const AxisPlan &ap : ctx->passes) shortest = std::min(shortest, ap.n);
+    ctx->unit_bs = M / shortest;
+    for (int i = 0; i < 4; ++i)
+      if (!alloc((void **)&ctx->units[i], sizeof(int16_t) * ctx->unit_bs * B))
+        return fail(SCFT_ERR_NO_MEMORY, "device allocation failed");
   }
   if (upload_gains(ctx)) return fail(SCFT_ERR_CUDA, "gain table upload failed: " + ctx->err);
   // x and y both as their own passes (no length-1 axis among them) and small

@@ -76,12 +76,10 @@ struct scft_ctx {
   bool tc_want[3] = {false, false, false};
   bool tc_planes = false;       // fused steps run the x and y passes on whole planes
   const void *dtc_pass[3] = {nullptr, nullptr, nullptr};
-  // the fused 64-bit march (run_chain_fixed): factors as integers and their
-  // largest exponent per instance, exponent bounds per step [2 chains], and
-  // log2 of the filters' growth
-  int64_t *wfix[2] = {nullptr, nullptr};
-  int *eref[2] = {nullptr, nullptr}, *ex[2] = {nullptr, nullptr}, *kbits = nullptr;
-  double row_sum[3] = {1.0, 1.0, 1.0};
+  // the fused 64-bit march (run_chain_fixed): the units of the intermediates' lines,
+  // one array [batch][unit_bs] for each tmp; null where it does not run
+  int16_t *units[4] = {nullptr, nullptr, nullptr, nullptr};
+  long long unit_bs = 0;
   int march_epoch = 0;          // plan_epoch that march_exec was captured with
   int plan_epoch = 0;           // bumped when a pass changes kernels (captured graphs are stale)
   struct AdjointState *adj = nullptr;   // adjoint / stress work buffers (lazy)

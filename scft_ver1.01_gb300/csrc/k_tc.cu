@@ -2,18 +2,21 @@
 //
 // k_real: one axis pass on working reals, out = post * K (pre * in), and for
 // FP32 the fused step pair.  k_fix: the fused march of FP64 contexts,
-// whose intermediates between passes stay 64-bit integers of one unit
-// per instance and step, so that a pass costs no conversion to or from the
-// working real (those were about half of a pass's 142 instructions per point):
-//   first  v0 = W q0 and the first filter        real in, fixed out
-//   mid    one filter                            fixed in, fixed out
+// whose intermediates between passes stay 64-bit integers, so that a pass costs no
+// conversion to or from the working real (those were about half of a pass's 142
+// instructions per point):
+//   first  v0 = W q0 and the first filter        real in, integers out
+//   mid    one filter                            integers in and out
 //   pair   filter, q = W y (stored), v = W q, filter
-//   last   filter, q = W y (stored)              fixed in, real out
-// The unit must be known before the values are: every kernel that forms v
-// reports the largest exponent (ex), and the next one scales by that times the
-// growth one step can bring (W^2 and the kernels' row sums, kbits).  Integers
-// stay below 2^59 (2^61 in registers); each line is rescaled to the digits' 2^54
-// by its own largest value, so a line keeps the accuracy of its own scale.
+//   last   filter, q = W y (stored)              integers in, real out
+// A filtered line goes out as it comes from the products, its unit (a power of two,
+// 16 bits) into an array by lines; the next pass, along another axis, gives every
+// point the unit of the line that it came from, and rescales its own lines to the
+// digits' 2^54 by their largest value.  So a line keeps the accuracy of its own scale
+// wherever in the instance it lies, as with reals, and exponents have no range to
+// leave.  (One unit for an instance and step, from bounds, is about 10 % faster, 64^3 3.53
+// ms per SCF iteration with 200 steps against 3.92, but values far below the largest lose
+// their last bits to it: beside a well 4e-10 off where FFTs leave 2e-11.)
 #include "tc_core.cuh"
 
 #include <limits.h>
@@ -94,11 +97,6 @@ __device__ __forceinline__ void over_rows(int nt, int n, int nl, L &&load, F &&f
       }
     }
   }
-}
-template <typename F>
-__device__ __forceinline__ void over_rows(int nt, int n, int nl, const int64_t *src, F &&f) {
-  over_rows<4>(nt, n, nl,
-               [&](int i) { return (int64_t)__ldg(reinterpret_cast<const long long *>(src) + i); }, f);
 }
 template <typename T> struct WithFactor {
   T x, w;
@@ -204,7 +202,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
     xb[i] = to_fixed(bb[i], Eb);
   }
   // results come in units of 2^(unit + shift)
-  const int shift = (kNd<T> == 7 ? 55 : 23) - head.kshift;
+  const int shift = (kNd<T> == 7 ? 55 - kFine : 23) - head.kshift;
   int ue = unit_exp(T(0.0f), Eb) + shift;
 
   if constexpr (PAIR) {
@@ -343,146 +341,246 @@ __global__ void __launch_bounds__(MAXT, 1) k_real(Lines ln, const void *table_, 
 // ------------------------------------------------------------------ k_fix
 enum { FIRST = 0, MID = 1, PAIR = 2, LAST = 3 };
 
-constexpr int kBadExp = 0x7fffffff;         // ex: the values are not finite
+// Units lie within +-5300 (values that are neither infinite nor 0 as reals, line_unit).
+// That of a line whose values are not finite: of its points, and what its integers are
+// rescaled to.
+constexpr int kBadUnit = 0x7fff, kBadLine = 1 << 21, kKeyBias = 1 << 22;
 
-__device__ __forceinline__ bool unit_bad(int s) { return s >= 0x40000000; }
 __device__ __forceinline__ int64_t ld64(const int64_t *p) {
   return __ldg(reinterpret_cast<const long long *>(p));
 }
-// r = W y as the stored slice's value, |r| in the range of from_fixed_fast or not
+__device__ __forceinline__ uint64_t ldw(const double *p) {
+  return (uint64_t)__ldg(reinterpret_cast<const long long *>(p));
+}
+// A point's exponent bound (|x| * 2^u <= 2^e) as a key of its line, and the unit of a
+// line's integers, |X| <= 2^54, from its largest key.  With 55 bits for every point that
+// unit is above all of theirs: they are only shifted to the right (7 instructions a point
+// instead of 12), and what that rounds off is below the rounding that the point of the
+// largest unit brings along.  Values of 2^1024 and more are infinite as reals; below
+// 2^-1100 they are 0.
+__device__ __forceinline__ int point_key(int64_t x, int u) { return u + bits_of(x) + kKeyBias; }
+__device__ __forceinline__ int line_unit(int key) {
+  const int e = max(key - kKeyBias, -1100);
+  return e > 1024 ? kBadLine : e - 54;
+}
+__device__ __forceinline__ int16_t short_unit(int u) { return (int16_t)min(u, kBadUnit); }
+// r * 2^ur as the stored slice's value
 __device__ __forceinline__ double slice_value(int64_t r, int ur) {
   const int h = (int)(r >> 32);
   if (h != (h >> 31) && fast_units(ur)) return from_fixed_fast(r, ur);
-  return from_fixed(r, ur, 0.0);
+  return ur >= kBadUnit / 2 ? bad_value(0.0) : from_fixed(r, ur, 0.0);
 }
+__device__ __forceinline__ Factor any_factor(uint64_t w) {
+  return factor_rare(w) ? factor_of_rare(w) : factor_of(w);
+}
+// The units of a thread's points, until their line's is known: two 16-bit numbers in a
+// register.
+template <int PP> struct Units {
+  uint32_t v[PP];
+  __device__ __forceinline__ void set(int i, int u0, int u1) {
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(v[i]) : "r"(u1), "r"(u0));
+  }
+  __device__ __forceinline__ int a(int i) const { return (int16_t)v[i]; }
+  __device__ __forceinline__ int b(int i) const { return (int)v[i] >> 16; }
+};
 // A thread's points of a column line: PP at off, off + sn, ..., and as many
 // another hs on; the first `lim` exist.
 struct Column {
   unsigned off, sn, hs;
   int lim;
 };
-// q = W y to the finished slice and x = W q for N/2 points (x[2j]: y of point
-// g + j of the column, x[2j + 1]: of its partner).  Without a branch in it, so
-// that the N chains (about 190 cycles each) run side by side; a value too small
-// for the fast conversion is stored again afterwards.  Returns the factors'
-// signs: a negative one is not finite.
+// q = W y to the finished slice and x = W q, in units of 2^u, for N/2 points (x[2j]: y of
+// point g + j of the column in units of 2^uo, x[2j + 1]: of its partner); returns the
+// largest key.  Without a branch in it, so that the N chains (about 190 cycles each) run
+// side by side: factors that are not normal numbers are set right before, values that
+// the fast conversion does not take are stored again afterwards.
 template <int N>
-__device__ __forceinline__ int factor_group(int64_t (&x)[N], const int64_t *wf, double *qo,
-                                            const Column &c, int g, int ur) {
+__device__ __forceinline__ int factor_group(int64_t (&x)[N], int (&u)[N], const double *w, double *qo,
+                                            const Column &c, int g, int uo) {
   auto at = [&](int i) { return c.off + (g + i / 2) * c.sn + (i & 1) * c.hs; };
-  int wneg = 0;
-  int64_t r[N], w[N];
+  uint64_t b[N];
+  Factor f[N];
+  bool rare = false, slow = (uint32_t)(uo + 490) >= 880u;   // (then ur is a fast unit)
 #pragma unroll
-  for (int i = 0; i < N; ++i) w[i] = g + i / 2 < c.lim ? ld64(wf + at(i)) : 0;
+  for (int i = 0; i < N; ++i) b[i] = g + i / 2 < c.lim ? ldw(w + at(i)) : 0x3ff0000000000000ULL;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    wneg |= (int)(w[i] >> 32);
-    r[i] = mul_w62(x[i], w[i]);
+    rare |= factor_rare(b[i]);
+    f[i] = factor_of(b[i]);
   }
-  bool slow = !fast_units(ur);
+  if (rare) {
+    slow = true;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (factor_rare(b[i])) f[i] = factor_of_rare(b[i]);
+  }
+  int64_t r[N];
+  int key = 0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const int h = (int)(r[i] >> 32);
+    r[i] = mul_w62(x[i], f[i]);
+    const int ur = uo + f[i].e - 1022, h = (int)(r[i] >> 32);
     const bool on = g + i / 2 < c.lim;
     slow |= on && h == (h >> 31);
     const double q = from_fixed_fast(r[i], ur);
     if (on) qo[at(i)] = q;
-    x[i] = mul_w62(r[i], w[i]);
+    x[i] = mul_w62(r[i], f[i]);
+    u[i] = ur + f[i].e - 1022;
+    key = max(key, on ? point_key(x[i], u[i]) : 0);
   }
   if (slow) {
 #pragma unroll 1
     for (int i = 0; i < N; ++i) {
       int64_t ri = r[0];
+      int ui = f[0].e;
 #pragma unroll
-      for (int j = 1; j < N; ++j) ri = i == j ? r[j] : ri;
-      if (g + i / 2 < c.lim) qo[at(i)] = slice_value(ri, ur);
+      for (int j = 1; j < N; ++j) {
+        ri = i == j ? r[j] : ri;
+        ui = i == j ? f[j].e : ui;
+      }
+      if (g + i / 2 < c.lim) qo[at(i)] = slice_value(ri, uo + ui - 1022);
     }
   }
-  return wneg;
+  return key;
 }
 // The same for all of a thread's points.
 template <int PP>
-__device__ __forceinline__ int factor_points(int64_t (&xa)[PP], int64_t (&xb)[PP],
-                                             const int64_t *wf, double *qo, const Column &c,
-                                             int ur) {
-  int wneg = 0;
+__device__ __forceinline__ int factor_points(int64_t (&xa)[PP], int64_t (&xb)[PP], Units<PP> &un,
+                                             const double *w, double *qo, const Column &c, int uo) {
+  int key = 0;
 #pragma unroll
   for (int g = 0; g < PP; g += 4) {
     int64_t x[8];
+    int u[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       x[2 * i] = xa[g + i];
       x[2 * i + 1] = xb[g + i];
     }
-    wneg |= factor_group(x, wf, qo, c, g, ur);
+    key = max(key, factor_group(x, u, w, qo, c, g, uo));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       xa[g + i] = x[2 * i];
       xb[g + i] = x[2 * i + 1];
+      un.set(g + i, u[2 * i], u[2 * i + 1]);
     }
   }
-  return wneg;
+  return key;
 }
 // A thread's points (16 and their partners) in the staging memory, where they
 // cost no registers: as unrolled code over registers the factor step of 16
 // points spilled 560-800 bytes a thread.
 struct Staged {
   int64_t *own;
+  int16_t *units;
   int stride;
   __device__ __forceinline__ int64_t &a(int i) const { return own[2 * i * stride]; }
   __device__ __forceinline__ int64_t &b(int i) const { return own[(2 * i + 1) * stride]; }
-  __device__ __forceinline__ int factor(const int64_t *wf, double *qo, const Column &c,
-                                        int ur) const {
-    int wneg = 0;
+  __device__ __forceinline__ int ua(int i) const { return units[2 * i * stride]; }
+  __device__ __forceinline__ int ub(int i) const { return units[(2 * i + 1) * stride]; }
+  __device__ __forceinline__ int factor(const double *w, double *qo, const Column &c, int uo) const {
+    int key = 0;
 #pragma unroll 1
     for (int g = 0; g < 16; g += 4) {
       int64_t x[8];
+      int u[8];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         x[2 * i] = a(g + i);
         x[2 * i + 1] = b(g + i);
       }
-      wneg |= factor_group(x, wf, qo, c, g, ur);
+      key = max(key, factor_group(x, u, w, qo, c, g, uo));
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         a(g + i) = x[2 * i];
         b(g + i) = x[2 * i + 1];
+        units[2 * (g + i) * stride] = short_unit(u[2 * i]);
+        units[(2 * (g + i) + 1) * stride] = short_unit(u[2 * i + 1]);
       }
     }
-    return wneg;
+    return key;
   }
 };
-// NaN where the input or the factor is not finite (rare)
-__device__ __forceinline__ void spoil_points(bool bad, const int64_t *wf, double *qo,
-                                             const Column &c, int pp) {
-  for (int i = 0; i < c.lim && i < pp; ++i) {
-    const unsigned o = c.off + i * c.sn;
-    if (bad || wf[o] < 0) qo[o] = bad_value(0.0);
-    if (bad || wf[o + c.hs] < 0) qo[o + c.hs] = bad_value(0.0);
-  }
-}
-// the largest magnitude key of a thread's points
+
+// v0 = W q0 for all of a thread's points, as factor_group does it.
 template <int PP>
-__device__ __forceinline__ int points_key(const int64_t (&xa)[PP], const int64_t (&xb)[PP]) {
+__device__ __forceinline__ int first_points(int64_t (&xa)[PP], int64_t (&xb)[PP], Units<PP> &un,
+                                            const double *in, const double *w, const Column &c) {
   int key = 0;
 #pragma unroll
-  for (int i = 0; i < PP; ++i) key = max(key, max(hi_key(xa[i]), hi_key(xb[i])));
+  for (int g = 0; g < PP; g += 2) {
+    uint64_t b[4], q[4];
+    Factor f[4];
+    int64_t x[4];
+    int u[4];
+    bool rare = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned o = c.off + (g + i / 2) * c.sn + (i & 1) * c.hs;
+      const bool on = g + i / 2 < c.lim;
+      b[i] = on ? ldw(w + o) : 0x3ff0000000000000ULL;
+      q[i] = on ? ldw(in + o) : 0x3ff0000000000000ULL;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      rare |= factor_rare(b[i]) || real_rare(q[i]);
+      f[i] = factor_of(b[i]);
+      x[i] = split_real(q[i], u[i]);
+    }
+    if (rare) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        f[i] = any_factor(b[i]);
+        if (real_rare(q[i])) x[i] = split_real_rare(q[i], u[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool on = g + i / 2 < c.lim;
+      x[i] = on ? mul_w62(x[i], f[i]) : 0;
+      u[i] += f[i].e - 1022;
+      key = max(key, on ? point_key(x[i], u[i]) : 0);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      xa[g + j] = x[2 * j];
+      xb[g + j] = x[2 * j + 1];
+      un.set(g + j, u[2 * j], u[2 * j + 1]);
+    }
+  }
   return key;
 }
-// a line's values, largest key `clz`, to the digits' 2^54; the unit's change
-template <int PP> __device__ __forceinline__ int to_line_scale(int64_t (&xa)[PP], int64_t (&xb)[PP],
-                                             int clz) {
+// A thread's points, x(i, half) in units of 2^u(i, half), and their largest key.
+template <int PP, typename X, typename U>
+__device__ __forceinline__ int load_points(int64_t (&xa)[PP], int64_t (&xb)[PP], Units<PP> &un, int lim,
+                                           X &&x, U &&u) {
+  int key = 0;
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
-    xa[i] = to_digits54(xa[i], clz - 2);
-    xb[i] = to_digits54(xb[i], clz - 2);
+    xa[i] = i < lim ? x(i, 0) : 0;
+    xb[i] = i < lim ? x(i, 1) : 0;
   }
-  return 10 - clz;
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    int u0 = 0, u1 = 0;
+    if (i < lim) {
+      u0 = u(i, 0);
+      u1 = u(i, 1);
+      key = max(key, max(point_key(xa[i], u0), point_key(xb[i], u1)));
+    }
+    un.set(i, u0, u1);
+  }
+  return key;
 }
-// reports the exponent bound of the CTA's lines (x per line, INT_MIN: none)
-__device__ __forceinline__ void report_exp(int *ex, int x) {
-  x = __reduce_max_sync(0xffffffffu, x);
-  if ((threadIdx.x & 31) == 0 && x != INT_MIN) atomicMax(ex, x);
+// ... to the unit of their line.
+template <int PP>
+__device__ __forceinline__ void scale_points(int64_t (&xa)[PP], int64_t (&xb)[PP], const Units<PP> &un,
+                                             int ue) {
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    xa[i] = shifted(xa[i], ue - un.a(i));
+    xb[i] = shifted(xb[i], ue - un.b(i));
+  }
 }
 
 template <int PP, bool XP, int MODE>
@@ -496,7 +594,6 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
   const unsigned line0 = blockIdx.x * e.ln;
   const int nl = (int)min((long long)e.ln, ln.lines - line0);
   const unsigned H = ln.sh.half[0];
-  const int kbits = *fp.kbits;
   pdl_wait();      // the input is the previous pass's output
   pdl_release();
   if (e.issuer) {
@@ -505,8 +602,7 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
     return;
   }
   e.run_compute();
-  const int eref = fp.eref[b];
-  // element offsets within an instance fit 32 bits (at most 128^3 points)
+  // element offsets within an instance fit 32 bits (lines of at most 128 points)
   const unsigned c = line0 + e.line, rl = (unsigned)ln.row_len;
   const unsigned base = XP ? c * ln.n : (c / rl) * (unsigned)ln.s_outer + c % rl;
   const unsigned sn = XP ? 1 : (unsigned)ln.s_n;
@@ -518,76 +614,46 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
   int64_t *stg = reinterpret_cast<int64_t *>(smem_raw);
   int64_t *row = stg + e.line * P + k0;                 // its points in the staging tile
   int *ur_row = reinterpret_cast<int *>(smem_raw + e.lay.ur_off);
-  const int64_t *wf = fp.w + b * fp.w_bs;
-  // units: 2^u_in of the input, 2^u_out of the output
-  const int s_in = MODE == FIRST ? 0 : fp.u_in[b], s_out = MODE == LAST ? 0 : fp.u_out[b];
-  bool bad = unit_bad(s_in) || unit_bad(s_out);   // (FIRST: u_out is the input's own)
-  const int u_in = s_in + fp.w_in * (eref - 1022) + kbits - 59;
-  const int u_out = s_out + fp.w_out * (eref - 1022) + kbits - 59;
-  const int shift = 55 - head.kshift;
+  int16_t *us = reinterpret_cast<int16_t *>(smem_raw + ln.sh.units_off);
+  int16_t *urow = us + e.line * P + k0;                 // rows' units, as the points lie
+  const double *w = fp.w + b * fp.w_bs;
+  const int shift = 55 - kFine - head.kshift;
 
   int64_t xa[PP], xb[PP];
-  int ue;                       // xa, xb in units of 2^ue
+  Units<PP> un;
+  int key = 0;
   if constexpr (MODE == FIRST) {
     // real slice times the factor; a handful of launches per iteration, so the
     // x pass reads its rows without staging
-    const double *in = static_cast<const double *>(fp.in) + b * fp.in_bs;
-    double a[PP], bb[PP];
-    int key = 0;
-#pragma unroll
-    for (int i = 0; i < PP; ++i) {
-      a[i] = i < lim ? ldg(in + (off + i * sn)) : 0.0;
-      bb[i] = i < lim ? ldg(in + (off + i * sn + hs)) : 0.0;
-      key = max(key, max(mag_key(a[i]), mag_key(bb[i])));
-    }
-    e.start();   // TMEM address, cleared keys
-    key = e.line_key(0, key);
-    const int Eb = line_exp(0.0, key);
-#pragma unroll
-    for (int i = 0; i < PP; ++i) {
-      const int64_t w0 = i < lim ? wf[off + i * sn] : 0, w1 = i < lim ? wf[off + i * sn + hs] : 0;
-      bad |= w0 < 0 || w1 < 0;
-      xa[i] = mul_w62(to_fixed(a[i], Eb) << 6, w0);
-      xb[i] = mul_w62(to_fixed(bb[i], Eb) << 6, w1);
-    }
-    bad = e.any(bad);
-    ue = unit_exp(0.0, Eb) - 6 + eref - 1022;
+    key = first_points(xa, xb, un, static_cast<const double *>(fp.in) + b * fp.in_bs, w, col);
   } else {
     const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs;
     if constexpr (XP) {
-      over_rows(e.ncomp, ln.n, nl, in + tile,
-                [&](int r, int cc, int, int64_t x) { stg[r * P + cc] = x; });
+      over_rows<4>(e.ncomp, ln.n, nl, [&](int i) { return ld64(in + tile + i); },
+                   [&](int r, int cc, int, int64_t x) { stg[r * P + cc] = x; });
       e.sync();
     }
-#pragma unroll
-    for (int i = 0; i < PP; ++i) {
-      xa[i] = xb[i] = 0;
-      if (i < lim) {
-        xa[i] = XP ? row[i] : ld64(in + (off + i * sn));
-        xb[i] = XP ? row[i + H] : ld64(in + (off + i * sn + hs));
-      }
-    }
-    int key = points_key(xa, xb);
-    e.start();   // TMEM address, cleared keys; the staging tile is read
-    key = e.line_key(0, key);
-    ue = u_in + to_line_scale(xa, xb, clz32((uint32_t)key | 1u));
+    const int16_t *u_in = fp.u_in + b * fp.u_in_bs + (c / fp.u_div) * fp.u_quo + (c % fp.u_div) * fp.u_rem +
+                      k0 * fp.u_step;
+    key = load_points(
+        xa, xb, un, lim,
+        [&](int i, int half) { return XP ? row[i + half * H] : ld64(in + (off + i * sn + half * hs)); },
+        [&](int i, int half) { return (int)__ldg(u_in + (i + half * H) * fp.u_step); });
   }
+  e.start();   // TMEM address, cleared keys; the staging tile is read
 
   // The filters and what follows each.  One copy of the code serves both
   // filters of a pair: with two a pair was 7450 instructions long (119 KB at
   // N = 128) and waited for them.
   int64_t *out = static_cast<int64_t *>(fp.out) + b * fp.out_bs;
   constexpr bool kStaged = PP == 16 && !XP && (MODE == PAIR || MODE == LAST);
-  const Staged sp{stg + threadIdx.x, e.ncomp};
+  const Staged sp{stg + threadIdx.x, us + threadIdx.x, e.ncomp};
+  int uo = 0;                   // the unit of the filtered line
 #pragma unroll 1
   for (int f = 0; f < (MODE == PAIR ? 2 : 1); ++f) {
-    if (MODE == FIRST || (MODE == PAIR && f == 1)) {
-      // the formed v: report its exponent, rescale the lines
-      const int key = e.line_key(1, points_key(xa, xb));   // (its barrier: the staging tile is read)
-      const int clz = clz32((uint32_t)key | 1u);
-      if (e.blk == 0) report_exp(fp.ex + b, bad ? kBadExp : (e.line < nl ? ue + 64 - clz : INT_MIN));
-      ue += to_line_scale(xa, xb, clz);
-    }
+    key = e.line_key(f, key);   // (its barrier: the staging tile is read)
+    const int ue = line_unit(key);
+    scale_points(xa, xb, un, ue);
     if constexpr (kStaged) {
       e.filter(xa, xb, []() {}, [&](int i, int64_t p, int64_t q) {
         if (i < 8) {
@@ -606,13 +672,12 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
     } else {
       e.filter(xa, xb, []() {});
     }
+    uo = ue == kBadLine ? kBadUnit : ue + shift;
     if (MODE == LAST || (MODE == PAIR && f == 0)) {
-      const int ur = ue + shift + eref - 1022;            // unit of r = W y
       double *qo = static_cast<double *>(fp.q) + b * fp.q_bs;
-      int wneg = 0;
       if constexpr (XP) {
         e.sync();   // A is free
-        if (e.blk == 0) ur_row[e.line] = ur;
+        if (e.blk == 0) ur_row[e.line] = uo;
 #pragma unroll
         for (int i = 0; i < PP; ++i) {
           if (i < lim) {
@@ -621,53 +686,55 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
           }
         }
         e.sync();
-        over_rows(e.ncomp, ln.n, nl, wf + tile, [&](int r, int cc, int i, int64_t w) {
-          wneg |= (int)(w >> 32);
-          const int64_t v = mul_w62(stg[r * P + cc], w);
-          qo[tile + i] = slice_value(v, ur_row[r]);
-          if (MODE == PAIR) stg[r * P + cc] = mul_w62(v, w);
+        over_rows<4>(e.ncomp, ln.n, nl, [&](int i) { return ldw(w + tile + i); },
+                     [&](int r, int cc, int i, uint64_t wb) {
+          const Factor fa = any_factor(wb);
+          const int ur = ur_row[r] + fa.e - 1022;
+          const int64_t v = mul_w62(stg[r * P + cc], fa);
+          qo[tile + i] = slice_value(v, ur);
+          if (MODE == PAIR) {
+            stg[r * P + cc] = mul_w62(v, fa);
+            us[r * P + cc] = short_unit(ur + fa.e - 1022);
+          }
         });
-        if (bad || wneg < 0)
-          over_rows(e.ncomp, ln.n, nl, wf + tile, [&](int, int, int i, int64_t w) {
-            if (bad || w < 0) qo[tile + i] = bad_value(0.0);
-          });
         if constexpr (MODE == PAIR) {
-          if (e.any(wneg < 0)) bad = true;
+          e.sync();
+          key = 0;
 #pragma unroll
           for (int i = 0; i < PP; ++i) {
-            xa[i] = i < lim ? row[i] : 0;
-            xb[i] = i < lim ? row[i + H] : 0;
+            xa[i] = xb[i] = 0;
+            if (i < lim) {
+              xa[i] = row[i];
+              xb[i] = row[i + H];
+              const int u0 = urow[i], u1 = urow[i + H];
+              un.set(i, u0, u1);
+              key = max(key, max(point_key(xa[i], u0), point_key(xb[i], u1)));
+            }
           }
         }
-      } else {
-        if constexpr (kStaged) {
-          wneg = sp.factor(wf, qo, col, ur);
+      } else if constexpr (kStaged) {
+        key = sp.factor(w, qo, col, uo);
 #pragma unroll
-          for (int i = 0; i < PP && MODE == PAIR; ++i) {
-            xa[i] = sp.a(i);
-            xb[i] = sp.b(i);
-          }
-        } else {
-          wneg = factor_points(xa, xb, wf, qo, col, ur);
+        for (int i = 0; i < PP && MODE == PAIR; ++i) {
+          xa[i] = sp.a(i);
+          xb[i] = sp.b(i);
+          un.set(i, sp.ua(i), sp.ub(i));
         }
-        if (bad || wneg < 0) spoil_points(bad, wf, qo, col, PP);
-        if constexpr (MODE == PAIR) {
-          if (e.any(wneg < 0)) bad = true;
-        }
+      } else if constexpr (PP <= 8) {
+        key = factor_points(xa, xb, un, w, qo, col, uo);
       }
-      ue = ur + eref - 1022;   // v = W r (PAIR)
     }
   }
 
   if constexpr (MODE != LAST) {
-    const Rescale rs(u_out - (ue + shift));   // to the output's unit
+    if (e.blk == 0 && e.line < nl) fp.u_out[b * fp.u_out_bs + c] = (int16_t)uo;
     if constexpr (XP) {
       e.sync();   // A is free
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
         if (i < lim) {
-          row[i] = rs(xa[i]);
-          row[i + H] = rs(xb[i]);
+          row[i] = xa[i];
+          row[i + H] = xb[i];
         }
       }
       e.sync();
@@ -676,16 +743,16 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
 #pragma unroll 4
       for (int i = 0; i < PP; ++i) {
         if (i < lim) {
-          out[off + i * sn] = rs(sp.a(i));
-          out[off + i * sn + hs] = rs(sp.b(i));
+          out[off + i * sn] = sp.a(i);
+          out[off + i * sn + hs] = sp.b(i);
         }
       }
     } else {
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
         if (i < lim) {
-          out[off + i * sn] = rs(xa[i]);
-          out[off + i * sn + hs] = rs(xb[i]);
+          out[off + i * sn] = xa[i];
+          out[off + i * sn + hs] = xb[i];
         }
       }
     }
@@ -707,8 +774,8 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
 // FILM true (nz = 1): a whole march segment, step after step, in one launch of
 // one CTA per instance: nothing of a film leaves the CTA but its slices.
 //
-// Between its filters the planes lie in shared memory as integers of one unit
-// (rows of nx + 1: conflict-free along both axes).  q and W are read and written
+// Between its filters the planes lie in shared memory as integers of their lines'
+// units (rows of nx + 1: conflict-free along both axes).  q and W are read and written
 // from the y lines, where consecutive lines are consecutive in memory.
 struct PlaneArgs {
   Shape sh;
@@ -716,7 +783,6 @@ struct PlaneArgs {
   int steps;             // FILM: contour steps of the segment
   long long q_step;      // FILM: from one slice to the next
 };
-
 template <int PP, bool FILM>
 __global__ void __launch_bounds__(544, 1)
     k_planes(PlaneArgs pa, const void *tx, const void *ty, FixPass fp) {
@@ -724,10 +790,9 @@ __global__ void __launch_bounds__(544, 1)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   E e;
   e.setup(smem_raw, pa.sh, tx, ty);
-  const int shift_x = 55 - static_cast<const TcHead *>(tx)->kshift;
-  const int shift_y = 55 - static_cast<const TcHead *>(ty)->kshift;
+  const int shift_x = 55 - kFine - static_cast<const TcHead *>(tx)->kshift;
+  const int shift_y = 55 - kFine - static_cast<const TcHead *>(ty)->kshift;
   const long long b = blockIdx.z;
-  const int kbits = *fp.kbits;
   const int filters = FILM ? 2 * pa.steps : 4;
   auto axis_of = [](int f) { return FILM ? f & 1 : (f == 1 || f == 2 ? 1 : 0); };
   pdl_wait();
@@ -738,13 +803,15 @@ __global__ void __launch_bounds__(544, 1)
     return;
   }
   e.run_compute();
-  const int eref = fp.eref[b];
   const int nx = pa.nx, ny = pa.ny, P = nx + 1;
   const int z0 = blockIdx.x * pa.per, np = min(pa.per, pa.nz - z0);
   const unsigned tile = (unsigned)z0 * ny * nx;
   const int k0 = PP * e.blk, pl = e.line / nx, xx = e.line - pl * nx;
   int64_t *S = reinterpret_cast<int64_t *>(smem_raw);
-  const int64_t *wf = fp.w + b * fp.w_bs;
+  // units: of the lines last filtered along each axis, and of points that have their own
+  int16_t *ul = reinterpret_cast<int16_t *>(smem_raw + e.lay.ur_off);
+  int16_t *us = reinterpret_cast<int16_t *>(smem_raw + pa.sh.units_off);
+  const double *w = fp.w + b * fp.w_bs;
   // this thread's points as x line (row `line`) and as y line (plane pl, x)
   const int lim_x = e.line < np * ny ? pa.sh.half[0] - k0 : 0;
   const int lim_y = e.line < np * nx ? pa.sh.half[1] - k0 : 0;
@@ -752,94 +819,89 @@ __global__ void __launch_bounds__(544, 1)
   const Column col{tile + (unsigned)(pl * ny + k0) * nx + xx, (unsigned)nx,
                    (unsigned)(pa.sh.half[1] * nx), lim_y};
 
-  int us, u_out = 0;            // the unit of what lies in S
-  bool bad;
+  int64_t xa[PP], xb[PP];
+  Units<PP> un;
+  int key = 0;
   if constexpr (FILM) {
-    // v0 = W q0, scaled by the slice's largest magnitude
-    const double *in = static_cast<const double *>(fp.in) + b * fp.in_bs + tile;
-    int *top = reinterpret_cast<int *>(smem_raw + e.lay.ur_off);
-    if (threadIdx.x == 0) top[0] = top[1] = 0;
-    e.start();
-    int key = 0;
-    for (int i = threadIdx.x; i < ny * nx; i += e.ncomp) key = max(key, mag_key(ldg(in + i)));
-    key = __reduce_max_sync(0xffffffffu, key);
-    if ((threadIdx.x & 31) == 0) atomicMax(top, key);
-    e.sync();
-    key = top[0];
-    bad = key >= bad_key<double>();
-    const int Eb = line_exp(0.0, key);
-    bool wbad = false;
-    over_rows(e.ncomp, nx, ny, wf + tile, [&](int r, int cc, int i, int64_t w) {
-      wbad |= w < 0;
-      S[r * P + cc] = mul_w62(to_fixed(ldg(in + i), Eb) << 5, w);
-    });
-    if (e.any(wbad)) bad = true;
-    us = unit_exp(0.0, Eb) - 5 + eref - 1022;
+    // v0 = W q0 (once a segment: rows read as they lie)
+    key = first_points(xa, xb, un, static_cast<const double *>(fp.in) + b * fp.in_bs, w,
+                       Column{(unsigned)(e.line * nx + k0), 1u, (unsigned)pa.sh.half[0], lim_x});
   } else {
-    const int s_in = fp.u_in[b], s_out = fp.u_out[b];
-    bad = unit_bad(s_in) || unit_bad(s_out);
-    us = s_in + fp.w_in * (eref - 1022) + kbits - 59;
-    u_out = s_out + fp.w_out * (eref - 1022) + kbits - 59;
-    const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs;
-    over_rows(e.ncomp, nx, np * ny, in + tile,
-              [&](int r, int cc, int, int64_t x) { S[r * P + cc] = x; });
-    e.start();
+    // the units of the z lines that the points came from: the same for every plane
+    const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs + tile;
+    const int16_t *u_in = fp.u_in + b * fp.u_in_bs;
+    const int nt = e.ncomp, total = np * ny * nx, plane = ny * nx, dr = nt / nx, dc = nt % nx, dp = nt % plane;
+    int r = (int)threadIdx.x / nx, cc = (int)threadIdx.x % nx, ip = (int)threadIdx.x % plane;
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < total; i0 += 4 * nt) {
+      int64_t x[4];
+      int16_t u[4];
+      int p = ip;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool on = i0 + j * nt < total;
+        x[j] = on ? ld64(in + i0 + j * nt) : 0;
+        u[j] = on ? __ldg(u_in + p) : (int16_t)0;
+        p += dp;
+        if (p >= plane) p -= plane;
+      }
+      ip = p;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (i0 + j * nt < total) {
+          S[r * P + cc] = x[j];
+          us[r * P + cc] = u[j];
+        }
+        r += dr;
+        cc += dc;
+        if (cc >= nx) {
+          cc -= nx;
+          ++r;
+        }
+      }
+    }
   }
+  e.start();
 
   double *qo = static_cast<double *>(fp.q) + b * fp.q_bs;
-  int64_t xa[PP], xb[PP];
-  int ue = us;
 #pragma unroll 1
   for (int f = 0; f < filters; ++f) {
     const int ax = axis_of(f);
     e.set_axis(ax);
     const int lim = ax ? lim_y : lim_x, at = ax ? at_y : at_x, st = ax ? P : 1, hs = e.H * st;
-    if (FILM || f != 2) {
-#pragma unroll
-      for (int i = 0; i < PP; ++i) {
-        xa[i] = i < lim ? S[at + i * st] : 0;
-        xb[i] = i < lim ? S[at + i * st + hs] : 0;
-      }
-      ue = us;
+    if (FILM ? f != 0 : f != 2) {
+      // a y line's points bring the units of their rows, an x line's their own, or in the
+      // last filter those of their columns
+      const bool own = ax == 0 && (FILM || f == 0);
+      const int16_t *ur = own ? us + at : (ax ? ul + pl * ny + k0 : ul + kLines + e.line / ny * nx + k0);
+      key = load_points(
+          xa, xb, un, lim, [&](int i, int half) { return S[at + i * st + half * hs]; },
+          [&](int i, int half) { return (int)ur[i + half * e.H]; });
     }
-    const int key = e.line_key(f & 3, points_key(xa, xb));   // (its barrier: S is read)
+    key = e.line_key(f & 3, key);   // (its barrier: S is read)
     if (e.blk == 0) e.clear_key((f + 2) & 3);
-    const int clz = clz32((uint32_t)key | 1u);
-    if (!FILM && f == 2 && e.blk == 0)
-      report_exp(fp.ex + b, bad ? kBadExp : (lim_y > 0 ? ue + 64 - clz : INT_MIN));
-    ue += to_line_scale(xa, xb, clz);
+    const int ue = line_unit(key);
+    scale_points(xa, xb, un, ue);
     e.filter(xa, xb, []() {});
-    ue += ax ? shift_y : shift_x;
-    int target = us;
-    if (FILM ? ax == 1 : f == 1) {
-      const int ur = ue + eref - 1022;
-      const int wneg = factor_points(xa, xb, wf, qo, col, ur);
-      if (bad || wneg < 0) spoil_points(bad, wf, qo, col, PP);
-      if (e.any(wneg < 0)) bad = true;
-      ue = ur + eref - 1022;
+    const int uo = ue == kBadLine ? kBadUnit : ue + (ax ? shift_y : shift_x);
+    const bool slice = FILM ? ax == 1 : f == 1;
+    if (slice) {
+      key = factor_points(xa, xb, un, w, qo, col, uo);
       if (!FILM) continue;     // v goes on along y
       if (f + 1 == filters) break;
       qo += pa.q_step;
-      // the next unit from the largest v (two slots in turn)
-      int *top = reinterpret_cast<int *>(smem_raw + e.lay.ur_off) + 2;
-      const int slot = f >> 1 & 1;
-      int x = ue + 64 - clz32((uint32_t)points_key(xa, xb) | 1u);
-      x = __reduce_max_sync(0xffffffffu, lim > 0 ? x : INT_MIN);
-      if (threadIdx.x == 0) top[slot ^ 1] = INT_MIN;
-      if (f == 1 && threadIdx.x == 0) top[slot] = INT_MIN;
-      e.sync();
-      if ((threadIdx.x & 31) == 0) atomicMax(top + slot, x);
-      e.sync();
-      target = us = top[slot] + kbits - 59;
-    } else if (!FILM && f >= 2) {
-      target = us = u_out;
+    } else if (e.blk == 0) {
+      ul[ax * kLines + e.line] = (int16_t)uo;
     }
-    const Rescale rs(target - ue);
 #pragma unroll
     for (int i = 0; i < PP; ++i) {
       if (i < lim) {
-        S[at + i * st] = rs(xa[i]);
-        S[at + i * st + hs] = rs(xb[i]);
+        S[at + i * st] = xa[i];
+        S[at + i * st + hs] = xb[i];
+        if (FILM && ax) {
+          us[at + i * st] = (int16_t)un.a(i);
+          us[at + i * st + hs] = (int16_t)un.b(i);
+        }
       }
     }
     e.sync();
@@ -847,6 +909,7 @@ __global__ void __launch_bounds__(544, 1)
   if constexpr (!FILM) {
     int64_t *out = static_cast<int64_t *>(fp.out) + b * fp.out_bs;
     over_rows(e.ncomp, nx, np * ny, [&](int r, int cc, int i) { out[tile + i] = S[r * P + cc]; });
+    if (threadIdx.x < np * ny) fp.u_out[b * fp.u_out_bs + z0 * ny + threadIdx.x] = ul[threadIdx.x];
   }
   e.finish(fp.err);
 }
@@ -967,43 +1030,6 @@ __global__ void __launch_bounds__(544, 1)
   e.finish(ps.err);
 }
 
-// ------------------------------------------------- factors and slice exponents
-// The largest biased FP64 exponent of each instance's finite factors.
-__global__ void k_wexp(const double *__restrict__ W, long long M, int *__restrict__ eref) {
-  const double *w = W + (long long)blockIdx.y * M;
-  int e = 0;
-  stream_loop<4>(M, [&](long long i) { return w[i]; }, [&](long long, double x) {
-    if (mag_key(x) < bad_key<double>()) e = max(e, line_exp(x, mag_key(x)));
-  });
-  e = __reduce_max_sync(0xffffffffu, e);
-  if ((threadIdx.x & 31) == 0) atomicMax(eref + blockIdx.y, e);
-}
-// W as packed integers: W = wf * 2^(eref - 1084), wf < 2^62; negative where not
-// finite.
-__global__ void k_wfix(const double *__restrict__ W, long long M, const int *__restrict__ eref_,
-                       int64_t *__restrict__ wf) {
-  const long long o = (long long)blockIdx.y * M;
-  const int eref = eref_[blockIdx.y];
-  stream_loop<4>(M, [&](long long i) { return W[o + i]; }, [&](long long i, double x) {
-    // from units of 2^(eref - 1076)
-    wf[o + i] = mag_key(x) >= bad_key<double>() ? -1 : pack_w62(to_fixed(x, eref) << 8);
-  });
-}
-// Exponent bound of a slice: every |q| < 2^ex[b]; kBadExp when not finite.
-__global__ void k_slice_exp(const double *__restrict__ q, long long bs, long long M,
-                            int *__restrict__ ex) {
-  const double *x = q + (long long)blockIdx.y * bs;
-  int key = 0;
-  stream_loop<4>(M, [&](long long i) { return x[i]; },
-                 [&](long long, double v) { key = max(key, mag_key(v)); });
-  key = __reduce_max_sync(0xffffffffu, key);
-  if ((threadIdx.x & 31) == 0 && key != 0) {
-    int e = kBadExp;
-    if (key < bad_key<double>()) e = unit_exp(0.0, line_exp(0.0, key)) + 55;
-    atomicMax(ex + blockIdx.y, e);
-  }
-}
-
 // Geometry of a pass, or false when the kernels do not take it.
 bool lines_of(const AxisPlan &ap, int nd, Lines &ln) {
   if (!ap.tc || !tc_line_possible(ap.n, nd) || ap.n_real < 1 || ap.n_outer < 1) return false;
@@ -1097,9 +1123,16 @@ cudaError_t launch_fix_t(Lines ln, const void *tc, const FixPass &fp, cudaStream
   const int lc = lines_per_cta(ln.sh);
   dim3 grid((unsigned)((ln.lines + lc - 1) / lc), 1, fp.batch);
   // x passes stage rows; column passes with 16 points per thread the factor step
-  if (XP) ln.sh.stage = lc * (ln.n + 1) * 8;
-  else if (ln.sh.pp == 16 && (MODE == PAIR || MODE == LAST))
-    ln.sh.stage = kLines * ln.sh.kg[0] * 256;
+  // (and 2 bytes for each point's unit)
+  if (XP) {
+    ln.sh.stage = lc * (ln.n + 1) * 8;
+    ln.sh.units = lc * (ln.n + 1) * 2;
+  } else if (ln.sh.pp == 16) {
+    if (MODE == PAIR || MODE == LAST) {
+      ln.sh.stage = kLines * ln.sh.kg[0] * 256;
+      ln.sh.units = kLines * ln.sh.kg[0] * 64;
+    }
+  }
   ln.sh.finish();
   const size_t smem = ln.sh.lay.total;
   if (ln.sh.pp == 4)
@@ -1132,6 +1165,7 @@ void plane_shape(int nx, int ny, int nz, int nd, int batch, bool film, PlaneArgs
   const int lc = lines_per_cta(pa.sh);
   pa.per = lc / m;
   pa.sh.stage = lc * (nx + 1) * (nd == 7 ? 8 : 4);
+  pa.sh.units = nd == 7 ? lc * (nx + 1) * 2 : 0;
   pa.sh.finish();
 }
 // ... of passes apx (x) and apy (lines nx apart), or false.
@@ -1256,9 +1290,11 @@ bool build_scaled(const std::vector<dd> &K, int nd, int kg, int less,
                   std::vector<unsigned char> &table) {
   const int n = (int)K.size(), H = n / 2, kp = 16 * kg;
   const int bits = 8 * nd;
-  double mx = 0.0;
-  for (int d = 0; d < H; ++d)
+  double mx = 0.0, l1 = 0.0;
+  for (int d = 0; d < H; ++d) {
     for (int s = -1; s <= 1; s += 2) mx = fmax(mx, fabs(K[d].h + s * K[d + H].h));
+    l1 += fabs(K[d].h) + fabs(K[d + H].h);
+  }
   TcHead head;
   memset(&head, 0, sizeof head);
   int shift = 0;
@@ -1268,6 +1304,8 @@ bool build_scaled(const std::vector<dd> &K, int nd, int kg, int less,
     shift = bits - 1 - ex;
     // a top digit of at most 127 with any others behind it
     if (ldexp(mx, shift) > ldexp(126.9, bits - 8)) --shift;
+    // results |2 y| <= sum |K'| * 2^(kFine - 1) below 2^61
+    while (nd == 7 && ldexp(l1, shift) > 0x1.fp61 / (1 << kFine)) --shift;
   }
   shift -= less;
   if (shift > 900 || shift < -900) return false;
@@ -1487,10 +1525,9 @@ cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double, kStepSet> &ps, b
 
 cudaError_t launch_fix(const AxisPlan &ap, int mode, const FixPass &fp, cudaStream_t st) {
   Lines ln;
-  if (!lines_of(ap, 7, ln) || fp.batch < 1 || fp.batch > 65535 || !fp.in || !fp.eref || !fp.kbits ||
-      (mode != LAST && (!fp.out || !fp.u_out)) || (mode != FIRST && !fp.u_in) ||
-      (mode != MID && !fp.w) || ((mode == PAIR || mode == LAST) && !fp.q) ||
-      ((mode == FIRST || mode == PAIR) && !fp.ex))
+  if (!lines_of(ap, 7, ln) || fp.batch < 1 || fp.batch > 65535 || !fp.in ||
+      (mode != LAST && (!fp.out || !fp.u_out)) || (mode != FIRST && (!fp.u_in || fp.u_div < 1)) ||
+      (mode != MID && !fp.w) || ((mode == PAIR || mode == LAST) && !fp.q))
     return cudaErrorInvalidValue;
   const bool x = ap.n_fast != 0;
   switch (mode) {
@@ -1529,9 +1566,9 @@ cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSe
 cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPass &fp, int steps,
                           long long q_step, cudaStream_t st) {
   PlaneArgs pa;
-  if (!planes_of(apx, apy, 7, fp.batch, steps > 0, pa) || fp.batch < 1 || fp.batch > 65535 || !fp.in || !fp.eref ||
-      !fp.kbits || !fp.w || !fp.q || (steps == 0 && (!fp.u_in || !fp.u_out || !fp.ex || !fp.out)) ||
-      steps < 0 || (steps > 0 && pa.nz != 1))
+  if (!planes_of(apx, apy, 7, fp.batch, steps > 0, pa) || fp.batch < 1 || fp.batch > 65535 || !fp.in ||
+      !fp.w || !fp.q || (steps == 0 && (!fp.u_in || !fp.u_out || !fp.out)) || steps < 0 ||
+      (steps > 0 && pa.nz != 1))
     return cudaErrorInvalidValue;
   pa.steps = steps;
   pa.q_step = q_step;
@@ -1540,26 +1577,6 @@ cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPas
   auto k = steps ? (pa.sh.pp == 4 ? k_planes<4, true> : k_planes<8, true>)
                  : (pa.sh.pp == 4 ? k_planes<4, false> : k_planes<8, false>);
   return launch_pdl(k, grid, dim3(pa.sh.threads), smem, st, pa, apx.tc, apy.tc, fp);
-}
-
-// Factors in integers: eref[b] and wf from W (two launches).
-cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
-                        cudaStream_t st) {
-  if (batch > 65535) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(eref, 0, sizeof(int) * batch, st);
-  if (e != cudaSuccess) return e;
-  const unsigned g = (unsigned)std::min<long long>((M + 1023) / 1024, 608);
-  k_wexp<<<dim3(g, batch), 256, 0, st>>>(W, M, eref);
-  k_wfix<<<dim3(g, batch), 256, 0, st>>>(W, M, eref, wf);
-  return cudaGetLastError();
-}
-// ex[b] (cleared by the caller) from a slice.
-cudaError_t launch_slice_exp(const double *q, long long bs, long long M, int batch, int *ex,
-                             cudaStream_t st) {
-  if (batch > 65535) return cudaErrorInvalidValue;
-  const unsigned g = (unsigned)std::min<long long>((M + 1023) / 1024, 608);
-  k_slice_exp<<<dim3(g, batch), 256, 0, st>>>(q, bs, M, ex);
-  return cudaGetLastError();
 }
 
 }  // namespace scft

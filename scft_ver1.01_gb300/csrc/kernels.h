@@ -159,21 +159,19 @@ cudaError_t launch_tc(const AxisPlan &ap, const PassSet<float, kStepSet> &ps, bo
                       cudaStream_t st);
 cudaError_t launch_tc(const AxisPlan &ap, const PassSet<double, kStepSet> &ps, bool pair,
                       cudaStream_t st);
-// One pass of the fused FP64 march, whose intermediates are
-// 64-bit integers (batch instances; strides in elements).  The unit of an
-// intermediate is 2^(u[b] + w * (eref[b] - 1022) + kbits - 59): u the exponent
-// bound of the values it was formed from, w the factors applied since.
+// One pass of the fused FP64 march, whose intermediates are 64-bit integers (batch
+// instances; strides in elements): a point's value is its integer times 2^u, u that of
+// the line that the pass before filtered it in.
 struct FixPass {
   const void *in;            // FIRST: FP64, else integers
   void *out;                 // integers (not LAST)
   void *q;                   // PAIR, LAST: the finished slice
-  const int64_t *w;          // the factors as integers (launch_wfix)
-  const int *eref;           // their largest exponent per instance
-  const int *kbits;          // log2 bound of one step's filters' growth
-  const int *u_in, *u_out;   // exponent bounds, [batch]
-  int w_in, w_out;
-  int *ex;                   // FIRST, PAIR: exponent bound of the formed W q (atomic max)
-  long long in_bs, out_bs, q_bs, w_bs;
+  const double *w;           // the factors
+  const int16_t *u_in;       // units by lines of the pass before ...
+  int16_t *u_out;            // ... and of this one, in the order of their offsets
+  // point k of line c: (c / u_div) * u_quo + (c % u_div) * u_rem + k * u_step
+  int u_div, u_quo, u_rem, u_step;
+  long long in_bs, out_bs, q_bs, w_bs, u_in_bs, u_out_bs;
   int batch;
   unsigned *err;             // device error word (bounded-wait timeouts)
 };
@@ -186,10 +184,6 @@ cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy,
                           const PassSet<float, kStepSet> &ps, cudaStream_t st);
 cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const FixPass &fp, int steps,
                           long long q_step, cudaStream_t st);
-cudaError_t launch_wfix(const double *W, long long M, int batch, int *eref, int64_t *wf,
-                        cudaStream_t st);
-cudaError_t launch_slice_exp(const double *q, long long bs, long long M, int batch, int *ex,
-                             cudaStream_t st);
 
 // Generic mixed-radix Stockham line filter (any n whose prime factors are
 // <= 61).  in/out may not alias.  pre multiplies the input, post the output

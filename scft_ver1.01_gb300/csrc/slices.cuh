@@ -62,17 +62,77 @@ SL_HD int clz32(uint32_t u) {
   return u ? __builtin_clz(u) : 32;
 #endif
 }
-// y * w / 2^62 rounded to nearest (within 2^-29 of a unit), |y| < 2^61, with the
-// factor 0 <= w < 2^62 packed as two 31-bit halves (high word, low word):
-// three 32-bit products.
-SL_HD int64_t mul_w62(int64_t y, int64_t wp) {
-  const int wh = (int)(wp >> 32), wl = (int)wp;
-  const int yh = (int)(y >> 31), yl = (int)((uint32_t)y & 0x7fffffffu);
-  const int64_t t = (int64_t)yh * wl + ((int64_t)yl * wh + (1 << 30));
-  return (int64_t)yh * wh + (t >> 31);
+// A factor W > 0: W = (h * 2^31 + l) * 2^(e - 1022 - 62), h and l two 31-bit halves of its
+// 53 bits, normalised (h >= 2^30).
+struct Factor {
+  int h, l, e;
+};
+// e of a factor that is not a finite positive number (or of such a real, below):
+// far above any other exponent
+constexpr int kBadFactor = 1 << 18;
+SL_HD bool factor_rare(uint64_t w) {   // not within 2^-500 .. 2^500
+  return (uint32_t)(w >> 32) - ((1023u - 500u) << 20) >= 1000u << 20;
 }
-SL_HD int64_t pack_w62(int64_t w) {
-  return (int64_t)((uint64_t)(w >> 31) << 32 | (uint64_t)(w & 0x7fffffff));
+SL_HD Factor factor_of(uint64_t w) {   // (a normal number)
+  const uint32_t hi = (uint32_t)(w >> 32), lo = (uint32_t)w;
+  Factor f;
+  f.e = (int)(hi >> 20);
+  f.h = (int)(((hi & 0x000fffffu) | 0x00100000u) << 10 | lo >> 22);
+  f.l = (int)((lo << 9) & 0x7fffffffu);
+  return f;
+}
+static __host__ __device__ __noinline__ Factor factor_of_rare(uint64_t w) {
+  Factor f = {0, 0, 0};
+  if (w - 0x0010000000000000ULL < 0x7fe0000000000000ULL) {
+    f = factor_of(w);
+  } else if (w >= 0x7ff0000000000000ULL) {   // negative, infinite, NaN
+    f.e = w == 0x8000000000000000ULL ? 0 : kBadFactor;
+  } else if (w != 0) {
+    const int lz = clz64(w) - 11;      // denormal: its leading bit to bit 52
+    const uint64_t m = w << (lz + 9);
+    f.e = 1 - lz;
+    f.h = (int)(m >> 31);
+    f.l = (int)(m & 0x7fffffff);
+  }
+  return f;
+}
+// y * (h * 2^31 + l) / 2^62, |y| < 2^61, rounded to nearest but for the product of the
+// low halves, which counts with its mean (half of l: within half a unit).
+SL_HD int64_t mul_w62(int64_t y, const Factor &w) {
+  const int yh = (int)(y >> 31), yl = (int)((uint32_t)y & 0x7fffffffu);
+  const int64_t t = (int64_t)yh * w.l + ((int64_t)yl * w.h + (int64_t)((1u << 30) + ((uint32_t)w.l >> 1)));
+  return (int64_t)yh * w.h + (t >> 31);
+}
+// x = m * 2^u, |m| in [2^60, 2^61) or 0; u of kBadFactor: not finite
+SL_HD bool real_rare(uint64_t x) {   // zero, denormal, not finite
+  return ((uint32_t)(x >> 32) & 0x7fffffffu) - 0x00100000u >= 0x7fe00000u;
+}
+SL_HD int64_t split_real(uint64_t x, int &u) {   // (a normal number)
+  u = ((int)(x >> 52) & 0x7ff) - 1083;
+  const int64_t m = (int64_t)(((x & 0xfffffffffffffULL) | 0x10000000000000ULL) << 8), s = (int64_t)x >> 63;
+  return (m ^ s) - s;
+}
+static __host__ __device__ __noinline__ int64_t split_real_rare(uint64_t x, int &u) {
+  const uint64_t a = x & 0x7fffffffffffffffULL;
+  const int lz = a ? clz64(a) - 11 : 0;          // denormal: its leading bit to bit 52
+  u = a >= 0x7ff0000000000000ULL ? kBadFactor : 1 - lz - 1083;
+  const int64_t m = a >= 0x7ff0000000000000ULL ? 0 : (int64_t)(a << (lz + 8));
+  return (int64_t)x < 0 ? -m : m;
+}
+// |x| <= 2^bits_of(x), at least 55
+SL_HD int bits_of(int64_t x) {
+  const int h = (int)(x >> 32);
+  return 64 - clz32((uint32_t)(h ^ (h >> 31)) | 0x400000u);
+}
+// x * 2^-s rounded to nearest (halves up), s > 0
+SL_HD int64_t shifted(int64_t x, int s) {
+#ifdef __CUDA_ARCH__
+  int64_t r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s - 1));   // (63 and more: the sign)
+  return (r + 1) >> 1;
+#else
+  return ((x >> (s > 64 ? 63 : s - 1)) + 1) >> 1;
+#endif
 }
 
 // 2^e as a float, e clamped to the normal range.
@@ -148,7 +208,7 @@ SL_HD double from_fixed_fast(int64_t y, int ue) {
   const uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(1085 + ue - lz) << 20);
   return u2d((uint64_t)(hi | (sg & 0x80000000u)) << 32 | (uint32_t)m);
 }
-SL_HD bool fast_units(int ue) { return ue > -1000 && ue < 900; }
+SL_HD bool fast_units(int ue) { return (uint32_t)(ue + 1000) < 1900u; }   // -1000 .. 899
 // The signed base-256 digits of X (digit i weighs 256^(ND-1-i)) as bytes plus
 // 128: all but the top one are in [0, 255]; the top one, in the high half word,
 // is in [0, 256] (7 digits) or [64, 192] (4 digits).

@@ -13,7 +13,11 @@
 // accumulate in FP32 in one TMEM accumulator per g.  The host checks for each
 // table that no accumulator can reach 2^22 (2^24 for FP32), so every partial
 // sum is an integer that FP32 holds exactly and the order of the sums does not
-// matter.  What is left out (i + j >= ND) is below the last digit's unit.
+// matter.  What is left out (i + j >= ND, for 7 digits i + j >= 8: groups 0 .. 7 are kept)
+// is below the last digit's unit.  The eighth group and an output unit 4 bits finer
+// (kFine) leave less at the small values of a line than an FFT does: with
+// seven groups and the coarser unit values 2^-90 of a line's largest were up to 5 times
+// further off.
 //
 // Tile: the 128 rows (M) of one tcgen05.mma x N points per CTA.  A row holds one
 // of LN = 128/rep lines; with rep > 1 every line stands in rep rows, because a
@@ -23,9 +27,9 @@
 // k + H: it writes their digits as A operands, once per copy (K-major core
 // matrices of 8 rows x 16 bytes, unswizzled), and reads the same outputs back.
 // B holds the digits of Kc or Kd stacked along its rows (digit j, output n), so
-// one instruction multiplies x's digit i with all of K's digits 0 .. ND-1-i and
-// adds into the accumulators i .. ND-1 side by side: up to 256 columns per
-// instruction.  (One instruction per digit pair, 32 or 64 columns wide, took
+// one instruction multiplies x's digit i with all of K's digits that it meets (the
+// first ND-i; 7 digits: 8-i, at most 7) and adds into the accumulators from i on side
+// by side: up to 256 columns per instruction.  (One instruction per digit pair, 32 or 64 columns wide, took
 // about 76 cycles each whatever its width.)  Lines above 128 points (FP32) have
 // no room for that B; there its 8x8 core matrix (bn, bk), which depends only on
 // bn - bk, is shared by descriptor: with A's k blocks in reverse order both
@@ -53,6 +57,11 @@ struct TcHead {
   int kshift;    // K' = K * 2^kshift
   int pad[3];
 };
+// 7 digits: bits of a result below 256^7, the unit of K' X / 256^6 / 256.  Its 61 bits
+// bound K': sum |K'| < 2^(62 - kFine).
+constexpr int kFine = 4;
+// accumulators (digit groups) of a product
+__host__ __device__ constexpr int groups(int nd) { return nd == 7 ? 8 : nd; }
 
 // 16-point blocks of a half line
 __host__ __device__ constexpr int line_blocks(int n) { return (n / 2 + 15) / 16; }
@@ -62,7 +71,7 @@ __host__ __device__ constexpr int pairs_per_thread(int kg) { return kg <= 2 ? 8 
 __host__ __device__ constexpr bool dense_b(int kg) { return kg <= 4; }
 // Accumulators come in two TMEM buffers, so that one is read while the tensor
 // core fills the other.  A buffer holds all outputs of c or d (whose A operands
-// then lie side by side); for 7 digits and 16 points per thread TMEM and shared
+// then lie side by side); for 7 digits (8 accumulators) and 16 points per thread TMEM and shared
 // memory have no room for that: a buffer holds half of the outputs (8 of each
 // thread's 16), a half takes two rounds, and c's operand memory serves d.
 __host__ __device__ constexpr bool split_rows(int nd, int kg) { return nd == 7 && kg > 2; }
@@ -104,6 +113,7 @@ struct Shape {
   int nd, pp, rep, axes;
   int half[2], kg[2];    // H, and 16-point blocks of it
   int stage;             // staging memory, bytes (aliases the A operands)
+  int units, units_off;  // bytes for points' units behind it
   Smem lay;
   int cols, threads;     // TMEM columns
   int a_digit[2], b_half[2];   // bytes of a digit's A operand, of a half's table
@@ -115,7 +125,7 @@ struct Shape {
       a_digit[i] = kLines * kg[i] * 32;
       b_half[i] = b_half_bytes(nd, kg[i]);
       const int a = nd * a_digit[i] * (both_halves(nd, kg[i]) ? 2 : 1);
-      const int c = nd * group_cols(nd, kg[i]) * (dense_b(kg[i]) ? 2 : 1);
+      const int c = groups(nd) * group_cols(nd, kg[i]) * (dense_b(kg[i]) ? 2 : 1);
       big = a > big ? a : big;
       bsum += (res ? 2 : 1) * b_half[i];
       need = c > need ? c : need;
@@ -125,10 +135,11 @@ struct Shape {
       a_digit[i] = a_digit[0];
       b_half[i] = b_half[0];
     }
-    lay.b_off = (big + 127) / 128 * 128;
+    units_off = (big + 15) / 16 * 16;
+    lay.b_off = (units_off + units + 127) / 128 * 128;
     lay.key_off = lay.b_off + bsum;
     lay.ur_off = lay.key_off + kKeySlots * kLines * 4;   // line keys
-    lay.bar_off = lay.ur_off + kLines * 4;               // per-line units, or CTA scratch
+    lay.bar_off = lay.ur_off + 2 * kLines * 4;           // lines' units (planes: of both axes)
     lay.total = lay.bar_off + 64;                        // six mbarriers, TMEM address
     for (cols = 32; cols < need;) cols *= 2;
     threads = kLines * ((16 * blocks + pp * rep - 1) / (pp * rep)) + issuer_threads(pp);
@@ -264,43 +275,23 @@ __device__ __forceinline__ void digit_words(int a, int b, uint32_t (&o)[4]) {
 }
 
 // ---- accumulators -> result
-// 7 digits: sum_g D_g 256^(6-g) / 256, rounded.  D_g + 1.5*2^23 has the integer
-// D_g in its low bits (|D_g| < 2^22).
-__device__ __forceinline__ int64_t combine(const float (&D)[7]) {
+// 7 digits: sum_g D_g 256^(6-g) / 256 * 2^kFine, rounded.  D_g + 1.5*2^23 has the
+// integer D_g in its low bits (|D_g| < 2^22).
+__device__ __forceinline__ int64_t combine(const float (&D)[8]) {
   constexpr uint32_t C = 0x4B400000u;
-  uint32_t I[7];
+  uint32_t I[8];
 #pragma unroll
-  for (int g = 0; g < 7; ++g) I[g] = __float_as_uint(D[g] + 12582912.f);
+  for (int g = 0; g < 8; ++g) I[g] = __float_as_uint(D[g] + 12582912.f);
   const uint32_t p01 = I[0] * 256u + I[1] - C * 257u;
   const int p23 = (int)(I[2] * 256u + I[3] - C * 257u);
   const int p45 = (int)(I[4] * 256u + I[5] - C * 257u);
-  const int l6 = ((int)(I[6] - C) + 128) >> 8;
-  return (int64_t)((uint64_t)p01 << 32) + (int64_t)p23 * 65536 + (int64_t)(p45 + l6);
+  const int p67 = (int)(I[6] * 256u + I[7] - C * 257u + (0x8000u >> kFine)) >> (16 - kFine);
+  return (int64_t)((uint64_t)(p01 << kFine) << 32) + p67 + (int64_t)p45 * (1 << kFine) +
+         (int64_t)p23 * (65536 << kFine);
 }
 __device__ __forceinline__ float combine(const float (&D)[4]) {
   return fmaf(fmaf(fmaf(D[0], 256.f, D[1]), 256.f, D[2]), 256.f, D[3]);
 }
-
-// x << lz, then / 256 rounded to nearest: a line's values from below 2^(62-lz)
-// to the digits' 2^54.
-__device__ __forceinline__ int64_t to_digits54(int64_t x, int lz) {
-  return (int64_t)(((uint64_t)x << lz) + 128) >> 8;
-}
-// A filter result to another unit: p * 2^-s, rounded to nearest.
-struct Rescale {
-  int l, r;
-  int64_t half;
-  __device__ __forceinline__ explicit Rescale(int s) {
-    l = s < 0 ? -s & 63 : 0;
-    r = s < 0 ? 0 : (s > 62 ? 62 : s);
-    half = r ? 1LL << (r - 1) : 0;
-  }
-  __device__ __forceinline__ int64_t operator()(int64_t p) const {
-    return (int64_t)(((uint64_t)p << l) + half) >> r;
-  }
-};
-// high word of |x|, as a magnitude key
-__device__ __forceinline__ int hi_key(int64_t x) { return (int)((uint64_t)(x ^ (x >> 63)) >> 32); }
 
 // mbarriers of a CTA
 enum { kFull0 = 0, kFull1 = 1, kEmpty = 2, kDone0 = 3, kDone1 = 4, kTable = 5 };
@@ -328,6 +319,7 @@ template <int ND, int PP> struct Tile {
   bool ok, both, issuer;
   static constexpr bool kSplit = ND == 7 && PP == 16;   // split_rows
   static constexpr bool kRes = ND == 4 || PP <= 8;   // both halves' tables resident
+  static constexpr int NG = groups(ND);
 
   __device__ __forceinline__ uint32_t bar(int i) const { return sm32(smem + lay.bar_off) + 8 * i; }
 
@@ -521,18 +513,26 @@ template <int ND, int PP> struct Tile {
       constexpr uint32_t blbo = ND * gc * 16 * (kSplit ? 2 : 1), adig = kLines * KG * 32;
       const uint64_t ad = smem_desc(a, kLines * 16, 128);
       const uint64_t bd = smem_desc(b + (kSplit ? buf * ND * gc * 16 : 0), blbo, 128);
-      const uint32_t d = tmem + buf * ND * gc;
+      const uint32_t d = tmem + buf * NG * gc;
 #pragma unroll
-      for (int s = 0; s < KG; ++s)
-#pragma unroll
-        for (int i = 0; i < ND; ++i) {
-          constexpr uint32_t kstep = 2 * kLines * 16 >> 4, bstep = 2 * blbo >> 4;
-          const uint32_t rows = (ND - i) * gc, n0 = rows < 256 ? rows : 256;
-          const uint64_t ai = ad + (s * kstep + (i * adig >> 4)), bs = bd + s * bstep;
-          mma_f16(d + i * gc, ai, bs, id0 | ((n0 >> 3) << 17), s + i != 0);
-          if (rows > 256)
-            mma_f16(d + i * gc + 256, ai, bs + 256, id0 | ((rows - 256) >> 3 << 17), s + i != 0);
+      for (int s = 0; s < KG; ++s) {
+        constexpr uint32_t kstep = 2 * kLines * 16 >> 4, bstep = 2 * blbo >> 4;
+        const uint64_t as = ad + s * kstep, bs = bd + s * bstep;
+        // K's first `rows` rows from row r0 on times x's digit i, from accumulator i on
+        auto mma = [&](int i, uint32_t r0, uint32_t rows, int accumulate) {
+          mma_f16(d + i * gc + r0, as + (i * adig >> 4), bs + r0, id0 | ((rows >> 3) << 17), accumulate);
+        };
+        // the first to write an accumulator overwrites it: with an eighth one, which
+        // digit 0 does not meet, that is digit 1 for all but the first
+        if (NG > ND && s == 0) {
+          mma(1, 0, ND * gc, 0);
+          mma(0, 0, gc, 0);
+          mma(0, gc, (ND - 1) * gc, 1);
         }
+#pragma unroll
+        for (int i = NG > ND && s == 0 ? 2 : 0; i < ND; ++i)
+          mma(i, 0, (NG - i < ND ? NG - i : ND) * gc, s + i != 0);
+      }
     }
   }
   // lines above 128 points: one instruction per digit pair (see the top)
@@ -553,27 +553,27 @@ template <int ND, int PP> struct Tile {
   }
 
   // GO outputs of this thread from accumulator buffer `buf`, starting at column
-  // `col` of each group (with 16 points per thread four at a time: 28
-  // accumulators in registers instead of 56, which spilled)
+  // `col` of each group (with 16 points per thread four at a time: 32
+  // accumulators in registers instead of 64, which spilled)
   static constexpr int GO = PP < 8 ? PP : 8;
   __device__ __forceinline__ void get(int buf, int col, Acc (&y)[GO]) {
     constexpr int L = PP == 16 ? 4 : GO;
     const uint32_t gc = group_cols(ND, kg);
     const uint32_t lane0 = tmem + ((uint32_t)(warp & 3) << 21);
-    uint32_t addr = lane0 + (dense_b(kg) ? buf * ND * gc : 0) + col;
+    uint32_t addr = lane0 + (dense_b(kg) ? buf * NG * gc : 0) + col;
     if (col >= (int)gc) addr = lane0;   // (no such outputs: not used)
 #pragma unroll
     for (int h = 0; h < GO; h += L) {
-      float D[ND][L];
+      float D[NG][L];
       __syncwarp();
 #pragma unroll
-      for (int g = 0; g < ND; ++g) tm_ld(addr + g * gc + h, D[g]);
+      for (int g = 0; g < NG; ++g) tm_ld(addr + g * gc + h, D[g]);
       tm_wait_ld();
 #pragma unroll
       for (int i = 0; i < L; ++i) {
-        float d[ND];
+        float d[NG];
 #pragma unroll
-        for (int g = 0; g < ND; ++g) d[g] = D[g][i];
+        for (int g = 0; g < NG; ++g) d[g] = D[g][i];
         y[h + i] = combine(d);
       }
     }

@@ -99,7 +99,7 @@ CASES = [((24, 16, 12), 0, 2), ((64, 12, 10), 0, 1), ((96, 10, 6), 0, 1), ((10, 
 
 
 @pytest.mark.parametrize("fused", [True, False])
-@pytest.mark.parametrize("kind", ["low"])
+@pytest.mark.parametrize("kind", ["rough", "well", "low"])
 @pytest.mark.parametrize("grid,prec,batch", CASES)
 def test_every_value_is_as_good_as_by_ffts(pkg, grid, prec, batch, kind, fused):
     ds, f = (0.1, 0.4) if kind == "rough" else (0.02, 0.3)
