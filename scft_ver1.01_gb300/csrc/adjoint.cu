@@ -20,8 +20,9 @@
 //   <q+(s), W (dK/dL_a) W q(s-1)> = <W^-1 D_a W q+(s), q(s)> :
 // one pass an axis and step instead of one an axis for every axis.  The whole
 // operator W K D_a W is applied where W or 1/W leaves 2^-60 .. 2^60, since the
-// quotient could lose what q(s) has left, and on axes that the tensor cores filter,
-// which have the one table of K_a D_a.
+// quotient could lose what q(s) has left, where W is rough (k_rough), since D_a
+// without K multiplies the roundings of high wave numbers, and on axes that the
+// tensor cores filter, which have the one table of K_a D_a.
 #include <math.h>
 #include <string.h>
 
@@ -141,24 +142,53 @@ __global__ void __launch_bounds__(kT) k_dots(DotArgs<R> d, const R *__restrict__
   }
 }
 
-// out = 1 / W; *wide is set where W is not within 2^-60 .. 2^60.
+// out = 1 / W
 __device__ __forceinline__ float inverse(float w) { return 1.0f / w; }
 __device__ __forceinline__ double inverse(double w) { return 1.0 / w; }
 __device__ __forceinline__ scft::dfloat inverse(scft::dfloat w) {
   return scft::dfloat(1.0 / (double)w);
 }
-__device__ __forceinline__ double size_of(float w) { return w; }
-__device__ __forceinline__ double size_of(double w) { return w; }
-__device__ __forceinline__ double size_of(scft::dfloat w) { return w.hi; }
 template <typename R>
-__global__ void k_inverse(const R *__restrict__ W, R *__restrict__ out, long long n,
-                          int *__restrict__ wide) {
+__global__ void k_inverse(const R *__restrict__ W, R *__restrict__ out, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    out[i] = inverse(W[i]);
+}
+// *flag is set where W is not within 2^-60 .. 2^60, or where D_a W^2, by second
+// differences (c[a] = 2 ds / L_a (n_a / L_a)^2; 0: not asked), is above kRough of W^2
+// itself.  Fields of a solve come to 0.001 - 0.02 (smooth patterns, or noise of 0.02 on
+// them); with noise of +-15 they come to 5, and the quotient's stress was 25 - 250 times
+// further off than the whole operator's (64^3: FP32 1.1e-5 against 3.9e-7, double-float
+// 4.9e-13 against 1.9e-15), in proportion to it.
+constexpr float kRough = 0.05f;
+__device__ __forceinline__ float approx(float w) { return w; }
+__device__ __forceinline__ float approx(double w) { return (float)w; }
+__device__ __forceinline__ float approx(scft::dfloat w) { return w.hi; }
+struct Axes {
+  int n[3];
+  float c[3];
+};
+template <typename R>
+__global__ void k_rough(const R *__restrict__ W, Axes g, long long n, int *__restrict__ flag) {
+  bool bad = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const R w = W[i];
-    if (!(size_of(w) > 0x1p-60 && size_of(w) < 0x1p60)) *wide = 1;
-    out[i] = inverse(w);
+    const float w = approx(W[i]);
+    bad |= !(w > 0x1p-60f && w < 0x1p60f);
+    long long at = i, st = 1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int m = g.n[a], k = (int)(at % m);
+      if (g.c[a] != 0.0f) {
+        const float up = approx(W[k + 1 < m ? i + st : i - (m - 1) * st]);
+        const float dn = approx(W[k > 0 ? i - st : i + (m - 1) * st]);
+        bad |= !(g.c[a] * fabsf(up * up + dn * dn - 2.0f * w * w) <= kRough * w * w);
+      }
+      at /= m;
+      st *= m;
+    }
   }
+  if (bad) *flag = 1;
 }
 
 // out[b] = sum_k partial[b*nblk + k]
@@ -401,21 +431,38 @@ int ensure_adjoint(scft_ctx *ctx, int K) {
   return SCFT_OK;
 }
 
-// Whether axis pass pi takes W K D_a W; out = that of `in` (s0, s1: scratch, `out`
-// the result's place among them).
+// Whether axis pass pi takes W K D_a W.
 bool whole_axis(const scft_ctx *ctx, int pi, int wide) { return wide || ctx->passes[pi].tc; }
+// ... for all of them: the FFT axes too, where these factors do not allow the quotient
+// (flag: device scratch).
+template <typename R>
+int whole_wanted(scft_ctx *ctx, const R *const (&W)[2], int *flag, int *wide) {
+  const double L[3] = {ctx->p.lx, ctx->p.ly, ctx->p.lz};
+  cudaStream_t st = ctx->st;
+  Axes g = {{ctx->p.nx, ctx->p.ny, ctx->p.nz}, {0.0f, 0.0f, 0.0f}};
+  *wide = 1;
+  for (size_t pi = 0; pi < ctx->passes.size(); ++pi) {
+    if (ctx->passes[pi].tc) continue;
+    const int a = ctx->pass_axis[pi];
+    g.c[a] = (float)(2.0 * ctx->p.ds0 / L[a] * (g.n[a] / L[a]) * (g.n[a] / L[a]));
+    *wide = 0;
+  }
+  if (*wide) return SCFT_OK;
+  CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  for (int f = 0; f < 2; ++f) {
+    k_rough<R><<<grid_for(ctx->M * ctx->batch), kT, 0, st>>>(W[f], g, ctx->M * ctx->batch, flag);
+    ++ctx->launches;
+  }
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  return SCFT_OK;
+}
+// out = W K D_a W in, a the axis of pass pi (s0, s1: scratch).
 template <typename R>
 int whole_term(scft_ctx *ctx, int pi, const R *in, long long in_bs, const R *W, long long w_bs,
-               int nb, R *t, R *s0, R *s1, const R **out, cudaStream_t st) {
-  const long long M = ctx->M;
-  if (ctx->passes[pi].tc) {
-    *out = t;
-    return scft_internal_filter(ctx, in, in_bs, t, M, W, W, w_bs, nb, pi, s0, s1, st);
-  }
-  RC(scft_internal_deriv(ctx, pi, in, in_bs, t, M, W, nullptr, w_bs, nb, st));
-  R *o = ctx->passes.size() == 1 ? s0 : t;
-  *out = o;
-  return scft_internal_filter(ctx, t, M, o, M, nullptr, W, w_bs, nb, -1, o == s0 ? s1 : s0, s1, st);
+               int nb, R *out, R *s0, R *s1, cudaStream_t st) {
+  return scft_internal_filter(ctx, in, in_bs, out, ctx->M, W, W, w_bs, nb, pi, s0, s1, st);
 }
 
 template <typename R>
@@ -582,19 +629,17 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
     return pt;
   };
 
-  // the box derivatives' 1/W (the marching pair is free), and whether it will do
+  // the box derivatives' 1/W (the marching pair is free), where it will do
   R *Winv[2] = {va, vb};
   int wide = 0;
   if (want_L) {
-    int *flag = reinterpret_cast<int *>(A.small + 4 * B);
-    CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
-    for (int f = 0; f < 2; ++f) {
-      k_inverse<R><<<grid_for(M * B), kT, 0, st>>>(W[f], Winv[f], M * B, flag);
+    const R *const Wc[2] = {W[0], W[1]};
+    RC(whole_wanted<R>(ctx, Wc, reinterpret_cast<int *>(A.small + 4 * B), &wide));
+    for (int f = 0; f < 2 && !wide; ++f) {
+      k_inverse<R><<<grid_for(M * B), kT, 0, st>>>(W[f], Winv[f], M * B);
       ++ctx->launches;
     }
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
   }
 
   // ---- the sweeps: the q chain's in reverse (s = N .. 1, q+ marched alongside),
@@ -622,13 +667,12 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
       if (want_L) {
         const int L = q_chain ? ACC_L1 : ACC_L2;
         for (int pi = 0; pi < np; ++pi) {
-          const R *d = t;
           const bool whole = whole_axis(ctx, pi, wide);
           if (whole)   // <a, W K D W x0>
-            RC(whole_term<R>(ctx, pi, x0, bs0, W[f], M, B, t, s0, s1, &d, st));
+            RC(whole_term<R>(ctx, pi, x0, bs0, W[f], M, B, t, s0, s1, st));
           else         // = <A a, W^-1 D W x0>
             RC(scft_internal_deriv(ctx, pi, x0, bs0, t, M, W[f], Winv[f], M, B, st));
-          CK(dot(d, M, whole ? a : p, M, q_chain ? (whole ? co : co_n) : nullptr, M, accp(L + pi),
+          CK(dot(t, M, whole ? a : p, M, q_chain ? (whole ? co : co_n) : nullptr, M, accp(L + pi),
                  q_chain ? accp(ACC_Q + pi) : nullptr));
         }
         if (has_unit)
@@ -703,7 +747,7 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
 // W^-1 D_a W q+(s) contracted with q(s) in FP64, or (whole_axis) W K D_a W q(s-1)
 // with q+(s).
 template <typename R>
-int stress_sums(scft_ctx *ctx, bool wide, double *acc, int *flag) {
+int stress_sums(scft_ctx *ctx, bool wide, double *acc) {
   AdjointState &A = *ctx->adj;
   const long long M = ctx->M;
   const int B = ctx->batch, nblk = kDotBlocks, np = (int)ctx->passes.size();
@@ -737,7 +781,7 @@ int stress_sums(scft_ctx *ctx, bool wide, double *acc, int *flag) {
     for (int b = 0; b < B && bl.ns > 0; ++b) {
       const R *W = static_cast<const R *>(ctx->W[bl.f]) + b * M;
       if (quotient) {
-        k_inverse<R><<<grid_for(M), kT, 0, st>>>(W, winv, M, flag);
+        k_inverse<R><<<grid_for(M), kT, 0, st>>>(W, winv, M);
         ++ctx->launches;
         CK(cudaGetLastError());
       }
@@ -751,7 +795,8 @@ int stress_sums(scft_ctx *ctx, bool wide, double *acc, int *flag) {
         for (int pi = 0; pi < np; ++pi) {
           if (!whole_axis(ctx, pi, wide)) continue;
           DotArgs<R> one = {};
-          RC(whole_term<R>(ctx, pi, qin, M, W, 0, cnt, t[0], t[1], t[2], &one.x[0], st));
+          RC(whole_term<R>(ctx, pi, qin, M, W, 0, cnt, t[0], t[1], t[2], st));
+          one.x[0] = t[0];
           one.acc[0] = slots(pi);
           one.n = 1;
           CK(dots(one, qcs, cnt));
@@ -784,20 +829,17 @@ int stress_impl(scft_ctx *ctx, double *h_out) {
   double *acc = reinterpret_cast<double *>(static_cast<unsigned char *>(A.smem) + A.sacc_off);
   double *sums = acc + (size_t)4 * B * nblk;
   int *flag = reinterpret_cast<int *>(sums + 4 * B);
-  CK(cudaMemsetAsync(flag, 0, sizeof(int), st));
   std::vector<double> s_h(4 * (size_t)B), hQ(B);
   int wide = 0;
-  for (int again = 0; again < 2; ++again) {
-    RC(stress_sums<R>(ctx, again != 0, acc, flag));
-    k_sum_slots<<<4 * B, kT, 0, st>>>(acc, nblk, sums);
-    ++ctx->launches;
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(s_h.data(), sums, 8 * 4 * B, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hQ.data(), ctx->Q, 8 * B, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&wide, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    RC(scft_internal_sync_check(ctx));
-    if (!wide) break;
-  }
+  const R *const W[2] = {static_cast<const R *>(ctx->W[0]), static_cast<const R *>(ctx->W[1])};
+  RC(whole_wanted<R>(ctx, W, flag, &wide));
+  RC(stress_sums<R>(ctx, wide != 0, acc));
+  k_sum_slots<<<4 * B, kT, 0, st>>>(acc, nblk, sums);
+  ++ctx->launches;
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(s_h.data(), sums, 8 * 4 * B, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(hQ.data(), ctx->Q, 8 * B, cudaMemcpyDeviceToHost, st));
+  RC(scft_internal_sync_check(ctx));
   for (int b = 0; b < B; ++b) {
     const double scale = -1.0 / ((double)M * hQ[b]);   // -d ln Q / dL
     for (int a = 0; a < 3; ++a) h_out[3 * b + a] = 0.0;

@@ -76,9 +76,9 @@ int upload_tc(scft_ctx *ctx, int pi, const std::vector<double> &g, const std::ve
 // exp(-ds0 k^2)/n, with the constant factors of length-1 axes folded into the
 // first pass) and their logarithmic box derivatives: d/dL_a of exp(-ds0 k_a^2) is
 // exp(-ds0 k_a^2) * 2 ds0 k_a^2 / L_a because k_a is proportional to 1/L_a; dgain
-// holds (2 ds0 k_a^2 / L_a) / n, the operator D_a with dK/dL_a = K D_a, and the
-// tensor-core table of an axis K_a D_a (D_a's own range of sizes would leave its
-// low wave numbers few bits: stresses 1e-13 off instead of 1e-15).
+// holds (2 ds0 k_a^2 / L_a) / n, the operator D_a with dK/dL_a = K D_a, and K_a D_a of
+// every pass, which is also the tensor-core table of an axis (D_a's own range of sizes
+// would leave its low wave numbers few bits: stresses 1e-13 off instead of 1e-15).
 // Rewritten in place when the box changes.
 int upload_gains(scft_ctx *ctx) {
   const scft_params &p = ctx->p;
@@ -95,7 +95,7 @@ int upload_gains(scft_ctx *ctx) {
     }
   }
   size_t dbytes = 0;
-  for (const AxisPlan &ap : ctx->passes) dbytes += ((size_t)ap.n * rb + 255) & ~(size_t)255;
+  for (const AxisPlan &ap : ctx->passes) dbytes += 2 * (((size_t)ap.n * rb + 255) & ~(size_t)255);
   if (!ctx->dgain) CK(cudaMalloc(&ctx->dgain, dbytes));
   size_t doff = 0;
   for (size_t pi = 0; pi < ctx->passes.size(); ++pi) {
@@ -109,20 +109,23 @@ int upload_gains(scft_ctx *ctx) {
       dg[m] = 2.0 * p.ds0 * k2[m] / lens[a] / ap.n;
       kdg[m] = g[m] * 2.0 * p.ds0 * k2[m] / lens[a];
     }
-    void *dptr = static_cast<unsigned char *>(ctx->dgain) + doff;
-    ctx->dgain_pass[pi] = dptr;
-    doff += ((size_t)ap.n * rb + 255) & ~(size_t)255;
-    if (rb == 4) {
-      std::vector<float> gf(g.begin(), g.end()), dgf(dg.begin(), dg.end());
-      CK(cudaMemcpy(const_cast<void *>(ap.gain), gf.data(), 4 * ap.n, cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(dptr, dgf.data(), 4 * ap.n, cudaMemcpyHostToDevice));
-    } else if (ctx->rkind == kRealDF) {
-      std::vector<scft::dfloat> gd(g.begin(), g.end()), dgd(dg.begin(), dg.end());
-      CK(cudaMemcpy(const_cast<void *>(ap.gain), gd.data(), 8 * ap.n, cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(dptr, dgd.data(), 8 * ap.n, cudaMemcpyHostToDevice));
-    } else {
-      CK(cudaMemcpy(const_cast<void *>(ap.gain), g.data(), 8 * ap.n, cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(dptr, dg.data(), 8 * ap.n, cudaMemcpyHostToDevice));
+    auto place = [&]() {
+      void *at = static_cast<unsigned char *>(ctx->dgain) + doff;
+      doff += ((size_t)ap.n * rb + 255) & ~(size_t)255;
+      return at;
+    };
+    ctx->dgain_pass[pi] = place();
+    ctx->kdgain_pass[pi] = place();
+    const std::vector<double> *tables[3] = {&g, &dg, &kdg};
+    const void *dst[3] = {ap.gain, ctx->dgain_pass[pi], ctx->kdgain_pass[pi]};
+    for (int k = 0; k < 3; ++k) {
+      const int rc = with_real(ctx, [&](auto r) {
+        using R = decltype(r);
+        const std::vector<R> t(tables[k]->begin(), tables[k]->end());
+        CK(cudaMemcpy(const_cast<void *>(dst[k]), t.data(), sizeof(R) * ap.n, cudaMemcpyHostToDevice));
+        return (int)SCFT_OK;
+      });
+      if (rc) return rc;
     }
     if (ctx->tc_want[pi]) {
       const int rc = upload_tc(ctx, (int)pi, g, kdg);
@@ -1015,7 +1018,7 @@ int scft_internal_get_conc(scft_ctx *ctx) { return get_conc(ctx); }
 namespace {
 template <typename R>
 int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long out_bs,
-                const R *pre, const R *post, long long w_bs, int nb, int tc_deriv, R *s0, R *s1,
+                const R *pre, const R *post, long long w_bs, int nb, int deriv, R *s0, R *s1,
                 cudaStream_t st) {
   const long long M = ctx->M;
   const int np = (int)ctx->passes.size();
@@ -1032,7 +1035,10 @@ int filter_impl(scft_ctx *ctx, const R *in, long long in_bs, R *out, long long o
     p.pre[0] = pi == 0 ? pre : nullptr;
     p.post[0] = pi == np - 1 ? post : nullptr;
     AxisPlan ap = ctx->passes[pi];
-    if (pi == tc_deriv) ap.tc = ctx->dtc_pass[pi];
+    if (pi == deriv) {
+      ap.gain = ctx->kdgain_pass[pi];
+      ap.tc = ctx->dtc_pass[pi];
+    }
     int rc = launch_set(ctx, ap, p, st);
     if (rc) return rc;
   }
@@ -1085,11 +1091,11 @@ int scft_internal_steps(scft_ctx *ctx, const StepIO *io, int n, long long w_bs, 
 
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,
-                         int nb, int tc_deriv, void *s0, void *s1, cudaStream_t st) {
+                         int nb, int deriv, void *s0, void *s1, cudaStream_t st) {
   return with_real(ctx, [&](auto r) {
     using R = decltype(r);
     return filter_impl<R>(ctx, (const R *)in, in_bs, (R *)out, out_bs, (const R *)pre,
-                          (const R *)post, w_bs, nb, tc_deriv, (R *)s0, (R *)s1, st);
+                          (const R *)post, w_bs, nb, deriv, (R *)s0, (R *)s1, st);
   });
 }
 

@@ -64,10 +64,11 @@ struct scft_ctx {
   void *tables = nullptr;
   std::vector<scft::AxisPlan> passes;
   int pass_axis[3] = {0, 0, 0};       // grid axis (0 x, 1 y, 2 z) of each pass
-  // box derivatives: per pass the gain times d(-ds k^2)/dL of its axis,
+  // box derivatives: per pass d(-ds k^2)/dL of its axis, D_a, and the gain times that,
   // and for length-1 axes (no pass) the constant d(-ds k^2)/dL
   void *dgain = nullptr;
   const void *dgain_pass[3] = {nullptr, nullptr, nullptr};
+  const void *kdgain_pass[3] = {nullptr, nullptr, nullptr};
   double unit_c[3] = {0.0, 0.0, 0.0};
   // tensor-core tables (k_tc.cu) of the passes that run there, for the gain
   // and its box derivative; slot 2*pass + derivative, 0 where a pass has none
@@ -120,13 +121,13 @@ std::string scft_internal_wait_message(unsigned word);
 
 // One application of the step operator's diffusion part to nb slices:
 // out = post * K (pre * in), K = the per-axis line filters of the context
-// (x, y, z passes, no plane fusion).  tc_deriv >= 0: pass tc_deriv (on the tensor
-// cores) with its table of K_a D_a, D_a = d ln K / dL_a.  s0 and s1 hold the
+// (x, y, z passes, no plane fusion).  deriv >= 0: pass deriv with K_a D_a for K_a,
+// D_a = d ln K / dL_a.  s0 and s1 hold the
 // intermediates (nb slices of M each); in, out, s0 and s1 must not overlap (with
 // one or two passes s1 is not used).  Working precision.
 int scft_internal_filter(scft_ctx *ctx, const void *in, long long in_bs, void *out,
                          long long out_bs, const void *pre, const void *post, long long w_bs,
-                         int nb, int tc_deriv, void *s0, void *s1, cudaStream_t st);
+                         int nb, int deriv, void *s0, void *s1, cudaStream_t st);
 // out = post * D_a (pre * in): one FFT pass along pass pi's axis.
 int scft_internal_deriv(scft_ctx *ctx, int pi, const void *in, long long in_bs, void *out,
                         long long out_bs, const void *pre, const void *post, long long w_bs, int nb,
