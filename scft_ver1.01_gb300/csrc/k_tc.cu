@@ -15,7 +15,7 @@
 // digits' 2^54 by their largest value.  So a line keeps the accuracy of its own scale
 // wherever in the instance it lies, as with reals, and exponents have no range to
 // leave.  (One unit for an instance and step, from bounds, is about 10 % faster, 64^3 3.53
-// ms per SCF iteration with 200 steps against 3.92, but values far below the largest lose
+// ms per SCF iteration with 200 steps against 3.83, but values far below the largest lose
 // their last bits to it: beside a well 4e-10 off where FFTs leave 2e-11.)
 #include "tc_core.cuh"
 
@@ -550,26 +550,30 @@ __device__ __forceinline__ int first_points(int64_t (&xa)[PP], int64_t (&xb)[PP]
   }
   return key;
 }
-// A thread's points, x(i, half) in units of 2^u(i, half), and their largest key.
+// A thread's points, x(i, half) in units of 2^u(i, half), and their largest key.  Units
+// first: with 16 points the registers do not hold the loads of both at once, and units
+// behind the points came in several rounds of their own.
 template <int PP, typename X, typename U>
 __device__ __forceinline__ int load_points(int64_t (&xa)[PP], int64_t (&xb)[PP], Units<PP> &un, int lim,
                                            X &&x, U &&u) {
   int key = 0;
 #pragma unroll
   for (int i = 0; i < PP; ++i) {
-    xa[i] = i < lim ? x(i, 0) : 0;
-    xb[i] = i < lim ? x(i, 1) : 0;
-  }
-#pragma unroll
-  for (int i = 0; i < PP; ++i) {
     int u0 = 0, u1 = 0;
     if (i < lim) {
       u0 = u(i, 0);
       u1 = u(i, 1);
-      key = max(key, max(point_key(xa[i], u0), point_key(xb[i], u1)));
     }
     un.set(i, u0, u1);
   }
+#pragma unroll
+  for (int i = 0; i < PP; ++i) {
+    xa[i] = i < lim ? x(i, 0) : 0;
+    xb[i] = i < lim ? x(i, 1) : 0;
+  }
+#pragma unroll
+  for (int i = 0; i < PP; ++i)
+    if (i < lim) key = max(key, max(point_key(xa[i], un.a(i)), point_key(xb[i], un.b(i))));
   return key;
 }
 // ... to the unit of their line.
