@@ -743,9 +743,9 @@ int adjoint_impl(scft_ctx *ctx, const double *h_pbA, const double *h_pbB, const 
 }
 
 // Box stress from the propagators stored by the last getConc (200 steps, ms: 128 x
-// 128 x 64 pairs 22.2 -> 10.2, FP64 24 x 32 x 32 0.81 -> 0.50): for every contour step s (all independent, so batched `chunk` steps per launch) and axis a,
-// W^-1 D_a W q+(s) contracted with q(s) in FP64, or (whole_axis) W K D_a W q(s-1)
-// with q+(s).
+// 128 x 64 pairs 22.2 -> 10.2, FP64 24 x 32 x 32 0.81 -> 0.50): for every contour step s
+// (all independent, so batched `chunk` steps per launch) and axis a, W^-1 D_a W q+(s)
+// contracted with q(s) in FP64, or (whole_axis) W K D_a W q(s-1) with q+(s).
 template <typename R>
 int stress_sums(scft_ctx *ctx, bool wide, double *acc) {
   AdjointState &A = *ctx->adj;

@@ -904,7 +904,7 @@ int autotune(scft_ctx *ctx) {
       for (int pipe = 0; pipe < (has_fast_col ? 2 : 1); ++pipe)
       for (int fs = 0; fs < (can_fs ? 2 : 1); ++fs) {
         // fused step pairs run only on two-stream chains and the plain column
-        // kernels (with the x+y plane, or with three register-resident passes)
+        // kernels (which passes: fused_possible)
         if (fs && (!two || pipe)) continue;
         ctx->two_streams = two;
         ctx->fuse_xy = can_xy && xy;
@@ -1372,10 +1372,12 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
   if (cudaMemcpy(ctx->tables, host.data(), tab_bytes, cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(SCFT_ERR_CUDA, "table upload failed");
   // Passes on the tensor cores: every FP64 line they take, and FP32 lines without
-  // a register kernel.  Measured, ms per SCF iteration with 200 contour steps:
-  // FP64 64^3 22 -> 3.5, 128^3 107 -> 22; FP32 100x80x60 24 -> 4.2.  FP32 and
-  // double-float lines with a register kernel keep it (64^3: FP32 1.2; double-float
-  // 4.0 against 5.5 on passes of the first form).
+  // a register kernel.  Measured, ms per SCF iteration with 200 contour steps, FFT
+  // passes and these: FP64 64^3 22 / 3.8, 128^3 107 / 26; FP32 100x80x60 24 / 4.2.  FP32
+  // lines with a register kernel keep it (1.17 / 1.97 at 48^3; with the x+y planes beside
+  // them 1.14 / 1.51 at 64^3, 4.30 / 6.08 at 128^3).  Double-float contexts keep theirs: 20.3
+  // at 128^3, where FP64 on the tensor cores takes 26; up to 64^3 FP64 is the faster of the
+  // two (32^3 2.80 / 2.17, 64^3 3.95 / 3.81), and pairs on the same passes are not built.
   size_t tc_bytes = 0;
   if (ctx->rkind != kRealDF && scft::tc_prepare() != cudaSuccess)
     return fail(SCFT_ERR_CUDA, "kernel attribute set-up failed");
@@ -1412,8 +1414,8 @@ int scft_create(const scft_params *pin, scft_ctx **out) {
   ctx->fuse_xy = rb == 4 && (p.flags & SCFT_FLAG_NO_XY) == 0 && ctx->passes.size() >= 2 &&
                  axes[0] == 0 && axes[1] == 1 &&
                  scft::xy_fusable(ctx->passes[0], ctx->passes[1]);
-  // fused step pairs need three passes: the x+y plane kernel and a
-  // register-resident z pass, or three register-resident axis passes
+  // fused step pairs: the x+y plane kernel and a z pass with a pair kernel, two or
+  // three tensor-core passes, or three passes with a pair kernel each
   ctx->fuse_steps = (p.flags & SCFT_FLAG_NO_FUSED_STEPS) == 0;
   ctx->fuse_steps = fused_possible(ctx);
   // With fused step pairs the two-stream chains win at every size the plane

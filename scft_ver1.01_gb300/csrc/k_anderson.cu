@@ -411,9 +411,10 @@ __global__ void k_anderson_solve(const double *__restrict__ G, const double *__r
   }
 }
 
-// Anderson step: w_new = sum_j a_j u_j over the listed slots, in pair
-// arithmetic, two points a thread (128^3, 20 slots: 126 us -> 101, 6.6 TB/s); simple step (mode 0): w_new = w + lam d_c in FP64 from the live
-// fields.  kUChunk slots' loads are in flight per element.
+// Anderson step: w_new = sum_j a_j u_j over the listed slots, in pair arithmetic, two
+// points a thread (128^3, 20 slots: 126 us -> 101, 6.6 TB/s); simple step (mode 0):
+// w_new = w + lam d_c in FP64 from the live fields.  kUChunk slots' loads are in flight
+// per element.
 struct SlotRing {
   const dfloat *u[kMaxSlots];
   int idx[kMaxSlots];

@@ -768,10 +768,10 @@ __global__ void __launch_bounds__(PP == 16 ? 640 : 544, 1) k_fix(Lines ln, const
 // Whole planes per CTA (up to 64 points a line): both axes of a step in one
 // launch.  What a launch costs beside its filters (2.7 us until the next one may
 // read, 1.5 us to load and store a tile) was about half of a 64^3 step.  ms per
-// SCF iteration with 200 steps, one launch per pass against planes: FP64 32^3 2.5 /
-// 2.1, 64^3 3.86 / 3.48.  Above 64 points the planes' one CTA each takes as long as the
-// passes' more evenly filled ones (128^3 22.5 / 22.4, 96^3 10.1 / 12.3; FP32 80^3 5.4 /
-// 6.2): those keep their passes.
+// SCF iteration with 200 steps, one launch per pass against planes: FP64 32^3 2.54 /
+// 2.17, 64^3 4.22 / 3.81.  Above 64 points the planes' one CTA each takes as long as the
+// passes' more evenly filled ones (with one unit per instance: 128^3 22.5 / 22.4, 96^3
+// 10.1 / 12.3; FP32 80^3 5.4 / 6.2): those keep their passes.
 //
 // FILM false: x filter, y filter, q = W y (stored), v = W q, y filter, x filter
 // (the middle pass, the pair and the next middle pass of k_fix's schedule).
@@ -834,7 +834,8 @@ __global__ void __launch_bounds__(544, 1)
     // the units of the z lines that the points came from: the same for every plane
     const int64_t *in = static_cast<const int64_t *>(fp.in) + b * fp.in_bs + tile;
     const int16_t *u_in = fp.u_in + b * fp.u_in_bs;
-    const int nt = e.ncomp, total = np * ny * nx, plane = ny * nx, dr = nt / nx, dc = nt % nx, dp = nt % plane;
+    const int nt = e.ncomp, plane = ny * nx, total = np * plane;
+    const int dr = nt / nx, dc = nt % nx, dp = nt % plane;
     int r = (int)threadIdx.x / nx, cc = (int)threadIdx.x % nx, ip = (int)threadIdx.x % plane;
 #pragma unroll 1
     for (int i0 = threadIdx.x; i0 < total; i0 += 4 * nt) {
@@ -1064,8 +1065,9 @@ bool lines_of(const AxisPlan &ap, int nd, Lines &ln) {
 // Copies of each line per CTA, and with them 4 points per thread, so that small
 // launches of lines of up to 64 points spread over the SMs: doubled while both
 // chains' CTAs still fit there side by side (ms per SCF iteration, one copy
-// against this: FP64 16^3 3.3 / 2.4, 32^3 3.6 / 2.6, 64^3 5.1 / 4.1).  With 16 points per
-// thread two copies were slower (FP32 100 x 80 x 60 5.7 against 5.2).
+// against this: FP64 16^3 3.34 / 2.05, 32^3 3.87 / 2.24, 64^3 5.57 / 3.88, 64 x 64 x 1 3.37 /
+// 2.18).  With 16 points per thread two copies were slower (FP32 100 x 80 x 60 5.7 against
+// 5.2).
 void spread(Shape &sh, long long lines) {
   if (sh.pp == 16) return;
   const int kg = sh.axes == 2 ? std::max(sh.kg[0], sh.kg[1]) : sh.kg[0];
@@ -1410,16 +1412,17 @@ long long tc_pass_ctas(const AxisPlan &ap, int nd) {
 
 // Whether a step's x and y passes run on whole planes.  A film's do when a
 // segment can stay in one CTA's 128 threads' reach, that is at up to 32 x 32
-// (ms per SCF iteration with 200 steps, planes against passes: 32 x 32 1.17 / 1.53,
-// 500 of them 4.6 / 8.1; 40 x 36 1.95 / 1.84, 64 x 64 2.01 / 1.94).  Otherwise
+// (ms per SCF iteration with 200 steps, planes against passes: 32 x 32 1.32 / 1.69,
+// 500 of them 5.0 / 9.1; with one unit per instance 40 x 36 1.95 / 1.84, 64 x 64 2.01 /
+// 1.94).  Otherwise
 // planes save two launches in two steps, but a plane does not split over CTAs,
 // its lines leave part of the 128 rows idle, and its CTAs may need one wave
 // more.  The filters' time on both sides is taken as the waves of both chains'
 // CTAs times 2 + 4/rep; in that unit (0.6 us for 7 digits, 0.35 us for 4) a launch
-// saved is worth 2 and 4.  Measured: 64^3 FP64 3.48 / 3.86 and 60^3 FP32 2.31 / 2.82,
-// 48^3 FP64 3.20 / 3.43, 36^3 FP32 1.84 / 2.17; against planes (12, 20, 28) x 8 FP64
-// 2.63 / 2.31, (64, 40, 30) x 4 FP64 4.55 / 4.23, (36, 36, 38) x 20 FP64 14.2 / 12.9
-// and FP32 8.8 / 8.6.
+// saved is worth 2 and 4.  Measured: for planes FP64 32^3 2.17 / 2.54, 56^3 3.81 / 4.05,
+// 64^3 3.81 / 4.22 and FP32 60^3 2.13 / 2.50, 36^3 1.81 / 2.05; against them FP64 48^3 3.47 /
+// 3.38, 40^3 3.30 / 3.27, and with one unit per instance (12, 20, 28) x 8 2.63 / 2.31,
+// (64, 40, 30) x 4 4.55 / 4.23, (36, 36, 38) x 20 14.2 / 12.9 and FP32 8.8 / 8.6.
 bool tc_planes_wanted(int nx, int ny, int nz, int nd, int batch) {
   if (nx > kLines / 2 || ny > kLines / 2 || nx < 2 || ny < 2) return false;
   if (nz == 1) return nx <= 32 && ny <= 32;
@@ -1563,7 +1566,8 @@ cudaError_t launch_planes(const AxisPlan &apx, const AxisPlan &apy, const PassSe
       return cudaErrorInvalidValue;
   dim3 grid((pa.nz + pa.per - 1) / pa.per, 1, (unsigned)sets);
   const size_t smem = pa.sh.lay.total;
-  return launch_pdl(pa.sh.pp == 4 ? k_planes_f32<4> : k_planes_f32<8>, grid, dim3(pa.sh.threads), smem, st, pa, apx.tc, apy.tc, ps);
+  return launch_pdl(pa.sh.pp == 4 ? k_planes_f32<4> : k_planes_f32<8>, grid, dim3(pa.sh.threads),
+                    smem, st, pa, apx.tc, apy.tc, ps);
 }
 // steps 0: the fused step on planes; else a film's segment of that many steps
 // (fp.q: the first finished slice, q_step to the next one).
