@@ -860,15 +860,13 @@ void free_all(scft_ctx *ctx) {
 }  // namespace
 
 int scft_internal_sync_check(scft_ctx *ctx) {
-  CK(cudaStreamSynchronize(ctx->st));
   unsigned w = 0;
-  CK(cudaMemcpy(&w, ctx->dev_err, sizeof(w), cudaMemcpyDeviceToHost));
-  if (w) {
-    CK(cudaMemset(ctx->dev_err, 0, sizeof(unsigned)));
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
-    return scft_internal_wait_failed(ctx, w);
-  }
-  return SCFT_OK;
+  CK(cudaMemcpyAsync(&w, ctx->dev_err, sizeof w, cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  if (!w) return SCFT_OK;
+  CK(cudaMemsetAsync(ctx->dev_err, 0, sizeof w, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  return scft_internal_wait_failed(ctx, w);
 }
 int scft_internal_wait_failed(scft_ctx *ctx, unsigned word) {
   ctx->have_conc = false;   // the propagators may be that launch's
